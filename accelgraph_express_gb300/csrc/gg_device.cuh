@@ -28,13 +28,6 @@ template <> __device__ __forceinline__ __half from_f32<__half>(float x) { return
 
 /* ---- fixed point (Q32.32 / Q16.16 / Q4.12 / Q2.6), same as the oracle ---- */
 
-__device__ __forceinline__ uint64_t fx64_from_double(double x)
-{
-    double t = __dmul_rn(x, 4294967296.0);
-    if (!(t > 0.0)) return 0ull;
-    if (t >= 18446744073709551615.0) return ~0ull;
-    return __double2ull_rz(t);
-}
 __device__ __forceinline__ double fx64_to_double(uint64_t f) { return __dmul_rn(__ull2double_rn(f), 1.0 / 4294967296.0); }
 __device__ __forceinline__ uint64_t fx64_mul(uint64_t a, uint64_t b)
 {
@@ -43,16 +36,31 @@ __device__ __forceinline__ uint64_t fx64_mul(uint64_t a, uint64_t b)
     uint64_t hi = __umul64hi(a, b);
     return (hi << 32) | (lo >> 32);
 }
-__device__ __forceinline__ uint32_t fx_from_float(float x, double scale, uint32_t maxv)
+/* The conversions below use no FP64: sm_103a issues FP64 at about 1/64 of the
+ * FP32 rate, and a few FP64 operations per vertex or edge were what the
+ * passes that call them spent their time on.  The scales are powers of two,
+ * so the FP32 products are exact and the results are those of the FP64 form. */
+
+/* trunc(x * 2^32) in 64 bits, saturating; NaN and negatives give 0 */
+__device__ __forceinline__ uint64_t fx64_from_float(float x)
 {
-    double t = __dmul_rn((double)x, scale);
-    if (!(t > 0.0)) return 0u;
-    if (t >= (double)maxv) return maxv;
-    return __double2uint_rz(t);
+    if (!(x > 0.0f)) return 0ull;
+    if (x >= 4294967296.0f) return ~0ull;
+    return __float2ull_rz(__fmul_rn(x, 4294967296.0f));
 }
-__device__ __forceinline__ float fx_to_float(uint64_t f, double inv_scale)
+/* trunc(x * scale), at most maxv; scale a power of two */
+__device__ __forceinline__ uint32_t fx_from_float(float x, float scale, uint32_t maxv)
 {
-    return __double2float_rn(__dmul_rn(__ull2double_rn(f), inv_scale));
+    const float t = __fmul_rn(x, scale);
+    if (!(t > 0.0f)) return 0u;
+    return min(__float2uint_rz(t), maxv);
+}
+/* f * inv_scale rounded once to FP32; inv_scale a power of two.  From 2^53 on
+ * the FP64 form rounds twice, which is kept. */
+__device__ __forceinline__ float fx_to_float(uint64_t f, float inv_scale)
+{
+    if (f >> 53) return __double2float_rn(__dmul_rn(__ull2double_rn(f), (double)inv_scale));
+    return __fmul_rn(f >> 32 ? __ull2float_rn(f) : __uint2float_rn((uint32_t)f), inv_scale);
 }
 
 /* Clear a sum slot that was just read.  The store is made to wait for the
@@ -89,24 +97,54 @@ template <class T> __device__ __forceinline__ T warp_sum(T v)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-/* Block-wide sum of (double, uint32) pairs; the result is valid in thread 0. */
+/* A running sum of floats held as hi + lo (Knuth's two-sum: every rounding
+ * error of hi is kept in lo), about 48 bits, in FP32 operations: the passes
+ * that summed a residual per vertex in FP64 were bound by its issue rate
+ * (k_pr_update of a 16.7M-vertex graph: 78 -> 60 us). */
+struct Sum2
+{
+    float hi, lo;
+    __device__ __forceinline__ Sum2() : hi(0.0f), lo(0.0f) {}
+    __device__ __forceinline__ void add(float x)
+    {
+        const float t = __fadd_rn(hi, x), z = __fsub_rn(t, hi);
+        lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, z)), __fsub_rn(x, z)));
+        hi = t;
+    }
+    /* an overflowed or NaN sum has no meaningful lo */
+    __device__ __forceinline__ double value() const
+    {
+        return fabsf(hi) <= 3.402823466e38f ? (double)hi + (double)lo : (double)hi;
+    }
+};
+
+/* Block-wide sum of (Sum2, uint32) pairs in FP64; the result is valid in thread 0. */
 template <int NT>
-__device__ __forceinline__ void block_sum2(double &a, uint32_t &b)
+__device__ __forceinline__ void block_sum2(Sum2 s, uint32_t b, double &a, uint32_t &n)
 {
     __shared__ double sa[NT / 32];
     __shared__ uint32_t sb[NT / 32];
-    a = warp_sum(a);
-    b = warp_sum(b);
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    /* within the warp in two-sum arithmetic, across warps in FP64 */
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+    {
+        const float h = __shfl_down_sync(0xffffffffu, s.hi, o), e = __shfl_down_sync(0xffffffffu, s.lo, o);
+        s.add(h);
+        s.lo = __fadd_rn(s.lo, e);
+    }
+    b = warp_sum(b);
     __syncthreads();
-    if (l == 0) { sa[w] = a; sb[w] = b; }
+    if (l == 0) { sa[w] = s.value(); sb[w] = b; }
     __syncthreads();
+    a = 0.0;
+    n = 0u;
     if (w == 0)
     {
         a = l < NT / 32 ? sa[l] : 0.0;
-        b = l < NT / 32 ? sb[l] : 0u;
+        n = l < NT / 32 ? sb[l] : 0u;
         a = warp_sum(a);
-        b = warp_sum(b);
+        n = warp_sum(n);
     }
 }
 

@@ -90,7 +90,7 @@ __device__ __forceinline__ uint32_t graph_iterations(const GraphsArgs &a, unsign
                                  reinterpret_cast<float *>(stage + S::OFF_BYTES + S::VAL_BYTES), w, warps, a.off,
                                  a.adj, a.V, a.coord + cb, ntiles, sm - vb, GraphsGather{c - vb});
         __syncthreads();
-        double e_sum = 0.0;
+        Sum2 es;
         uint32_t n_act = 0;
         constexpr uint32_t U = 2; /* measured: 4 was slower, and spills at IPT 9 */
         for (uint32_t v0 = threadIdx.x; v0 < Vg; v0 += U * blockDim.x)
@@ -118,13 +118,14 @@ __device__ __forceinline__ uint32_t graph_iterations(const GraphsArgs &a, unsign
                     const float nr = __fadd_rn(base, __fmul_rn(a.damp, sv[k]));
                     a.rank[vb + v] = nr;
                     const float e = fabsf(__fsub_rn(nr, pr[k]));
-                    e_sum += (double)e;
+                    es.add(e);
                     n_act += e >= a.eps_f ? 1u : 0u;
                     c[v] = contrib_of_f(nr, dg[k]);
                 }
             }
         }
         /* CTA sums of the residual and the active count */
+        double e_sum = es.value();
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1)
         {

@@ -84,13 +84,13 @@ __device__ __forceinline__ typename Fmt<K>::CT encode(float c, uint32_t deg)
     if constexpr (K == K_F32 || K == K_BF16 || K == K_F16)
         return from_f32<typename Fmt<K>::CT>(c);
     else if constexpr (K == K_FX64)
-        return deg ? fx64_from_double((double)c) : 0ull;
+        return deg ? fx64_from_float(c) : 0ull;
     else if constexpr (K == K_FX32)
-        return deg ? fx_from_float(c, 65536.0, 0xffffffffu) : 0u;
+        return deg ? fx_from_float(c, 65536.0f, 0xffffffffu) : 0u;
     else if constexpr (K == K_FX16)
-        return (uint16_t)(deg ? fx_from_float(c, 4096.0, 0xffffu) : 0u);
+        return (uint16_t)(deg ? fx_from_float(c, 4096.0f, 0xffffu) : 0u);
     else if constexpr (K == K_FX8)
-        return (uint8_t)(deg ? fx_from_float(c, 64.0, 0xffu) : 0u);
+        return (uint8_t)(deg ? fx_from_float(c, 64.0f, 0xffu) : 0u);
     else
         return 0; /* quantised formats are written by k_quantize */
 }
@@ -113,11 +113,11 @@ __device__ __forceinline__ float next_rank(float base, float damp, typename Fmt<
     else if constexpr (K == K_FX64)
         return __double2float_rn(__dadd_rn((double)base, __dmul_rn((double)damp, fx64_to_double(sum))));
     else if constexpr (K == K_FX32)
-        return __fadd_rn(base, __fmul_rn(damp, fx_to_float(sum, 1.0 / 65536.0)));
+        return __fadd_rn(base, __fmul_rn(damp, fx_to_float(sum, 1.0f / 65536.0f)));
     else if constexpr (K == K_FX16)
-        return __fadd_rn(base, __fmul_rn(damp, fx_to_float(sum, 1.0 / 4096.0)));
+        return __fadd_rn(base, __fmul_rn(damp, fx_to_float(sum, 1.0f / 4096.0f)));
     else if constexpr (K == K_FX8)
-        return __fadd_rn(base, __fmul_rn(damp, fx_to_float(sum, 1.0 / 64.0)));
+        return __fadd_rn(base, __fmul_rn(damp, fx_to_float(sum, 1.0f / 64.0f)));
     else
         return __fadd_rn(base, __fmul_rn(damp, __fmul_rn(qscale, __ull2float_rn(sum))));
 }
@@ -132,10 +132,14 @@ __device__ __forceinline__ float quant_scale(uint32_t maxbits, int bits)
 {
     float mx = __uint_as_float(maxbits);
     if (!(mx > 0.0f)) return 0.0f;
+    /* 8 and 16 bits: the levels are an FP32 number and mx / levels lies at
+     * least 2^-41 (relative) from any rounding boundary it is not on, so
+     * rounding the quotient once gives what rounding it through FP64 gives */
+    if (bits <= 16) return __fdiv_rn(mx, (float)((1u << bits) - 1u));
     double levels = (double)((1ull << bits) - 1);
     return __double2float_rn(__ddiv_rn((double)mx, levels));
 }
-__device__ __forceinline__ uint32_t quantize(float x, float scale, uint32_t zero, int bits)
+__device__ __forceinline__ uint32_t quantize_f64(float x, float scale, uint32_t zero, int bits)
 {
     double maxq = (double)((1ull << bits) - 1);
     if (scale == 0.0f) return zero;
@@ -143,6 +147,33 @@ __device__ __forceinline__ uint32_t quantize(float x, float scale, uint32_t zero
     if (t < 0.0) return 0u;
     if (t > maxq) return (uint32_t)maxq;
     return (uint32_t)t;
+}
+/* floor(x / scale + 0.5) + zero, clipped to the format's range.  For 8 and
+ * 16 bits without an FP64 division per value: a candidate from the
+ * reciprocal is within one of the result, and the sign of x - (n +- 0.5) *
+ * scale, which one FMA gives exactly (n + 0.5 has at most 18 bits), moves it
+ * to the right side.  The FP64 form rounds the quotient, which cannot move
+ * it across a boundary: a quotient below 2^16 not on n + 0.5 is at least
+ * 2^-25 away from it.  32-bit values keep the FP64 form.  rscale = 1 / scale,
+ * 0 to use the FP64 form (a scale whose products could leave the FP32
+ * range).  700K vertices: 49.5 -> 5.1 us a pass. */
+template <int BITS>
+__device__ __forceinline__ uint32_t quantize(float x, float scale, float rscale, uint32_t zero)
+{
+    if (BITS > 16 || rscale == 0.0f) return quantize_f64(x, scale, zero, BITS);
+    constexpr float MAXQ = (float)((1ull << (BITS > 16 ? 16 : BITS)) - 1);
+    float n = floorf(__fadd_rn(__fmul_rn(x, rscale), 0.5f));
+    n = fminf(fmaxf(n, 0.0f), MAXQ + 1.0f);
+    if (__fmaf_rn(-__fsub_rn(n, 0.5f), scale, x) < 0.0f)
+        n -= 1.0f;
+    else if (__fmaf_rn(-__fadd_rn(n, 0.5f), scale, x) >= 0.0f)
+        n += 1.0f;
+    n = fminf(fmaxf(n, 0.0f) + (float)zero, MAXQ);
+    return __float2uint_rz(n);
+}
+__device__ __forceinline__ float quant_rscale(float scale)
+{
+    return scale >= 1e-30f && scale <= 1e30f ? __frcp_rn(scale) : 0.0f;
 }
 __device__ __forceinline__ uint32_t quant_zero(uint32_t maxbits, float scale, int bits)
 {
@@ -330,40 +361,80 @@ __global__ void k_pr_init(float *__restrict__ rank, const uint32_t *__restrict__
     if constexpr (Fmt<K>::quant) block_max_bits<256>(tmax, &rec[0].maxbits);
 }
 
-/* q[v] = quantize(contrib[v]) with the scale of iteration `it`
- * (pageRank.c:2212-2226); bits = 8 with a zero point is the push variant
- * (pageRank.c:2727-2737) */
-template <class QT>
-__global__ void k_quantize(const float *__restrict__ cf, QT *__restrict__ q, uint32_t V, int bits, int with_zero,
-                           IterRec *rec, uint32_t it, uint32_t *zero_out)
+/* two adjacent elements moved by one access */
+template <class T>
+struct alignas(2 * sizeof(T)) Two
 {
+    T x, y;
+};
+
+/* q[v] = quantize(contrib[v]) with the scale of iteration `it`
+ * (pageRank.c:2212-2226); WITH_ZERO (8 bits) is the push variant with a zero
+ * point (pageRank.c:2727-2737).  Two adjacent vertices per step; every array
+ * is a whole allocation. */
+template <class QT, bool WITH_ZERO>
+__global__ void k_quantize(const float *__restrict__ cf, QT *__restrict__ q, uint32_t V, IterRec *rec, uint32_t it,
+                           uint32_t *zero_out)
+{
+    constexpr int BITS = 8 * (int)sizeof(QT);
+    pdl_wait();
     if (it > 0 && rec[it - 1].active == 0u) return;
     const uint32_t mb = rec[it].maxbits;
-    const float scale = quant_scale(mb, bits);
-    const uint32_t zero = with_zero ? quant_zero(mb, scale, bits) : 0u;
-    if (zero_out && blockIdx.x == 0 && threadIdx.x == 0) zero_out[it] = zero;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
-        q[v] = (QT)quantize(cf[v], scale, zero, bits);
+    const float scale = quant_scale(mb, BITS), rscale = quant_rscale(scale);
+    uint32_t zero = 0u;
+    if constexpr (WITH_ZERO)
+    {
+        /* FP64: once per block */
+        __shared__ uint32_t s_zero;
+        if (threadIdx.x == 0) s_zero = quant_zero(mb, scale, BITS);
+        __syncthreads();
+        zero = s_zero;
+        if (blockIdx.x == 0 && threadIdx.x == 0) zero_out[it] = zero;
+    }
+    const uint32_t P = V >> 1, stride = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t p = tid; p < P; p += stride)
+    {
+        const float2 c = reinterpret_cast<const float2 *>(cf)[p];
+        reinterpret_cast<Two<QT> *>(q)[p] = Two<QT>{(QT)quantize<BITS>(c.x, scale, rscale, zero),
+                                                    (QT)quantize<BITS>(c.y, scale, rscale, zero)};
+    }
+    if ((V & 1u) && tid == 0) q[V - 1] = (QT)quantize<BITS>(cf[V - 1], scale, rscale, zero);
+    pdl_trigger();
 }
 
-/* final normalisation and sum (pageRank.c:1080-1085) */
+/* final normalisation and sum (pageRank.c:1080-1085), two adjacent vertices
+ * per step */
 __global__ void k_pr_finalize(float *__restrict__ rank, uint32_t V, int divide, double *sum)
 {
     pdl_wait();
-    double s = 0.0;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
+    Sum2 s;
+    const float fv = __uint2float_rn(V);
+    const uint32_t P = V >> 1, stride = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t p = tid; p < P; p += stride)
     {
-        float r = rank[v];
+        float2 r = reinterpret_cast<const float2 *>(rank)[p];
         if (divide)
         {
-            r = __fdiv_rn(r, __uint2float_rn(V));
-            rank[v] = r;
+            r = make_float2(__fdiv_rn(r.x, fv), __fdiv_rn(r.y, fv));
+            reinterpret_cast<float2 *>(rank)[p] = r;
         }
-        s += (double)r;
+        s.add(r.x);
+        s.add(r.y);
     }
-    uint32_t dummy = 0;
-    block_sum2<256>(s, dummy);
-    if (threadIdx.x == 0 && s != 0.0) atomicAdd(sum, s);
+    if ((V & 1u) && tid == 0)
+    {
+        float r = rank[V - 1];
+        if (divide)
+        {
+            r = __fdiv_rn(r, fv);
+            rank[V - 1] = r;
+        }
+        s.add(r);
+    }
+    double total;
+    uint32_t none;
+    block_sum2<256>(s, 0u, total, none);
+    if (threadIdx.x == 0 && total != 0.0) atomicAdd(sum, total);
 }
 
 /* final normalisation of a batch of graphs (vertex ranges voff[g] ..
@@ -371,7 +442,7 @@ __global__ void k_pr_finalize(float *__restrict__ rank, uint32_t V, int divide, 
 __global__ void k_pr_finalize_seg(float *__restrict__ rank, uint32_t V, const uint32_t *__restrict__ voff,
                                   uint32_t ngraphs, double *sum)
 {
-    double s = 0.0;
+    Sum2 s;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
     {
         /* graph of v: the last g with voff[g] <= v */
@@ -386,11 +457,12 @@ __global__ void k_pr_finalize_seg(float *__restrict__ rank, uint32_t V, const ui
         }
         const float r = __fdiv_rn(rank[v], __uint2float_rn(voff[lo + 1] - voff[lo]));
         rank[v] = r;
-        s += (double)r;
+        s.add(r);
     }
-    uint32_t dummy = 0;
-    block_sum2<256>(s, dummy);
-    if (threadIdx.x == 0 && s != 0.0) atomicAdd(sum, s);
+    double total;
+    uint32_t none;
+    block_sum2<256>(s, 0u, total, none);
+    if (threadIdx.x == 0 && total != 0.0) atomicAdd(sum, total);
 }
 
 /* ---- push: scatter + vertex update ---------------------------------------------- */
@@ -458,75 +530,88 @@ __global__ void __launch_bounds__(GG_TILE_NT) k_pr_push_q(const uint32_t *__rest
 
 /* vertex update from the gathered (pull) or scattered (push) sums
  * (pageRank.c:1055-1069 and :2067-2081), fused with the next iteration's
- * contribution pass (pageRank.c:1026-1033); clears sums for the next launch */
+ * contribution pass (pageRank.c:1026-1033); clears sums for the next launch.
+ * Bound by HBM (20-32 bytes per vertex) once no FP64 runs per vertex: two
+ * adjacent vertices per step, every array a whole allocation. */
+template <int K>
+struct UpdateStep
+{
+    typedef typename Fmt<K>::Acc Acc;
+    float base, damp, eps_f, qscale;
+    Sum2 err;
+    uint32_t act = 0, tmax = 0;
+    /* pageRank.c:1057-1067: |rank' - rank| is a float difference; the sum of
+     * the differences is divided by V once on the host (the reference
+     * divides each term), and `error >= epsilon` is the same test as
+     * e >= eps_f in FP32 */
+    __device__ __forceinline__ float rank(Acc s, float old)
+    {
+        float nr;
+        if constexpr (K == K_Q8Z)
+            nr = __fadd_rn(base, __fmul_rn(damp, (float)s));
+        else
+            nr = next_rank<K>(base, damp, s, qscale);
+        const float e = fabsf(__fsub_rn(nr, old));
+        err.add(e);
+        if (e >= eps_f) act++;
+        return nr;
+    }
+    __device__ __forceinline__ float contribution(float nr, uint32_t deg)
+    {
+        const float c = contrib_of(nr, deg);
+        if constexpr (Fmt<K>::quant) tmax = max(tmax, __float_as_uint(c));
+        return c;
+    }
+};
+
 template <int K>
 __global__ void k_pr_update(PrCommon c, typename Fmt<K>::Acc *sums, typename Fmt<K>::CT *cout, float *cf)
 {
+    typedef typename Fmt<K>::Acc Acc;
+    typedef typename Fmt<K>::CT CT;
     pdl_wait();
     if (c.skip()) return;
-    double err = 0.0;
-    uint32_t act = 0, tmax = 0;
-    float qscale = 0.0f;
-    if constexpr (Fmt<K>::quant && K != K_Q8Z) qscale = quant_scale(c.rec[c.it].maxbits, Fmt<K>::bits);
-    typename Fmt<K>::Acc *__restrict__ sv = sums;
+    UpdateStep<K> st;
+    st.base = c.base;
+    st.damp = c.damp;
+    st.eps_f = c.eps_f;
+    st.qscale = 0.0f;
+    if constexpr (Fmt<K>::quant && K != K_Q8Z) st.qscale = quant_scale(c.rec[c.it].maxbits, Fmt<K>::bits);
+    Acc *__restrict__ sv = sums;
     float *__restrict__ rank = c.rank;
     const uint32_t *__restrict__ outdeg = c.outdeg;
-    uint32_t v0 = 0;
-    if constexpr (K == K_F32)
+    const uint32_t P = c.V >> 1, stride = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t p = tid; p < P; p += stride)
     {
-        /* FP32: two adjacent vertices per step in 8-byte loads and stores
-         * (more loads in flight; every array is a whole allocation), the
-         * same arithmetic per vertex as the loop below */
-        const uint32_t P = c.V >> 1;
-        for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x)
-        {
-            const float2 s = reinterpret_cast<const float2 *>(sv)[p];
-            const float2 pr = reinterpret_cast<const float2 *>(rank)[p];
-            const uint2 d = reinterpret_cast<const uint2 *>(outdeg)[p];
-            if (s.x != 0.0f || s.y != 0.0f) reinterpret_cast<float2 *>(sv)[p] = make_float2(0.0f, 0.0f);
-            const float2 nr = make_float2(next_rank<K>(c.base, c.damp, s.x, 0.0f), next_rank<K>(c.base, c.damp, s.y, 0.0f));
-            reinterpret_cast<float2 *>(rank)[p] = nr;
-            const float e0 = fabsf(__fsub_rn(nr.x, pr.x)), e1 = fabsf(__fsub_rn(nr.y, pr.y));
-            err += (double)e0;
-            err += (double)e1;
-            act += (e0 >= c.eps_f) + (e1 >= c.eps_f);
-            reinterpret_cast<float2 *>(cout)[p] = make_float2(encode<K>(contrib_of(nr.x, d.x), d.x),
-                                                              encode<K>(contrib_of(nr.y, d.y), d.y));
-        }
-        v0 = P * 2;
-    }
-    for (uint32_t v = v0 + blockIdx.x * blockDim.x + threadIdx.x; v < c.V; v += gridDim.x * blockDim.x)
-    {
-        const typename Fmt<K>::Acc s = sv[v];
-        const float pr = rank[v];
-        const uint32_t d = outdeg[v];
-        float nr;
-        if constexpr (K == K_Q8Z)
-            nr = __fadd_rn(c.base, __fmul_rn(c.damp, (float)s));
-        else
-            nr = next_rank<K>(c.base, c.damp, s, qscale);
-        clear_after_read(&sv[v], s);
-        rank[v] = nr;
-        /* pageRank.c:1057-1067: |rank' - rank| is a float difference, exact
-         * in FP64; the FP64 sum of the differences is divided by V once on
-         * the host (the reference divides each term), and `error >= epsilon`
-         * is the same test as e >= eps_f in FP32, so no FP64 division or
-         * compare runs per vertex (FP64 is a small fraction of the FP32 rate
-         * here) */
-        const float e = fabsf(__fsub_rn(nr, pr));
-        err += (double)e;
-        if (e >= c.eps_f) act++;
-        float ctb = contrib_of(nr, d);
+        const Two<Acc> s = reinterpret_cast<const Two<Acc> *>(sv)[p];
+        const float2 pr = reinterpret_cast<const float2 *>(rank)[p];
+        const uint2 d = reinterpret_cast<const uint2 *>(outdeg)[p];
+        if (s.x != Acc(0) || s.y != Acc(0)) reinterpret_cast<Two<Acc> *>(sv)[p] = Two<Acc>{Acc(0), Acc(0)};
+        const float2 nr = make_float2(st.rank(s.x, pr.x), st.rank(s.y, pr.y));
+        reinterpret_cast<float2 *>(rank)[p] = nr;
+        const float c0 = st.contribution(nr.x, d.x), c1 = st.contribution(nr.y, d.y);
         if constexpr (Fmt<K>::quant)
-        {
+            reinterpret_cast<float2 *>(cf)[p] = make_float2(c0, c1);
+        else
+            reinterpret_cast<Two<CT> *>(cout)[p] = Two<CT>{encode<K>(c0, d.x), encode<K>(c1, d.y)};
+    }
+    if ((c.V & 1u) && tid == 0)
+    {
+        const uint32_t v = c.V - 1, d = outdeg[v];
+        const Acc s = sv[v];
+        clear_after_read(&sv[v], s);
+        const float nr = st.rank(s, rank[v]);
+        rank[v] = nr;
+        const float ctb = st.contribution(nr, d);
+        if constexpr (Fmt<K>::quant)
             cf[v] = ctb;
-            tmax = max(tmax, __float_as_uint(ctb));
-        }
         else
             cout[v] = encode<K>(ctb, d);
     }
-    if constexpr (Fmt<K>::quant) block_max_bits<256>(tmax, &c.rec[c.it + 1].maxbits);
-    block_sum2<256>(err, act);
+    if constexpr (Fmt<K>::quant) block_max_bits<256>(st.tmax, &c.rec[c.it + 1].maxbits);
+    double err;
+    uint32_t act;
+    block_sum2<256>(st.err, st.act, err, act);
     if (threadIdx.x == 0) c.reduce(err, act);
     pdl_trigger();
 }
@@ -607,8 +692,8 @@ struct DeltaStep
     float base, damp, init, in_inv, eps_f;
     int k;
     bool first;
-    double err;
-    uint32_t act, tmax;
+    Sum2 err;
+    uint32_t act = 0, tmax = 0;
     __device__ __forceinline__ void operator()(float ds, float &s, float &ch, uint32_t deg, float &nr, CT &q)
     {
         const float s_old = s;
@@ -619,7 +704,7 @@ struct DeltaStep
         const float pr = first ? init : __fadd_rn(base, __fmul_rn(damp, s_old));
         nr = __fadd_rn(base, __fmul_rn(damp, s));
         const float e = fabsf(__fsub_rn(nr, pr));
-        err += (double)e;
+        err.add(e);
         if (e >= eps_f) act++;
         const float d = __fsub_rn(contrib_of(nr, deg), ch);
         ch = __fadd_rn(ch, store_delta<K>(d, k, &q));
@@ -652,8 +737,14 @@ __global__ void k_pr_update_delta(PrCommon c, float init, float *__restrict__ ds
     typedef typename Fmt<K>::CT CT;
     pdl_wait();
     if (c.skip()) return;
-    DeltaStep<K> st{c.base, c.damp, init, c.rec[c.it].qinv, c.eps_f,
-                    K == K_F16 ? f16_scale_exp(c.rec[c.it].maxbits) : 0, c.it == 0, 0.0, 0u, 0u};
+    DeltaStep<K> st;
+    st.base = c.base;
+    st.damp = c.damp;
+    st.init = init;
+    st.in_inv = c.rec[c.it].qinv;
+    st.eps_f = c.eps_f;
+    st.k = K == K_F16 ? f16_scale_exp(c.rec[c.it].maxbits) : 0;
+    st.first = c.it == 0;
     float *__restrict__ rank = c.rank;
     const uint32_t *__restrict__ outdeg = c.outdeg;
     const uint32_t P = c.V >> 1, stride = gridDim.x * blockDim.x;
@@ -686,8 +777,10 @@ __global__ void k_pr_update_delta(PrCommon c, float init, float *__restrict__ ds
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) c.rec[c.it + 1].qinv = pow2f(-st.k);
     block_max_bits<256>(st.tmax, &c.rec[c.it + 1].maxbits);
-    block_sum2<256>(st.err, st.act);
-    if (threadIdx.x == 0) c.reduce(st.err, st.act);
+    double err;
+    uint32_t act;
+    block_sum2<256>(st.err, st.act, err, act);
+    if (threadIdx.x == 0) c.reduce(err, act);
     pdl_trigger();
 }
 
@@ -725,8 +818,8 @@ __global__ void k_dd_update(PrCommon c, float *sums, const uint8_t *__restrict__
                             const uint32_t *__restrict__ out_off, const uint32_t *__restrict__ out_adj)
 {
     if (c.skip()) return;
-    double err = 0.0;
-    uint32_t act = 0;
+    Sum2 es;
+    uint32_t na = 0;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < c.V; v += gridDim.x * blockDim.x)
     {
         const float sum = sums[v];
@@ -734,15 +827,17 @@ __global__ void k_dd_update(PrCommon c, float *sums, const uint8_t *__restrict__
         if (!wl_curr[v]) continue;
         float nr = __fadd_rn(c.base, __fmul_rn(c.damp, sum));
         float e = fabsf(__fsub_rn(nr, c.rank[v]));
-        err += (double)e;
+        es.add(e);
         if (e >= c.eps_f)
         {
             c.rank[v] = nr;
             for (uint32_t j = out_off[v]; j < out_off[v + 1]; j++) wl_next[out_adj[j]] = 1;
-            act++;
+            na++;
         }
     }
-    block_sum2<256>(err, act);
+    double err;
+    uint32_t act;
+    block_sum2<256>(es, na, err, act);
     if (threadIdx.x == 0) c.reduce(err, act);
 }
 
@@ -779,8 +874,8 @@ __global__ void k_dd_push(PrCommon c, int pullpush, const uint32_t *__restrict__
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    double err = 0.0;
-    uint32_t act = 0;
+    Sum2 es;
+    uint32_t na = 0;
     for (uint32_t v = warp; v < c.V; v += nwarps)
     {
         if (!wl_curr[v]) continue;
@@ -811,7 +906,7 @@ __global__ void k_dd_push(PrCommon c, int pullpush, const uint32_t *__restrict__
         if (lane == 0)
         {
             float fv = __uint2float_rn(c.V);
-            err += fabs((double)__fsub_rn(__fdiv_rn(new_pr, fv), __fdiv_rn(old_pr, fv)));
+            es.add(fabsf(__fsub_rn(__fdiv_rn(new_pr, fv), __fdiv_rn(old_pr, fv))));
             c.rank[v] = new_pr;
         }
         uint32_t deg = c.outdeg[v];
@@ -822,13 +917,15 @@ __global__ void k_dd_push(PrCommon c, int pullpush, const uint32_t *__restrict__
             float prev = atomicAdd(&resid[u], delta);
             if (fabsf(__fadd_rn(prev, delta)) >= c.eps_f && prev <= c.eps_fl)
             {
-                act++;
+                na++;
                 if (pullpush) atomicAdd(&resid[u], delta);
                 wl_next[u] = 1;
             }
         }
     }
-    block_sum2<256>(err, act);
+    double err;
+    uint32_t act;
+    block_sum2<256>(es, na, err, act);
     if (threadIdx.x == 0) c.reduce(err, act);
 }
 
@@ -903,7 +1000,8 @@ gg_status run_pull(Run &R, IterRec *rec, float *rank, uint32_t iters, float base
     {
         if constexpr (Fmt<K>::quant)
         {
-            k_quantize<CT><<<grid_v(V), 256, 0, R.s>>>((const float *)cf, cb[0], V, Fmt<K>::bits, 0, rec, it, nullptr);
+            GG_CUDA(gg_launch_pdl(k_quantize<CT, false>, dim3(grid_v(V)), dim3(256), 0, R.s, (const float *)cf, cb[0], V,
+                                  rec, it, nullptr));
             R.launches++;
         }
         const CT *cin = Fmt<K>::quant ? cb[0] : cb[it & 1];
@@ -1005,8 +1103,8 @@ gg_status run_push(Run &R, IterRec *rec, float *rank, uint32_t iters, float base
         GG_CHECK(timed_begin(R));
         if constexpr (K == K_Q8Z)
         {
-            k_quantize<uint8_t><<<grid_v(V), 256, 0, R.s>>>((const float *)cf, (uint8_t *)c0, V, 8, 1, rec, it,
-                                                           (uint32_t *)zeros);
+            k_quantize<uint8_t, true><<<grid_v(V), 256, 0, R.s>>>((const float *)cf, (uint8_t *)c0, V, rec, it,
+                                                                  (uint32_t *)zeros);
             k_pr_push_q<<<gg_persistent_grid((const void *)k_pr_push_q, t->ntiles), GG_TILE_NT, 0, R.s>>>(
                 g->out_off, g->out_adj, t->coord, t->ntiles, V, (const uint8_t *)c0,
                                                            (const uint32_t *)zeros, (float *)nx, rec, it);

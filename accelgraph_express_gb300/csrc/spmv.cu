@@ -139,7 +139,7 @@ struct SpmvFxGather
     __device__ __forceinline__ Raw load(uint32_t e, uint32_t u) const { return Raw{ldg_val(w + e), ldg_val(x32 + u)}; }
     __device__ __forceinline__ unsigned long long value(const Raw &r) const
     {
-        return ((unsigned long long)r.x * fx_from_float(r.w, 65536.0, 0xffffffffu)) >> 16;
+        return ((unsigned long long)r.x * fx_from_float(r.w, 65536.0f, 0xffffffffu)) >> 16;
     }
 };
 
@@ -156,7 +156,7 @@ __global__ void k_spmv_fx_pull_out(unsigned long long *y64, float *y, uint32_t V
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
     {
         const unsigned long long s = y64[v];
-        y[v] = fx_to_float(s, 1.0 / 65536.0);
+        y[v] = fx_to_float(s, 1.0f / 65536.0f);
         clear_after_read(&y64[v], s);
     }
 }
@@ -195,7 +195,7 @@ __global__ void __launch_bounds__(GG_TILE_NT) k_spmv_push_fx(const uint32_t *__r
         __device__ __forceinline__ unsigned long long row_value(uint32_t r) const { return x64[r]; }
         __device__ __forceinline__ void scatter(unsigned long long xv, uint32_t e, uint32_t dst) const
         {
-            atomicAdd(&y64[dst], fx64_mul(fx64_from_double((double)w[e]), xv));
+            atomicAdd(&y64[dst], fx64_mul(fx64_from_float(w[e]), xv));
         }
     } op{w, x64, y64};
     warp_push<GG_TILE_IPT, GG_TILE_WARPS>(off, adj, V, coord, ntiles, op);
@@ -219,8 +219,8 @@ __global__ void k_spmv_x(const uint32_t *__restrict__ outdeg, const float *xin, 
         }
         xf[v] = xv;
         if (xs) xs[v] = from_f32<T>(xv);
-        if (x32) x32[v] = fx_from_float(xv, 65536.0, 0xffffffffu);
-        if (x64) x64[v] = fx64_from_double((double)xv);
+        if (x32) x32[v] = fx_from_float(xv, 65536.0f, 0xffffffffu);
+        if (x64) x64[v] = fx64_from_float(xv);
         y[v] = 0.0f;
     }
 }
@@ -228,21 +228,44 @@ __global__ void k_spmv_x(const uint32_t *__restrict__ outdeg, const float *xin, 
 __global__ void k_spmv_fx64_out(const unsigned long long *y64, float *y, uint32_t V)
 {
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
-        y[v] = __double2float_rn(fx64_to_double(y64[v]));
+        y[v] = fx_to_float(y64[v], 1.0f / 4294967296.0f);
 }
 
-/* sum of round2(y) as the reference prints it (SPMV.c:727-730) */
-__global__ void k_spmv_checksum(const float *y, uint32_t V, double *out)
+/* (int)(x * 100 + 0.5) in FP64, as the reference's round2 takes it; below
+ * 2^22 from the exact fraction of the FP32 product, without FP64 */
+__device__ __forceinline__ int round2_int(float y)
 {
-    double s = 0.0;
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
+    const float f = __fmul_rn(y, 100.0f), a = fabsf(f);
+    if (!(a < 4194304.0f)) return (int)__dadd_rn((double)f, 0.5);
+    const int i = __float2int_rz(a);
+    const bool up = __fsub_rn(a, (float)i) >= 0.5f;
+    if (f >= 0.0f) return up ? i + 1 : i;
+    const int n = up ? i : i - 1; /* truncation towards zero of f + 0.5 */
+    return n > 0 ? -n : 0;
+}
+
+/* sum of round2(y) as the reference prints it (SPMV.c:727-730), in
+ * hundredths: whole numbers, summed exactly (an FP64 division per vertex had
+ * made this pass 197 us at 5M vertices; 31 now) */
+__global__ void k_spmv_checksum(const float *__restrict__ y, uint32_t V, unsigned long long *out)
+{
+    long long s = 0;
+    const uint32_t P = V >> 2, stride = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
+    for (uint32_t p = tid; p < P; p += stride)
     {
-        double t = __dadd_rn((double)__fmul_rn(y[v], 100.0f), 0.5);
-        s += (double)(int)t / 100.0;
+        const float4 v = reinterpret_cast<const float4 *>(y)[p];
+        s += (long long)round2_int(v.x) + round2_int(v.y) + round2_int(v.z) + round2_int(v.w);
     }
-    uint32_t dummy = 0;
-    block_sum2<256>(s, dummy);
-    if (threadIdx.x == 0 && s != 0.0) atomicAdd(out, s);
+    if (tid < (V & 3u)) s += round2_int(y[P * 4 + tid]);
+    __shared__ long long part[8];
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = s;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        for (int k = 1; k < 8; k++) s += part[k];
+        if (s) atomicAdd(out, (unsigned long long)s);
+    }
 }
 
 int grid_v(uint32_t V) { int b = (int)((V + 255) / 256); int cap = gg_sm_count() * 8; return b < 1 ? 1 : (b > cap ? cap : b); }
@@ -409,17 +432,17 @@ extern "C" gg_status gg_spmv(gg_graph *g, const gg_spmv_params *p, const float *
                 launches++;
             }
         }
-        k_spmv_checksum<<<grid_v(V), 256, 0, s>>>((const float *)yv, V, (double *)chk);
+        k_spmv_checksum<<<grid_v(V), 256, 0, s>>>((const float *)yv, V, (unsigned long long *)chk);
         launches++;
         GG_CUDA(cudaGetLastError());
     }
-    double checksum = 0.0;
+    long long hundredths = 0;
     GG_CHECK(gg_wait(s)); /* bounded, before a copy to pageable memory */
-    GG_CUDA(cudaMemcpyAsync(&checksum, chk, 8, cudaMemcpyDeviceToHost, s));
+    GG_CUDA(cudaMemcpyAsync(&hundredths, chk, 8, cudaMemcpyDeviceToHost, s));
     if (y && V) GG_CHECK(gg_copy_d2h(y, yv, (size_t)V * 4, s));
     if (x_out && V) GG_CHECK(gg_copy_d2h(x_out, xf, (size_t)V * 4, s));
     GG_CHECK(gg_wait(s));
-    res.checksum = checksum;
+    res.checksum = (double)hundredths / 100.0;
     res.launches = launches;
     res.spmv_launches = timed;
     if (p->profile)
