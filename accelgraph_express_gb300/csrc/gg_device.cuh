@@ -320,7 +320,12 @@ __device__ __forceinline__ uint32_t tile_rows(uint2 c0, uint2 c1, uint32_t V)
 /*
  * The pull engine: sums[r] = sum over the CSC row r of op's edge terms, for
  * every row, by persistent warps over merge-path tiles.  Op supplies:
- *   typedef Acc;                       float or unsigned long long
+ *   typedef Acc;                       float, uint32_t or unsigned long long:
+ *                                      sums within a tile
+ *   typedef Sum;                       the type of sums[] (Acc, or 64 bits
+ *                                      where a tile's sums fit 32: 8- and
+ *                                      16-bit formats, whose tile of at most
+ *                                      2^10 edges sums to less than 2^26)
  *   typedef Raw;                       what one edge's gather loads
  *   Raw load(uint32_t e, uint32_t u) const;
  *                                      issue the loads of edge e with
@@ -362,9 +367,10 @@ __device__ __forceinline__ void warp_pull_sums_core(uint32_t *s_offs, typename O
                                                     typename Op::Acc *s_row, uint32_t tile, uint32_t nw,
                                                     const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
                                                     uint32_t V, const uint2 *__restrict__ coord, uint32_t ntiles,
-                                                    typename Op::Acc *sums, const Op &op)
+                                                    typename Op::Sum *sums, const Op &op)
 {
     typedef typename Op::Acc Acc;
+    typedef typename Op::Sum Sum;
     typedef typename Op::Raw Raw;
     constexpr uint32_t TW = PullStage<IPT, Acc>::TW;
     constexpr uint32_t OFFW = PullStage<IPT, Acc>::OFFW;
@@ -501,12 +507,12 @@ __device__ __forceinline__ void warp_pull_sums_core(uint32_t *s_offs, typename O
         {
             if (k == 0 && s_off[0] < j0)
             {
-                if (s_off[1] > j0) atomic_add_acc(&sums[i0], s_row[0]);
+                if (s_off[1] > j0) atomic_add_acc(&sums[i0], (Sum)s_row[0]);
             }
             else
                 sums[i0 + k] = s_row[k];
         }
-        if (lane == 0 && i1 < V && s_off[nend] < j1) atomic_add_acc(&sums[i1], s_row[nend]);
+        if (lane == 0 && i1 < V && s_off[nend] < j1) atomic_add_acc(&sums[i1], (Sum)s_row[nend]);
         __syncwarp();
 
         /* C's offsets into A's buffer; rotate */
@@ -526,7 +532,7 @@ __device__ __forceinline__ void warp_pull_sums_core(uint32_t *s_offs, typename O
 template <int IPT, int WARPS, class Op>
 __device__ __forceinline__ void warp_pull_sums(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
                                                uint32_t V, const uint2 *__restrict__ coord, uint32_t ntiles,
-                                               typename Op::Acc *sums, const Op &op)
+                                               typename Op::Sum *sums, const Op &op)
 {
     typedef typename Op::Acc Acc;
     constexpr uint32_t TW = PullStage<IPT, Acc>::TW, OFFW = PullStage<IPT, Acc>::OFFW;
@@ -544,7 +550,7 @@ template <int IPT, class Op>
 __device__ __forceinline__ void warp_pull_sums_dyn(unsigned char *base, const uint32_t *__restrict__ off,
                                                    const uint32_t *__restrict__ adj, uint32_t V,
                                                    const uint2 *__restrict__ coord, uint32_t ntiles,
-                                                   typename Op::Acc *sums, const Op &op)
+                                                   typename Op::Sum *sums, const Op &op)
 {
     typedef typename Op::Acc Acc;
     typedef PullStage<IPT, Acc> S;

@@ -63,6 +63,7 @@ struct GraphsArgs
 struct GraphsGather
 {
     typedef float Acc;
+    typedef float Sum;
     typedef float Raw;
     const float *base;
     __device__ __forceinline__ Raw load(uint32_t, uint32_t u) const { return base[u]; }

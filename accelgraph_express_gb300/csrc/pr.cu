@@ -63,18 +63,18 @@ struct IterRec
 enum Kind { K_F32, K_BF16, K_F16, K_FX64, K_FX32, K_FX16, K_FX8, K_Q32, K_Q16, K_Q8, K_Q8Z };
 
 template <int K> struct Fmt;
-template <> struct Fmt<K_F32> { typedef float CT; typedef float Acc; static constexpr bool quant = false; };
-template <> struct Fmt<K_BF16> { typedef __nv_bfloat16 CT; typedef float Acc; static constexpr bool quant = false; };
-template <> struct Fmt<K_F16> { typedef __half CT; typedef float Acc; static constexpr bool quant = false; };
-template <> struct Fmt<K_FX64> { typedef unsigned long long CT; typedef unsigned long long Acc; static constexpr bool quant = false; };
-template <> struct Fmt<K_FX32> { typedef uint32_t CT; typedef unsigned long long Acc; static constexpr bool quant = false; };
-template <> struct Fmt<K_FX16> { typedef uint16_t CT; typedef unsigned long long Acc; static constexpr bool quant = false; };
-template <> struct Fmt<K_FX8> { typedef uint8_t CT; typedef unsigned long long Acc; static constexpr bool quant = false; };
-template <> struct Fmt<K_Q32> { typedef uint32_t CT; typedef unsigned long long Acc; static constexpr bool quant = true; static constexpr int bits = 32; };
-template <> struct Fmt<K_Q16> { typedef uint16_t CT; typedef unsigned long long Acc; static constexpr bool quant = true; static constexpr int bits = 16; };
-template <> struct Fmt<K_Q8> { typedef uint8_t CT; typedef unsigned long long Acc; static constexpr bool quant = true; static constexpr int bits = 8; };
+template <> struct Fmt<K_F32> { typedef float CT; typedef float Acc; typedef float Tile; static constexpr bool quant = false; };
+template <> struct Fmt<K_BF16> { typedef __nv_bfloat16 CT; typedef float Acc; typedef float Tile; static constexpr bool quant = false; };
+template <> struct Fmt<K_F16> { typedef __half CT; typedef float Acc; typedef float Tile; static constexpr bool quant = false; };
+template <> struct Fmt<K_FX64> { typedef unsigned long long CT; typedef unsigned long long Acc; typedef unsigned long long Tile; static constexpr bool quant = false; };
+template <> struct Fmt<K_FX32> { typedef uint32_t CT; typedef unsigned long long Acc; typedef unsigned long long Tile; static constexpr bool quant = false; };
+template <> struct Fmt<K_FX16> { typedef uint16_t CT; typedef unsigned long long Acc; typedef uint32_t Tile; static constexpr bool quant = false; };
+template <> struct Fmt<K_FX8> { typedef uint8_t CT; typedef unsigned long long Acc; typedef uint32_t Tile; static constexpr bool quant = false; };
+template <> struct Fmt<K_Q32> { typedef uint32_t CT; typedef unsigned long long Acc; typedef unsigned long long Tile; static constexpr bool quant = true; static constexpr int bits = 32; };
+template <> struct Fmt<K_Q16> { typedef uint16_t CT; typedef unsigned long long Acc; typedef uint32_t Tile; static constexpr bool quant = true; static constexpr int bits = 16; };
+template <> struct Fmt<K_Q8> { typedef uint8_t CT; typedef unsigned long long Acc; typedef uint32_t Tile; static constexpr bool quant = true; static constexpr int bits = 8; };
 /* push variant of the quantised mode: 8 bits with a zero point, FP32 scatter */
-template <> struct Fmt<K_Q8Z> { typedef uint8_t CT; typedef float Acc; static constexpr bool quant = true; static constexpr int bits = 8; };
+template <> struct Fmt<K_Q8Z> { typedef uint8_t CT; typedef float Acc; typedef float Tile; static constexpr bool quant = true; static constexpr int bits = 8; };
 
 /* stored contribution of a vertex from its new rank (pageRank.c:1028-1031
  * and the fixed-point forms at :1373, :1553, :1730, :1911) */
@@ -96,12 +96,12 @@ __device__ __forceinline__ typename Fmt<K>::CT encode(float c, uint32_t deg)
 }
 
 template <int K>
-__device__ __forceinline__ typename Fmt<K>::Acc decode(typename Fmt<K>::CT x)
+__device__ __forceinline__ typename Fmt<K>::Tile decode(typename Fmt<K>::CT x)
 {
     if constexpr (K == K_F32 || K == K_BF16 || K == K_F16)
         return to_f32(x);
     else
-        return (unsigned long long)x;
+        return (typename Fmt<K>::Tile)x;
 }
 
 /* rank' from the gathered sum (pageRank.c:1057, :1400, :1581, :1758, :1939, :2252) */
@@ -229,7 +229,8 @@ struct PrCommon
 template <int K>
 struct PrGather
 {
-    typedef typename Fmt<K>::Acc Acc;
+    typedef typename Fmt<K>::Tile Acc;
+    typedef typename Fmt<K>::Acc Sum;
     typedef typename Fmt<K>::CT Raw;
     const Raw *cin;
     __device__ __forceinline__ Raw load(uint32_t, uint32_t u) const { return ldg_val(cin + u); }
@@ -240,7 +241,8 @@ struct PrGather
 template <int K>
 struct PrGatherHot
 {
-    typedef typename Fmt<K>::Acc Acc;
+    typedef typename Fmt<K>::Tile Acc;
+    typedef typename Fmt<K>::Acc Sum;
     typedef typename Fmt<K>::CT Raw;
     const Raw *cin;
     const Raw *s_hot;
@@ -262,7 +264,7 @@ __host__ __device__ constexpr uint32_t hot_entries()
 template <int K>
 __host__ __device__ constexpr size_t hot_stage_bytes(uint32_t warps)
 {
-    return (size_t)warps * PullStage<GG_HOT_IPT, typename Fmt<K>::Acc>::BYTES;
+    return (size_t)warps * PullStage<GG_HOT_IPT, typename Fmt<K>::Tile>::BYTES;
 }
 template <int K>
 __host__ __device__ constexpr size_t hot_smem_bytes(uint32_t warps)
@@ -800,6 +802,7 @@ __global__ void k_dd_contrib(const float *__restrict__ rank, const uint32_t *__r
 struct DdGather
 {
     typedef float Acc;
+    typedef float Sum;
     typedef float Raw;
     const float *cf;
     __device__ __forceinline__ float load(uint32_t, uint32_t u) const { return ldg_val(cf + u); }

@@ -31,6 +31,7 @@ template <class T>
 struct SpmvGather
 {
     typedef float Acc;
+    typedef float Sum;
     struct Raw { T w, x; };
     const T *w;
     const T *x;
@@ -52,6 +53,7 @@ template <class T>
 struct SpmvGatherHot
 {
     typedef float Acc;
+    typedef float Sum;
     typedef typename SpmvGather<T>::Raw Raw;
     const T *w;
     const T *x;
@@ -133,6 +135,7 @@ int spmv_hot_grid(uint32_t ntiles, uint32_t warps)
 struct SpmvFxGather
 {
     typedef unsigned long long Acc;
+    typedef unsigned long long Sum;
     struct Raw { float w; uint32_t x; };
     const float *w;
     const uint32_t *x32;
