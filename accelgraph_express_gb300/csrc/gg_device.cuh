@@ -544,23 +544,6 @@ __device__ __forceinline__ void warp_pull_sums(const uint32_t *__restrict__ off,
                              V, coord, ntiles, sums, op);
 }
 
-/* the engine with per-warp staging carved from dynamic shared memory at
- * `base` (blockDim.x / 32 warps of PullStage<IPT, Acc>::BYTES each) */
-template <int IPT, class Op>
-__device__ __forceinline__ void warp_pull_sums_dyn(unsigned char *base, const uint32_t *__restrict__ off,
-                                                   const uint32_t *__restrict__ adj, uint32_t V,
-                                                   const uint2 *__restrict__ coord, uint32_t ntiles,
-                                                   typename Op::Sum *sums, const Op &op)
-{
-    typedef typename Op::Acc Acc;
-    typedef PullStage<IPT, Acc> S;
-    const uint32_t w = threadIdx.x >> 5, warps = blockDim.x >> 5;
-    unsigned char *p = base + (size_t)w * S::BYTES;
-    warp_pull_sums_core<IPT>(reinterpret_cast<uint32_t *>(p), reinterpret_cast<Acc *>(p + S::OFF_BYTES),
-                             reinterpret_cast<Acc *>(p + S::OFF_BYTES + S::VAL_BYTES), blockIdx.x * warps + w,
-                             gridDim.x * warps, off, adj, V, coord, ntiles, sums, op);
-}
-
 /*
  * The push engine: the same warp tiles over the out-CSR; every edge
  * (row -> dst) applies op.scatter(row value, edge, dst).  Per-row data is

@@ -46,7 +46,7 @@ struct gg_buf
  * gg_autotune, or found in the tuning cache for a graph like this one. */
 struct gg_pull_shape
 {
-    uint32_t hot = 2;        /* hot-vertex table: 0 off, 1 on, 2 by size (from 1M vertices) */
+    uint32_t hot = 2;        /* hot-vertex table: 0 off, 1 on, 2 by size (GG_HOT_MIN_E) */
     uint32_t ctas = 5;       /* plain kernel: resident CTAs per SM (GG_PULL_CTAS_PER_SM) */
     uint32_t hot_warps = 32; /* hot kernel: warps of its one CTA per SM (GG_HOT_WARPS) */
 };
@@ -106,7 +106,7 @@ struct gg_graph
     void *out_w16[3] = {nullptr, nullptr, nullptr};
 
     /* work buffers, grown on demand */
-    gg_buf work[32];
+    gg_buf work[34];
     /* merge-path tiles of the batched PageRank gather (own tile size) */
     gg_tiles ppr_tiles;
     const float *ppr_ranks = nullptr;
@@ -116,7 +116,9 @@ struct gg_graph
     uint32_t *hot_list = nullptr;  /* GG_HOT_ENTRIES slots */
     uint32_t hot_n = 0;            /* slots in use */
     uint32_t hot_cap = 0;          /* table capacity the encoding was made for */
-    gg_tiles hot_tiles;            /* tiles of 32 * GG_HOT_IPT items over the CSC */
+    uint32_t *hot_rows = nullptr;  /* the rows with edges, in order (V + GG_HOT_ROW_PAD entries) */
+    uint32_t *hot_seg0 = nullptr;  /* per tile of hot_tile edges: its first row end (gg_hot.cuh) */
+    uint32_t hot_ntiles = 0, hot_tile = 0; /* tiles and edges per tile */
     /* page-locked host scratch for small per-step read-backs */
     void *pinned = nullptr;
     size_t pinned_bytes = 0;
@@ -208,8 +210,8 @@ gg_status gg_apply_labels(const uint32_t *ids, uint64_t n, const uint32_t *label
 /* the mapping's page-locked host scratch, at least `bytes` long */
 gg_status gg_pinned(gg_graph *g, size_t bytes, void **out);
 /* build the hot-vertex table of the mapping for a table of `cap` entries
- * (<= GG_HOT_ENTRIES; rebuilt only when cap changes; needs GG_MAP_IN), and
- * the tiles of the hot kernels */
+ * (<= GG_HOT_ENTRIES; rebuilt only when cap changes; needs GG_MAP_IN and
+ * gg_hot_fits), and the rows and tiles of the hot kernels */
 gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap);
 cudaStream_t gg_stream(gg_graph *g, void *user_stream);
 /* host wait on all work queued on `s`, bounded by the wait limit */
@@ -276,18 +278,33 @@ int gg_occupancy(const void *kernel, int threads, size_t smem);
 /* device-side wait limit of the grid barriers, in ns (gg_set_barrier_limit_us) */
 unsigned long long gg_barrier_limit_ns();
 
-/* Hot-vertex table of the pull gather (hot.cu): up to GG_HOT_ENTRIES
- * vertices with the most out-edges are read from a shared-memory table of
- * GG_HOT_TABLE_BYTES (as many entries as the stored value type fits: 8K FP32,
- * 16K BF16/FP16); a copy of the CSC ids marks them as GG_HOT_FLAG | slot.
- * The kernels that use it run one CTA of GG_HOT_WARPS warps per SM sharing
- * the table (measured on R-MAT-24: many warps per SM matter more than a
- * bigger table or longer tiles). */
+/* Hot-vertex table of the pull gather (hot.cu, gg_hot.cuh): the vertices with
+ * the most out-edges, as many as GG_HOT_TABLE_BYTES of their stored values
+ * hold (40K FP32, 80K of 16 bits), are read from shared memory.  A copy of the
+ * CSC ids carries them as GG_HOT_FLAG | slot, and GG_HOT_END on the last edge
+ * of each row.  The kernels run one CTA of up to GG_HOT_WARPS warps per SM;
+ * the table and 32 warps' landing slots take 224 KB of shared memory. */
 #define GG_HOT_FLAG 0x80000000u
-#define GG_HOT_ENTRIES 16384u
-#define GG_HOT_TABLE_BYTES 32768u
+#define GG_HOT_END 0x40000000u
+#define GG_HOT_ID 0x3fffffffu
+#define GG_HOT_SLOT 0x1ffffu /* GG_HOT_ENTRIES slots and the pad slot after them */
+#define GG_HOT_TABLE_BYTES 163840u
+#define GG_HOT_ENTRIES 81920u
 #define GG_HOT_WARPS 32
-#define GG_HOT_IPT 7
+#define GG_HOT_TILE_MAX 2048u
+#define GG_HOT_ROW_PAD 64u
+/* From this many edges the pull gathers use the table by default.  Measured
+ * per FP32 gather, table off -> on (its filling included): R-MAT with 4.2M
+ * edges 20.5 -> 21.2 us, 11.2M 44.5 -> 35.0, 16.8M 63.5 -> 47.5, 67M 241 ->
+ * 157, 268M 1,000 -> 662; uniform random graphs 28.7 -> 28.6, 61.5 -> 58.1,
+ * 88 -> 78, 320 -> 268, 1,259 -> 1,043.  Below, the 25 MB of table that 152
+ * SMs read per launch cost more than the requests they save. */
+#define GG_HOT_MIN_E (1u << 23)
+/* ids need two flag bits; edge numbers a tile round's headroom in 32 bits */
+#define GG_HOT_MAX_V 0x40000000u
+#define GG_HOT_MAX_E 0xfc000000u
+/* whether the hot-vertex gather can run on a graph of these sizes */
+inline bool gg_hot_fits(uint32_t V, uint32_t E) { return V > 0 && E > 0 && V < GG_HOT_MAX_V && E <= GG_HOT_MAX_E; }
 /* many-graphs PageRank (graphs.cu): tile coordinates and size order for the
  * graph boundaries h_voff (cached on the mapping), and the one launch */
 gg_status gg_graphs_prepare(gg_graph *g, uint32_t ngraphs, const uint32_t *h_voff, uint32_t items, cudaStream_t s);

@@ -6,15 +6,17 @@
  * contributions a pull gather reads most often -- get slots 0..H-1, and a
  * copy of the CSC neighbour ids carries them as 0x80000000 | slot, so a
  * gather kernel can serve those reads from a table in shared memory filled
- * once per launch.  On R-MAT graphs in natural order the 16K hottest of 16.7M
- * vertices receive 30% of all gathers, and their sectors sit on a few L2
- * slices that otherwise saturate first.
+ * per launch.  On R-MAT graphs in natural order the 32K hottest of 16.7M
+ * vertices receive 37% of all gathers, the 64K hottest 48%.
  *
  * Preparation, once per mapping: a histogram of out-degrees (clamped at
  * 65535) read back to the host gives the threshold degree T; vertices above
  * T and, up to H, vertices at T take slots by atomics (which of the ties win
  * does not matter: the table holds exact copies); one pass over the CSC
- * writes the encoded ids.
+ * writes the encoded ids.  The gather (gg_hot.cuh) finds rows through the ids
+ * themselves: three passes over the row offsets list the rows that have
+ * edges, mark each one's last edge in the encoded ids, and note for every
+ * tile of edges which row end comes first in it.
  */
 #include <cuda_runtime.h>
 
@@ -70,19 +72,20 @@ __global__ void k_hot_mark(const uint32_t *__restrict__ outdeg, uint32_t V, uint
 /* ids -> encoded ids.  Every CTA first puts the hot vertices into a Bloom
  * filter in shared memory (BLOOM_BITS bits, two hashes): an id whose two
  * bits are not both set is not hot and is copied as it is, and only the
- * others (the hot ones, ~22% of the edges of R-MAT-24, and rare false
+ * others (the hot ones, 37-48% of the edges of R-MAT-24, and rare false
  * positives) read their slot.  Reading the slot of every id at random had
  * made the pass ~0.9 ms of L2 requests at R-MAT-24.  The ids stream in
  * 16-byte loads, four in flight per thread. */
-constexpr uint32_t BLOOM_BITS = 1u << 19; /* 64 KB */
+constexpr uint32_t BLOOM_LOG2 = 20;
+constexpr uint32_t BLOOM_BITS = 1u << BLOOM_LOG2; /* 128 KB: 1.4% false positives at 64K hot vertices */
 
-__device__ __forceinline__ uint32_t bloom_h1(uint32_t u) { return (u * 0x9E3779B1u) >> 13; }
-__device__ __forceinline__ uint32_t bloom_h2(uint32_t u) { return (u * 0x85EBCA77u + 0x165667B1u) >> 13; }
+__device__ __forceinline__ uint32_t bloom_h1(uint32_t u) { return (u * 0x9E3779B1u) >> (32 - BLOOM_LOG2); }
+__device__ __forceinline__ uint32_t bloom_h2(uint32_t u) { return (u * 0x85EBCA77u + 0x165667B1u) >> (32 - BLOOM_LOG2); }
 
 __global__ void __launch_bounds__(1024) k_hot_encode(const uint32_t *__restrict__ adj, uint64_t n,
                                                      const uint32_t *__restrict__ slot_of,
                                                      const uint32_t *__restrict__ hot_list,
-                                                     const uint32_t *__restrict__ counters, uint32_t H,
+                                                     const uint32_t *__restrict__ counters, uint32_t H, uint32_t cap,
                                                      uint32_t *__restrict__ out)
 {
     extern __shared__ uint32_t bloom[];
@@ -137,25 +140,163 @@ __global__ void __launch_bounds__(1024) k_hot_encode(const uint32_t *__restrict_
         const uint64_t e = nv * 4 + threadIdx.x;
         out[e] = enc(adj[e]);
     }
+    /* the pads after the last id read the table's zero entry */
+    if (blockIdx.x == 0 && threadIdx.x < GG_EDGE_PAD) out[n + threadIdx.x] = GG_HOT_FLAG | cap;
+}
+
+/* ---- rows with edges ---- */
+
+constexpr uint32_t ROW_BLOCK = 256, ROW_PER = 8, ROW_TILE = ROW_BLOCK * ROW_PER;
+
+/* inclusive sum over the block of one value per thread; total in *all */
+__device__ __forceinline__ uint32_t block_scan(uint32_t v, uint32_t *all)
+{
+    __shared__ uint32_t part[ROW_BLOCK / 32];
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= (uint32_t)o) v += y;
+    }
+    if (lane == 31) part[w] = v;
+    __syncthreads();
+    uint32_t base = 0, total = 0;
+    for (uint32_t k = 0; k < ROW_BLOCK / 32; k++)
+    {
+        if (k < w) base += part[k];
+        total += part[k];
+    }
+    __syncthreads();
+    *all = total;
+    return v + base;
+}
+
+/* thread t of a block takes rows first + t, first + t + 256, ... so that the
+ * offsets are read coalesced; bit k of the result: row first + t + 256 k has
+ * edges */
+__device__ __forceinline__ uint32_t rows_with_edges(const uint32_t *__restrict__ off, uint32_t V, uint32_t first)
+{
+    uint32_t bits = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < ROW_PER; k++)
+    {
+        const uint32_t v = first + k * ROW_BLOCK + threadIdx.x;
+        if (v < V && off[v + 1] > off[v]) bits |= 1u << k;
+    }
+    return bits;
+}
+
+__global__ void __launch_bounds__(ROW_BLOCK) k_rows_count(const uint32_t *__restrict__ off, uint32_t V,
+                                                          uint32_t *__restrict__ counts)
+{
+    uint32_t all;
+    block_scan((uint32_t)__popc(rows_with_edges(off, V, blockIdx.x * ROW_TILE)), &all);
+    if (threadIdx.x == 0) counts[blockIdx.x] = all;
+}
+
+/* exclusive scan of the block counts, in place, by one block */
+__global__ void __launch_bounds__(ROW_BLOCK) k_rows_scan(uint32_t *counts, uint32_t n)
+{
+    uint32_t base = 0;
+    for (uint32_t at = 0; at < n; at += ROW_TILE)
+    {
+        uint32_t c[ROW_PER], sum = 0;
+#pragma unroll
+        for (uint32_t k = 0; k < ROW_PER; k++)
+        {
+            const uint32_t i = at + threadIdx.x * ROW_PER + k;
+            c[k] = i < n ? counts[i] : 0u;
+            sum += c[k];
+        }
+        uint32_t all;
+        uint32_t run = base + block_scan(sum, &all) - sum;
+#pragma unroll
+        for (uint32_t k = 0; k < ROW_PER; k++)
+        {
+            const uint32_t i = at + threadIdx.x * ROW_PER + k;
+            if (i < n) counts[i] = run;
+            run += c[k];
+        }
+        base += all;
+    }
+}
+
+/* rows[r] = the r-th row with edges; seg0 of the tiles that begin in it */
+__global__ void __launch_bounds__(ROW_BLOCK) k_rows_write(const uint32_t *__restrict__ off, uint32_t V,
+                                                          const uint32_t *__restrict__ base,
+                                                          uint32_t *__restrict__ rows, uint32_t *__restrict__ seg0,
+                                                          uint32_t tile)
+{
+    const uint32_t first = blockIdx.x * ROW_TILE;
+    uint32_t r0 = base[blockIdx.x];
+    for (uint32_t k = 0; k < ROW_PER; k++)
+    {
+        const uint32_t v = first + k * ROW_BLOCK + threadIdx.x;
+        uint32_t a = 0, b = 0;
+        if (v < V)
+        {
+            a = off[v];
+            b = off[v + 1];
+        }
+        uint32_t all;
+        const uint32_t r = r0 + block_scan(b > a ? 1u : 0u, &all) - 1u;
+        if (b > a)
+        {
+            rows[r] = v;
+            /* tiles whose first edge lies in [a, b) */
+            for (uint64_t t = ((uint64_t)a + tile - 1) / tile; t * tile < b; t++)
+                seg0[t] = r | (t * tile > a ? 0x80000000u : 0u);
+        }
+        r0 += all;
+    }
+}
+
+/* the last edge of every row in the encoded ids */
+__global__ void k_rows_mark(const uint32_t *__restrict__ off, uint32_t V, uint32_t *__restrict__ ids)
+{
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
+    {
+        const uint32_t a = off[v], b = off[v + 1];
+        if (b > a) ids[b - 1] |= GG_HOT_END;
+    }
 }
 
 } // namespace
+
+/* edges per tile: the tiles are dealt round robin to 32 warps on every SM, so
+ * a few tiles per warp leave the last round nearly empty (R-MAT-20, 3,450
+ * edges per warp: 49 us with tiles of 2048) and many cost an atomic add each.
+ * At least eight tiles per warp, from 256 to GG_HOT_TILE_MAX edges. */
+static uint32_t hot_tile_for(uint32_t E)
+{
+    uint32_t tile = 256;
+    while (tile < GG_HOT_TILE_MAX && (uint64_t)tile * 2 * 8 * 32 * (uint32_t)gg_sm_count() <= E) tile *= 2;
+    return tile;
+}
 
 gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap)
 {
     if (!g->in_adj || !g->out_deg) return gg_fail(GG_ERR_INVALID, "the hot-vertex table needs GG_MAP_IN");
     const uint32_t V = g->V, E = g->E;
-    if (V >= GG_HOT_FLAG) return gg_fail(GG_ERR_INVALID, "graph too large for flag-encoded ids");
+    if (!gg_hot_fits(V, E)) return gg_fail(GG_ERR_INVALID, "graph too large for flag-encoded ids");
     if (cap < 1 || cap > GG_HOT_ENTRIES) return gg_fail(GG_ERR_INVALID, "hot table capacity out of range");
-    gg_tiles &t = g->hot_tiles;
-    if (!t.coord)
+    if (!g->hot_seg0)
     {
-        const uint32_t items = 32u * GG_HOT_IPT;
-        const uint64_t nt = ((uint64_t)V + E + items - 1) / items;
-        if (nt >= 0xffffffffull) return gg_fail(GG_ERR_INVALID, "graph too large for 32-bit tile ids");
-        t.ntiles = (uint32_t)(nt ? nt : 1);
-        GG_CHECK(gg_dev_alloc(g, (void **)&t.coord, ((size_t)t.ntiles + 1) * sizeof(uint2)));
-        GG_CHECK(gg_launch_tile_coords(g->in_off, V, E, t.ntiles, t.coord, s, items));
+        const uint32_t nb = (uint32_t)(((uint64_t)V + ROW_TILE - 1) / ROW_TILE);
+        const uint32_t tile = hot_tile_for(E);
+        const uint32_t nt = (uint32_t)(((uint64_t)E + tile - 1) / tile);
+        void *counts;
+        GG_CHECK(gg_work(g, 33, (size_t)nb * 4, &counts));
+        if (!g->hot_rows) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_rows, ((size_t)V + GG_HOT_ROW_PAD) * 4));
+        g->hot_ntiles = nt;
+        g->hot_tile = tile;
+        GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_seg0, (size_t)nt * 4));
+        k_rows_count<<<nb, ROW_BLOCK, 0, s>>>(g->in_off, V, (uint32_t *)counts);
+        k_rows_scan<<<1, ROW_BLOCK, 0, s>>>((uint32_t *)counts, nb);
+        k_rows_write<<<nb, ROW_BLOCK, 0, s>>>(g->in_off, V, (const uint32_t *)counts, g->hot_rows, g->hot_seg0,
+                                             tile);
+        GG_CUDA(cudaGetLastError());
     }
     if (g->hot_adj && g->hot_cap == cap) return GG_OK;
     const uint32_t H = V < cap ? V : cap;
@@ -190,7 +331,8 @@ gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap)
      * whole allocations, 16-byte aligned for the vector loads */
     GG_CUDA(cudaFuncSetAttribute(k_hot_encode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BLOOM_BITS / 8)));
     k_hot_encode<<<gg_sm_count(), 1024, BLOOM_BITS / 8, s>>>(g->in_adj, (uint64_t)E, (const uint32_t *)slot_of,
-                                                              g->hot_list, (const uint32_t *)cnt, H, g->hot_adj);
+                                                              g->hot_list, (const uint32_t *)cnt, H, cap, g->hot_adj);
+    k_rows_mark<<<grid, 256, 0, s>>>(g->in_off, V, g->hot_adj);
     GG_CUDA(cudaGetLastError());
     std::vector<uint32_t> c(4);
     GG_CHECK(gg_wait(s));

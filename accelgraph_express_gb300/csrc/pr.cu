@@ -27,7 +27,7 @@
  * stores the rounding of (contribution - stored so far) and no rounding
  * error accumulates (k_pr_update_delta).
  *
- * From 1M vertices the FP pull gather reads the contributions of the
+ * From 8M edges the pull gather reads the contributions of the
  * vertices with the most out-edges from a shared-memory table
  * (k_pr_pull_hot, table built by hot.cu).  With GG_PR_CUDA_GRAPH the whole
  * call is captured once into a CUDA graph kept on the mapping and relaunched
@@ -42,7 +42,7 @@
 #include <cstring>
 #include <vector>
 
-#include "gg_device.cuh"
+#include "gg_hot.cuh"
 
 namespace {
 
@@ -237,92 +237,54 @@ struct PrGather
     __device__ __forceinline__ Acc value(const Raw &r) const { return decode<K>(r); }
 };
 
-/* the gather with the hot-vertex table: flagged ids read the table */
-template <int K>
-struct PrGatherHot
+/* the hot vertices' stored contributions, contiguous, for k_pr_pull_hot */
+template <class CT>
+__global__ void k_pr_hot_fill(const CT *__restrict__ cin, const uint32_t *__restrict__ hot_list, uint32_t n,
+                              uint32_t cap, CT *__restrict__ out, const IterRec *rec, uint32_t it)
 {
-    typedef typename Fmt<K>::Tile Acc;
-    typedef typename Fmt<K>::Acc Sum;
-    typedef typename Fmt<K>::CT Raw;
-    const Raw *cin;
-    const Raw *s_hot;
-    __device__ __forceinline__ Raw load(uint32_t, uint32_t u) const
-    {
-        if (u & GG_HOT_FLAG) return s_hot[u & ~GG_HOT_FLAG];
-        return ldg_val(cin + u);
-    }
-    __device__ __forceinline__ Acc value(const Raw &r) const { return decode<K>(r); }
-};
-
-template <int K>
-__host__ __device__ constexpr uint32_t hot_entries()
-{
-    return GG_HOT_TABLE_BYTES / sizeof(typename Fmt<K>::CT) < GG_HOT_ENTRIES
-               ? (uint32_t)(GG_HOT_TABLE_BYTES / sizeof(typename Fmt<K>::CT))
-               : GG_HOT_ENTRIES;
-}
-template <int K>
-__host__ __device__ constexpr size_t hot_stage_bytes(uint32_t warps)
-{
-    return (size_t)warps * PullStage<GG_HOT_IPT, typename Fmt<K>::Tile>::BYTES;
-}
-template <int K>
-__host__ __device__ constexpr size_t hot_smem_bytes(uint32_t warps)
-{
-    return hot_stage_bytes<K>(warps) + ((size_t)hot_entries<K>() * sizeof(typename Fmt<K>::CT) + 15) / 16 * 16;
-}
-
-/* one CTA per SM (up to GG_HOT_WARPS warps, the tuned count): the CTA fills
- * the table with the hot vertices' stored contributions, then its warps run
- * the engine */
-template <int K>
-__global__ void __launch_bounds__(GG_HOT_WARPS * 32, 1)
-    k_pr_pull_hot(const uint32_t *__restrict__ off, const uint32_t *__restrict__ hot_adj,
-                  const uint2 *__restrict__ coord, uint32_t ntiles, uint32_t V, typename Fmt<K>::Acc *sums,
-                  const typename Fmt<K>::CT *__restrict__ cin, const uint32_t *__restrict__ hot_list, uint32_t hot_n,
-                  const IterRec *rec, uint32_t it)
-{
-    typedef typename Fmt<K>::CT CT;
-    extern __shared__ __align__(16) unsigned char gg_dyn[];
     pdl_wait();
     if (it > 0 && rec[it - 1].active == 0u) return;
-    CT *s_hot = reinterpret_cast<CT *>(gg_dyn + hot_stage_bytes<K>(blockDim.x >> 5));
-    for (uint32_t i = threadIdx.x; i < hot_n; i += blockDim.x) s_hot[i] = cin[hot_list[i]];
-    __syncthreads();
-    warp_pull_sums_dyn<GG_HOT_IPT>(gg_dyn, off, hot_adj, V, coord, ntiles, sums, PrGatherHot<K>{cin, s_hot});
+    hot_table_fill(cin, hot_list, n, cap, out);
     pdl_trigger();
 }
 
-/* grid of k_pr_pull_hot<K> with `warps` warps: one CTA per SM, the
- * carve-out sized to its shared memory (the rest of the array stays L1) */
+/* the pull gather through the hot-vertex table (gg_hot.cuh): one CTA per SM
+ * of up to GG_HOT_WARPS warps (the tuned count).  The first ids are on their
+ * way before the wait for the previous kernel: they do not depend on it. */
+template <int K>
+__global__ void __launch_bounds__(GG_HOT_WARPS * 32, 1)
+    k_pr_pull_hot(HotArgs a, const typename Fmt<K>::CT *__restrict__ cin,
+                  const typename Fmt<K>::CT *__restrict__ table_src, typename Fmt<K>::Acc *sums, const IterRec *rec,
+                  uint32_t it)
+{
+    typedef typename Fmt<K>::CT CT;
+    extern __shared__ __align__(16) unsigned char gg_dyn[];
+    const uint32_t table = (uint32_t)__cvta_generic_to_shared(gg_dyn);
+    const uint32_t warps = blockDim.x >> 5, w = threadIdx.x >> 5;
+    hot_pull_sums<CT, typename Fmt<K>::Tile, typename Fmt<K>::Acc, false>(
+        table + hot_table_bytes<CT>() + w * HOT_RING, table, hot_cap<CT>(), a, w * gridDim.x + blockIdx.x,
+        gridDim.x * warps, cin, (const CT *)nullptr, sums, [&] {
+            pdl_wait();
+            if (it > 0 && rec[it - 1].active == 0u) return false;
+            hot_table_load(table, table_src, hot_table_bytes<CT>());
+            return true;
+        });
+    pdl_trigger();
+}
+
+/* grid of k_pr_pull_hot<K> with `warps` warps: one CTA per SM */
 template <int K>
 int hot_grid(uint32_t ntiles, uint32_t warps)
 {
     static int ok = -1;
-    static uint32_t applied = 0;
-    int dev = 0, smem_sm = 0;
     if (ok < 0)
     {
-        const size_t most = hot_smem_bytes<K>(GG_HOT_WARPS);
-        cudaError_t e = cudaFuncSetAttribute(k_pr_pull_hot<K>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        cudaError_t e = cudaFuncSetAttribute(k_pr_pull_hot<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)hot_smem_bytes<typename Fmt<K>::CT>(GG_HOT_WARPS));
         ok = e == cudaSuccess ? 1 : 0;
         if (!ok) cudaGetLastError();
     }
     if (!ok) return 0;
-    if (applied != warps)
-    {
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-        if (smem_sm > 0)
-        {
-            const int pct = (int)ceil(100.0 * (double)(hot_smem_bytes<K>(warps) + 1024) / (double)smem_sm);
-            if (cudaFuncSetAttribute(k_pr_pull_hot<K>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     pct > 100 ? 100 : pct) == cudaSuccess)
-                applied = warps;
-            else
-                cudaGetLastError();
-        }
-    }
     const uint32_t need = (ntiles + warps - 1) / warps;
     const uint32_t cap = (uint32_t)gg_sm_count();
     return (int)(need < cap ? (need ? need : 1) : cap);
@@ -986,12 +948,13 @@ gg_status run_pull(Run &R, IterRec *rec, float *rank, uint32_t iters, float base
     CT *cb[2] = {(CT *)c0, (CT *)c1};
     /* 16-bit storage: FP32 running sums and stored-so-far values */
     constexpr bool delta = K == K_BF16 || K == K_F16;
-    void *Sb = nullptr, *chb = nullptr;
+    void *Sb = nullptr, *chb = nullptr, *hot_tab = nullptr;
     if (delta)
     {
         GG_CHECK(gg_work(g, 28, ((size_t)V + 16) * 4, &Sb));
         GG_CHECK(gg_work(g, 29, ((size_t)V + 16) * 4, &chb));
     }
+    if (R.use_hot) GG_CHECK(gg_work(g, 32, GG_HOT_TABLE_BYTES + 16, &hot_tab));
 
     if constexpr (delta)
         k_pr_init_delta<K><<<grid_v(V), 256, 0, R.s>>>(rank, g->out_deg, V, init, cb[0], (float *)Sb, (float *)chb, rec);
@@ -1011,22 +974,30 @@ gg_status run_pull(Run &R, IterRec *rec, float *rank, uint32_t iters, float base
         GG_CHECK(timed_begin(R));
         int hg = 0;
         const uint32_t hw = R.shape.hot_warps;
-        if constexpr (sizeof(Acc) == 4)
-            if (R.use_hot && g->hot_cap == hot_entries<K>()) hg = hot_grid<K>(g->hot_tiles.ntiles, hw);
+        if (R.use_hot) hg = hot_grid<K>(g->hot_ntiles, hw);
         /* gather and update as programmatic dependent launches (each kernel
          * waits for the one before it; its launch overlaps that kernel's
          * tail), except when they are timed one by one */
         const bool pdl = !R.p->profile;
         if (hg)
         {
+            const HotArgs ha{g->hot_adj, g->hot_rows, g->hot_seg0, g->E, g->hot_ntiles, g->hot_tile};
+            CT *tab = (CT *)hot_tab;
+            const size_t smem = hot_smem_bytes<CT>(hw);
+            const int fg = (int)((hot_cap<CT>() + 255) / 256);
             if (pdl)
-                GG_CUDA(gg_launch_pdl(k_pr_pull_hot<K>, dim3(hg), dim3(hw * 32), hot_smem_bytes<K>(hw), R.s, g->in_off,
-                                      g->hot_adj, g->hot_tiles.coord, g->hot_tiles.ntiles, V, (Acc *)sums, cin,
-                                      g->hot_list, g->hot_n, (const IterRec *)rec, it));
+            {
+                GG_CUDA(gg_launch_pdl(k_pr_hot_fill<CT>, dim3(fg), dim3(256), 0, R.s, cin, g->hot_list, g->hot_n,
+                                      hot_cap<CT>(), tab, (const IterRec *)rec, it));
+                GG_CUDA(gg_launch_pdl(k_pr_pull_hot<K>, dim3(hg), dim3(hw * 32), smem, R.s, ha, cin, (const CT *)tab,
+                                      (Acc *)sums, (const IterRec *)rec, it));
+            }
             else
-                k_pr_pull_hot<K><<<hg, hw * 32, hot_smem_bytes<K>(hw), R.s>>>(
-                    g->in_off, g->hot_adj, g->hot_tiles.coord, g->hot_tiles.ntiles, V, (Acc *)sums, cin, g->hot_list,
-                    g->hot_n, rec, it);
+            {
+                k_pr_hot_fill<CT><<<fg, 256, 0, R.s>>>(cin, g->hot_list, g->hot_n, hot_cap<CT>(), tab, rec, it);
+                k_pr_pull_hot<K><<<hg, hw * 32, smem, R.s>>>(ha, cin, tab, (Acc *)sums, rec, it);
+            }
+            R.launches++;
         }
         else
         {
@@ -1209,6 +1180,21 @@ gg_status run_dd(Run &R, int mode, IterRec *rec, float *rank, uint32_t iters, fl
     return GG_OK;
 }
 
+/* bytes of a stored contribution of the topology-driven pull modes; 0 for
+ * the other modes */
+uint32_t value_bytes(const gg_pr_params *p)
+{
+    switch (p->mode)
+    {
+    case GG_PR_PULL: return p->storage == GG_STORE_F32 ? 4u : 2u;
+    case GG_PR_PULL_FX64: return 8u;
+    case GG_PR_PULL_FX32: case GG_PR_PULL_Q32: return 4u;
+    case GG_PR_PULL_FX16: case GG_PR_PULL_Q16: return 2u;
+    case GG_PR_PULL_FX8: case GG_PR_PULL_Q8: return 1u;
+    default: return 0u;
+    }
+}
+
 /* every launch of one PageRank run, queued on R.s */
 gg_status pagerank_enqueue(Run &R, const gg_pr_params *p, IterRec *rec, float *rank, void *sum_v, uint32_t ngraphs,
                            const uint32_t *voff)
@@ -1372,16 +1358,18 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
         GG_CUDA(cudaMemcpyAsync(voff_v, h_voff, ((size_t)ngraphs + 1) * 4, cudaMemcpyHostToDevice, R.s));
     }
 
-    /* the hot-vertex table for the FP pull modes (prepared before any
-     * capture: preparation reads back to the host) */
+    /* the hot-vertex table of the pull modes (prepared before any capture: preparation reads back to the host) */
     gg_tune_lookup(g, R.s);
     R.shape = g->pr_shape;
-    const bool hot_default = R.shape.hot == 2 ? V >= (1u << 20) : R.shape.hot == 1;
-    if (p->mode == GG_PR_PULL && !(p->flags & GG_PR_HOT_OFF) && ((p->flags & GG_PR_HOT_ON) || hot_default) &&
-        V < GG_HOT_FLAG && V > 0)
+    const bool hot_default = R.shape.hot == 2 ? g->E >= GG_HOT_MIN_E : R.shape.hot == 1;
+    if (value_bytes(p) && !(p->flags & GG_PR_HOT_OFF) && ((p->flags & GG_PR_HOT_ON) || hot_default) &&
+        gg_hot_fits(V, g->E))
     {
-        const uint32_t cap = GG_HOT_TABLE_BYTES / (p->storage == GG_STORE_F32 ? 4u : 2u);
-        GG_CHECK(gg_hot_prepare(g, R.s, cap < GG_HOT_ENTRIES ? cap : GG_HOT_ENTRIES));
+        const uint32_t vb = value_bytes(p);
+        GG_CHECK(gg_hot_prepare(g, R.s, vb == 8   ? hot_cap<unsigned long long>()
+                                        : vb == 4 ? hot_cap<uint32_t>()
+                                        : vb == 2 ? hot_cap<uint16_t>()
+                                                  : hot_cap<uint8_t>()));
         R.use_hot = true;
     }
 

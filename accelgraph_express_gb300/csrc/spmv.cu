@@ -20,7 +20,7 @@
 #include <string>
 #include <vector>
 
-#include "gg_device.cuh"
+#include "gg_hot.cuh"
 
 namespace {
 
@@ -47,84 +47,43 @@ __global__ void __launch_bounds__(GG_TILE_NT) k_spmv_pull(const uint32_t *__rest
     warp_pull_sums<GG_TILE_IPT, GG_TILE_WARPS>(off, adj, V, coord, ntiles, y, op);
 }
 
-/* the pull product with the hot-vertex table: x of the flagged in-neighbours
- * comes from shared memory (the same table as the PageRank gather's) */
+/* x of the hot vertices, contiguous (once per call: x does not change) */
 template <class T>
-struct SpmvGatherHot
+__global__ void k_spmv_hot_fill(const T *__restrict__ x, const uint32_t *__restrict__ hot_list, uint32_t n,
+                                uint32_t cap, T *__restrict__ out)
 {
-    typedef float Acc;
-    typedef float Sum;
-    typedef typename SpmvGather<T>::Raw Raw;
-    const T *w;
-    const T *x;
-    const T *s_hot;
-    __device__ __forceinline__ Raw load(uint32_t e, uint32_t u) const
-    {
-        const T wv = ldg_val(w + e);
-        if (u & GG_HOT_FLAG) return Raw{wv, s_hot[u & ~GG_HOT_FLAG]};
-        return Raw{wv, ldg_val(x + u)};
-    }
-    __device__ __forceinline__ float value(const Raw &r) const { return __fmul_rn(to_f32(r.w), to_f32(r.x)); }
-};
-
-template <class T>
-__host__ __device__ constexpr size_t spmv_hot_stage_bytes(uint32_t warps)
-{
-    return (size_t)warps * PullStage<GG_HOT_IPT, float>::BYTES;
-}
-template <class T>
-__host__ __device__ constexpr uint32_t spmv_hot_entries()
-{
-    return GG_HOT_TABLE_BYTES / sizeof(T) < GG_HOT_ENTRIES ? (uint32_t)(GG_HOT_TABLE_BYTES / sizeof(T)) : GG_HOT_ENTRIES;
-}
-template <class T>
-__host__ __device__ constexpr size_t spmv_hot_smem_bytes(uint32_t warps)
-{
-    return spmv_hot_stage_bytes<T>(warps) + ((size_t)spmv_hot_entries<T>() * sizeof(T) + 15) / 16 * 16;
+    hot_table_fill(x, hot_list, n, cap, out);
 }
 
+/* the pull product through the hot-vertex table (gg_hot.cuh) */
 template <class T>
 __global__ void __launch_bounds__(GG_HOT_WARPS * 32, 1)
-    k_spmv_pull_hot(const uint32_t *__restrict__ off, const uint32_t *__restrict__ hot_adj,
-                    const uint2 *__restrict__ coord, uint32_t ntiles, uint32_t V, float *y, const T *w,
-                    const T *__restrict__ x, const uint32_t *__restrict__ hot_list, uint32_t hot_n)
+    k_spmv_pull_hot(HotArgs a, const T *__restrict__ x, const T *__restrict__ w, const T *__restrict__ table_src,
+                    float *y)
 {
     extern __shared__ __align__(16) unsigned char gg_dyn[];
-    T *s_hot = reinterpret_cast<T *>(gg_dyn + spmv_hot_stage_bytes<T>(blockDim.x >> 5));
-    for (uint32_t i = threadIdx.x; i < hot_n; i += blockDim.x) s_hot[i] = x[hot_list[i]];
-    __syncthreads();
-    warp_pull_sums_dyn<GG_HOT_IPT>(gg_dyn, off, hot_adj, V, coord, ntiles, y, SpmvGatherHot<T>{w, x, s_hot});
+    const uint32_t table = (uint32_t)__cvta_generic_to_shared(gg_dyn);
+    const uint32_t warps = blockDim.x >> 5, wid = threadIdx.x >> 5;
+    hot_pull_sums<T, float, float, true>(table + hot_table_bytes<T>() + wid * HOT_RING, table, hot_cap<T>(), a,
+                           wid * gridDim.x + blockIdx.x, gridDim.x * warps, x, w, y, [&] {
+                               hot_table_load(table, table_src, hot_table_bytes<T>());
+                               return true;
+                           });
 }
 
-/* one CTA of `warps` warps per SM, carve-out sized to its shared memory */
+/* one CTA of `warps` warps per SM */
 template <class T>
 int spmv_hot_grid(uint32_t ntiles, uint32_t warps)
 {
     static int ok = -1;
-    static uint32_t applied = 0;
     if (ok < 0)
     {
-        const size_t most = spmv_hot_smem_bytes<T>(GG_HOT_WARPS);
-        cudaError_t e = cudaFuncSetAttribute(k_spmv_pull_hot<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most);
+        cudaError_t e = cudaFuncSetAttribute(k_spmv_pull_hot<T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)hot_smem_bytes<T>(GG_HOT_WARPS));
         ok = e == cudaSuccess ? 1 : 0;
         if (!ok) cudaGetLastError();
     }
     if (!ok) return 0;
-    if (applied != warps)
-    {
-        int dev = 0, smem_sm = 0;
-        cudaGetDevice(&dev);
-        cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-        if (smem_sm > 0)
-        {
-            const int pct = (int)ceil(100.0 * (double)(spmv_hot_smem_bytes<T>(warps) + 1024) / (double)smem_sm);
-            if (cudaFuncSetAttribute(k_spmv_pull_hot<T>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                     pct > 100 ? 100 : pct) == cudaSuccess)
-                applied = warps;
-            else
-                cudaGetLastError();
-        }
-    }
     const uint32_t need = (ntiles + warps - 1) / warps;
     const uint32_t cap = (uint32_t)gg_sm_count();
     return (int)(need < cap ? (need ? need : 1) : cap);
@@ -297,15 +256,19 @@ gg_status spmv_fp(gg_graph *g, const gg_spmv_params *p, const float *x_dev, floa
     k_spmv_x<T><<<grid_v(V), 256, 0, s>>>(g->out_deg, x_dev, xf, (T *)xs, nullptr, nullptr, y, V);
     launches++;
     const T *xv = sizeof(T) == 4 ? (const T *)xf : (const T *)xs;
-    /* the hot-vertex table (as for the PageRank pull): by default from 1M vertices */
+    /* the hot-vertex table, as for the PageRank pull */
     bool use_hot = false;
+    void *hot_tab = nullptr;
     gg_tune_lookup(g, s);
     const gg_pull_shape shape = g->spmv_shape;
-    const bool hot_default = shape.hot == 2 ? V >= (1u << 20) : shape.hot == 1;
-    if (pull && !(p->flags & GG_PR_HOT_OFF) && ((p->flags & GG_PR_HOT_ON) || hot_default) && V < GG_HOT_FLAG)
+    const bool hot_default = shape.hot == 2 ? g->E >= GG_HOT_MIN_E : shape.hot == 1;
+    if (pull && !(p->flags & GG_PR_HOT_OFF) && ((p->flags & GG_PR_HOT_ON) || hot_default) && gg_hot_fits(V, g->E))
     {
-        GG_CHECK(gg_hot_prepare(g, s, spmv_hot_entries<T>()));
-        use_hot = g->hot_cap == spmv_hot_entries<T>();
+        GG_CHECK(gg_hot_prepare(g, s, hot_cap<T>()));
+        GG_CHECK(gg_work(g, 32, GG_HOT_TABLE_BYTES + 16, &hot_tab));
+        k_spmv_hot_fill<T><<<(hot_cap<T>() + 255) / 256, 256, 0, s>>>(xv, g->hot_list, g->hot_n, hot_cap<T>(), (T *)hot_tab);
+        launches++;
+        use_hot = true;
     }
     for (uint32_t it = 0; it < p->iterations; it++)
     {
@@ -321,10 +284,10 @@ gg_status spmv_fp(gg_graph *g, const gg_spmv_params *p, const float *x_dev, floa
             /* y is the row-sum array: zero, then the gather stores rows and
              * adds the partials of rows spanning tiles */
             GG_CUDA(cudaMemsetAsync(y, 0, (size_t)V * sizeof(float), s));
-            const int hg = use_hot ? spmv_hot_grid<T>(g->hot_tiles.ntiles, shape.hot_warps) : 0;
+            const int hg = use_hot ? spmv_hot_grid<T>(g->hot_ntiles, shape.hot_warps) : 0;
             if (hg)
-                k_spmv_pull_hot<T><<<hg, shape.hot_warps * 32, spmv_hot_smem_bytes<T>(shape.hot_warps), s>>>(
-                    g->in_off, g->hot_adj, g->hot_tiles.coord, g->hot_tiles.ntiles, V, y, w, xv, g->hot_list, g->hot_n);
+                k_spmv_pull_hot<T><<<hg, shape.hot_warps * 32, hot_smem_bytes<T>(shape.hot_warps), s>>>(
+                    HotArgs{g->hot_adj, g->hot_rows, g->hot_seg0, g->E, g->hot_ntiles, g->hot_tile}, xv, w, (const T *)hot_tab, y);
             else
                 k_spmv_pull<T><<<gg_persistent_grid((const void *)k_spmv_pull<T>, t->ntiles, (int)shape.ctas),
                                  GG_TILE_NT, 0, s>>>(g->in_off, g->in_adj, t->coord, t->ntiles, V, y, SpmvGather<T>{w, xv});

@@ -159,7 +159,7 @@ gg_status tune_pull(gg_graph *g, bool spmv, uint32_t storage, uint32_t reps, cud
         x.ctas = ctas;
         cands.push_back(x);
     }
-    if (g->V < GG_HOT_FLAG)
+    if (gg_hot_fits(g->V, g->E))
         for (uint32_t w : {16u, 24u, 32u})
         {
             gg_pull_shape x;

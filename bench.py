@@ -10,7 +10,7 @@ value      GTEPS with the graph resident in HBM, device time (CUDA events on
 e2e        the same metric through the drop-in pageRankGraphCSR call on host
            arrays: every step uploads the CSC (offsets, neighbour ids) and
            out-degrees and reads the ranks back.
-roofline   the gather kernel (k_pr_pull_hot from 1M vertices: the pull gather
+roofline   the gather kernel (k_pr_pull_hot from 8M edges: the pull gather
            with the hot-vertex table; k_pr_pull below): algorithmic bytes per launch
            4E + 4(V+1) + sV + 4V with s = 4 bytes of FP32 contribution (CSC
            ids, CSC offsets, each contribution once, the row sums written),

@@ -186,10 +186,11 @@ typedef struct gg_pr_params
  * freed since (another algorithm regrowing a shared work buffer), in which
  * case it is captured again. */
 #define GG_PR_CUDA_GRAPH 0x1u
-/* The pull gather of the FP32/BF16/FP16 modes serves the contributions of
- * the 16K vertices with the most out-edges from a shared-memory table (built
- * once per mapping; an extra copy of the CSC ids).  By default from 1M
- * vertices up; HOT_OFF never, HOT_ON on any graph.  Results are the same. */
+/* The pull gather (every pull mode; SpMV pull in FP) serves the values of the
+ * vertices with the most out-edges -- 40K FP32, 80K 16- or 8-bit, 20K 64-bit
+ * ones -- from a shared-memory table (built once per mapping; an extra copy of
+ * the CSC ids).  By default from 8M edges up; HOT_OFF never, HOT_ON on any
+ * graph with edges (below 2^30 vertices).  Results are the same. */
 #define GG_PR_HOT_OFF 0x2u
 #define GG_PR_HOT_ON 0x4u
 /* gg_pagerank_batch: run the ordinary pull over the union of the graphs
