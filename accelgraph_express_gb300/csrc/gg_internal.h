@@ -107,8 +107,12 @@ struct gg_graph
 
     /* work buffers, grown on demand */
     gg_buf work[34];
-    /* merge-path tiles of the batched PageRank gather (own tile size) */
-    gg_tiles ppr_tiles;
+    /* the rows (of the CSC) that have edges, in order: rows_list[0 .. n), then
+     * GG_ROW_PAD entries of V, and n itself at rows_list[V + GG_ROW_PAD] */
+    uint32_t *rows_list = nullptr;
+    /* batched PageRank: first row end of every tile of ppr_tiles_items edges */
+    uint32_t *ppr_seg0 = nullptr;
+    uint32_t ppr_ntiles = 0;
     const float *ppr_ranks = nullptr;
     uint32_t ppr_stride = 0;
     /* hot-vertex table: flag-encoded copy of in_adj and the slot -> vertex list */
@@ -116,7 +120,6 @@ struct gg_graph
     uint32_t *hot_list = nullptr;  /* GG_HOT_ENTRIES slots */
     uint32_t hot_n = 0;            /* slots in use */
     uint32_t hot_cap = 0;          /* table capacity the encoding was made for */
-    uint32_t *hot_rows = nullptr;  /* the rows with edges, in order (V + GG_HOT_ROW_PAD entries) */
     uint32_t *hot_seg0 = nullptr;  /* per tile of hot_tile edges: its first row end (gg_hot.cuh) */
     uint32_t hot_ntiles = 0, hot_tile = 0; /* tiles and edges per tile */
     /* page-locked host scratch for small per-step read-backs */
@@ -150,7 +153,7 @@ struct gg_graph
      * threshold, the batched PPR tile; tuned = bit per family */
     gg_pull_shape pr_shape, spmv_shape;
     uint32_t bfs_heavy = 64;
-    uint32_t ppr_tile = 512, ppr_tiles_items = 0;
+    uint32_t ppr_tile = 0, ppr_tiles_items = 0; /* 0: by size (gg_ppr_tile) */
     uint32_t tuned = 0;
     bool tune_looked_up = false;
 };
@@ -213,6 +216,12 @@ gg_status gg_pinned(gg_graph *g, size_t bytes, void **out);
  * (<= GG_HOT_ENTRIES; rebuilt only when cap changes; needs GG_MAP_IN and
  * gg_hot_fits), and the rows and tiles of the hot kernels */
 gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap);
+/* rows_list of the mapping, and for tiles of `tile` edges the first row end in
+ * each (bit 31: that row began in an earlier tile) in a new allocation of
+ * *ntiles words; adds its launches to *launches (hot.cu) */
+#define GG_ROW_PAD 128u
+gg_status gg_rows_tiles(gg_graph *g, cudaStream_t s, uint32_t tile, uint32_t **seg0, uint32_t *ntiles,
+                        uint32_t *launches);
 cudaStream_t gg_stream(gg_graph *g, void *user_stream);
 /* host wait on all work queued on `s`, bounded by the wait limit */
 gg_status gg_wait(cudaStream_t s);
@@ -292,7 +301,6 @@ unsigned long long gg_barrier_limit_ns();
 #define GG_HOT_ENTRIES 81920u
 #define GG_HOT_WARPS 32
 #define GG_HOT_TILE_MAX 2048u
-#define GG_HOT_ROW_PAD 64u
 /* From this many edges the pull gathers use the table by default.  Measured
  * per FP32 gather, table off -> on (its filling included): R-MAT with 4.2M
  * edges 20.5 -> 21.2 us, 11.2M 44.5 -> 35.0, 16.8M 63.5 -> 47.5, 67M 241 ->
@@ -335,6 +343,8 @@ struct gg_ppr_round_args
     float *slots = nullptr;
     float damp = 0.85f;
 };
+/* edges per tile of the batched PageRank on this mapping */
+uint32_t gg_ppr_tile(const gg_graph *g);
 /* tiles and the two contribution buffers (zeroed) and the tile slots */
 gg_status gg_ppr_round_prepare(gg_graph *g, uint32_t rs, int bf16, void **cb0, void **cb1, float **slots,
                                cudaStream_t s);

@@ -1075,10 +1075,10 @@ extern "C" gg_status gg_graph_unmap(gg_graph *g)
     }
     free_tiles(g, g->in_tiles, idle);
     free_tiles(g, g->out_tiles, idle);
-    free_tiles(g, g->ppr_tiles, idle);
+    dev_release(g, g->rows_list, ((size_t)g->V + GG_ROW_PAD + 4) * 4, idle);
+    dev_release(g, g->ppr_seg0, (size_t)g->ppr_ntiles * 4, idle);
     dev_release(g, g->hot_adj, ((size_t)g->E + GG_EDGE_PAD) * 4, idle);
     dev_release(g, g->hot_list, (size_t)GG_HOT_ENTRIES * 4, idle);
-    dev_release(g, g->hot_rows, ((size_t)g->V + GG_HOT_ROW_PAD) * 4, idle);
     dev_release(g, g->hot_seg0, (size_t)g->hot_ntiles * 4, idle);
     for (auto &b : g->work) dev_release(g, b.ptr, b.bytes, idle);
     dev_release(g, g->graphs.coord, g->graphs.bytes, idle);

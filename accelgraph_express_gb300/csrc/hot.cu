@@ -14,8 +14,7 @@
  * T and, up to H, vertices at T take slots by atomics (which of the ties win
  * does not matter: the table holds exact copies); one pass over the CSC
  * writes the encoded ids.  The gather (gg_hot.cuh) finds rows through the ids
- * themselves: three passes over the row offsets list the rows that have
- * edges, mark each one's last edge in the encoded ids, and note for every
+ * themselves: passes over the row offsets list the rows that have edges, mark each one's last edge in the encoded ids, and note for every
  * tile of edges which row end comes first in it.
  */
 #include <cuda_runtime.h>
@@ -187,17 +186,25 @@ __device__ __forceinline__ uint32_t rows_with_edges(const uint32_t *__restrict__
     return bits;
 }
 
+/* rows with edges per block of ROW_TILE rows; the block that finishes last
+ * turns the counts into their exclusive prefix, in place, and stores the total
+ * (ticket: zeroed before the launch) */
 __global__ void __launch_bounds__(ROW_BLOCK) k_rows_count(const uint32_t *__restrict__ off, uint32_t V,
-                                                          uint32_t *__restrict__ counts)
+                                                          uint32_t *counts, uint32_t *ticket, uint32_t *total)
 {
+    __shared__ bool s_last;
     uint32_t all;
     block_scan((uint32_t)__popc(rows_with_edges(off, V, blockIdx.x * ROW_TILE)), &all);
-    if (threadIdx.x == 0) counts[blockIdx.x] = all;
-}
-
-/* exclusive scan of the block counts, in place, by one block */
-__global__ void __launch_bounds__(ROW_BLOCK) k_rows_scan(uint32_t *counts, uint32_t n)
-{
+    if (threadIdx.x == 0)
+    {
+        counts[blockIdx.x] = all;
+        __threadfence();
+        s_last = atomicAdd(ticket, 1u) == gridDim.x - 1;
+    }
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    const uint32_t n = gridDim.x;
     uint32_t base = 0;
     for (uint32_t at = 0; at < n; at += ROW_TILE)
     {
@@ -206,10 +213,9 @@ __global__ void __launch_bounds__(ROW_BLOCK) k_rows_scan(uint32_t *counts, uint3
         for (uint32_t k = 0; k < ROW_PER; k++)
         {
             const uint32_t i = at + threadIdx.x * ROW_PER + k;
-            c[k] = i < n ? counts[i] : 0u;
+            c[k] = i < n ? __ldcg(counts + i) : 0u;
             sum += c[k];
         }
-        uint32_t all;
         uint32_t run = base + block_scan(sum, &all) - sum;
 #pragma unroll
         for (uint32_t k = 0; k < ROW_PER; k++)
@@ -220,13 +226,19 @@ __global__ void __launch_bounds__(ROW_BLOCK) k_rows_scan(uint32_t *counts, uint3
         }
         base += all;
     }
+    if (threadIdx.x == 0) *total = base;
 }
 
-/* rows[r] = the r-th row with edges; seg0 of the tiles that begin in it */
+/* tiles whose first edge lies in row r = [a, b) (r-th with edges) */
+__device__ __forceinline__ void row_tiles(uint32_t a, uint32_t b, uint32_t r, uint32_t tile, uint32_t *seg0)
+{
+    for (uint64_t t = ((uint64_t)a + tile - 1) / tile; t * tile < b; t++) seg0[t] = r | (t * tile > a ? 0x80000000u : 0u);
+}
+
+/* rows[r] = the r-th row with edges, then the pads; seg0 of every tile */
 __global__ void __launch_bounds__(ROW_BLOCK) k_rows_write(const uint32_t *__restrict__ off, uint32_t V,
-                                                          const uint32_t *__restrict__ base,
-                                                          uint32_t *__restrict__ rows, uint32_t *__restrict__ seg0,
-                                                          uint32_t tile)
+                                                          const uint32_t *__restrict__ base, uint32_t *__restrict__ rows,
+                                                          uint32_t *__restrict__ seg0, uint32_t tile)
 {
     const uint32_t first = blockIdx.x * ROW_TILE;
     uint32_t r0 = base[blockIdx.x];
@@ -244,12 +256,21 @@ __global__ void __launch_bounds__(ROW_BLOCK) k_rows_write(const uint32_t *__rest
         if (b > a)
         {
             rows[r] = v;
-            /* tiles whose first edge lies in [a, b) */
-            for (uint64_t t = ((uint64_t)a + tile - 1) / tile; t * tile < b; t++)
-                seg0[t] = r | (t * tile > a ? 0x80000000u : 0u);
+            row_tiles(a, b, r, tile, seg0);
         }
         r0 += all;
     }
+    const uint32_t total = rows[V + GG_ROW_PAD];
+    if (blockIdx.x == 0 && threadIdx.x < GG_ROW_PAD) rows[total + threadIdx.x] = V;
+}
+
+/* seg0 alone, for another tile size */
+__global__ void k_rows_seg0(const uint32_t *__restrict__ off, uint32_t V, const uint32_t *__restrict__ rows,
+                            uint32_t *__restrict__ seg0, uint32_t tile)
+{
+    const uint32_t n = rows[V + GG_ROW_PAD];
+    for (uint32_t r = blockIdx.x * blockDim.x + threadIdx.x; r < n; r += gridDim.x * blockDim.x)
+        row_tiles(off[rows[r]], off[rows[r] + 1], r, tile, seg0);
 }
 
 /* the last edge of every row in the encoded ids */
@@ -263,6 +284,33 @@ __global__ void k_rows_mark(const uint32_t *__restrict__ off, uint32_t V, uint32
 }
 
 } // namespace
+
+gg_status gg_rows_tiles(gg_graph *g, cudaStream_t s, uint32_t tile, uint32_t **seg0, uint32_t *ntiles,
+                        uint32_t *launches)
+{
+    const uint32_t V = g->V, E = g->E;
+    const uint32_t nt = (uint32_t)(((uint64_t)E + tile - 1) / tile);
+    GG_CHECK(gg_dev_alloc(g, (void **)seg0, (size_t)nt * 4));
+    *ntiles = nt;
+    if (g->rows_list)
+    {
+        k_rows_seg0<<<gg_sm_count() * 8, 256, 0, s>>>(g->in_off, V, g->rows_list, *seg0, tile);
+        GG_CUDA(cudaGetLastError());
+        *launches += 1;
+        return GG_OK;
+    }
+    const uint32_t nb = (uint32_t)(((uint64_t)V + ROW_TILE - 1) / ROW_TILE);
+    void *counts;
+    GG_CHECK(gg_work(g, 33, ((size_t)nb + 4) * 4, &counts));
+    uint32_t *ticket = (uint32_t *)counts + nb;
+    GG_CUDA(cudaMemsetAsync(ticket, 0, 4, s));
+    GG_CHECK(gg_dev_alloc(g, (void **)&g->rows_list, ((size_t)V + GG_ROW_PAD + 4) * 4));
+    k_rows_count<<<nb, ROW_BLOCK, 0, s>>>(g->in_off, V, (uint32_t *)counts, ticket, g->rows_list + V + GG_ROW_PAD);
+    k_rows_write<<<nb, ROW_BLOCK, 0, s>>>(g->in_off, V, (const uint32_t *)counts, g->rows_list, *seg0, tile);
+    GG_CUDA(cudaGetLastError());
+    *launches += 2;
+    return GG_OK;
+}
 
 /* edges per tile: the tiles are dealt round robin to 32 warps on every SM, so
  * a few tiles per warp leave the last round nearly empty (R-MAT-20, 3,450
@@ -283,20 +331,9 @@ gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap)
     if (cap < 1 || cap > GG_HOT_ENTRIES) return gg_fail(GG_ERR_INVALID, "hot table capacity out of range");
     if (!g->hot_seg0)
     {
-        const uint32_t nb = (uint32_t)(((uint64_t)V + ROW_TILE - 1) / ROW_TILE);
-        const uint32_t tile = hot_tile_for(E);
-        const uint32_t nt = (uint32_t)(((uint64_t)E + tile - 1) / tile);
-        void *counts;
-        GG_CHECK(gg_work(g, 33, (size_t)nb * 4, &counts));
-        if (!g->hot_rows) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_rows, ((size_t)V + GG_HOT_ROW_PAD) * 4));
-        g->hot_ntiles = nt;
-        g->hot_tile = tile;
-        GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_seg0, (size_t)nt * 4));
-        k_rows_count<<<nb, ROW_BLOCK, 0, s>>>(g->in_off, V, (uint32_t *)counts);
-        k_rows_scan<<<1, ROW_BLOCK, 0, s>>>((uint32_t *)counts, nb);
-        k_rows_write<<<nb, ROW_BLOCK, 0, s>>>(g->in_off, V, (const uint32_t *)counts, g->hot_rows, g->hot_seg0,
-                                             tile);
-        GG_CUDA(cudaGetLastError());
+        uint32_t launches = 0;
+        g->hot_tile = hot_tile_for(E);
+        GG_CHECK(gg_rows_tiles(g, s, g->hot_tile, &g->hot_seg0, &g->hot_ntiles, &launches));
     }
     if (g->hot_adj && g->hot_cap == cap) return GG_OK;
     const uint32_t H = V < cap ? V : cap;

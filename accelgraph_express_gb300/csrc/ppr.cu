@@ -10,21 +10,40 @@
  *     rank'[v][k]   = (1-d) c_k(v) / |S_k| + d * sum over in-edges (u,v) of contrib[u][k]
  *
  * Layout: contributions vertex-major, [V][KP] with KP = K rounded up to 16,
- * 32 or 64, stored in FP32 or BF16 and summed in FP32.  At KP = 64 BF16 one
- * vertex's contributions are one 128-byte line, so every edge of the CSC
- * gathers one full line.  A group of KP/4 lanes owns a merge-path tile and
- * walks it edge by edge, each lane summing four vectors from one 8-byte
- * (BF16) or 16-byte (FP32) load; several groups share a warp, and a batch of
- * edges' rows is in flight while the previous ones are summed.  Rows are
- * finished where they end: rank = teleport + d * sum (the teleport row comes
- * through a per-vertex seed index), contribution = rank * (1 / outdeg) with
- * the reciprocal computed once per vertex (within an ulp of the division:
- * the division, 4 per lane per row end, had made the row ends the bulk of
- * the work); FP32 ranks are only written by the last iteration.  A row
- * spanning tiles leaves its partial sum in per-tile slots (the tile where it began or that it crosses: `tail`;
- * the tile where it ends: `head`) and k_ppr_fixup adds them in tile order, so
- * every vector's result is deterministic and independent of the vectors
- * batched with it.
+ * 32 or 64, stored in FP32 or BF16 and summed in FP32, so an edge gathers one
+ * contiguous row of 32 to 256 bytes.
+ *
+ * The gather.  Little's law bounds it: at ~1 us under load an SM needs 50 KB
+ * and more of rows in flight, and a warp that holds rows in registers has room
+ * for a few (four to six were in flight per half warp, 25 KB per SM).  So rows
+ * land in shared memory: a warp owns a tile of edges, asks for the rows of a
+ * chunk of up to 32 edges with 16-byte asynchronous copies (cp.async.cg: L2
+ * only, so rows rewritten inside the persistent launch are read fresh), and
+ * sums a chunk while the next ones arrive; 8 KB of landing space per warp, 24
+ * warps per SM.  The half warps take alternate edges, each lane KP / 16
+ * columns, so one shared-memory read serves two edges and the additions are
+ * packed (add.f32x2): issue slots are what is left to bound the loop.  The two
+ * halves' sums are exchanged and added where the row ends, for every KP: the
+ * order of a vector's additions does not depend on the vectors batched with it.
+ *
+ * Rows are finished where they end: rank = teleport + d * sum (the teleport
+ * row comes through a per-vertex seed index), contribution = rank *
+ * (1 / outdeg) with the reciprocal computed once per vertex (within an ulp of
+ * the division); FP32 ranks are only written by the last iteration.  The rows
+ * with edges are listed once per mapping (hot.cu); a warp keeps the next 64
+ * rows' ends, seed indices and reciprocals in registers and turns the ends
+ * into one bit mask per chunk.  A row spanning tiles leaves its partial sum in
+ * per-tile slots (the tile where it began or that it crosses: `tail`; the tile
+ * where it ends: `head`) and the fix-up adds them in tile order, so every
+ * vector's result is deterministic.  The fix-up also writes the rows without
+ * in-edges.
+ *
+ * Landing rows must be 128-byte aligned in shared memory: 16 bytes off, the
+ * asynchronous copies ran at half the rate.
+ *
+ * Measured, 20 iterations, K = 64 BF16 / FP32 and K = 16 FP32, against rows held
+ * in registers: R-MAT-20 17.2 / 20.3 / 15.1 -> 7.3 / 8.6 / 6.0 ms; R-MAT-16
+ * 3.6 / 3.6 / 5.6 -> 1.6 / 1.8 / 1.2 ms.
  */
 #include <cuda_runtime.h>
 #include <cuda_bf16.h>
@@ -42,171 +61,114 @@ using namespace gg;
 
 constexpr uint32_t NO_SEED = 0xffffffffu;
 
-/* VPL stored values per lane, read in one access of 4, 8 or 16 bytes */
-template <class CT, int VPL> struct VecIO;
-template <int VPL> struct Bf16IO
-{
-    static constexpr int W = VPL / 2; /* 32-bit words per lane */
-    struct Raw
-    {
-        uint32_t w[W];
-    };
-    static __device__ __forceinline__ Raw load(const __nv_bfloat16 *p)
-    {
-        Raw r;
-        if constexpr (W == 4)
-            asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]) : "l"(p));
-        else if constexpr (W == 2)
-            asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(r.w[0]), "=r"(r.w[1]) : "l"(p));
-        else
-            asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(r.w[0]) : "l"(p));
-        return r;
-    }
-    /* through L2 only: contributions rewritten inside the persistent launch */
-    static __device__ __forceinline__ Raw load_cg(const __nv_bfloat16 *p)
-    {
-        Raw r;
-        if constexpr (W == 4)
-            asm volatile("ld.global.cg.v4.u32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(r.w[0]), "=r"(r.w[1]), "=r"(r.w[2]), "=r"(r.w[3]) : "l"(p));
-        else if constexpr (W == 2)
-            asm volatile("ld.global.cg.v2.u32 {%0, %1}, [%2];" : "=r"(r.w[0]), "=r"(r.w[1]) : "l"(p));
-        else
-            asm volatile("ld.global.cg.u32 %0, [%1];" : "=r"(r.w[0]) : "l"(p));
-        return r;
-    }
-    /* element 2i is the low half of word i (little-endian); BF16 -> FP32 is exact */
-    static __device__ __forceinline__ void add(float *acc, const Raw &r)
-    {
-#pragma unroll
-        for (int i = 0; i < W; i++)
-        {
-            acc[2 * i] += __uint_as_float(r.w[i] << 16);
-            acc[2 * i + 1] += __uint_as_float(r.w[i] & 0xffff0000u);
-        }
-    }
-    static __device__ __forceinline__ void store(__nv_bfloat16 *p, const float *c)
-    {
-        uint32_t w[W];
-#pragma unroll
-        for (int i = 0; i < W; i++)
-        {
-            const __nv_bfloat162 h = __floats2bfloat162_rn(c[2 * i], c[2 * i + 1]);
-            w[i] = *reinterpret_cast<const uint32_t *>(&h);
-        }
-        if constexpr (W == 4)
-            *reinterpret_cast<uint4 *>(p) = make_uint4(w[0], w[1], w[2], w[3]);
-        else if constexpr (W == 2)
-            *reinterpret_cast<uint2 *>(p) = make_uint2(w[0], w[1]);
-        else
-            *reinterpret_cast<uint32_t *>(p) = w[0];
-    }
-};
-template <int VPL> struct F32IO
-{
-    struct Raw
-    {
-        float v[VPL];
-    };
-    static __device__ __forceinline__ Raw load(const float *p)
-    {
-        Raw r;
-        if constexpr (VPL == 4)
-            asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]) : "l"(p));
-        else
-            asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(r.v[0]), "=f"(r.v[1]) : "l"(p));
-        return r;
-    }
-    static __device__ __forceinline__ Raw load_cg(const float *p)
-    {
-        Raw r;
-        if constexpr (VPL == 4)
-            asm volatile("ld.global.cg.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(r.v[0]), "=f"(r.v[1]), "=f"(r.v[2]), "=f"(r.v[3]) : "l"(p));
-        else
-            asm volatile("ld.global.cg.v2.f32 {%0, %1}, [%2];" : "=f"(r.v[0]), "=f"(r.v[1]) : "l"(p));
-        return r;
-    }
-    static __device__ __forceinline__ void add(float *acc, const Raw &r)
-    {
-#pragma unroll
-        for (int i = 0; i < VPL; i++) acc[i] += r.v[i];
-    }
-    static __device__ __forceinline__ void store(float *p, const float *c)
-    {
-        if constexpr (VPL == 4)
-            *reinterpret_cast<float4 *>(p) = make_float4(c[0], c[1], c[2], c[3]);
-        else
-            *reinterpret_cast<float2 *>(p) = make_float2(c[0], c[1]);
-    }
-};
-template <int V> struct VecIO<__nv_bfloat16, V> : Bf16IO<V>
-{
-    static constexpr int VPL = V;
-};
-template <int V> struct VecIO<float, V> : F32IO<V>
-{
-    static constexpr int VPL = V;
-};
+/* the gather kernels: two CTAs of ten warps per SM (96 registers a thread;
+ * 24 warps at 80 registers spilled in the persistent kernel's loop) */
+constexpr int PPR_THREADS = 320, PPR_CTAS = 2, PPR_WARPS = PPR_THREADS / 32;
 
-/* values per lane of the PPR gather and edges per batch (rows in flight
- * per lane group, at most one per lane of the group), by storage and row
- * width KP, as measured on R-MAT-22 (20 iterations, GTEPS, BF16 / FP32):
- *   KP = 64: 4 per lane (one 8- or 16-byte load), batches of 6 / 4:
- *            2,249 / 1,856 (2 per lane: 2,037 / 1,330; 8 BF16 per lane
- *            with batches of 4: 2,032, of 8: 1,510)
- *   KP = 32: BF16 2 per lane, batches of 8: 1,427 (4 per lane: 1,406);
- *            FP32 4 per lane, batches of 4: 1,281 (2 per lane: 1,253)
- *   KP = 16: 2 per lane, batches of 8: 908 / 782 (4 per lane: 712 / 671) */
-template <class CT, int KP> constexpr int ppr_vpl()
+/* a pair of FP32 sums, added in one instruction (each sum rounded as FADD) */
+struct F2
 {
-    return (KP == 16 || (sizeof(CT) == 2 && KP == 32)) ? 2 : 4;
+    float x, y;
+};
+__device__ __forceinline__ F2 add2(F2 a, F2 b)
+{
+    F2 r;
+    asm("{\n\t.reg .b64 ra, rb, rc;\n\t"
+        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+        "add.rn.f32x2 rc, ra, rb;\n\tmov.b64 {%0, %1}, rc;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
 }
-template <class CT, int KP> using PprIO = VecIO<CT, ppr_vpl<CT, KP>()>;
 
-/* VPL consecutive floats (aligned to 4 * min(VPL, 4) bytes) */
-template <int VPL>
+/* One row of KP stored values, seen by a half warp: lane l of 16 reads the
+ * columns from l * VPL on.  At a row's end the lane keeps OUT of them: the
+ * lower half the first OUT, the upper half the rest (nothing at KP = 16). */
+template <class CT, int KP>
+struct PprRow
+{
+    static constexpr uint32_t BYTES = KP * sizeof(CT);
+    static constexpr uint32_t VPL = KP / 16;
+    static constexpr uint32_t OUT = VPL == 1 ? 1 : VPL / 2;
+    static constexpr uint32_t CHUNK = 4096 / BYTES < 32 ? 4096 / BYTES : 32; /* edges per chunk */
+    static constexpr uint32_t STAGE = CHUNK * BYTES;
+    static constexpr uint32_t DEPTH = 8192 / STAGE < 4 ? 8192 / STAGE : 4;   /* chunks in flight */
+    static constexpr uint32_t RING = DEPTH * STAGE;               /* landing bytes per warp */
+    static constexpr uint32_t LPR = BYTES / 16;                   /* lanes that copy one row */
+    static constexpr uint32_t RPI = 32 / LPR;                     /* rows per copy instruction */
+    static constexpr uint32_t F2S = (VPL + 1) / 2;
+
+    /* first column this lane keeps at a row's end, and whether it keeps any */
+    static __device__ __forceinline__ uint32_t out_col(uint32_t lane)
+    {
+        return (lane & 15) * VPL + (VPL > 1 ? (lane >> 4) * OUT : 0);
+    }
+    static __device__ __forceinline__ bool keeps(uint32_t lane) { return VPL > 1 || lane < 16; }
+
+    /* this lane's columns of the row landed at shared address `at` (the
+     * lane's own offset included); BF16 -> FP32 is exact, the low half is the
+     * lower column */
+    static __device__ __forceinline__ void read(uint32_t at, F2 *v)
+    {
+        if constexpr (sizeof(CT) == 4 && VPL == 4)
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v[0].x), "=f"(v[0].y), "=f"(v[1].x), "=f"(v[1].y) : "r"(at) : "memory");
+        else if constexpr (sizeof(CT) == 4 && VPL == 2)
+            asm volatile("ld.shared.v2.f32 {%0, %1}, [%2];" : "=f"(v[0].x), "=f"(v[0].y) : "r"(at) : "memory");
+        else if constexpr (sizeof(CT) == 4)
+        {
+            asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v[0].x) : "r"(at) : "memory");
+            v[0].y = 0.0f;
+        }
+        else if constexpr (VPL == 4)
+        {
+            uint32_t a, b;
+            asm volatile("ld.shared.v2.u32 {%0, %1}, [%2];" : "=r"(a), "=r"(b) : "r"(at) : "memory");
+            v[0] = F2{__uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u)};
+            v[1] = F2{__uint_as_float(b << 16), __uint_as_float(b & 0xffff0000u)};
+        }
+        else if constexpr (VPL == 2)
+        {
+            uint32_t a;
+            asm volatile("ld.shared.u32 %0, [%1];" : "=r"(a) : "r"(at) : "memory");
+            v[0] = F2{__uint_as_float(a << 16), __uint_as_float(a & 0xffff0000u)};
+        }
+        else
+        {
+            uint16_t a;
+            asm volatile("ld.shared.u16 %0, [%1];" : "=h"(a) : "r"(at) : "memory");
+            v[0] = F2{__uint_as_float((uint32_t)a << 16), 0.0f};
+        }
+    }
+    static __device__ __forceinline__ void store(CT *p, const float *c)
+    {
+        if constexpr (sizeof(CT) == 4 && OUT == 2)
+            *reinterpret_cast<float2 *>(p) = make_float2(c[0], c[1]);
+        else if constexpr (OUT == 2)
+            *reinterpret_cast<__nv_bfloat162 *>(p) = __floats2bfloat162_rn(c[0], c[1]);
+        else
+            *p = from_f32<CT>(c[0]);
+    }
+};
+
+template <uint32_t N>
 __device__ __forceinline__ void load_f32(const float *p, float *v)
 {
-    if constexpr (VPL % 4 == 0)
+    if constexpr (N == 2)
     {
-#pragma unroll
-        for (int i = 0; i < VPL; i += 4)
-        {
-            const float4 t = *reinterpret_cast<const float4 *>(p + i);
-            v[i] = t.x;
-            v[i + 1] = t.y;
-            v[i + 2] = t.z;
-            v[i + 3] = t.w;
-        }
+        const float2 t = *reinterpret_cast<const float2 *>(p);
+        v[0] = t.x;
+        v[1] = t.y;
     }
     else
-    {
-#pragma unroll
-        for (int i = 0; i < VPL; i += 2)
-        {
-            const float2 t = *reinterpret_cast<const float2 *>(p + i);
-            v[i] = t.x;
-            v[i + 1] = t.y;
-        }
-    }
+        v[0] = *p;
 }
-template <int VPL>
+template <uint32_t N>
 __device__ __forceinline__ void store_f32(float *p, const float *v)
 {
-    if constexpr (VPL % 4 == 0)
-    {
-#pragma unroll
-        for (int i = 0; i < VPL; i += 4)
-            *reinterpret_cast<float4 *>(p + i) = make_float4(v[i], v[i + 1], v[i + 2], v[i + 3]);
-    }
+    if constexpr (N == 2)
+        *reinterpret_cast<float2 *>(p) = make_float2(v[0], v[1]);
     else
-    {
-#pragma unroll
-        for (int i = 0; i < VPL; i += 2) *reinterpret_cast<float2 *>(p + i) = make_float2(v[i], v[i + 1]);
-    }
+        *p = v[0];
 }
 
 template <class CT>
@@ -214,9 +176,10 @@ struct PprArgs
 {
     const uint32_t *off, *adj, *seed_idx;
     const float *inv_deg; /* 1 / out-degree, 0 for out-degree 0 */
-    const uint2 *coord;
+    const uint32_t *rows; /* the rows with edges, padded with V */
+    const uint32_t *seg0; /* per tile: its first row end; bit 31: the row began earlier */
     uint32_t ntiles, V, E;
-    uint32_t tile_log2; /* merge items per tile, a power of two (512 by default, the tuned size otherwise) */
+    uint32_t tile; /* edges per tile, a power of two from 256 (512 by default, the tuned size otherwise) */
     const CT *cin;
     CT *cout;
     float *rank;       /* [V][rs]: ranks of the vectors in rank_mask are written here */
@@ -241,215 +204,406 @@ struct PprIter
 };
 
 /* the stores of a row end in an iteration where some vectors write their
- * ranks or retire (rare: kept out of line so the unrolled edge loop, which
- * inlines the row end at every edge of a batch, stays small; inlined, it
- * cost the K = 64 gather 20% on R-MAT-22) */
+ * ranks or retire (rare: the loops have an instance of their own for it) */
 template <int KP, class CT>
-__device__ __noinline__ void ppr_store_masked(CT *cout, float *rank, unsigned long long rank_mask,
+__device__ __forceinline__ void ppr_store_masked(CT *cout, float *rank, unsigned long long rank_mask,
                                               unsigned long long zero_mask, size_t o, const float *r, float *c,
-                                              uint32_t gl)
+                                              uint32_t col)
 {
-    constexpr int VPL = PprIO<CT, KP>::VPL;
-    const uint32_t zero = (uint32_t)(zero_mask >> (VPL * gl)) & ((1u << VPL) - 1u);
-    const uint32_t want = (uint32_t)(rank_mask >> (VPL * gl)) & ((1u << VPL) - 1u);
+    constexpr uint32_t VPL = PprRow<CT, KP>::OUT;
+    const uint32_t zero = (uint32_t)(zero_mask >> col) & ((1u << VPL) - 1u);
+    const uint32_t want = (uint32_t)(rank_mask >> col) & ((1u << VPL) - 1u);
 #pragma unroll
-    for (int k = 0; k < VPL; k++)
+    for (uint32_t k = 0; k < VPL; k++)
         if (zero >> k & 1u) c[k] = 0.0f;
-    PprIO<CT, KP>::store(cout + o, c);
-    if (want == (1u << VPL) - 1u)
-        store_f32<VPL>(rank + o, r);
-    else
+    PprRow<CT, KP>::store(cout + o, c);
 #pragma unroll
-        for (int k = 0; k < VPL; k++)
-            if (want >> k & 1u) rank[o + k] = r[k];
+    for (uint32_t k = 0; k < VPL; k++)
+        if (want >> k & 1u) rank[o + k] = r[k];
 }
 
-/* rank and contribution of row r from its sums (VPL vectors of this lane):
- * contribution = rank * (1 / out-degree), the reciprocal computed once per
- * vertex (within an ulp of rank / out-degree; 0 without out-edges).
- * RS: values per vertex row of cin / cout / rank / tele -- KP, or 64 when
- * only the first KP of wider rows are run (the server's continuous batch) */
-template <int KP, int RS, class CT>
+/* rank and contribution of row r from its sums (this lane's columns, from
+ * `col`; every lane of the warp calls it, at KP = 16 the upper half stores
+ * nothing): contribution = rank * (1 / out-degree).  RS: values per vertex
+ * row of cin / cout / rank / tele -- KP, or 64 when only the first KP of
+ * wider rows are run (the server's continuous batch).  MASKED: some vectors
+ * write their ranks or retire in this iteration */
+template <int KP, int RS, bool MASKED, class CT>
 __device__ __forceinline__ void ppr_finish(const PprArgs<CT> &a, const PprIter<CT> &it, uint32_t r, const float *s,
-                                           uint32_t si, float inv, uint32_t gl)
+                                           uint32_t si, float inv, uint32_t col, bool mine)
 {
-    constexpr int VPL = PprIO<CT, KP>::VPL;
+    constexpr uint32_t VPL = PprRow<CT, KP>::OUT;
     float rr[VPL], c[VPL];
 #pragma unroll
-    for (int k = 0; k < VPL; k++) rr[k] = __fmul_rn(a.damp, s[k]);
+    for (uint32_t k = 0; k < VPL; k++) rr[k] = __fmul_rn(a.damp, s[k]);
     if (si != NO_SEED)
     {
         float t[VPL];
-        load_f32<VPL>(a.tele + (size_t)si * RS + VPL * gl, t);
+        load_f32<VPL>(a.tele + (size_t)si * RS + col, t);
 #pragma unroll
-        for (int k = 0; k < VPL; k++) rr[k] = __fadd_rn(t[k], rr[k]);
+        for (uint32_t k = 0; k < VPL; k++) rr[k] = __fadd_rn(t[k], rr[k]);
     }
 #pragma unroll
-    for (int k = 0; k < VPL; k++) c[k] = __fmul_rn(rr[k], inv);
-    const size_t o = (size_t)r * RS + VPL * gl;
-    if ((it.rank_mask | a.zero_mask) == 0ull)
-        PprIO<CT, KP>::store(it.cout + o, c);
-    else
-        ppr_store_masked<KP, CT>(it.cout, a.rank, it.rank_mask, a.zero_mask, o, rr, c, gl);
-}
-
-template <int KP, int VPL>
-__device__ __forceinline__ void ppr_slot(float *slots, uint32_t tile, const float *s, uint32_t gl)
-{
-    store_f32<VPL>(slots + (size_t)tile * KP + VPL * gl, s);
-}
-
-/* one group of KP/VPL lanes per tile, each lane VPL vectors with one
- * 16-byte access per edge; U edges' rows in flight per batch (one id per
- * lane); COHERENT: contributions read through L2 only (they are rewritten
- * inside the launch by the persistent kernel; the read-only path may keep
- * stale lines from an earlier iteration) */
-template <int KP, int RS, class CT, int U, bool COHERENT>
-__device__ __forceinline__ void ppr_gather_tiles(const PprArgs<CT> &a, const PprIter<CT> &it)
-{
-    typedef PprIO<CT, KP> IO;
-    constexpr uint32_t VPL = IO::VPL;
-    constexpr uint32_t LPE = KP / VPL;
-    static_assert(U <= (int)LPE, "one id load per batch");
-    static_assert(LPE >= 1 && LPE <= 32 && (32 % LPE) == 0, "lane groups tile the warp");
-    const uint32_t lane = threadIdx.x & 31, gl = lane % LPE;
-    const unsigned gmask = LPE == 32 ? 0xffffffffu : (((1u << LPE) - 1u) << (lane - gl));
-    const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) / LPE;
-    const uint32_t ngroups = (gridDim.x * blockDim.x) / LPE;
-    for (uint32_t tile = gid; tile < a.ntiles; tile += ngroups)
+    for (uint32_t k = 0; k < VPL; k++) c[k] = __fmul_rn(rr[k], inv);
+    const size_t o = (size_t)r * RS + col;
+    if constexpr (MASKED)
     {
-        const uint2 c0 = a.coord[tile], c1 = a.coord[tile + 1];
-        const uint32_t i0 = c0.x, j0 = c0.y, i1 = c1.x, j1 = c1.y;
-        /* rows rb .. rb+LPE-1, one per lane: end offset, seed index, 1 / out-degree */
-        uint32_t rb = i0, w_end = 0, w_seed = NO_SEED;
-        float w_inv = 0.0f;
-        auto fetch = [&](uint32_t base) {
-            rb = base;
-            const uint32_t row = base + gl;
-            w_end = a.E;
-            w_seed = NO_SEED;
-            w_inv = 0.0f;
-            if (row < a.V)
-            {
-                w_end = a.off[row + 1];
-                w_seed = a.seed_idx[row];
-                w_inv = a.inv_deg[row];
-            }
-        };
-        fetch(i0);
-        /* row i0 began in an earlier tile when its first edge precedes j0 */
-        const uint32_t start0 = i0 < a.V ? a.off[i0] : a.E;
-        uint32_t r = i0;
-        uint32_t re = __shfl_sync(gmask, w_end, 0, LPE);
-        float acc[VPL];
-#pragma unroll
-        for (uint32_t k = 0; k < VPL; k++) acc[k] = 0.0f;
-        /* finish row r (it ends in this tile) and move to r+1 */
-        auto next_row = [&]() {
-            const uint32_t k = r - rb;
-            const uint32_t si = __shfl_sync(gmask, w_seed, k, LPE);
-            const float inv = __shfl_sync(gmask, w_inv, k, LPE);
-            if (r == i0 && start0 < j0)
-                ppr_slot<KP, VPL>(a.head, tile, acc, gl);
-            else
-                ppr_finish<KP, RS, CT>(a, it, r, acc, si, inv, gl);
-#pragma unroll
-            for (uint32_t q = 0; q < VPL; q++) acc[q] = 0.0f;
-            r++;
-            if (r - rb >= LPE) fetch(r);
-            re = __shfl_sync(gmask, w_end, r - rb, LPE);
-        };
-        /* the ids of a batch are loaded while the previous batch's rows are
-         * in flight, so a batch waits for one memory latency, not two */
-        uint32_t myid = 0;
-        if (j0 < j1 && gl < min((uint32_t)U, j1 - j0)) myid = ldg_stream(a.adj + j0 + gl);
-        for (uint32_t e = j0; e < j1; e += U)
+        if (mine) ppr_store_masked<KP, CT>(it.cout, a.rank, it.rank_mask, a.zero_mask, o, rr, c, col);
+    }
+    else if (mine)
+        PprRow<CT, KP>::store(it.cout + o, c);
+}
+
+/* the next rows with edges, one per lane: id, end offset, seed index, 1 / out-degree */
+struct PprWindow
+{
+    uint32_t row, end, seed;
+    float inv;
+};
+template <class CT>
+__device__ __forceinline__ PprWindow ppr_window(const PprArgs<CT> &a, uint32_t row)
+{
+    PprWindow w{row, 0xffffffffu, NO_SEED, 0.0f};
+    if (row < a.V)
+    {
+        w.end = a.off[row + 1];
+        w.seed = a.seed_idx[row];
+        w.inv = a.inv_deg[row];
+    }
+    return w;
+}
+
+/* `next`: hands out the tiles after each warp's first (zero on entry) -- a
+ * tile of one-edge rows takes several times as long as one of a hub's edges,
+ * and dealt round robin the slowest warp held the others up by a third */
+template <int KP, int RS, bool MASKED, class CT>
+__device__ __forceinline__ void ppr_gather_tiles(const PprArgs<CT> &a, const PprIter<CT> &it, uint32_t ring,
+                                                 uint32_t *next)
+{
+    typedef PprRow<CT, KP> R;
+    constexpr uint32_t CH = R::CHUNK, D = R::DEPTH, OUT = R::OUT, F2S = R::F2S;
+    const uint32_t lane = threadIdx.x & 31, half = lane >> 4;
+    const uint32_t col = R::out_col(lane);
+    const bool mine = R::keeps(lane);
+    const uint32_t nw = gridDim.x * (blockDim.x >> 5);
+    uint32_t tile = (threadIdx.x >> 5) * gridDim.x + blockIdx.x;
+    if (tile >= a.ntiles) return;
+    /* positions count chunks: 32 bits hold them for any E */
+    const uint32_t per = a.tile / CH, pmask = per - 1u;
+    const uint32_t nchunks = (a.E - 1u) / CH + 1u;
+    /* the chunk after c: in the same tile, or the first of the next one, which
+     * lane 0 took from the counter when the current one began */
+    uint32_t taken = 0, ntile = 0;
+    auto take = [&]() {
+        if (lane == 0) taken = nw + atomicAdd(next, 1u);
+    };
+    auto after = [&](uint32_t c) -> uint32_t {
+        const uint32_t n = c + 1u;
+        if (n & pmask) return n;
+        ntile = __shfl_sync(0xffffffffu, taken, 0);
+        return ntile * per;
+    };
+    take();
+    auto ids_at = [&](uint32_t c) -> uint32_t {
+        const uint32_t i = c * CH + lane;
+        return (lane < CH && c < nchunks && i < a.E) ? ldg_stream(a.adj + i) : 0u;
+    };
+    /* ask for the rows of chunk c into landing slot `slot`; rows past E land
+     * as zeros */
+    const uint32_t sub = lane / R::LPR;
+    const unsigned char *src0 = reinterpret_cast<const unsigned char *>(it.cin) + (lane % R::LPR) * 16;
+    auto ask = [&](uint32_t c, uint32_t ids, uint32_t slot) {
+        const uint32_t dst = ring + slot * R::STAGE + lane * 16;
+        if (c + 1u < nchunks)
         {
-            const uint32_t nb = min((uint32_t)U, j1 - e);
-            typename IO::Raw v[U];
 #pragma unroll
-            for (int i = 0; i < U; i++)
+            for (uint32_t i = 0; i < CH / R::RPI; i++)
             {
-                const uint32_t u = __shfl_sync(gmask, myid, i, LPE);
-                if ((uint32_t)i < nb)
-                    v[i] = COHERENT ? IO::load_cg(it.cin + (size_t)u * RS + VPL * gl)
-                                    : IO::load(it.cin + (size_t)u * RS + VPL * gl);
+                const uint32_t u = __shfl_sync(0xffffffffu, ids, i * R::RPI + sub);
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + i * 512u),
+                             "l"(src0 + (uint64_t)u * (uint32_t)(RS * sizeof(CT))) : "memory");
             }
-            const uint32_t en = e + U;
-            myid = 0;
-            if (en < j1 && gl < min((uint32_t)U, j1 - en)) myid = ldg_stream(a.adj + en + gl);
-#pragma unroll
-            for (int i = 0; i < U; i++)
+        }
+        else if (c < nchunks)
+        {
+            const uint32_t n = a.E - c * CH;
+#pragma unroll 1
+            for (uint32_t i = 0; i < CH / R::RPI; i++)
             {
-                if ((uint32_t)i < nb)
+                const uint32_t r = i * R::RPI + sub, u = __shfl_sync(0xffffffffu, ids, r);
+                if (r < n)
+                    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst + i * 512u),
+                                 "l"(src0 + (uint64_t)u * (uint32_t)(RS * sizeof(CT))) : "memory");
+                else
+                    asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};\n" ::"r"(dst + i * 512u), "r"(0u) : "memory");
+            }
+        }
+        cp_async_commit();
+    };
+
+    uint32_t c = tile * per;
+    uint32_t ahead = c; /* the chunk whose rows are asked for next, its ids in idn */
+    uint32_t idn = ids_at(ahead);
+#pragma unroll
+    for (uint32_t d = 0; d < D; d++)
+    {
+        const uint32_t n = after(ahead), ids = idn;
+        idn = ids_at(n);
+        ask(ahead, ids, d);
+        ahead = n;
+    }
+    uint32_t s0 = a.seg0[tile];
+    uint32_t seg = s0 & 0x7fffffffu, wb = seg;
+    bool open = s0 >> 31;
+    PprWindow cur = ppr_window(a, a.rows[wb + lane]), nxt = ppr_window(a, a.rows[wb + 32 + lane]);
+    uint32_t row2 = a.rows[wb + 64 + lane];
+    uint32_t seeded = __ballot_sync(0xffffffffu, cur.seed != NO_SEED);
+    F2 acc[F2S];
+#pragma unroll
+    for (uint32_t k = 0; k < F2S; k++) acc[k] = F2{0.0f, 0.0f};
+
+    /* the row's sum in the columns this lane keeps */
+    auto total = [&](float *t) {
+        if constexpr (R::VPL == 4)
+        {
+            const F2 give = half ? acc[0] : acc[1], keep = half ? acc[1] : acc[0];
+            t[0] = __fadd_rn(keep.x, __shfl_xor_sync(0xffffffffu, give.x, 16));
+            t[1] = __fadd_rn(keep.y, __shfl_xor_sync(0xffffffffu, give.y, 16));
+        }
+        else if constexpr (R::VPL == 2)
+        {
+            const float give = half ? acc[0].x : acc[0].y, keep = half ? acc[0].y : acc[0].x;
+            t[0] = __fadd_rn(keep, __shfl_xor_sync(0xffffffffu, give, 16));
+        }
+        else
+            t[0] = __fadd_rn(acc[0].x, __shfl_xor_sync(0xffffffffu, acc[0].x, 16));
+    };
+    auto finish = [&]() {
+        float t[OUT];
+        total(t);
+        const uint32_t k = seg - wb;
+        if (open)
+        {
+            if (mine) store_f32<OUT>(a.head + (size_t)tile * KP + col, t);
+            open = false;
+        }
+        else
+        {
+            uint32_t si = NO_SEED;
+            if (seeded >> k & 1u) si = __shfl_sync(0xffffffffu, cur.seed, k);
+            ppr_finish<KP, RS, MASKED, CT>(a, it, __shfl_sync(0xffffffffu, cur.row, k), t, si,
+                                           __shfl_sync(0xffffffffu, cur.inv, k), col, mine);
+        }
+        seg++;
+        if (k == 31u)
+        {
+            wb += 32;
+            cur = nxt;
+            seeded = __ballot_sync(0xffffffffu, cur.seed != NO_SEED);
+            nxt = ppr_window(a, row2);
+            row2 = a.rows[wb + 64 + lane];
+        }
+    };
+
+    const uint32_t read0 = ring + half * R::BYTES + (lane & 15) * (R::VPL * (uint32_t)sizeof(CT));
+    uint32_t slot = 0;
+    for (;;)
+    {
+        /* row ends of the chunk: bit i = its edge i is the last of its row */
+        const uint32_t b0 = cur.end - 1u - c * CH, b1 = nxt.end - 1u - c * CH;
+        const uint32_t m = __reduce_or_sync(0xffffffffu, (cur.row < a.V && b0 < CH ? 1u << b0 : 0u) |
+                                                             (nxt.row < a.V && b1 < CH ? 1u << b1 : 0u));
+        asm volatile("cp.async.wait_group %0;\n" ::"n"((int)D - 1) : "memory");
+        __syncwarp();
+        const uint32_t at = read0 + slot * R::STAGE;
+        constexpr uint32_t B = 8; /* edges per step: four pairs */
+#pragma unroll 1
+        for (uint32_t i0 = 0; i0 < CH; i0 += B)
+        {
+            F2 v[B / 2][F2S];
+#pragma unroll
+            for (uint32_t i = 0; i < B / 2; i++) R::read(at + (i0 + 2 * i) * R::BYTES, v[i]);
+            const uint32_t mm = (m >> i0) & 0xffu;
+            if (mm == 0u)
+            {
+#pragma unroll
+                for (uint32_t i = 0; i < B / 2; i++)
+#pragma unroll
+                    for (uint32_t k = 0; k < F2S; k++) acc[k] = add2(acc[k], v[i][k]);
+            }
+            else
+            {
+#pragma unroll
+                for (uint32_t i = 0; i < B / 2; i++)
                 {
-                    /* rows ending before this edge, zero-degree rows included */
-                    while (e + i >= re) next_row();
-                    IO::add(acc, v[i]);
+                    /* row ends after the even and the odd edge of the pair;
+                     * selects, not branches, keep the half warps together
+                     * (x + 0 is x: sums here are never -0) */
+                    const uint32_t two = (mm >> (2 * i)) & 3u;
+                    if (two & 1u)
+                    {
+#pragma unroll
+                        for (uint32_t k = 0; k < F2S; k++)
+                            acc[k] = add2(acc[k], half ? F2{0.0f, 0.0f} : v[i][k]);
+                        finish();
+#pragma unroll
+                        for (uint32_t k = 0; k < F2S; k++) acc[k] = half ? v[i][k] : F2{0.0f, 0.0f};
+                    }
+                    else
+#pragma unroll
+                        for (uint32_t k = 0; k < F2S; k++) acc[k] = add2(acc[k], v[i][k]);
+                    if (two & 2u)
+                    {
+                        finish();
+#pragma unroll
+                        for (uint32_t k = 0; k < F2S; k++) acc[k] = F2{0.0f, 0.0f};
+                    }
                 }
             }
         }
-        /* rows whose end items follow the tile's last edge */
-        while (r < i1) next_row();
-        /* row i1 continues in the next tile: leave what it gathered here */
-        if (i1 < a.V && j1 > j0)
+        __syncwarp(); /* every lane has read the slot that is asked for again */
         {
-            const uint32_t o = a.off[i1];
-            if (o < j1) ppr_slot<KP, VPL>(a.tail, tile, acc, gl);
+            const uint32_t n = after(ahead), ids = idn;
+            idn = ids_at(n);
+            ask(ahead, ids, slot);
+            ahead = n;
         }
+        slot = slot + 1 == D ? 0 : slot + 1;
+        if (((c + 1u) & pmask) == 0u || c + 1u >= nchunks)
+        {
+            /* a row open at the tile's end leaves what the tile had of it
+             * (edge E - 1 ends its row) */
+            if (c + 1u < nchunks && !(m >> (CH - 1) & 1u))
+            {
+                float t[OUT];
+                total(t);
+                if (mine) store_f32<OUT>(a.tail + (size_t)tile * KP + col, t);
+#pragma unroll
+                for (uint32_t k = 0; k < F2S; k++) acc[k] = F2{0.0f, 0.0f};
+            }
+            if (c + 1u >= nchunks) break; /* the last tile may be short of a full one */
+            tile = ntile; /* set when the chunks asked for reached it */
+            if (tile >= a.ntiles) break;
+            take();
+            s0 = a.seg0[tile];
+            seg = wb = s0 & 0x7fffffffu;
+            open = s0 >> 31;
+            cur = ppr_window(a, a.rows[wb + lane]);
+            nxt = ppr_window(a, a.rows[wb + 32 + lane]);
+            row2 = a.rows[wb + 64 + lane];
+            seeded = __ballot_sync(0xffffffffu, cur.seed != NO_SEED);
+            c = tile * per;
+        }
+        else
+            c++;
     }
+    cp_async_wait_all();
 }
 
-template <int KP, int RS, class CT, int U>
-__global__ void __launch_bounds__(256) k_ppr_pull(PprArgs<CT> a)
+template <int KP, int RS, bool MASKED, class CT>
+__global__ void __launch_bounds__(PPR_THREADS, PPR_CTAS) k_ppr_pull(PprArgs<CT> a, uint32_t *next)
 {
-    ppr_gather_tiles<KP, RS, CT, U, false>(a, PprIter<CT>{a.cin, a.cout, a.rank_mask});
+    extern __shared__ __align__(1024) unsigned char gg_dyn[];
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(gg_dyn) + (threadIdx.x >> 5) * PprRow<CT, KP>::RING;
+    ppr_gather_tiles<KP, RS, MASKED, CT>(a, PprIter<CT>{a.cin, a.cout, a.rank_mask}, ring, next);
 }
 
 /* finish the rows spanning tiles: the row that begins in tile t and is
- * still open at t's end (row coord[t+1].x) sums tail[t], the tails of the
- * tiles it crosses and the head of the tile where it ends, in tile order */
-template <int KP, int RS, class CT>
-__device__ __forceinline__ void ppr_fixup_tiles(const PprArgs<CT> &a, const PprIter<CT> &it)
+ * still open at t's end sums tail[t], the tails of the tiles it crosses and
+ * the head of the tile where it ends, in tile order; and, with `empty`, the
+ * rows without in-edges (their sum is zero).  One warp per row, one row at a
+ * time: four at once, or a function of its own, made the persistent kernel's
+ * gather spill (R-MAT-20, K = 64 BF16, 7.3 -> 8.0 and 7.6 ms). */
+template <int KP, int RS, bool MASKED, class CT>
+__device__ __forceinline__ void ppr_fixup_tiles(const PprArgs<CT> &a, const PprIter<CT> &it, bool empty)
 {
-    constexpr uint32_t VPL = PprIO<CT, KP>::VPL;
-    constexpr uint32_t LPE = KP / VPL, B = 32 / VPL; /* tails in flight per lane: 32 floats */
-    const uint32_t lane = threadIdx.x & 31, gl = lane % LPE;
-    const uint32_t gid = (blockIdx.x * blockDim.x + threadIdx.x) / LPE;
-    const uint32_t ngroups = (gridDim.x * blockDim.x) / LPE;
-    for (uint32_t t = gid; t < a.ntiles; t += ngroups)
+    typedef PprRow<CT, KP> R;
+    constexpr uint32_t VPL = R::OUT, B = 16 / VPL; /* tails in flight per lane */
+    const uint32_t lane = threadIdx.x & 31;
+    const uint32_t col = R::out_col(lane);
+    const bool mine = R::keeps(lane);
+    const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+    /* the tiles are spread over all warps, at most 32 per warp and round; a
+     * lane looks at one, with what its row's end needs, and the warp then
+     * takes the spanning rows found */
+    const uint32_t group = min(32u, (a.ntiles + nw - 1) / nw);
+    for (uint32_t t0 = warp * group; t0 + 1 < a.ntiles; t0 += nw * group)
     {
-        const uint32_t r = a.coord[t + 1].x;
-        if (r >= a.V) continue;
-        if ((((uint64_t)r + a.off[r]) >> a.tile_log2) != t) continue;
-        /* the tile of the row's end item */
-        const uint32_t t_last = (uint32_t)(((uint64_t)r + a.off[r + 1]) >> a.tile_log2);
-        float tot[VPL];
-        load_f32<VPL>(a.tail + (size_t)t * KP + VPL * gl, tot);
-        for (uint32_t m = t + 1; m < t_last; m += B)
+        const uint32_t t = t0 + lane;
+        uint32_t row = a.V, last = 0, seed = NO_SEED;
+        float inv = 0.0f;
+        if (lane < group && t + 1 < a.ntiles)
         {
-            float v[B][VPL];
-#pragma unroll
-            for (uint32_t i = 0; i < B; i++)
-                if (m + i < t_last) load_f32<VPL>(a.tail + (size_t)(m + i) * KP + VPL * gl, v[i]);
-#pragma unroll
-            for (uint32_t i = 0; i < B; i++)
-                if (m + i < t_last)
-#pragma unroll
-                    for (uint32_t k = 0; k < VPL; k++) tot[k] += v[i][k];
+            const uint32_t s = a.seg0[t + 1];
+            if (s >> 31)
+            {
+                const uint32_t r = a.rows[s & 0x7fffffffu];
+                if (a.off[r] / a.tile == t)
+                {
+                    row = r;
+                    last = (a.off[r + 1] - 1u) / a.tile;
+                    seed = a.seed_idx[r];
+                    inv = a.inv_deg[r];
+                }
+            }
         }
-        float h[VPL];
-        load_f32<VPL>(a.head + (size_t)t_last * KP + VPL * gl, h);
+        for (uint32_t todo = __ballot_sync(0xffffffffu, row < a.V); todo; todo &= todo - 1)
+        {
+            const int src = __ffs(todo) - 1;
+            const uint32_t r = __shfl_sync(0xffffffffu, row, src), tt = t0 + src;
+            const uint32_t t_last = __shfl_sync(0xffffffffu, last, src);
+            float tot[VPL], h[VPL];
+            load_f32<VPL>(a.tail + (size_t)tt * KP + col, tot);
+            load_f32<VPL>(a.head + (size_t)t_last * KP + col, h);
+            for (uint32_t m = tt + 1; m < t_last; m += B)
+            {
+                float v[B][VPL];
 #pragma unroll
-        for (uint32_t k = 0; k < VPL; k++) tot[k] += h[k];
-        ppr_finish<KP, RS, CT>(a, it, r, tot, a.seed_idx[r], a.inv_deg[r], gl);
+                for (uint32_t i = 0; i < B; i++)
+                    if (m + i < t_last) load_f32<VPL>(a.tail + (size_t)(m + i) * KP + col, v[i]);
+#pragma unroll
+                for (uint32_t i = 0; i < B; i++)
+                    if (m + i < t_last)
+#pragma unroll
+                        for (uint32_t k = 0; k < VPL; k++) tot[k] += v[i][k];
+            }
+#pragma unroll
+            for (uint32_t k = 0; k < VPL; k++) tot[k] += h[k];
+            ppr_finish<KP, RS, MASKED, CT>(a, it, r, tot, __shfl_sync(0xffffffffu, seed, src),
+                                           __shfl_sync(0xffffffffu, inv, src), col, mine);
+        }
+    }
+    if (!empty) return;
+    for (uint64_t v0 = (uint64_t)warp * 32; v0 < a.V; v0 += (uint64_t)nw * 32)
+    {
+        const uint32_t v = (uint32_t)v0 + lane;
+        bool none = false;
+        uint32_t si = NO_SEED;
+        float inv = 0.0f;
+        if (v0 + lane < a.V && a.off[v] == a.off[v + 1])
+        {
+            none = true;
+            si = a.seed_idx[v];
+            inv = a.inv_deg[v];
+        }
+        for (uint32_t todo = __ballot_sync(0xffffffffu, none); todo; todo &= todo - 1)
+        {
+            const int src = __ffs(todo) - 1;
+            float zero[VPL];
+#pragma unroll
+            for (uint32_t k = 0; k < VPL; k++) zero[k] = 0.0f;
+            ppr_finish<KP, RS, MASKED, CT>(a, it, (uint32_t)v0 + src, zero, __shfl_sync(0xffffffffu, si, src),
+                                   __shfl_sync(0xffffffffu, inv, src), col, mine);
+        }
     }
 }
 
-template <int KP, int RS, class CT>
-__global__ void __launch_bounds__(256) k_ppr_fixup(PprArgs<CT> a)
+/* `next` is the gather's tile counter, cleared for the next gather */
+template <int KP, int RS, bool MASKED, class CT>
+__global__ void __launch_bounds__(256) k_ppr_fixup(PprArgs<CT> a, uint32_t *next)
 {
-    ppr_fixup_tiles<KP, RS, CT>(a, PprIter<CT>{a.cin, a.cout, a.rank_mask});
+    if (blockIdx.x == 0 && threadIdx.x == 0) *next = 0u;
+    ppr_fixup_tiles<KP, RS, MASKED, CT>(a, PprIter<CT>{a.cin, a.cout, a.rank_mask}, true);
 }
 
 /* every iteration in one cooperative launch: gather, grid barrier, fix-up
@@ -463,45 +617,63 @@ struct PprLoop
     uint32_t iterations;
     char *ctl;
     unsigned int *err;
+    uint32_t *next; /* a zeroed tile counter per iteration */
     unsigned long long limit_ns;
 };
 
-/* resident CTAs of the persistent kernel: its gather, fix-up and barrier
- * take ~120 registers per thread without spills, so 2 CTAs of 256 per SM
- * (3, with spills, measured the same) */
-template <class CT> constexpr int ppr_persist_ctas() { return 2; }
-
-template <int KP, class CT> constexpr int ppr_batch()
+template <int KP, class CT>
+__global__ void __launch_bounds__(PPR_THREADS, PPR_CTAS) k_ppr_persist(const __grid_constant__ PprArgs<CT> a,
+                                                        const __grid_constant__ PprLoop<CT> L)
 {
-    constexpr int lpe = KP / ppr_vpl<CT, KP>();
-    constexpr int umax = ppr_vpl<CT, KP>() == 2 ? 8 : (sizeof(CT) == 2 ? 6 : 4);
-    return lpe < umax ? lpe : umax;
-}
-
-template <int KP, class CT, int U>
-__global__ void __launch_bounds__(256, ppr_persist_ctas<CT>()) k_ppr_persist(const __grid_constant__ PprArgs<CT> a,
-                                                                             const __grid_constant__ PprLoop<CT> L)
-{
+    extern __shared__ __align__(1024) unsigned char gg_dyn[];
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(gg_dyn) + (threadIdx.x >> 5) * PprRow<CT, KP>::RING;
     unsigned int gen = 0;
     for (uint32_t i = 0; i < L.iterations; i++)
     {
         const PprIter<CT> it{(i & 1) ? L.cb1 : L.cb0, (i & 1) ? L.cb0 : L.cb1, i + 1 == L.iterations ? ~0ull : 0ull};
-        ppr_gather_tiles<KP, KP, CT, U, true>(a, it);
+        const bool last = i + 1 == L.iterations; /* writes the ranks */
+        if (last)
+            ppr_gather_tiles<KP, KP, true, CT>(a, it, ring, L.next + i);
+        else
+            ppr_gather_tiles<KP, KP, false, CT>(a, it, ring, L.next + i);
         if (!grid_barrier(L.ctl, L.err, L.limit_ns, gen)) return;
-        ppr_fixup_tiles<KP, KP, CT>(a, it);
-        if (i + 1 < L.iterations && !grid_barrier(L.ctl, L.err, L.limit_ns, gen)) return;
+        /* a row without in-edges keeps its contribution: both buffers hold it
+         * after two iterations, and the last one writes the ranks */
+        if (last)
+            ppr_fixup_tiles<KP, KP, true, CT>(a, it, true);
+        else
+            ppr_fixup_tiles<KP, KP, false, CT>(a, it, i < 2);
+        if (!last && !grid_barrier(L.ctl, L.err, L.limit_ns, gen)) return;
     }
+}
+
+/* dynamic shared memory of the gather kernels: the warps' landing space */
+template <int KP, class CT> constexpr size_t ppr_smem() { return (size_t)PPR_WARPS * PprRow<CT, KP>::RING; }
+
+/* allow a kernel its dynamic shared memory (once per kernel) */
+gg_status ppr_allow(const void *kernel, size_t smem)
+{
+    GG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    return GG_OK;
 }
 
 /* contributions of the seed vertices at iteration 0 (the rest is zero), and
  * their seed indices; rows of rs values, of which vectors in `fresh` are
  * written (all of them for gg_ppr; the newly admitted slots for the
  * server, whose other columns hold running vectors) */
+/* with `inv`, also inv[v] = 1 / out-degree (correctly rounded), 0 without
+ * out-edges */
 template <class CT>
 __global__ void k_ppr_seed_init(const uint32_t *__restrict__ seed_vertex, uint32_t nseeds,
                                 const float *__restrict__ init, const uint32_t *__restrict__ outdeg, CT *cin,
-                                uint32_t *seed_idx, uint32_t rs, unsigned long long fresh)
+                                uint32_t *seed_idx, uint32_t rs, unsigned long long fresh, uint32_t V, float *inv)
 {
+    if (inv)
+        for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
+        {
+            const uint32_t d = outdeg[v];
+            inv[v] = d ? __frcp_rn(__uint2float_rn(d)) : 0.0f;
+        }
     const uint64_t n = (uint64_t)nseeds * (rs / 2);
     for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
     {
@@ -546,16 +718,50 @@ gg_status ppr_inv_deg(gg_graph *g, cudaStream_t s, const float **out)
     return GG_OK;
 }
 
-template <class K>
-int occupancy_grid(K kernel, int threads, size_t work_groups, int lanes_per_group)
+/* persistent grid of a kernel with one warp per work item */
+int occupancy_grid(const void *kernel, int threads, size_t smem, size_t warps)
 {
-    int bps = gg_occupancy((const void *)kernel, threads, 0);
+    int bps = gg_occupancy(kernel, threads, smem);
     if (bps < 1) bps = 1;
-    const size_t groups_per_block = (size_t)threads / lanes_per_group;
-    const size_t need = (work_groups + groups_per_block - 1) / groups_per_block;
-    const size_t cap = (size_t)gg_sm_count() * bps;
+    const size_t need = (warps + threads / 32 - 1) / (threads / 32), cap = (size_t)gg_sm_count() * bps;
     const size_t g = need < cap ? need : cap;
     return (int)(g < 1 ? 1 : g);
+}
+
+/* seg0 of the mapping for its PPR tile size */
+gg_status ppr_tiles(gg_graph *g, cudaStream_t s, uint32_t *launches)
+{
+    const uint32_t tile = gg_ppr_tile(g);
+    if (g->ppr_seg0 && g->ppr_tiles_items == tile) return GG_OK;
+    if (g->ppr_seg0) gg_dev_free(g, g->ppr_seg0, (size_t)g->ppr_ntiles * 4);
+    g->ppr_seg0 = nullptr;
+    GG_CHECK(gg_rows_tiles(g, s, tile, &g->ppr_seg0, &g->ppr_ntiles, launches));
+    g->ppr_tiles_items = tile;
+    return GG_OK;
+}
+
+/* one gather / fix-up as a launch of its own */
+template <int KP, int RS, class CT>
+gg_status launch_pull(const PprArgs<CT> &a, uint32_t *next, cudaStream_t s)
+{
+    if (!a.ntiles) return GG_OK;
+    constexpr size_t smem = ppr_smem<KP, CT>();
+    const bool masked = (a.rank_mask | a.zero_mask) != 0ull;
+    const void *fn = masked ? (const void *)k_ppr_pull<KP, RS, true, CT> : (const void *)k_ppr_pull<KP, RS, false, CT>;
+    GG_CHECK(ppr_allow(fn, smem));
+    void *args[] = {(void *)&a, &next};
+    GG_CUDA(cudaLaunchKernel(fn, dim3(occupancy_grid(fn, PPR_THREADS, smem, a.ntiles)), dim3(PPR_THREADS), args,
+                             smem, s));
+    return GG_OK;
+}
+template <int KP, int RS, class CT>
+gg_status launch_fixup(const PprArgs<CT> &a, uint32_t *next, cudaStream_t s)
+{
+    const bool masked = (a.rank_mask | a.zero_mask) != 0ull;
+    const void *fn = masked ? (const void *)k_ppr_fixup<KP, RS, true, CT> : (const void *)k_ppr_fixup<KP, RS, false, CT>;
+    void *args[] = {(void *)&a, &next};
+    GG_CUDA(cudaLaunchKernel(fn, dim3(occupancy_grid(fn, 256, 0, ((size_t)a.V + 31) / 32)), dim3(256), args, 0, s));
+    return GG_OK;
 }
 
 template <int KP, class CT>
@@ -563,63 +769,51 @@ gg_status run_ppr(gg_graph *g, const gg_ppr_params *p, uint32_t nseedv, const ui
                   const float *d_tele, uint32_t *d_seed_idx, float *d_rank, cudaStream_t s, gg_ppr_result &res,
                   std::vector<cudaEvent_t> &evs, void **ctl_out)
 {
-    constexpr int LPE = KP / PprIO<CT, KP>::VPL;
-    constexpr int U = ppr_batch<KP, CT>();
     const uint32_t V = g->V;
-    gg_tiles &t = g->ppr_tiles;
-    const uint32_t tile = g->ppr_tile;
-    if (t.coord && g->ppr_tiles_items != tile)
-    {
-        gg_dev_free(g, t.coord, ((size_t)t.ntiles + 1) * sizeof(uint2));
-        t.coord = nullptr;
-    }
-    if (!t.coord)
-    {
-        const uint64_t nt = ((uint64_t)V + g->E + tile - 1) / tile;
-        if (nt >= 0xffffffffull) return gg_fail(GG_ERR_INVALID, "graph too large for 32-bit tile ids");
-        t.ntiles = (uint32_t)(nt ? nt : 1);
-        GG_CHECK(gg_dev_alloc(g, (void **)&t.coord, ((size_t)t.ntiles + 1) * sizeof(uint2)));
-        GG_CHECK(gg_launch_tile_coords(g->in_off, V, g->E, t.ntiles, t.coord, s, tile));
-        g->ppr_tiles_items = tile;
-        res.launches++;
-    }
+    GG_CHECK(ppr_tiles(g, s, &res.launches));
+    const uint32_t ntiles = g->ppr_ntiles;
     void *c0, *c1, *slots;
     GG_CHECK(gg_work(g, 16, (size_t)V * KP * sizeof(CT), &c0));
     GG_CHECK(gg_work(g, 17, (size_t)V * KP * sizeof(CT), &c1));
-    GG_CHECK(gg_work(g, 18, (size_t)t.ntiles * KP * sizeof(float) * 2, &slots));
+    GG_CHECK(gg_work(g, 18, ((size_t)ntiles * KP * 2 + 4) * sizeof(float), &slots));
+    uint32_t *next = (uint32_t *)((float *)slots + (size_t)ntiles * KP * 2);
+    void *inv;
+    GG_CHECK(gg_work(g, 15, (size_t)V * 4 + 16, &inv));
     GG_CUDA(cudaMemsetAsync(c0, 0, (size_t)V * KP * sizeof(CT), s));
     GG_CUDA(cudaMemsetAsync(d_seed_idx, 0xff, (size_t)V * sizeof(uint32_t), s));
-    k_ppr_seed_init<CT><<<gg_sm_count() * 2, 256, 0, s>>>(d_seedv, nseedv, d_init, g->out_deg, (CT *)c0, d_seed_idx,
-                                                          KP, ~0ull);
+    k_ppr_seed_init<CT><<<gg_sm_count() * 4, 256, 0, s>>>(d_seedv, nseedv, d_init, g->out_deg, (CT *)c0, d_seed_idx,
+                                                          KP, ~0ull, V, (float *)inv);
     res.launches++;
 
     PprArgs<CT> a;
     a.off = g->in_off; a.adj = g->in_adj; a.seed_idx = d_seed_idx;
-    GG_CHECK(ppr_inv_deg(g, s, &a.inv_deg));
-    res.launches++;
-    a.coord = t.coord; a.ntiles = t.ntiles; a.V = V; a.E = g->E; a.tile_log2 = (uint32_t)__builtin_ctz(tile);
+    a.inv_deg = (const float *)inv;
+    a.rows = g->rows_list; a.seg0 = g->ppr_seg0; a.ntiles = ntiles; a.V = V; a.E = g->E; a.tile = g->ppr_tiles_items;
     a.rank = d_rank; a.rank_mask = 0; a.zero_mask = 0;
     a.tele = d_tele; a.damp = p->damp;
     a.head = (float *)slots;
-    a.tail = (float *)slots + (size_t)t.ntiles * KP;
+    a.tail = (float *)slots + (size_t)ntiles * KP;
+    constexpr size_t smem = ppr_smem<KP, CT>();
     CT *cb[2] = {(CT *)c0, (CT *)c1};
     if (!p->profile)
     {
         /* all iterations in one cooperative launch: every block resident */
-        const int per_sm = gg_occupancy((const void *)k_ppr_persist<KP, CT, U>, 256, 0);
+        const void *fn = (const void *)k_ppr_persist<KP, CT>;
+        GG_CHECK(ppr_allow(fn, smem));
+        const int per_sm = gg_occupancy(fn, PPR_THREADS, smem);
         if (per_sm < 1) return gg_fail(GG_ERR_CUDA, "k_ppr_persist cannot be resident");
-        const size_t groups_per_block = 256 / LPE;
-        const size_t need = ((size_t)t.ntiles + groups_per_block - 1) / groups_per_block;
-        const size_t cap = (size_t)gg_sm_count() * (size_t)per_sm;
-        const int grid = (int)(need < cap ? (need ? need : 1) : cap);
+        /* a warp per tile, or per 32 vertices (the rows without in-edges) */
+        const int grid = occupancy_grid(fn, PPR_THREADS, smem, std::max<size_t>(ntiles, ((size_t)V + 31) / 32));
         void *ctl;
-        GG_CHECK(gg_work(g, 30, GG_BAR_BYTES, &ctl));
-        GG_CUDA(cudaMemsetAsync(ctl, 0, GG_BAR_BYTES, s));
+        const size_t ctl_bytes = GG_BAR_BYTES + (size_t)p->iterations * 4;
+        GG_CHECK(gg_work(g, 30, ctl_bytes, &ctl));
+        GG_CUDA(cudaMemsetAsync(ctl, 0, ctl_bytes, s));
         PprLoop<CT> L;
         L.cb0 = cb[0]; L.cb1 = cb[1]; L.iterations = p->iterations;
         L.ctl = (char *)ctl; L.err = (unsigned int *)ctl; L.limit_ns = gg_barrier_limit_ns();
+        L.next = (uint32_t *)((char *)ctl + GG_BAR_BYTES);
         void *args[] = {&a, &L};
-        GG_CUDA(cudaLaunchCooperativeKernel((const void *)k_ppr_persist<KP, CT, U>, dim3(grid), dim3(256), args, 0, s));
+        GG_CUDA(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(PPR_THREADS), args, smem, s));
         res.launches++;
         res.gather_launches = p->iterations;
         res.persistent = 1;
@@ -627,8 +821,7 @@ gg_status run_ppr(gg_graph *g, const gg_ppr_params *p, uint32_t nseedv, const ui
         GG_CUDA(cudaGetLastError());
         return GG_OK;
     }
-    const int grid = occupancy_grid(k_ppr_pull<KP, KP, CT, U>, 256, t.ntiles, LPE);
-    const int fgrid = occupancy_grid(k_ppr_fixup<KP, KP, CT>, 256, t.ntiles, LPE);
+    GG_CUDA(cudaMemsetAsync(next, 0, 4, s));
     for (uint32_t it = 0; it < p->iterations; it++)
     {
         a.cin = cb[it & 1];
@@ -641,7 +834,7 @@ gg_status run_ppr(gg_graph *g, const gg_ppr_params *p, uint32_t nseedv, const ui
             GG_CUDA(cudaEventRecord(e, s));
             evs.push_back(e);
         }
-        k_ppr_pull<KP, KP, CT, U><<<grid, 256, 0, s>>>(a);
+        GG_CHECK((launch_pull<KP, KP, CT>(a, next, s)));
         if (p->profile)
         {
             cudaEvent_t e;
@@ -649,7 +842,7 @@ gg_status run_ppr(gg_graph *g, const gg_ppr_params *p, uint32_t nseedv, const ui
             GG_CUDA(cudaEventRecord(e, s));
             evs.push_back(e);
         }
-        k_ppr_fixup<KP, KP, CT><<<fgrid, 256, 0, s>>>(a);
+        GG_CHECK((launch_fixup<KP, KP, CT>(a, next, s)));
         res.launches += 2;
         res.gather_launches++;
     }
@@ -666,55 +859,50 @@ namespace {
 template <int KP, class CT>
 gg_status round_run(gg_graph *g, const gg_ppr_round_args &r, cudaStream_t s)
 {
-    constexpr int LPE = KP / PprIO<CT, KP>::VPL;
-    constexpr int U = ppr_batch<KP, CT>();
-    gg_tiles &t = g->ppr_tiles;
+    const uint32_t ntiles = g->ppr_ntiles;
     PprArgs<CT> a;
     a.off = g->in_off; a.adj = g->in_adj; a.seed_idx = r.seed_idx;
     void *inv;
     GG_CHECK(gg_work(g, 15, (size_t)g->V * 4 + 16, &inv)); /* filled by gg_ppr_round_prepare */
     a.inv_deg = (const float *)inv;
-    a.coord = t.coord; a.ntiles = t.ntiles; a.V = g->V; a.E = g->E;
-    a.tile_log2 = (uint32_t)__builtin_ctz(g->ppr_tiles_items);
+    a.rows = g->rows_list; a.seg0 = g->ppr_seg0; a.ntiles = ntiles; a.V = g->V; a.E = g->E;
+    a.tile = g->ppr_tiles_items;
     a.cin = (const CT *)r.cin; a.cout = (CT *)r.cout; a.rank = r.rank;
     a.rank_mask = r.rank_mask; a.zero_mask = r.zero_mask;
     a.tele = r.tele; a.damp = r.damp;
     a.head = r.slots;
-    a.tail = r.slots + (size_t)t.ntiles * KP;
-    const int grid = occupancy_grid(k_ppr_pull<KP, 64, CT, U>, 256, t.ntiles, LPE);
-    const int fgrid = occupancy_grid(k_ppr_fixup<KP, 64, CT>, 256, t.ntiles, LPE);
-    k_ppr_pull<KP, 64, CT, U><<<grid, 256, 0, s>>>(a);
-    k_ppr_fixup<KP, 64, CT><<<fgrid, 256, 0, s>>>(a);
+    a.tail = r.slots + (size_t)ntiles * KP;
+    uint32_t *next = (uint32_t *)(r.slots + (size_t)ntiles * 64 * 2); /* cleared by gg_ppr_round_prepare */
+    GG_CHECK((launch_pull<KP, 64, CT>(a, next, s)));
+    GG_CHECK((launch_fixup<KP, 64, CT>(a, next, s)));
     GG_CUDA(cudaGetLastError());
     return GG_OK;
 }
 
 } // namespace
 
+/* edges per tile: the tuned size, or by the graph's.  A tile runs on one warp,
+ * so a graph of few tiles per warp (3,040 resident) ends with the slowest:
+ * 256 below four 512-edge tiles per warp (R-MAT-16, K = 64
+ * BF16: 96 -> 78 us an iteration), 512 above (fewer rows
+ * span tiles). */
+uint32_t gg_ppr_tile(const gg_graph *g)
+{
+    if (g->ppr_tile) return g->ppr_tile;
+    return g->E < 4u * 512u * (uint32_t)(PPR_CTAS * PPR_WARPS) * (uint32_t)gg_sm_count() ? 256u : 512u;
+}
+
 gg_status gg_ppr_round_prepare(gg_graph *g, uint32_t rs, int bf16, void **cb0, void **cb1, float **slots,
                                cudaStream_t s)
 {
-    gg_tiles &t = g->ppr_tiles;
-    const uint32_t tile = g->ppr_tile;
     const uint32_t V = g->V;
-    if (t.coord && g->ppr_tiles_items != tile)
-    {
-        gg_dev_free(g, t.coord, ((size_t)t.ntiles + 1) * sizeof(uint2));
-        t.coord = nullptr;
-    }
-    if (!t.coord)
-    {
-        const uint64_t nt = ((uint64_t)V + g->E + tile - 1) / tile;
-        if (nt >= 0xffffffffull) return gg_fail(GG_ERR_INVALID, "graph too large for 32-bit tile ids");
-        t.ntiles = (uint32_t)(nt ? nt : 1);
-        GG_CHECK(gg_dev_alloc(g, (void **)&t.coord, ((size_t)t.ntiles + 1) * sizeof(uint2)));
-        GG_CHECK(gg_launch_tile_coords(g->in_off, V, g->E, t.ntiles, t.coord, s, tile));
-        g->ppr_tiles_items = tile;
-    }
+    uint32_t launches = 0;
+    GG_CHECK(ppr_tiles(g, s, &launches));
     const size_t cb = (size_t)V * rs * (bf16 ? 2 : 4);
     GG_CHECK(gg_work(g, 16, cb, cb0));
     GG_CHECK(gg_work(g, 17, cb, cb1));
-    GG_CHECK(gg_work(g, 18, (size_t)t.ntiles * rs * sizeof(float) * 2, (void **)slots));
+    GG_CHECK(gg_work(g, 18, ((size_t)g->ppr_ntiles * rs * 2 + 4) * sizeof(float), (void **)slots));
+    GG_CUDA(cudaMemsetAsync(*slots + (size_t)g->ppr_ntiles * rs * 2, 0, 4, s));
     GG_CUDA(cudaMemsetAsync(*cb0, 0, cb, s));
     GG_CUDA(cudaMemsetAsync(*cb1, 0, cb, s));
     const float *inv;
@@ -728,10 +916,10 @@ gg_status gg_ppr_round_seed(gg_graph *g, uint32_t rs, int bf16, void *cin, const
     if (!nseedv) return GG_OK;
     if (bf16)
         k_ppr_seed_init<__nv_bfloat16><<<gg_sm_count() * 2, 256, 0, s>>>(d_seedv, nseedv, d_init, g->out_deg,
-                                                                         (__nv_bfloat16 *)cin, d_seed_idx, rs, fresh);
+                                                                         (__nv_bfloat16 *)cin, d_seed_idx, rs, fresh, 0, nullptr);
     else
         k_ppr_seed_init<float><<<gg_sm_count() * 2, 256, 0, s>>>(d_seedv, nseedv, d_init, g->out_deg, (float *)cin,
-                                                                 d_seed_idx, rs, fresh);
+                                                                 d_seed_idx, rs, fresh, 0, nullptr);
     GG_CUDA(cudaGetLastError());
     return GG_OK;
 }

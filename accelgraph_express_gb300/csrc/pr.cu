@@ -981,7 +981,7 @@ gg_status run_pull(Run &R, IterRec *rec, float *rank, uint32_t iters, float base
         const bool pdl = !R.p->profile;
         if (hg)
         {
-            const HotArgs ha{g->hot_adj, g->hot_rows, g->hot_seg0, g->E, g->hot_ntiles, g->hot_tile};
+            const HotArgs ha{g->hot_adj, g->rows_list, g->hot_seg0, g->E, g->hot_ntiles, g->hot_tile};
             CT *tab = (CT *)hot_tab;
             const size_t smem = hot_smem_bytes<CT>(hw);
             const int fg = (int)((hot_cap<CT>() + 255) / 256);

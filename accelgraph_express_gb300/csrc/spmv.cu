@@ -287,7 +287,7 @@ gg_status spmv_fp(gg_graph *g, const gg_spmv_params *p, const float *x_dev, floa
             const int hg = use_hot ? spmv_hot_grid<T>(g->hot_ntiles, shape.hot_warps) : 0;
             if (hg)
                 k_spmv_pull_hot<T><<<hg, shape.hot_warps * 32, hot_smem_bytes<T>(shape.hot_warps), s>>>(
-                    HotArgs{g->hot_adj, g->hot_rows, g->hot_seg0, g->E, g->hot_ntiles, g->hot_tile}, xv, w, (const T *)hot_tab, y);
+                    HotArgs{g->hot_adj, g->rows_list, g->hot_seg0, g->E, g->hot_ntiles, g->hot_tile}, xv, w, (const T *)hot_tab, y);
             else
                 k_spmv_pull<T><<<gg_persistent_grid((const void *)k_spmv_pull<T>, t->ntiles, (int)shape.ctas),
                                  GG_TILE_NT, 0, s>>>(g->in_off, g->in_adj, t->coord, t->ntiles, V, y, SpmvGather<T>{w, xv});

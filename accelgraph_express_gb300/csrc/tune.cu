@@ -290,8 +290,11 @@ gg_status tune_ppr(gg_graph *g, uint32_t storage, uint32_t reps, cudaStream_t s,
     const uint32_t K = (uint32_t)seeds.size();
     const uint32_t keep = g->ppr_tile;
     float best = INFINITY;
-    uint32_t pick = 512, n = 0;
-    for (uint32_t tile : {512u, 256u, 1024u})
+    /* the size that an untuned mapping uses comes first */
+    g->ppr_tile = 0;
+    const uint32_t dflt = gg_ppr_tile(g);
+    uint32_t pick = dflt, n = 0;
+    for (uint32_t tile : {dflt, dflt == 512u ? 256u : 512u, 1024u})
     {
         g->ppr_tile = tile;
         float ms = INFINITY;
@@ -584,7 +587,7 @@ extern "C" gg_status gg_tune_get(const gg_graph *g, uint32_t family, uint32_t *p
     case GG_TUNE_SPMV:
         params[0] = g->spmv_shape.hot; params[1] = g->spmv_shape.ctas; params[2] = g->spmv_shape.hot_warps; break;
     case GG_TUNE_BFS: params[0] = g->bfs_heavy; break;
-    case GG_TUNE_PPR: params[0] = g->ppr_tile; break;
+    case GG_TUNE_PPR: params[0] = gg_ppr_tile(g); break;
     case GG_TUNE_BATCH:
         params[0] = g->graphs_cfg.ipt; params[1] = g->graphs_cfg.warps; params[2] = g->graphs_cfg.smem_vmax;
         params[3] = g->graphs_cfg.ctas; params[4] = g->graphs_cfg.strategy; break;
