@@ -258,12 +258,11 @@ __global__ void __launch_bounds__(GG_HOT_WARPS * 32, 1)
                   uint32_t it)
 {
     typedef typename Fmt<K>::CT CT;
-    extern __shared__ __align__(16) unsigned char gg_dyn[];
-    const uint32_t table = (uint32_t)__cvta_generic_to_shared(gg_dyn);
+    extern __shared__ __align__(1024) unsigned char gg_dyn[];
     const uint32_t warps = blockDim.x >> 5, w = threadIdx.x >> 5;
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(gg_dyn), table = ring + warps * HOT_RING;
     hot_pull_sums<CT, typename Fmt<K>::Tile, typename Fmt<K>::Acc, false>(
-        table + hot_table_bytes<CT>() + w * HOT_RING, table, hot_cap<CT>(), a, w * gridDim.x + blockIdx.x,
-        gridDim.x * warps, cin, (const CT *)nullptr, sums, [&] {
+        ring + w * HOT_RING, table, hot_cap<CT>(), a, w * gridDim.x + blockIdx.x, gridDim.x * warps, cin, (const CT *)nullptr, sums, [&] {
             pdl_wait();
             if (it > 0 && rec[it - 1].active == 0u) return false;
             hot_table_load(table, table_src, hot_table_bytes<CT>());

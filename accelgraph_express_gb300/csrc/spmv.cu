@@ -61,10 +61,10 @@ __global__ void __launch_bounds__(GG_HOT_WARPS * 32, 1)
     k_spmv_pull_hot(HotArgs a, const T *__restrict__ x, const T *__restrict__ w, const T *__restrict__ table_src,
                     float *y)
 {
-    extern __shared__ __align__(16) unsigned char gg_dyn[];
-    const uint32_t table = (uint32_t)__cvta_generic_to_shared(gg_dyn);
+    extern __shared__ __align__(1024) unsigned char gg_dyn[];
     const uint32_t warps = blockDim.x >> 5, wid = threadIdx.x >> 5;
-    hot_pull_sums<T, float, float, true>(table + hot_table_bytes<T>() + wid * HOT_RING, table, hot_cap<T>(), a,
+    const uint32_t ring = (uint32_t)__cvta_generic_to_shared(gg_dyn), table = ring + warps * HOT_RING;
+    hot_pull_sums<T, float, float, true>(ring + wid * HOT_RING, table, hot_cap<T>(), a,
                            wid * gridDim.x + blockIdx.x, gridDim.x * warps, x, w, y, [&] {
                                hot_table_load(table, table_src, hot_table_bytes<T>());
                                return true;
