@@ -210,6 +210,9 @@ gg_status gg_relabel_device(gg_graph *g, uint32_t V, uint64_t E, const uint32_t 
                             uint32_t mode, uint64_t seed, uint32_t *label, cudaStream_t s);
 gg_status gg_check_permutation(gg_graph *g, const uint32_t *label, uint32_t V, cudaStream_t s);
 gg_status gg_apply_labels(const uint32_t *ids, uint64_t n, const uint32_t *label, uint32_t *out, cudaStream_t s);
+/* results of up to this many 4-byte values are read back through page-locked
+ * scratch, one wait for all of a call's results */
+#define GG_STAGE_VALUES ((size_t)65536)
 /* the mapping's page-locked host scratch, at least `bytes` long */
 gg_status gg_pinned(gg_graph *g, size_t bytes, void **out);
 /* build the hot-vertex table of the mapping for a table of `cap` entries
@@ -325,6 +328,13 @@ gg_graphs_config gg_graphs_choice(gg_graph *g, uint32_t ngraphs);
 /* tuning (tune.cu): apply the process's tuning cache to g once (the shapes
  * tuned earlier for a graph of the same size class on this GPU) */
 void gg_tune_lookup(gg_graph *g, cudaStream_t s);
+
+/* FP32 pull PageRank of a small graph in one launch (small.cu): whether the
+ * graph fits, and the run -- ranks (normalised), iteration records and the rank
+ * sum as the launches of pr.cu write them (rec and sum zeroed before) */
+bool gg_small_fits(const gg_graph *g);
+gg_status gg_small_pagerank(gg_graph *g, const gg_pr_params *p, float *rank, void *rec, double *sum, float base,
+                            float init, float eps_f, cudaStream_t s);
 
 /* One iteration of the batched personalised PageRank on caller-held state
  * (ppr.cu; the server's continuous batch): the first kp (16/32/64) vectors

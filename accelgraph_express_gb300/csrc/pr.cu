@@ -908,6 +908,7 @@ struct Run
     const gg_pr_params *p;
     float eps_f = 0.0f, eps_fl = 0.0f;
     bool use_hot = false; /* pull gather through the hot-vertex table */
+    bool small = false;   /* every iteration in one cluster (small.cu) */
     gg_pull_shape shape;  /* launch shape of the FP pull gather */
     uint32_t launches = 0;
     uint32_t gather_launches = 0;
@@ -1194,18 +1195,67 @@ uint32_t value_bytes(const gg_pr_params *p)
     }
 }
 
+/* the buffers and tiles that pagerank_enqueue will use, so that a capture of it
+ * neither allocates nor frees (growing a buffer frees the old one, which
+ * synchronises the device and would break the capture) */
+gg_status pagerank_reserve(gg_graph *g, const gg_pr_params *p, bool use_hot, cudaStream_t s)
+{
+    const size_t n = (size_t)g->V + 16;
+    void *b;
+    gg_tiles *t;
+    const uint32_t vb = value_bytes(p);
+    const bool quant = p->mode == GG_PR_PULL_Q32 || p->mode == GG_PR_PULL_Q16 || p->mode == GG_PR_PULL_Q8;
+    const bool push = p->mode == GG_PR_PUSH || p->mode == GG_PR_PUSH_FX64 || p->mode == GG_PR_PUSH_Q;
+    if (vb)
+    {
+        GG_CHECK(gg_tiles_get(g, 1, s, &t));
+        GG_CHECK(gg_work(g, 2, n * vb, &b));
+        GG_CHECK(gg_work(g, 3, n * vb, &b));
+        GG_CHECK(gg_work(g, 5, n * (p->mode == GG_PR_PULL ? 4u : 8u), &b));
+    }
+    else if (push)
+    {
+        GG_CHECK(gg_tiles_get(g, 0, s, &t));
+        GG_CHECK(gg_work(g, 2, n * (p->mode == GG_PR_PUSH_FX64 ? 8u : 4u), &b));
+        GG_CHECK(gg_work(g, 5, n * 8, &b));
+    }
+    else
+    {
+        if (p->mode == GG_PR_DD_PULL) GG_CHECK(gg_tiles_get(g, 1, s, &t));
+        GG_CHECK(gg_work(g, 5, n * 4, &b));
+        GG_CHECK(gg_work(g, 7, n, &b));
+        GG_CHECK(gg_work(g, 8, n, &b));
+        GG_CHECK(gg_work(g, 9, n * 4, &b));
+    }
+    if (quant || p->mode == GG_PR_PUSH_Q || !(vb || push)) GG_CHECK(gg_work(g, 4, n * 4, &b));
+    if (p->mode == GG_PR_PUSH_Q) GG_CHECK(gg_work(g, 6, ((size_t)p->max_iterations + 2) * 4, &b));
+    if ((p->mode == GG_PR_PULL || p->mode == GG_PR_PUSH) && p->storage != GG_STORE_F32)
+    {
+        GG_CHECK(gg_work(g, 28, n * 4, &b));
+        GG_CHECK(gg_work(g, 29, n * 4, &b));
+    }
+    if (use_hot) GG_CHECK(gg_work(g, 32, GG_HOT_TABLE_BYTES + 16, &b));
+    return GG_OK;
+}
+
 /* every launch of one PageRank run, queued on R.s */
 gg_status pagerank_enqueue(Run &R, const gg_pr_params *p, IterRec *rec, float *rank, void *sum_v, uint32_t ngraphs,
                            const uint32_t *voff)
 {
     const uint32_t V = R.g->V, iters = p->max_iterations;
-    GG_CUDA(cudaMemsetAsync(rec, 0, ((size_t)iters + 2) * sizeof(IterRec), R.s));
-    GG_CUDA(cudaMemsetAsync(sum_v, 0, 64, R.s));
+    GG_CUDA(cudaMemsetAsync(rec, 0, ((size_t)iters + 2) * sizeof(IterRec) + 64, R.s)); /* and the sum after them */
     const float damp = p->damp;
     const float base_pr = 1.0f - damp;
     const float base = p->init_one_over_n ? base_pr / (float)V : base_pr;
     const float init = p->init_one_over_n ? 1.0f / (float)V : base_pr;
 
+    if (R.small)
+    {
+        GG_CHECK(gg_small_pagerank(R.g, p, rank, rec, (double *)sum_v, base, init, R.eps_f, R.s));
+        R.launches++;
+        R.gather_launches += iters;
+        return GG_OK;
+    }
     if (V > 0)
     {
         gg_status st = GG_OK;
@@ -1347,8 +1397,10 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
 
     void *rank_v, *rec_v, *sum_v, *voff_v = nullptr;
     GG_CHECK(gg_work(g, 0, ((size_t)V + 16) * 4, &rank_v));
-    GG_CHECK(gg_work(g, 1, ((size_t)iters + 2) * sizeof(IterRec), &rec_v));
-    GG_CHECK(gg_work(g, 10, 64, &sum_v));
+    /* the records and, after them, the rank sum: cleared and read back together */
+    const size_t rec_bytes = ((size_t)iters + 2) * sizeof(IterRec);
+    GG_CHECK(gg_work(g, 1, rec_bytes + 64, &rec_v));
+    sum_v = (char *)rec_v + rec_bytes;
     IterRec *rec = (IterRec *)rec_v;
     float *rank = (float *)rank_v;
     if (ngraphs)
@@ -1372,13 +1424,19 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
         R.use_hot = true;
     }
 
+    /* a graph that fits one cluster's shared memory: faster at every size it
+     * takes (small.cu); timed runs time each gather launch, and a table asked
+     * for is used */
+    R.small = p->mode == GG_PR_PULL && p->storage == GG_STORE_F32 && !ngraphs && !p->profile && !R.use_hot &&
+              gg_small_fits(g);
+
     /* with GG_PR_CUDA_GRAPH everything from here to the final normalisation
-     * is captured into one CUDA graph (relaxed capture: buffers first used
-     * inside it are allocated during the capture) and instantiated; the
+     * is captured into one CUDA graph (over buffers reserved before) and
+     * instantiated; the
      * instance stays with the mapping and is launched again by calls with
      * the same parameters while no device memory of the mapping has been
      * freed since (the buffers it writes are then the same) */
-    const bool as_graph = (p->flags & GG_PR_CUDA_GRAPH) != 0;
+    const bool as_graph = (p->flags & GG_PR_CUDA_GRAPH) != 0 && !R.small;
     gg_status st = GG_OK;
     if (as_graph)
     {
@@ -1407,6 +1465,7 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
                 cudaGraphExecDestroy(g->pr_exec);
                 g->pr_exec = nullptr;
             }
+            GG_CHECK(pagerank_reserve(g, p, R.use_hot, R.s));
             GG_CUDA(cudaStreamBeginCapture(R.s, cudaStreamCaptureModeRelaxed));
             st = pagerank_enqueue(R, p, rec, rank, sum_v, ngraphs, (const uint32_t *)voff_v);
             cudaGraph_t graph = nullptr;
@@ -1440,17 +1499,40 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
         st = pagerank_enqueue(R, p, rec, rank, sum_v, ngraphs, (const uint32_t *)voff_v);
     if (st != GG_OK) return st;
 
-    std::vector<IterRec> h(iters + 2);
+    /* the records, the sum and the ranks of a small graph come back through the
+     * mapping's page-locked buffer, queued behind the iterations: one wait for
+     * everything (a copy to pageable memory blocks, so each had needed a wait
+     * before it, 8 us apiece; a call on 1,000 vertices 111 -> 83 us).  Larger
+     * ranks go to the caller's memory directly, their pages made resident
+     * while the iterations run; very many records as before */
+    std::vector<IterRec> many;
+    const IterRec *h;
     double sum = 0.0;
-    /* a bounded wait first: a copy to pageable memory would block until the
-     * iterations end, however long that is; the rank destination's pages are
-     * made resident while the iterations run */
-    if (ranks && V) gg_host_dst_prepare(ranks, (size_t)V * 4);
-    GG_CHECK(gg_wait(R.s));
-    GG_CUDA(cudaMemcpyAsync(h.data(), rec, ((size_t)iters + 2) * sizeof(IterRec), cudaMemcpyDeviceToHost, R.s));
-    GG_CUDA(cudaMemcpyAsync(&sum, sum_v, sizeof(double), cudaMemcpyDeviceToHost, R.s));
-    if (ranks && V) GG_CHECK(gg_copy_d2h(ranks, rank, (size_t)V * 4, R.s));
-    GG_CHECK(gg_wait(R.s));
+    const bool stage_rank = ranks && V && V <= GG_STAGE_VALUES;
+    if (ranks && V && !stage_rank) gg_host_dst_prepare(ranks, (size_t)V * 4);
+    if (rec_bytes <= GG_STAGE_VALUES * 4)
+    {
+        void *pin;
+        GG_CHECK(gg_pinned(g, GG_STAGE_VALUES * 8 + 64, &pin));
+        GG_CUDA(cudaMemcpyAsync(pin, rec, rec_bytes + 8, cudaMemcpyDeviceToHost, R.s));
+        float *pin_rank = (float *)((char *)pin + GG_STAGE_VALUES * 4 + 64);
+        if (stage_rank) GG_CUDA(cudaMemcpyAsync(pin_rank, rank, (size_t)V * 4, cudaMemcpyDeviceToHost, R.s));
+        GG_CHECK(gg_wait(R.s));
+        h = (const IterRec *)pin;
+        memcpy(&sum, (const char *)pin + rec_bytes, 8);
+        if (stage_rank) memcpy(ranks, pin_rank, (size_t)V * 4);
+    }
+    else
+    {
+        many.resize((size_t)iters + 2);
+        GG_CHECK(gg_wait(R.s)); /* bounded, before a copy to pageable memory */
+        GG_CUDA(cudaMemcpyAsync(many.data(), rec, rec_bytes, cudaMemcpyDeviceToHost, R.s));
+        GG_CUDA(cudaMemcpyAsync(&sum, sum_v, sizeof(double), cudaMemcpyDeviceToHost, R.s));
+        GG_CHECK(gg_wait(R.s));
+        h = many.data();
+        if (stage_rank) GG_CHECK(gg_copy_d2h(ranks, rank, (size_t)V * 4, R.s));
+    }
+    if (ranks && V && !stage_rank) GG_CHECK(gg_copy_d2h(ranks, rank, (size_t)V * 4, R.s));
 
     /* reference loop convention: iterations = index of the breaking
      * iteration, or max when the loop ran out (pageRank.c:1021-1075) */
