@@ -403,11 +403,26 @@ extern "C" gg_status gg_spmv(gg_graph *g, const gg_spmv_params *p, const float *
         GG_CUDA(cudaGetLastError());
     }
     long long hundredths = 0;
-    GG_CHECK(gg_wait(s)); /* bounded, before a copy to pageable memory */
-    GG_CUDA(cudaMemcpyAsync(&hundredths, chk, 8, cudaMemcpyDeviceToHost, s));
-    if (y && V) GG_CHECK(gg_copy_d2h(y, yv, (size_t)V * 4, s));
-    if (x_out && V) GG_CHECK(gg_copy_d2h(x_out, xf, (size_t)V * 4, s));
+    /* small results through the page-locked scratch, with one wait */
+    const bool stage = V <= GG_STAGE_VALUES;
+    void *pin;
+    GG_CHECK(gg_pinned(g, GG_STAGE_VALUES * 8 + 64, &pin));
+    float *pin_y = (float *)((char *)pin + 64), *pin_x = pin_y + GG_STAGE_VALUES;
+    GG_CUDA(cudaMemcpyAsync(pin, chk, 8, cudaMemcpyDeviceToHost, s));
+    if (stage && y && V) GG_CUDA(cudaMemcpyAsync(pin_y, yv, (size_t)V * 4, cudaMemcpyDeviceToHost, s));
+    if (stage && x_out && V) GG_CUDA(cudaMemcpyAsync(pin_x, xf, (size_t)V * 4, cudaMemcpyDeviceToHost, s));
     GG_CHECK(gg_wait(s));
+    memcpy(&hundredths, pin, 8);
+    if (stage)
+    {
+        if (y && V) memcpy(y, pin_y, (size_t)V * 4);
+        if (x_out && V) memcpy(x_out, pin_x, (size_t)V * 4);
+    }
+    else
+    {
+        if (y) GG_CHECK(gg_copy_d2h(y, yv, (size_t)V * 4, s));
+        if (x_out) GG_CHECK(gg_copy_d2h(x_out, xf, (size_t)V * 4, s));
+    }
     res.checksum = (double)hundredths / 100.0;
     res.launches = launches;
     res.spmv_launches = timed;
