@@ -21,8 +21,10 @@
  *         in-edges start visited), the source, and the device loop's
  *         control block and first bitmap cleared, in one pass
  *   k_compact  bitmap -> queue (block-wide scan, one atomic per block pass)
- * Step counters are added and read once per block, not per warp: atomics
- * and loads of one address from every warp queue at one L2 slice.
+ * Step counters are added and read once per block, not per warp, and the edges
+ * of deferred hubs (and the host-driven top-down steps) gather what a block
+ * claims in shared memory before they append it: atomics and loads of one
+ * address from every warp queue at one L2 slice.
  * The direction switch follows the reference's uint32 arithmetic (alpha 15,
  * beta 18, mu/mf/nf, BFS.c:555-650).  Without profiling, the
  * direction-optimised modes run the whole level loop in one cooperative
@@ -183,11 +185,64 @@ __device__ __forceinline__ void td_enqueue(bool claimed, uint32_t u, uint32_t la
     }
 }
 
+/* The vertices a block claims in a top-down step, in shared memory until the
+ * step ends: one append per block.  One per warp and 32 edges meant
+ * up to 275K atomics on one word for the 8.8M edges of 303 hubs (104 us; 37
+ * now).  What does not fit is appended as it is claimed.  n[0]:
+ * claimed, n[1]: the end of the local part once it overflows. */
+constexpr uint32_t TD_LOCAL = 1024;
+
+struct LocalQueue
+{
+    uint32_t item[TD_LOCAL], n[2], at;
+};
+__device__ __forceinline__ void local_clear(LocalQueue &L)
+{
+    L.n[0] = 0u;
+    L.n[1] = TD_LOCAL;
+}
+/* append the block's local part; every thread calls it after the last enqueue */
+__device__ __forceinline__ void local_append(LocalQueue &L, uint32_t *nq, Counters *c)
+{
+    __syncthreads();
+    const uint32_t mine = min(L.n[0], L.n[1]);
+    if (threadIdx.x == 0 && mine) L.at = atomicAdd(&c->qlen, mine);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < mine; i += blockDim.x) nq[L.at + i] = L.item[i];
+}
+
+__device__ __forceinline__ void td_enqueue_local(bool claimed, uint32_t u, uint32_t lane, uint32_t *nq, Counters *c,
+                                                 LocalQueue &L)
+{
+    const uint32_t m = __ballot_sync(0xffffffffu, claimed);
+    if (!m) return;
+    const uint32_t cnt = (uint32_t)__popc(m);
+    uint32_t base = 0;
+    if (lane == 0) base = atomicAdd(&L.n[0], cnt);
+    base = __shfl_sync(0xffffffffu, base, 0);
+    uint32_t *to = L.item;
+    if (base + cnt > TD_LOCAL)
+    {
+        if (lane == 0)
+        {
+            atomicMin(&L.n[1], base);
+            base = atomicAdd(&c->qlen, cnt);
+        }
+        base = __shfl_sync(0xffffffffu, base, 0);
+        to = nq;
+    }
+    if (claimed) to[base + __popc(m & ((1u << lane) - 1u))] = u;
+}
+
 /* frontier vertices with more out-edges than `heavy_thr` (64 by default,
  * the tuned value per mapping otherwise) go to k_td_heavy, at most
  * TD_MAX_HEAVY of them per step (further ones stay with their warp) */
 #define TD_MAX_HEAVY 4096u
 
+/* LOCAL: claims through the block's local queue.  Not inside the single-launch
+ * search, where its registers made the bottom-up steps spill: a search of
+ * R-MAT-22 lost 10 us while one of a graph without hubs won 55 */
+template <bool LOCAL>
 __device__ __forceinline__ void td_body(const uint32_t *q, uint32_t qlen,
                                         const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
                                         int32_t *parents, uint32_t *dist, uint32_t newdist, uint32_t *visited,
@@ -198,6 +253,12 @@ __device__ __forceinline__ void td_body(const uint32_t *q, uint32_t qlen,
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
     uint32_t mf = 0;
     unsigned long long edges = 0;
+    __shared__ LocalQueue L;
+    if (LOCAL)
+    {
+        if (threadIdx.x == 0) local_clear(L);
+        __syncthreads();
+    }
     for (uint32_t i = warp; i < qlen; i += nwarps)
     {
         const uint32_t v = q[i];
@@ -224,9 +285,13 @@ __device__ __forceinline__ void td_body(const uint32_t *q, uint32_t qlen,
                 u = adj[j];
                 claimed = td_claim(u, v, parents, dist, newdist, visited, nbm, mf);
             }
-            td_enqueue(claimed, u, lane, nq, c);
+            if (LOCAL)
+                td_enqueue_local(claimed, u, lane, nq, c, L);
+            else
+                td_enqueue(claimed, u, lane, nq, c);
         }
     }
+    if (LOCAL) local_append(L, nq, c);
     block_flush(&c->mf, mf, &c->edges, edges);
 }
 
@@ -240,7 +305,12 @@ __device__ __forceinline__ void td_heavy_body(const uint4 *heavy, const uint32_t
     __shared__ uint32_t pre[TD_MAX_HEAVY + 1];
     __shared__ uint32_t wsum[8];
     __shared__ uint32_t s_nh;
-    if (threadIdx.x == 0) s_nh = min(*(volatile uint32_t *)&c->nheavy, TD_MAX_HEAVY);
+    __shared__ LocalQueue L;
+    if (threadIdx.x == 0)
+    {
+        s_nh = min(*(volatile uint32_t *)&c->nheavy, TD_MAX_HEAVY);
+        local_clear(L);
+    }
     __syncthreads();
     const uint32_t nh = s_nh;
     if (nh == 0) return;
@@ -300,8 +370,9 @@ __device__ __forceinline__ void td_heavy_body(const uint4 *heavy, const uint32_t
             u = adj[h.y + (k - pre[lo])];
             claimed = td_claim(u, h.x, parents, dist, newdist, visited, nbm, mf);
         }
-        td_enqueue(claimed, u, lane, nq, c);
+        td_enqueue_local(claimed, u, lane, nq, c, L);
     }
+    local_append(L, nq, c);
     block_flush(&c->mf, mf, nullptr, 0ull);
 }
 
@@ -483,7 +554,7 @@ __global__ void __launch_bounds__(256) k_td(const uint32_t *__restrict__ q, uint
                                             uint32_t *nq, uint32_t *nbm, Counters *c, uint4 *heavy,
                                             uint32_t heavy_thr)
 {
-    td_body(q, qlen, off, adj, parents, dist, newdist, visited, nq, nbm, c, heavy, heavy_thr);
+    td_body<true>(q, qlen, off, adj, parents, dist, newdist, visited, nq, nbm, c, heavy, heavy_thr);
 }
 __global__ void __launch_bounds__(256) k_td_heavy(const uint4 *__restrict__ heavy, const uint32_t *__restrict__ adj,
                                                   int32_t *parents, uint32_t *dist, uint32_t newdist,
@@ -638,7 +709,7 @@ __global__ void __launch_bounds__(256, 6) k_bfs_do(DoArgs a)
             mu -= mf;
             Counters *cs = a.c + s % 3;
             clear_slot(a.c + (s + 1) % 3);
-            td_body(a.q[qcur], qlen, a.out_off, a.out_adj, a.parents, a.dist, level + 1, a.visited, a.q[qcur ^ 1],
+            td_body<false>(a.q[qcur], qlen, a.out_off, a.out_adj, a.parents, a.dist, level + 1, a.visited, a.q[qcur ^ 1],
                     nullptr, cs, a.heavy, a.heavy_thr);
             if (!(ok = grid_barrier(a.ctl, a.bar_limit_ns, gen))) break;
             /* the deferred high-degree vertices, when there are any (every
