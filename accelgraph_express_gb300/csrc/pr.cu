@@ -1409,19 +1409,25 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
         GG_CUDA(cudaMemcpyAsync(voff_v, h_voff, ((size_t)ngraphs + 1) * 4, cudaMemcpyHostToDevice, R.s));
     }
 
-    /* the hot-vertex table of the pull modes (prepared before any capture: preparation reads back to the host) */
+    /* before the launches: allocating it may wait for them */
+    void *pin;
+    GG_CHECK(gg_pinned(g, GG_STAGE_VALUES * 8 + 64, &pin));
+
+    /* the hot-vertex table of the pull modes (prepared before any capture) */
     gg_tune_lookup(g, R.s);
     R.shape = g->pr_shape;
-    const bool hot_default = R.shape.hot == 2 ? g->E >= GG_HOT_MIN_E : R.shape.hot == 1;
-    if (value_bytes(p) && !(p->flags & GG_PR_HOT_OFF) && ((p->flags & GG_PR_HOT_ON) || hot_default) &&
-        gg_hot_fits(V, g->E))
+    const uint32_t vb = value_bytes(p);
+    if (vb && gg_hot_fits(V, g->E))
     {
-        const uint32_t vb = value_bytes(p);
-        GG_CHECK(gg_hot_prepare(g, R.s, vb == 8   ? hot_cap<unsigned long long>()
-                                        : vb == 4 ? hot_cap<uint32_t>()
-                                        : vb == 2 ? hot_cap<uint16_t>()
-                                                  : hot_cap<uint8_t>()));
-        R.use_hot = true;
+        const uint32_t cap = vb == 8   ? hot_cap<unsigned long long>()
+                             : vb == 4 ? hot_cap<uint32_t>()
+                             : vb == 2 ? hot_cap<uint16_t>()
+                                       : hot_cap<uint8_t>();
+        if (gg_hot_wanted(g, p->flags, R.shape.hot, cap, p->max_iterations))
+        {
+            GG_CHECK(gg_hot_prepare(g, R.s, cap));
+            R.use_hot = true;
+        }
     }
 
     /* a graph that fits one cluster's shared memory: faster at every size it
@@ -1512,8 +1518,6 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
     if (ranks && V && !stage_rank) gg_host_dst_prepare(ranks, (size_t)V * 4);
     if (rec_bytes <= GG_STAGE_VALUES * 4)
     {
-        void *pin;
-        GG_CHECK(gg_pinned(g, GG_STAGE_VALUES * 8 + 64, &pin));
         GG_CUDA(cudaMemcpyAsync(pin, rec, rec_bytes + 8, cudaMemcpyDeviceToHost, R.s));
         float *pin_rank = (float *)((char *)pin + GG_STAGE_VALUES * 4 + 64);
         if (stage_rank) GG_CUDA(cudaMemcpyAsync(pin_rank, rank, (size_t)V * 4, cudaMemcpyDeviceToHost, R.s));

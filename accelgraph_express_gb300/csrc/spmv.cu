@@ -326,7 +326,8 @@ extern "C" gg_status gg_spmv(gg_graph *g, const gg_spmv_params *p, const float *
     const uint32_t V = g->V;
     gg_spmv_result res;
     memset(&res, 0, sizeof(res));
-    void *xf, *yv, *xin = nullptr, *chk;
+    void *xf, *yv, *xin = nullptr, *chk, *pin;
+    GG_CHECK(gg_pinned(g, GG_STAGE_VALUES * 8 + 64, &pin)); /* before the launches: allocating it may wait for them */
     GG_CHECK(gg_work(g, 0, ((size_t)V + 16) * 4, &xf));
     GG_CHECK(gg_work(g, 11, ((size_t)V + 16) * 4, &yv));
     GG_CHECK(gg_work(g, 10, 64, &chk));
@@ -405,8 +406,6 @@ extern "C" gg_status gg_spmv(gg_graph *g, const gg_spmv_params *p, const float *
     long long hundredths = 0;
     /* small results through the page-locked scratch, with one wait */
     const bool stage = V <= GG_STAGE_VALUES;
-    void *pin;
-    GG_CHECK(gg_pinned(g, GG_STAGE_VALUES * 8 + 64, &pin));
     float *pin_y = (float *)((char *)pin + 64), *pin_x = pin_y + GG_STAGE_VALUES;
     GG_CUDA(cudaMemcpyAsync(pin, chk, 8, cudaMemcpyDeviceToHost, s));
     if (stage && y && V) GG_CUDA(cudaMemcpyAsync(pin_y, yv, (size_t)V * 4, cudaMemcpyDeviceToHost, s));

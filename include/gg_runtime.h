@@ -151,8 +151,9 @@ size_t gg_graph_device_bytes(const gg_graph *g);
 /* Device memory the library has freed is kept for reuse (a mapping made
  * and dropped per call then pays no cudaMalloc / cudaFree), up to
  * GG_DEVICE_CACHE_MB (default 16384) MB; an allocation that fails empties
- * the cache first.  trim hands every cached block back to CUDA; bytes is
- * what the cache holds now. */
+ * the cache first.  Up to 16 small page-locked blocks are kept likewise.
+ * trim hands every kept block back to CUDA; bytes is what the device cache
+ * holds now. */
 void gg_device_cache_trim(void);
 size_t gg_device_cache_bytes(void);
 

@@ -1,5 +1,5 @@
 """BFS where a step's shared-memory structures reach their limits: a first
-bottom-up frontier around the size that gets a Bloom filter, blocks that claim
+bottom-up frontier from one vertex to a third of the graph, blocks that claim
 more vertices than their local queue holds, and hubs whose edges are dealt to
 the grid.  Levels are compared exactly with the oracle's or the known ones."""
 import numpy as np
