@@ -317,13 +317,21 @@ __device__ __forceinline__ void hot_pull_sums(uint32_t ring, uint32_t table, uin
     }
 }
 
-/* table[i] = x[hot_list[i]], zero from n to cap and in the pad entry, padded
+/* slots in use of the H there are, from the counts behind the hot list:
+ * vertices above the threshold degree and at it */
+__device__ __forceinline__ uint32_t hot_taken(const uint32_t *__restrict__ cnt, uint32_t H)
+{
+    return min(cnt[0] + cnt[1], H);
+}
+
+/* table[i] = x[hot_list[i]], zero from the slots in use to cap and in the pad entry, padded
  * to 16 bytes: the contiguous copy that every CTA of the gather reads (each
  * CTA gathering its own had cost 32K requests per SM and launch) */
 template <class CT>
 __device__ __forceinline__ void hot_table_fill(const CT *__restrict__ x, const uint32_t *__restrict__ hot_list,
-                                               uint32_t n, uint32_t cap, CT *__restrict__ out)
+                                               uint32_t H, uint32_t cap, CT *__restrict__ out)
 {
+    const uint32_t n = hot_taken(hot_list + GG_HOT_ENTRIES, H);
     const uint32_t all = cap + 16 / sizeof(CT);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < all; i += gridDim.x * blockDim.x)
         out[i] = i < n ? x[hot_list[i]] : CT(0);

@@ -117,9 +117,10 @@ struct gg_graph
     uint32_t ppr_stride = 0;
     /* hot-vertex table: flag-encoded copy of in_adj and the slot -> vertex list */
     uint32_t *hot_adj = nullptr;
-    uint32_t *hot_list = nullptr;  /* GG_HOT_ENTRIES slots */
-    uint32_t hot_n = 0;            /* slots in use */
+    uint32_t *hot_list = nullptr;  /* GG_HOT_ENTRIES slots, then the counts (hot_taken) */
+    uint32_t hot_slots = 0;        /* slots there are: hot_cap, or V if that is less */
     uint32_t hot_cap = 0;          /* table capacity the encoding was made for */
+    uint64_t plain_its = 0;        /* gathers done without the table since it was last made */
     uint32_t *hot_seg0 = nullptr;  /* per tile of hot_tile edges: its first row end (gg_hot.cuh) */
     uint32_t hot_ntiles = 0, hot_tile = 0; /* tiles and edges per tile */
     /* page-locked host scratch for small per-step read-backs */
@@ -219,6 +220,10 @@ gg_status gg_pinned(gg_graph *g, size_t bytes, void **out);
  * (<= GG_HOT_ENTRIES; rebuilt only when cap changes; needs GG_MAP_IN and
  * gg_hot_fits), and the rows and tiles of the hot kernels */
 gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap);
+/* whether a call of `iterations` gathers takes the table of `cap` entries:
+ * asked for by the flags, chosen by the tuner (hot 0/1), or by the rule of
+ * GG_HOT_MIN_E and GG_HOT_PAYS; the graph passes gg_hot_fits (hot.cu) */
+bool gg_hot_wanted(gg_graph *g, uint32_t flags, uint32_t hot, uint32_t cap, uint32_t iterations);
 /* rows_list of the mapping, and for tiles of `tile` edges the first row end in
  * each (bit 31: that row began in an earlier tile) in a new allocation of
  * *ntiles words; adds its launches to *launches (hot.cu) */
@@ -311,9 +316,17 @@ unsigned long long gg_barrier_limit_ns();
  * 88 -> 78, 320 -> 268, 1,259 -> 1,043.  Below, the 25 MB of table that 152
  * SMs read per launch cost more than the requests they save. */
 #define GG_HOT_MIN_E (1u << 23)
+/* ... and, while the table is not there, once the gathers done without it and
+ * those of the call make (gathers - 2) * E reach this.  Making the table
+ * costs what it saves in (R-MAT, PageRank and SpMV; uniform random) 3-4; 8-11
+ * gathers of 16.8M edges, 2-3; 3-5 of 67M, 2 of 268M: a mapping that is used
+ * for a product or two stays without it, and one that is used on pays for it
+ * at most twice. */
+#define GG_HOT_PAYS 50000000ull
 /* ids need two flag bits; edge numbers a tile round's headroom in 32 bits */
 #define GG_HOT_MAX_V 0x40000000u
 #define GG_HOT_MAX_E 0xfc000000u
+#define GG_HOT_LIST_BYTES (((size_t)GG_HOT_ENTRIES + 4) * 4)
 /* whether the hot-vertex gather can run on a graph of these sizes */
 inline bool gg_hot_fits(uint32_t V, uint32_t E) { return V > 0 && E > 0 && V < GG_HOT_MAX_V && E <= GG_HOT_MAX_E; }
 /* many-graphs PageRank (graphs.cu): tile coordinates and size order for the

@@ -442,6 +442,9 @@ gg_status gg_work(gg_graph *g, int slot, size_t bytes, void **out)
 
 gg_status gg_pinned(gg_graph *g, size_t bytes, void **out)
 {
+    /* one size for all uses: growing would wait on the device in
+     * cudaFreeHost, past the limit of gg_wait */
+    bytes = std::max(bytes, (size_t)GG_STAGE_VALUES * 8 + 64);
     if (g->pinned_bytes < bytes)
     {
         if (g->pinned) cudaFreeHost(g->pinned);
@@ -1127,7 +1130,7 @@ extern "C" gg_status gg_graph_unmap(gg_graph *g)
     dev_release(g, g->rows_list, ((size_t)g->V + GG_ROW_PAD + 4) * 4, idle);
     dev_release(g, g->ppr_seg0, (size_t)g->ppr_ntiles * 4, idle);
     dev_release(g, g->hot_adj, ((size_t)g->E + GG_EDGE_PAD) * 4, idle);
-    dev_release(g, g->hot_list, (size_t)GG_HOT_ENTRIES * 4, idle);
+    dev_release(g, g->hot_list, GG_HOT_LIST_BYTES, idle);
     dev_release(g, g->hot_seg0, (size_t)g->hot_ntiles * 4, idle);
     for (auto &b : g->work) dev_release(g, b.ptr, b.bytes, idle);
     dev_release(g, g->graphs.coord, g->graphs.bytes, idle);

@@ -9,8 +9,8 @@
  * per launch.  On R-MAT graphs in natural order the 32K hottest of 16.7M
  * vertices receive 37% of all gathers, the 64K hottest 48%.
  *
- * Preparation, once per mapping: a histogram of out-degrees (clamped at
- * 65535) read back to the host gives the threshold degree T; vertices above
+ * Preparation, once per mapping, without a wait on the host: a histogram of
+ * out-degrees (clamped at 65535) gives the threshold degree T; vertices above
  * T and, up to H, vertices at T take slots by atomics (which of the ties win
  * does not matter: the table holds exact copies); one pass over the CSC
  * writes the encoded ids.  The gather (gg_hot.cuh) finds rows through the ids
@@ -19,13 +19,13 @@
  */
 #include <cuda_runtime.h>
 
-#include <vector>
-
-#include "gg_internal.h"
+#include "gg_hot.cuh"
 
 namespace {
 
 constexpr uint32_t NO_SLOT = 0xffffffffu;
+
+using gg::hot_taken;
 
 /* out-degree histogram (clamped at 65535): degrees below 4096 -- nearly all
  * of them on skewed graphs, so global atomics on those bins would serialise
@@ -49,18 +49,72 @@ __global__ void __launch_bounds__(256) k_deg_hist(const uint32_t *__restrict__ o
         if (s[i]) atomicAdd(&hist[i], s[i]);
 }
 
-__global__ void k_hot_mark(const uint32_t *__restrict__ outdeg, uint32_t V, uint32_t T, uint32_t above,
-                           uint32_t H, uint32_t *slot_of, uint32_t *hot_list, uint32_t *counters)
+/* cnt[0] = vertices above T, cnt[1] = at T, cnt[2] = T, cnt[3] = vertices
+ * above T by the histogram: T is the degree with fewer than H vertices above
+ * it.  One block: its warps sum 2,048 bins each, then the chunk in which the
+ * count from the top reaches H is scanned bin by bin.  (Read back and
+ * scanned on the host, with a second read for the slots taken, preparation
+ * took 160 us longer than its kernels: 247 -> 89 us at R-MAT-20.) */
+__global__ void __launch_bounds__(1024) k_hot_threshold(const uint32_t *__restrict__ hist, uint32_t H, uint32_t *cnt)
 {
+    __shared__ uint32_t s_sum[32], s_chunk, s_before;
+    const uint32_t lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    /* chunk c holds bins 65535 - 2048 c downwards */
+    uint32_t n = 0;
+#pragma unroll 8
+    for (uint32_t k = 0; k < 64; k++) n += hist[65535u - (w * 2048u + k * 32u + lane)];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) n += __shfl_xor_sync(0xffffffffu, n, o);
+    if (lane == 0) s_sum[w] = n;
+    __syncthreads();
+    if (threadIdx.x == 0)
+    {
+        uint32_t c = 0, before = 0;
+        while (c < 31u && before + s_sum[c] < H) before += s_sum[c++];
+        s_chunk = c;
+        s_before = before;
+    }
+    __syncthreads();
+    const uint32_t top = 65535u - s_chunk * 2048u - threadIdx.x * 2u; /* this thread's bins: top, top - 1 */
+    const uint32_t n0 = hist[top], n1 = hist[top - 1u];
+    uint32_t incl = n0 + n1;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= (uint32_t)o) incl += y;
+    }
+    if (lane == 31) s_sum[w] = incl;
+    __syncthreads();
+    uint32_t before = s_before;
+    for (uint32_t k = 0; k < w; k++) before += s_sum[k];
+    before += incl - n0 - n1;
+    /* the first bin from the top at which the count reaches H; bin 0 if none */
+    if (before < H && before + n0 >= H)
+    {
+        cnt[2] = top;
+        cnt[3] = before;
+    }
+    else if (before + n0 < H && (before + n0 + n1 >= H || top == 1u))
+    {
+        cnt[2] = top - 1u;
+        cnt[3] = before + n0;
+    }
+}
+
+__global__ void k_hot_mark(const uint32_t *__restrict__ outdeg, uint32_t V, uint32_t H, uint32_t *slot_of,
+                           uint32_t *hot_list, uint32_t *cnt)
+{
+    const uint32_t T = cnt[2], above = cnt[3];
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
     {
         const uint32_t d = min(outdeg[v], 65535u);
         uint32_t slot = NO_SLOT;
         if (d > T)
-            slot = atomicAdd(&counters[0], 1u);
+            slot = atomicAdd(&cnt[0], 1u);
         else if (d == T && T > 0)
         {
-            const uint32_t k = atomicAdd(&counters[1], 1u);
+            const uint32_t k = atomicAdd(&cnt[1], 1u);
             if (above + k < H) slot = above + k;
         }
         slot_of[v] = slot;
@@ -90,8 +144,7 @@ __global__ void __launch_bounds__(1024) k_hot_encode(const uint32_t *__restrict_
     extern __shared__ uint32_t bloom[];
     for (uint32_t i = threadIdx.x; i < BLOOM_BITS / 32; i += blockDim.x) bloom[i] = 0u;
     __syncthreads();
-    const uint32_t taken = counters[0] + counters[1];
-    const uint32_t nh = taken < H ? taken : H;
+    const uint32_t nh = hot_taken(counters, H);
     for (uint32_t i = threadIdx.x; i < nh; i += blockDim.x)
     {
         const uint32_t u = hot_list[i], b1 = bloom_h1(u), b2 = bloom_h2(u);
@@ -323,6 +376,19 @@ static uint32_t hot_tile_for(uint32_t E)
     return tile;
 }
 
+bool gg_hot_wanted(gg_graph *g, uint32_t flags, uint32_t hot, uint32_t cap, uint32_t iterations)
+{
+    if (flags & GG_PR_HOT_OFF) return false;
+    if (flags & GG_PR_HOT_ON) return true;
+    if (hot != 2) return hot == 1;
+    if (g->E < GG_HOT_MIN_E) return false;
+    if (g->hot_adj && g->hot_cap == cap) return true;
+    const uint64_t its = g->plain_its + iterations;
+    if (its > 2 && (its - 2) * g->E >= GG_HOT_PAYS) return true;
+    g->plain_its = its;
+    return false;
+}
+
 gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap)
 {
     if (!g->in_adj || !g->out_deg) return gg_fail(GG_ERR_INVALID, "the hot-vertex table needs GG_MAP_IN");
@@ -337,46 +403,27 @@ gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap)
     }
     if (g->hot_adj && g->hot_cap == cap) return GG_OK;
     const uint32_t H = V < cap ? V : cap;
-    void *hist, *slot_of, *cnt;
+    void *hist, *slot_of;
     GG_CHECK(gg_work(g, 25, 65536 * 4, &hist));
     GG_CHECK(gg_work(g, 26, (size_t)V * 4, &slot_of));
-    GG_CHECK(gg_work(g, 27, 16, &cnt));
+    if (!g->hot_list) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_list, GG_HOT_LIST_BYTES));
+    if (!g->hot_adj) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_adj, ((size_t)E + GG_EDGE_PAD) * 4));
+    uint32_t *cnt = g->hot_list + GG_HOT_ENTRIES;
     GG_CUDA(cudaMemsetAsync(hist, 0, 65536 * 4, s));
     GG_CUDA(cudaMemsetAsync(cnt, 0, 16, s));
     const int grid = gg_sm_count() * 8;
     k_deg_hist<<<gg_sm_count() * 2, 256, 0, s>>>(g->out_deg, V, (uint32_t *)hist);
-    GG_CUDA(cudaGetLastError());
-    std::vector<uint32_t> h(65536);
-    GG_CHECK(gg_wait(s)); /* bounded, before a copy to pageable memory */
-    GG_CUDA(cudaMemcpyAsync(h.data(), hist, 65536 * 4, cudaMemcpyDeviceToHost, s));
-    GG_CHECK(gg_wait(s));
-    /* threshold: the degree T with fewer than H vertices above it */
-    uint32_t above = 0, T = 0;
-    for (int d = 65535; d >= 0; d--)
-    {
-        if (above + h[d] >= H || d == 0)
-        {
-            T = (uint32_t)d;
-            break;
-        }
-        above += h[d];
-    }
-    if (!g->hot_list) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_list, (size_t)GG_HOT_ENTRIES * 4));
-    if (!g->hot_adj) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_adj, ((size_t)E + GG_EDGE_PAD) * 4));
-    k_hot_mark<<<grid, 256, 0, s>>>(g->out_deg, V, T, above, H, (uint32_t *)slot_of, g->hot_list, (uint32_t *)cnt);
+    k_hot_threshold<<<1, 1024, 0, s>>>((const uint32_t *)hist, H, cnt);
+    k_hot_mark<<<grid, 256, 0, s>>>(g->out_deg, V, H, (uint32_t *)slot_of, g->hot_list, cnt);
     /* one CTA of 1024 threads per SM (60 registers a thread); adj and out are
      * whole allocations, 16-byte aligned for the vector loads */
     GG_CUDA(cudaFuncSetAttribute(k_hot_encode, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(BLOOM_BITS / 8)));
     k_hot_encode<<<gg_sm_count(), 1024, BLOOM_BITS / 8, s>>>(g->in_adj, (uint64_t)E, (const uint32_t *)slot_of,
-                                                              g->hot_list, (const uint32_t *)cnt, H, cap, g->hot_adj);
+                                                              g->hot_list, cnt, H, cap, g->hot_adj);
     k_rows_mark<<<grid, 256, 0, s>>>(g->in_off, V, g->hot_adj);
     GG_CUDA(cudaGetLastError());
-    std::vector<uint32_t> c(4);
-    GG_CHECK(gg_wait(s));
-    GG_CUDA(cudaMemcpyAsync(c.data(), cnt, 16, cudaMemcpyDeviceToHost, s));
-    GG_CHECK(gg_wait(s));
-    g->hot_n = T > 0 ? (c[0] + (c[1] < H - above ? c[1] : H - above)) : c[0];
-    if (g->hot_n > H) g->hot_n = H;
+    g->plain_its = 0;
+    g->hot_slots = H;
     g->hot_cap = cap;
     return GG_OK;
 }

@@ -239,12 +239,12 @@ struct PrGather
 
 /* the hot vertices' stored contributions, contiguous, for k_pr_pull_hot */
 template <class CT>
-__global__ void k_pr_hot_fill(const CT *__restrict__ cin, const uint32_t *__restrict__ hot_list, uint32_t n,
+__global__ void k_pr_hot_fill(const CT *__restrict__ cin, const uint32_t *__restrict__ hot_list, uint32_t H,
                               uint32_t cap, CT *__restrict__ out, const IterRec *rec, uint32_t it)
 {
     pdl_wait();
     if (it > 0 && rec[it - 1].active == 0u) return;
-    hot_table_fill(cin, hot_list, n, cap, out);
+    hot_table_fill(cin, hot_list, H, cap, out);
     pdl_trigger();
 }
 
@@ -987,14 +987,14 @@ gg_status run_pull(Run &R, IterRec *rec, float *rank, uint32_t iters, float base
             const int fg = (int)((hot_cap<CT>() + 255) / 256);
             if (pdl)
             {
-                GG_CUDA(gg_launch_pdl(k_pr_hot_fill<CT>, dim3(fg), dim3(256), 0, R.s, cin, g->hot_list, g->hot_n,
+                GG_CUDA(gg_launch_pdl(k_pr_hot_fill<CT>, dim3(fg), dim3(256), 0, R.s, cin, g->hot_list, g->hot_slots,
                                       hot_cap<CT>(), tab, (const IterRec *)rec, it));
                 GG_CUDA(gg_launch_pdl(k_pr_pull_hot<K>, dim3(hg), dim3(hw * 32), smem, R.s, ha, cin, (const CT *)tab,
                                       (Acc *)sums, (const IterRec *)rec, it));
             }
             else
             {
-                k_pr_hot_fill<CT><<<fg, 256, 0, R.s>>>(cin, g->hot_list, g->hot_n, hot_cap<CT>(), tab, rec, it);
+                k_pr_hot_fill<CT><<<fg, 256, 0, R.s>>>(cin, g->hot_list, g->hot_slots, hot_cap<CT>(), tab, rec, it);
                 k_pr_pull_hot<K><<<hg, hw * 32, smem, R.s>>>(ha, cin, tab, (Acc *)sums, rec, it);
             }
             R.launches++;

@@ -49,10 +49,10 @@ __global__ void __launch_bounds__(GG_TILE_NT) k_spmv_pull(const uint32_t *__rest
 
 /* x of the hot vertices, contiguous (once per call: x does not change) */
 template <class T>
-__global__ void k_spmv_hot_fill(const T *__restrict__ x, const uint32_t *__restrict__ hot_list, uint32_t n,
+__global__ void k_spmv_hot_fill(const T *__restrict__ x, const uint32_t *__restrict__ hot_list, uint32_t H,
                                 uint32_t cap, T *__restrict__ out)
 {
-    hot_table_fill(x, hot_list, n, cap, out);
+    hot_table_fill(x, hot_list, H, cap, out);
 }
 
 /* the pull product through the hot-vertex table (gg_hot.cuh) */
@@ -261,12 +261,11 @@ gg_status spmv_fp(gg_graph *g, const gg_spmv_params *p, const float *x_dev, floa
     void *hot_tab = nullptr;
     gg_tune_lookup(g, s);
     const gg_pull_shape shape = g->spmv_shape;
-    const bool hot_default = shape.hot == 2 ? g->E >= GG_HOT_MIN_E : shape.hot == 1;
-    if (pull && !(p->flags & GG_PR_HOT_OFF) && ((p->flags & GG_PR_HOT_ON) || hot_default) && gg_hot_fits(V, g->E))
+    if (pull && gg_hot_fits(V, g->E) && gg_hot_wanted(g, p->flags, shape.hot, hot_cap<T>(), p->iterations))
     {
         GG_CHECK(gg_hot_prepare(g, s, hot_cap<T>()));
         GG_CHECK(gg_work(g, 32, GG_HOT_TABLE_BYTES + 16, &hot_tab));
-        k_spmv_hot_fill<T><<<(hot_cap<T>() + 255) / 256, 256, 0, s>>>(xv, g->hot_list, g->hot_n, hot_cap<T>(), (T *)hot_tab);
+        k_spmv_hot_fill<T><<<(hot_cap<T>() + 255) / 256, 256, 0, s>>>(xv, g->hot_list, g->hot_slots, hot_cap<T>(), (T *)hot_tab);
         launches++;
         use_hot = true;
     }
