@@ -106,7 +106,7 @@ struct gg_graph
     void *out_w16[3] = {nullptr, nullptr, nullptr};
 
     /* work buffers, grown on demand */
-    gg_buf work[34];
+    gg_buf work[35];
     /* the rows (of the CSC) that have edges, in order: rows_list[0 .. n), then
      * GG_ROW_PAD entries of V, and n itself at rows_list[V + GG_ROW_PAD] */
     uint32_t *rows_list = nullptr;

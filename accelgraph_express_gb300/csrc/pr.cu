@@ -1430,8 +1430,8 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
         }
     }
 
-    /* a graph that fits one cluster's shared memory: faster at every size it
-     * takes (small.cu); timed runs time each gather launch, and a table asked
+    /* a graph of up to 2.5M edges and 262K vertices: every iteration in one
+     * launch, faster at every size it takes (small.cu); timed runs time each gather launch, and a table asked
      * for is used */
     R.small = p->mode == GG_PR_PULL && p->storage == GG_STORE_F32 && !ngraphs && !p->profile && !R.use_hot &&
               gg_small_fits(g);
@@ -1537,6 +1537,8 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
         if (stage_rank) GG_CHECK(gg_copy_d2h(ranks, rank, (size_t)V * 4, R.s));
     }
     if (ranks && V && !stage_rank) GG_CHECK(gg_copy_d2h(ranks, rank, (size_t)V * 4, R.s));
+
+    if (R.small && h[iters + 1].pad) return gg_fail(GG_ERR_KERNEL, "PageRank grid barrier timed out");
 
     /* reference loop convention: iterations = index of the breaking
      * iteration, or max when the loop ran out (pageRank.c:1021-1075) */
