@@ -550,12 +550,10 @@ __device__ __forceinline__ void warp_pull_sums(const uint32_t *__restrict__ off,
  * fetched once per lane segment through op.row_value(row).
  */
 template <int IPT, int WARPS, class Op>
-__device__ __forceinline__ void warp_push(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
-                                          uint32_t V, const uint2 *__restrict__ coord, uint32_t ntiles, Op &op)
+__device__ __forceinline__ void warp_push_staged(uint32_t *sm_off, uint32_t *sm_adj, const uint32_t *__restrict__ off,
+                                                 const uint32_t *__restrict__ adj, uint32_t V,
+                                                 const uint2 *__restrict__ coord, uint32_t ntiles, Op &op)
 {
-    constexpr uint32_t TW = 32 * IPT;
-    __shared__ __align__(16) uint32_t sm_off[WARPS][TW + 8];
-    __shared__ __align__(16) uint32_t sm_adj[WARPS][TW + 4];
     const uint32_t w = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t nw = gridDim.x * WARPS;
     for (uint32_t tile = blockIdx.x * WARPS + w; tile < ntiles; tile += nw)
@@ -563,8 +561,8 @@ __device__ __forceinline__ void warp_push(const uint32_t *__restrict__ off, cons
         TileGeom t;
         t.load(coord, tile, V);
         /* edge j0+i at s_adj[i], row i0+k's offset at s_off[k] */
-        const uint32_t *s_adj = sm_adj[w] + stage_words(sm_adj[w], adj, t.j0, t.nedges, lane);
-        const uint32_t *s_off = sm_off[w] + stage_words(sm_off[w], off, t.i0, t.nrows + 1, lane);
+        const uint32_t *s_adj = sm_adj + stage_words(sm_adj, adj, t.j0, t.nedges, lane);
+        const uint32_t *s_off = sm_off + stage_words(sm_off, off, t.i0, t.nrows + 1, lane);
         cp_async_wait_all();
         __syncwarp();
         const uint32_t d = lane * IPT;
@@ -595,6 +593,114 @@ __device__ __forceinline__ void warp_push(const uint32_t *__restrict__ off, cons
             }
         }
         __syncwarp();
+    }
+}
+
+template <int IPT, int WARPS, class Op>
+__device__ __forceinline__ void warp_push(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
+                                          uint32_t V, const uint2 *__restrict__ coord, uint32_t ntiles, Op &op)
+{
+    constexpr uint32_t TW = 32 * IPT;
+    __shared__ __align__(16) uint32_t sm_off[WARPS][TW + 8];
+    __shared__ __align__(16) uint32_t sm_adj[WARPS][TW + 4];
+    const uint32_t w = threadIdx.x >> 5;
+    warp_push_staged<IPT, WARPS>(sm_off[w], sm_adj[w], off, adj, V, coord, ntiles, op);
+}
+
+/*
+ * Table of the push scatters: the most frequent destinations (push.cu) are
+ * added up in shared memory, one table per block, and each block adds them to
+ * global memory once, at its end (shared-memory additions of FP32 run at 1 T/s
+ * over random slots and 10 ns apart on one).  Per scatter, without -> with, R-MAT
+ * with 16 edges per vertex: 1M edges 57 -> 22 us, 8M 204 -> 72; 33M (11 per
+ * vertex) 541 -> 236.  Half the slots: 22, 81, 259; twice: 24, 66, 228.
+ */
+__device__ __forceinline__ uint32_t push_slot(uint32_t dst) { return (dst * GG_PUSH_HASH) >> (32 - PUSH_LOG); }
+
+template <class T>
+struct PushTable
+{
+    uint32_t *tag; /* the destination of each slot */
+    T *val;
+    T *out;
+    /* smem: PUSH_SLOTS values, then as many tags */
+    __device__ __forceinline__ PushTable(unsigned char *smem, const uint32_t *__restrict__ tags, T *o) : out(o)
+    {
+        val = reinterpret_cast<T *>(smem);
+        tag = reinterpret_cast<uint32_t *>(val + PUSH_SLOTS);
+        for (uint32_t i = threadIdx.x; i < PUSH_SLOTS; i += PUSH_NT)
+        {
+            tag[i] = tags[i];
+            val[i] = T(0);
+        }
+        __syncthreads();
+    }
+    __device__ __forceinline__ void add(uint32_t dst, T v) const
+    {
+        const uint32_t slot = push_slot(dst);
+        if (tag[slot] == dst)
+            atomicAdd(&val[slot], v);
+        else
+            atomicAdd(&out[dst], v);
+    }
+    __device__ __forceinline__ void flush() const
+    {
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < PUSH_SLOTS; i += PUSH_NT)
+        {
+            const T v = val[i];
+            if (v != T(0)) atomicAdd(&out[tag[i]], v);
+        }
+    }
+};
+
+/* warp_push for blocks of PUSH_WARPS warps, staged in dynamic shared memory */
+constexpr size_t PUSH_STAGE = (size_t)PUSH_WARPS * (2 * GG_TILE_ITEMS + 12) * 4;
+template <class T>
+constexpr size_t push_smem()
+{
+    return PUSH_STAGE + (size_t)PUSH_SLOTS * (sizeof(T) + 4);
+}
+
+template <class T>
+struct PushDirect
+{
+    T *out;
+    __device__ __forceinline__ void add(uint32_t dst, T v) const { atomicAdd(&out[dst], v); }
+};
+
+template <class T, class Sink, class Row, class Term>
+struct PushOp
+{
+    typedef T RowVal;
+    Sink sink;
+    Row row;
+    Term term;
+    __device__ __forceinline__ T row_value(uint32_t r) const { return row(r); }
+    __device__ __forceinline__ void scatter(T rv, uint32_t e, uint32_t dst) const { sink.add(dst, term(rv, e)); }
+};
+
+/* out[dst] += term(row(r), e) over all edges e of every row r, by blocks of
+ * PUSH_NT threads with push_smem<T>() bytes of dynamic shared memory and the
+ * table, or of GG_TILE_NT threads without */
+template <bool TABLE, class T, class Row, class Term>
+__device__ __forceinline__ void push_scatter(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj, uint32_t V,
+                                             const uint2 *__restrict__ coord, uint32_t ntiles,
+                                             const uint32_t *__restrict__ tags, T *out, Row row, Term term)
+{
+    if constexpr (TABLE)
+    {
+        extern __shared__ __align__(1024) unsigned char gg_dyn[];
+        const PushTable<T> table(gg_dyn + PUSH_STAGE, tags, out);
+        PushOp<T, PushTable<T>, Row, Term> op{table, row, term};
+        uint32_t *st = reinterpret_cast<uint32_t *>(gg_dyn) + (threadIdx.x >> 5) * (2 * GG_TILE_ITEMS + 12);
+        warp_push_staged<GG_TILE_IPT, PUSH_WARPS>(st, st + GG_TILE_ITEMS + 8, off, adj, V, coord, ntiles, op);
+        table.flush();
+    }
+    else
+    {
+        PushOp<T, PushDirect<T>, Row, Term> op{PushDirect<T>{out}, row, term};
+        warp_push<GG_TILE_IPT, GG_TILE_WARPS>(off, adj, V, coord, ntiles, op);
     }
 }
 

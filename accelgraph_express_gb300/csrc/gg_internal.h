@@ -120,6 +120,9 @@ struct gg_graph
     uint32_t *hot_list = nullptr;  /* GG_HOT_ENTRIES slots, then the counts (hot_taken) */
     uint32_t hot_slots = 0;        /* slots there are: hot_cap, or V if that is less */
     uint32_t hot_cap = 0;          /* table capacity the encoding was made for */
+    uint32_t *push_tags = nullptr; /* frequent destinations (gg_push_tags) */
+    bool push_hubs = false;        /* they are frequent enough for the table */
+    uint64_t push_edges = 0;       /* edges scattered without them */
     uint64_t plain_its = 0;        /* gathers done without the table since it was last made */
     uint32_t *hot_seg0 = nullptr;  /* per tile of hot_tile edges: its first row end (gg_hot.cuh) */
     uint32_t hot_ntiles = 0, hot_tile = 0; /* tiles and edges per tile */
@@ -279,6 +282,19 @@ int gg_sm_count();
  * sets the kernel's shared-memory carve-out to just hold them, so the rest
  * of each SM's combined L1/shared array caches the gathered values. */
 int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm = 0);
+/* Push scatters through a table of frequent destinations (push.cu,
+ * gg_device.cuh) */
+#define PUSH_LOG 12
+#define PUSH_WARPS 16
+#define PUSH_NT (32 * PUSH_WARPS)
+#define PUSH_SLOTS (1u << PUSH_LOG)
+/* a destination's slot */
+#define GG_PUSH_HASH 0x9E3779B1u
+/* the destinations of the PUSH_SLOTS slots for a call of `iterations` scatters
+ * over the out-CSR; null when the table would not pay (or not yet) */
+gg_status gg_push_tags(gg_graph *g, uint32_t iterations, cudaStream_t s, const uint32_t **tags);
+/* its kernel's blocks (smem bytes of dynamic shared memory, set here too) */
+int gg_push_grid(const void *kernel, uint32_t ntiles, size_t smem);
 /* resident blocks per SM of `kernel` at this block size and dynamic shared
  * memory (cudaOccupancyMaxActiveBlocksPerMultiprocessor, remembered; 0 on
  * failure); for kernels whose attributes do not change between launches */

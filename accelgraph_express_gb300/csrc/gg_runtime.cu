@@ -116,6 +116,15 @@ int gg_occupancy(const void *kernel, int threads, size_t smem)
     return bps;
 }
 
+int gg_push_grid(const void *kernel, uint32_t ntiles, size_t smem)
+{
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) cudaGetLastError();
+    const int per_sm = gg_occupancy(kernel, PUSH_NT, smem);
+    const int cap = gg_sm_count() * (per_sm > 0 ? per_sm : 1);
+    const uint32_t need = ntiles / PUSH_WARPS + 1;
+    return need < (uint32_t)cap ? (int)need : cap;
+}
+
 int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm)
 {
     /* per (kernel, requested CTAs per SM): the resident CTAs per SM and the
@@ -1129,6 +1138,7 @@ extern "C" gg_status gg_graph_unmap(gg_graph *g)
     free_tiles(g, g->out_tiles, idle);
     dev_release(g, g->rows_list, ((size_t)g->V + GG_ROW_PAD + 4) * 4, idle);
     dev_release(g, g->ppr_seg0, (size_t)g->ppr_ntiles * 4, idle);
+    dev_release(g, g->push_tags, (PUSH_SLOTS + 4) * 4, idle);
     dev_release(g, g->hot_adj, ((size_t)g->E + GG_EDGE_PAD) * 4, idle);
     dev_release(g, g->hot_list, GG_HOT_LIST_BYTES, idle);
     dev_release(g, g->hot_seg0, (size_t)g->hot_ntiles * 4, idle);

@@ -430,65 +430,46 @@ __global__ void k_pr_finalize_seg(float *__restrict__ rank, uint32_t V, const ui
 
 /* ---- push: scatter + vertex update ---------------------------------------------- */
 
-template <int K>
-__global__ void __launch_bounds__(GG_TILE_NT) k_pr_push_f(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
-                                                          const uint2 *__restrict__ coord, uint32_t ntiles, uint32_t V,
-                                                          const typename Fmt<K>::CT *cin, float *next,
-                                                          IterRec *rec, uint32_t it)
+/* TABLE: with the frequent destinations in shared memory (push.cu) */
+template <int K, bool TABLE>
+__global__ void __launch_bounds__(TABLE ? PUSH_NT : GG_TILE_NT)
+    k_pr_push_f(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj, const uint2 *__restrict__ coord,
+                uint32_t ntiles, uint32_t V, const uint32_t *__restrict__ tags, const typename Fmt<K>::CT *cin,
+                float *next, IterRec *rec, uint32_t it)
 {
     if (it > 0 && rec[it - 1].active == 0u) return;
-    struct Op
-    {
-        typedef float RowVal;
-        const typename Fmt<K>::CT *cin;
-        float *next;
-        __device__ __forceinline__ float row_value(uint32_t r) const { return to_f32(cin[r]); }
-        __device__ __forceinline__ void scatter(float rv, uint32_t, uint32_t dst) const { atomicAdd(&next[dst], rv); }
-    } op{cin, next};
-    warp_push<GG_TILE_IPT, GG_TILE_WARPS>(off, adj, V, coord, ntiles, op);
+    push_scatter<TABLE>(
+        off, adj, V, coord, ntiles, tags, next, [=](uint32_t r) -> float { return to_f32(cin[r]); },
+        [](float v, uint32_t) { return v; });
 }
 
-__global__ void __launch_bounds__(GG_TILE_NT) k_pr_push_fx64(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
-                                                             const uint2 *__restrict__ coord, uint32_t ntiles, uint32_t V,
-                                                             const unsigned long long *cin, unsigned long long *next,
-                                                             IterRec *rec, uint32_t it)
+template <bool TABLE>
+__global__ void __launch_bounds__(TABLE ? PUSH_NT : GG_TILE_NT)
+    k_pr_push_fx64(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj, const uint2 *__restrict__ coord,
+                   uint32_t ntiles, uint32_t V, const uint32_t *__restrict__ tags, const unsigned long long *cin,
+                   unsigned long long *next, IterRec *rec, uint32_t it)
 {
     if (it > 0 && rec[it - 1].active == 0u) return;
-    struct Op
-    {
-        typedef unsigned long long RowVal;
-        const unsigned long long *cin;
-        unsigned long long *next;
-        __device__ __forceinline__ unsigned long long row_value(uint32_t r) const { return cin[r]; }
-        __device__ __forceinline__ void scatter(unsigned long long rv, uint32_t, uint32_t dst) const
-        {
-            atomicAdd(&next[dst], rv);
-        }
-    } op{cin, next};
-    warp_push<GG_TILE_IPT, GG_TILE_WARPS>(off, adj, V, coord, ntiles, op);
+    push_scatter<TABLE>(
+        off, adj, V, coord, ntiles, tags, next, [=](uint32_t r) -> unsigned long long { return cin[r]; },
+        [](unsigned long long v, uint32_t) { return v; });
 }
 
-__global__ void __launch_bounds__(GG_TILE_NT) k_pr_push_q(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
-                                                          const uint2 *__restrict__ coord, uint32_t ntiles, uint32_t V,
-                                                          const uint8_t *q, const uint32_t *zeros, float *next,
-                                                          IterRec *rec, uint32_t it)
+/* without the table: a sum in another order than the reference's moves the
+ * scale by an ulp, and with it whole groups of equal ranks to another step of
+ * the 8 bits */
+__global__ void __launch_bounds__(GG_TILE_NT)
+    k_pr_push_q(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj, const uint2 *__restrict__ coord,
+                uint32_t ntiles, uint32_t V, const uint8_t *q, const uint32_t *zeros, float *next, IterRec *rec, uint32_t it)
 {
     if (it > 0 && rec[it - 1].active == 0u) return;
-    struct Op
-    {
-        typedef float RowVal;
-        const uint8_t *q;
-        float scale;
-        uint32_t zero;
-        float *next;
-        /* pageRank.c:2753: scale * (q - zero) */
-        __device__ __forceinline__ float row_value(uint32_t r) const
-        {
-            return __fmul_rn(scale, (float)((long long)q[r] - (long long)zero));
-        }
-        __device__ __forceinline__ void scatter(float rv, uint32_t, uint32_t dst) const { atomicAdd(&next[dst], rv); }
-    } op{q, quant_scale(rec[it].maxbits, 8), zeros[it], next};
-    warp_push<GG_TILE_IPT, GG_TILE_WARPS>(off, adj, V, coord, ntiles, op);
+    const float scale = quant_scale(rec[it].maxbits, 8);
+    const uint32_t zero = zeros[it];
+    /* pageRank.c:2753: scale * (q - zero) */
+    push_scatter<false>(
+        off, adj, V, coord, ntiles, nullptr, next,
+        [=](uint32_t r) -> float { return __fmul_rn(scale, (float)((long long)q[r] - (long long)zero)); },
+        [](float v, uint32_t) { return v; });
 }
 
 /* vertex update from the gathered (pull) or scattered (push) sums
@@ -908,6 +889,7 @@ struct Run
     const gg_pr_params *p;
     float eps_f = 0.0f, eps_fl = 0.0f;
     bool use_hot = false; /* pull gather through the hot-vertex table */
+    const uint32_t *push_tags = nullptr; /* push scatter through the table of frequent destinations */
     bool small = false;   /* every iteration in one cluster (small.cu) */
     gg_pull_shape shape;  /* launch shape of the FP pull gather */
     uint32_t launches = 0;
@@ -1037,6 +1019,16 @@ gg_status run_pull(Run &R, IterRec *rec, float *rank, uint32_t iters, float base
     return GG_OK;
 }
 
+/* a push scatter: `with` the table of frequent destinations or `without` */
+template <class... P, class... A>
+void launch_push(Run &R, uint32_t ntiles, void (*with)(P...), void (*without)(P...), size_t smem, A... args)
+{
+    if (R.push_tags)
+        with<<<gg_push_grid((const void *)with, ntiles, smem), PUSH_NT, smem, R.s>>>(args...);
+    else
+        without<<<gg_persistent_grid((const void *)without, ntiles), GG_TILE_NT, 0, R.s>>>(args...);
+}
+
 template <int K>
 gg_status run_push(Run &R, IterRec *rec, float *rank, uint32_t iters, float base, float init)
 {
@@ -1080,22 +1072,21 @@ gg_status run_push(Run &R, IterRec *rec, float *rank, uint32_t iters, float base
             k_quantize<uint8_t, true><<<grid_v(V), 256, 0, R.s>>>((const float *)cf, (uint8_t *)c0, V, rec, it,
                                                                   (uint32_t *)zeros);
             k_pr_push_q<<<gg_persistent_grid((const void *)k_pr_push_q, t->ntiles), GG_TILE_NT, 0, R.s>>>(
-                g->out_off, g->out_adj, t->coord, t->ntiles, V, (const uint8_t *)c0,
-                                                           (const uint32_t *)zeros, (float *)nx, rec, it);
+                g->out_off, g->out_adj, t->coord, t->ntiles, V, (const uint8_t *)c0, (const uint32_t *)zeros, (float *)nx, rec,
+                it);
             R.launches += 2;
         }
         else if constexpr (K == K_FX64)
         {
-            k_pr_push_fx64<<<gg_persistent_grid((const void *)k_pr_push_fx64, t->ntiles), GG_TILE_NT, 0, R.s>>>(
-                g->out_off, g->out_adj, t->coord, t->ntiles, V,
-                                                              (const unsigned long long *)c0, (unsigned long long *)nx, rec, it);
+            launch_push(R, t->ntiles, k_pr_push_fx64<true>, k_pr_push_fx64<false>, push_smem<unsigned long long>(),
+                        g->out_off, g->out_adj, t->coord, t->ntiles, V, R.push_tags, (const unsigned long long *)c0,
+                        (unsigned long long *)nx, rec, it);
             R.launches++;
         }
         else
         {
-            k_pr_push_f<K><<<gg_persistent_grid((const void *)k_pr_push_f<K>, t->ntiles), GG_TILE_NT, 0, R.s>>>(
-                g->out_off, g->out_adj, t->coord, t->ntiles, V, (const CT *)c0,
-                                                              (float *)nx, rec, it);
+            launch_push(R, t->ntiles, k_pr_push_f<K, true>, k_pr_push_f<K, false>, push_smem<float>(), g->out_off,
+                        g->out_adj, t->coord, t->ntiles, V, R.push_tags, (const CT *)c0, (float *)nx, rec, it);
             R.launches++;
         }
         GG_CHECK(timed_end(R));
@@ -1430,6 +1421,9 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
         }
     }
 
+    if (p->mode == GG_PR_PUSH || p->mode == GG_PR_PUSH_FX64)
+        GG_CHECK(gg_push_tags(g, iters, R.s, &R.push_tags));
+
     /* a graph of up to 2.5M edges and 262K vertices: every iteration in one
      * launch, faster at every size it takes (small.cu); timed runs time each gather launch, and a table asked
      * for is used */
@@ -1448,7 +1442,7 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
     {
         struct Key
         {
-            uint32_t mode, storage, iters, init, flags, ngraphs, use_hot, V, E, ctas, hot_warps;
+            uint32_t mode, storage, iters, init, flags, ngraphs, use_hot, V, E, ctas, hot_warps, push;
             float damp;
             double eps;
         } key;
@@ -1456,7 +1450,7 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
         memset(&key, 0, sizeof(key));
         key.mode = p->mode; key.storage = p->storage; key.iters = iters; key.init = p->init_one_over_n;
         key.flags = p->flags; key.ngraphs = ngraphs; key.use_hot = R.use_hot ? 1u : 0u; key.V = V; key.E = g->E;
-        key.ctas = R.shape.ctas; key.hot_warps = R.shape.hot_warps;
+        key.ctas = R.shape.ctas; key.hot_warps = R.shape.hot_warps; key.push = R.push_tags ? 1u : 0u;
         key.damp = p->damp; key.eps = p->epsilon;
         if (g->pr_exec && g->pr_gen == g->mem_gen && memcmp(g->pr_key, &key, sizeof(key)) == 0)
         {

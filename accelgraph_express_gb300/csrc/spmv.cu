@@ -123,44 +123,26 @@ __global__ void k_spmv_fx_pull_out(unsigned long long *y64, float *y, uint32_t V
     }
 }
 
-template <class T>
-__global__ void __launch_bounds__(GG_TILE_NT) k_spmv_push(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
-                                                          const uint2 *__restrict__ coord, uint32_t ntiles, uint32_t V,
-                                                          const T *w, const T *x, float *y)
+/* TABLE: with the frequent destinations in shared memory (push.cu) */
+template <class T, bool TABLE>
+__global__ void __launch_bounds__(TABLE ? PUSH_NT : GG_TILE_NT)
+    k_spmv_push(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj, const uint2 *__restrict__ coord,
+                uint32_t ntiles, uint32_t V, const uint32_t *__restrict__ tags, const T *w, const T *x, float *y)
 {
-    struct Op
-    {
-        typedef float RowVal;
-        const T *w;
-        const T *x;
-        float *y;
-        __device__ __forceinline__ float row_value(uint32_t r) const { return to_f32(x[r]); }
-        __device__ __forceinline__ void scatter(float xv, uint32_t e, uint32_t dst) const
-        {
-            atomicAdd(&y[dst], __fmul_rn(to_f32(w[e]), xv));
-        }
-    } op{w, x, y};
-    warp_push<GG_TILE_IPT, GG_TILE_WARPS>(off, adj, V, coord, ntiles, op);
+    push_scatter<TABLE>(
+        off, adj, V, coord, ntiles, tags, y, [=](uint32_t r) -> float { return to_f32(x[r]); },
+        [=](float xv, uint32_t e) { return __fmul_rn(to_f32(w[e]), xv); });
 }
 
-__global__ void __launch_bounds__(GG_TILE_NT) k_spmv_push_fx(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
-                                                             const uint2 *__restrict__ coord, uint32_t ntiles, uint32_t V,
-                                                             const float *w, const unsigned long long *x64,
-                                                             unsigned long long *y64)
+template <bool TABLE>
+__global__ void __launch_bounds__(TABLE ? PUSH_NT : GG_TILE_NT)
+    k_spmv_push_fx(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj, const uint2 *__restrict__ coord,
+                   uint32_t ntiles, uint32_t V, const uint32_t *__restrict__ tags, const float *w,
+                   const unsigned long long *x64, unsigned long long *y64)
 {
-    struct Op
-    {
-        typedef unsigned long long RowVal;
-        const float *w;
-        const unsigned long long *x64;
-        unsigned long long *y64;
-        __device__ __forceinline__ unsigned long long row_value(uint32_t r) const { return x64[r]; }
-        __device__ __forceinline__ void scatter(unsigned long long xv, uint32_t e, uint32_t dst) const
-        {
-            atomicAdd(&y64[dst], fx64_mul(fx64_from_float(w[e]), xv));
-        }
-    } op{w, x64, y64};
-    warp_push<GG_TILE_IPT, GG_TILE_WARPS>(off, adj, V, coord, ntiles, op);
+    push_scatter<TABLE>(
+        off, adj, V, coord, ntiles, tags, y64, [=](uint32_t r) -> unsigned long long { return x64[r]; },
+        [=](unsigned long long xv, uint32_t e) { return fx64_mul(fx64_from_float(w[e]), xv); });
 }
 
 /* x[v] = 1/outdeg(v), or 0.001 when 0 (SPMV.c:696-701), unless given; the
@@ -269,6 +251,8 @@ gg_status spmv_fp(gg_graph *g, const gg_spmv_params *p, const float *x_dev, floa
         launches++;
         use_hot = true;
     }
+    const uint32_t *tags = nullptr;
+    if (!pull) GG_CHECK(gg_push_tags(g, p->iterations, s, &tags));
     for (uint32_t it = 0; it < p->iterations; it++)
     {
         if (p->profile)
@@ -292,8 +276,14 @@ gg_status spmv_fp(gg_graph *g, const gg_spmv_params *p, const float *x_dev, floa
                                  GG_TILE_NT, 0, s>>>(g->in_off, g->in_adj, t->coord, t->ntiles, V, y, SpmvGather<T>{w, xv});
         }
         else
-            k_spmv_push<T><<<gg_persistent_grid((const void *)k_spmv_push<T>, t->ntiles), GG_TILE_NT, 0, s>>>(
-                g->out_off, g->out_adj, t->coord, t->ntiles, V, w, xv, y);
+        {
+            if (tags)
+                k_spmv_push<T, true><<<gg_push_grid((const void *)k_spmv_push<T, true>, t->ntiles, push_smem<float>()), PUSH_NT,
+                                       push_smem<float>(), s>>>(g->out_off, g->out_adj, t->coord, t->ntiles, V, tags, w, xv, y);
+            else
+                k_spmv_push<T, false><<<gg_persistent_grid((const void *)k_spmv_push<T, false>, t->ntiles), GG_TILE_NT, 0, s>>>(
+                    g->out_off, g->out_adj, t->coord, t->ntiles, V, tags, w, xv, y);
+        }
         if (p->profile)
         {
             cudaEvent_t e;
@@ -361,6 +351,8 @@ extern "C" gg_status gg_spmv(gg_graph *g, const gg_spmv_params *p, const float *
                                                       pull ? (uint32_t *)xq : nullptr,
                                                       pull ? nullptr : (unsigned long long *)xq, (float *)yv, V);
             launches++;
+            const uint32_t *tags = nullptr;
+            if (!pull) GG_CHECK(gg_push_tags(g, p->iterations, s, &tags));
             for (uint32_t it = 0; it < p->iterations; it++)
             {
                 if (p->profile)
@@ -379,9 +371,17 @@ extern "C" gg_status gg_spmv(gg_graph *g, const gg_spmv_params *p, const float *
                     launches++;
                 }
                 else
-                    k_spmv_push_fx<<<gg_persistent_grid((const void *)k_spmv_push_fx, t->ntiles), GG_TILE_NT, 0, s>>>(
-                        g->out_off, g->out_adj, t->coord, t->ntiles, V, g->out_w, (const unsigned long long *)xq,
-                        (unsigned long long *)y64);
+                {
+                    constexpr size_t smem = push_smem<unsigned long long>();
+                    if (tags)
+                        k_spmv_push_fx<true><<<gg_push_grid((const void *)k_spmv_push_fx<true>, t->ntiles, smem), PUSH_NT, smem, s>>>(
+                            g->out_off, g->out_adj, t->coord, t->ntiles, V, tags, g->out_w, (const unsigned long long *)xq,
+                            (unsigned long long *)y64);
+                    else
+                        k_spmv_push_fx<false><<<gg_persistent_grid((const void *)k_spmv_push_fx<false>, t->ntiles), GG_TILE_NT, 0, s>>>(
+                            g->out_off, g->out_adj, t->coord, t->ntiles, V, tags, g->out_w, (const unsigned long long *)xq,
+                            (unsigned long long *)y64);
+                }
                 if (p->profile)
                 {
                     cudaEvent_t e;
