@@ -706,21 +706,18 @@ __device__ __forceinline__ void push_scatter(const uint32_t *__restrict__ off, c
 
 /*
  * Grid-wide barrier over the co-resident blocks of a cooperative launch, on
- * a control block `ctl` of GG_BAR_BYTES zeroed before the launch: the root
- * counter at 512, per group of blocks an arrival counter at 1024 + 128 g and
- * a release word at 4096 + 128 g (separate 128-byte lines, so the spinning
- * blocks of one group do not queue behind the arrivals or the other groups
- * at one L2 slice).  Two levels: blocks arrive at their group's counter, the
- * last of a group at the root, and the last at the root releases every
- * group.  The counters only grow (barrier `gen` completes a group at
- * (gen + 1) * group size arrivals and the root at (gen + 1) * groups), so
- * no arrival waits for a counter to be reset.  Ordering: each block's
- * writes are fenced before it arrives, the last arrivers fence before
- * passing on, and every block fences after it is released.  A wait gives up
- * after limit_ns (globaltimer) and sets *err; the block then reports false
- * and the caller leaves, so the other blocks give up at their next barrier
- * and the launch ends with *err set, the context intact.  Bytes 0..511 of
- * ctl are the caller's.
+ * a control block `ctl` of GG_BAR_BYTES zeroed before the launch: an arrival
+ * counter per group of blocks, at 1024 + 128 g (a 128-byte line each: one
+ * address takes an addition every 5 ns).  A block adds to its group's counter
+ * and the lanes of its first warp each poll one group's: two memory round trips
+ * (MEASURED_BAR).  The counters only grow (barrier `gen` completes a group
+ * at (gen + 1) * group size arrivals), so no arrival waits for a counter to be
+ * reset.  Ordering: the addition releases the block's writes, which the block
+ * barrier before it has gathered; the polls acquire, and the block barrier
+ * after them hands that on.  A wait gives up after limit_ns (globaltimer) and
+ * sets *err; the block then reports false and the caller leaves, so the other
+ * blocks give up at their next barrier and the launch ends with *err set, the
+ * context intact.  Bytes 0..1023 of ctl are the caller's.
  */
 constexpr unsigned int GG_BAR_GROUPS = 16;
 
@@ -736,43 +733,32 @@ __device__ __forceinline__ bool grid_barrier(char *ctl, unsigned int *err, unsig
 {
     __shared__ unsigned int s_ok;
     __syncthreads();
-    if (threadIdx.x == 0)
+    if (threadIdx.x < 32)
     {
-        unsigned int *root = (unsigned int *)(ctl + 512);
+        const unsigned int lane = threadIdx.x;
         const unsigned int G = gridDim.x < GG_BAR_GROUPS ? gridDim.x : GG_BAR_GROUPS;
-        const unsigned int grp = blockIdx.x % G;
-        const unsigned int gsize = (gridDim.x - grp + G - 1) / G;
-        unsigned int *count = (unsigned int *)(ctl + 1024 + 128 * grp);
-        unsigned int *rel = (unsigned int *)(ctl + 4096 + 128 * grp);
-        const unsigned int target = gen + 1;
-        bool released = false, ok = true;
-        __threadfence();
-        if (atomicAdd(count, 1u) == target * gsize - 1)
+        if (lane == 0)
+            asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(ctl + 1024 + 128 * (blockIdx.x % G)), "r"(1u)
+                         : "memory");
+        const char *word = ctl + 1024 + 128 * lane;
+        const unsigned int want = lane < G ? (gen + 1) * ((gridDim.x - lane + G - 1) / G) : 0u;
+        bool ok = true;
+        const unsigned long long t0 = global_ns();
+        for (;;)
         {
-            __threadfence();
-            if (atomicAdd(root, 1u) == target * G - 1)
+            unsigned int v = want;
+            if (lane < G) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
+            /* a counter past `want` has arrivals at the next barrier already */
+            if (__all_sync(0xffffffffu, (int)(v - want) >= 0)) break;
+            __nanosleep(20);
+            if (__shfl_sync(0xffffffffu, global_ns() - t0, 0) > limit_ns)
             {
-                __threadfence();
-                for (unsigned int k = 0; k < G; k++) atomicExch((unsigned int *)(ctl + 4096 + 128 * k), target);
-                released = true;
+                if (lane == 0) atomicExch(err, 1u);
+                ok = false;
+                break;
             }
         }
-        if (!released)
-        {
-            const unsigned long long t0 = global_ns();
-            while (*(volatile unsigned int *)rel != target)
-            {
-                if (global_ns() - t0 > limit_ns)
-                {
-                    atomicExch(err, 1u);
-                    ok = false;
-                    break;
-                }
-                __nanosleep(32);
-            }
-        }
-        __threadfence();
-        s_ok = ok ? 1u : 0u;
+        if (lane == 0) s_ok = ok ? 1u : 0u;
     }
     __syncthreads();
     gen++;

@@ -307,7 +307,7 @@ int gg_occupancy(const void *kernel, int threads, size_t smem);
 #define GG_PULL_CTAS_PER_SM 5
 
 /* control block bytes of gg::grid_barrier (gg_device.cuh) */
-#define GG_BAR_BYTES (4096 + 128 * 16)
+#define GG_BAR_BYTES (1024 + 128 * 16)
 /* device-side wait limit of the grid barriers, in ns (gg_set_barrier_limit_us) */
 unsigned long long gg_barrier_limit_ns();
 

@@ -888,8 +888,16 @@ gg_status round_run(gg_graph *g, const gg_ppr_round_args &r, cudaStream_t s)
  * span tiles). */
 uint32_t gg_ppr_tile(const gg_graph *g)
 {
-    if (g->ppr_tile) return g->ppr_tile;
-    return g->E < 4u * 512u * (uint32_t)(PPR_CTAS * PPR_WARPS) * (uint32_t)gg_sm_count() ? 256u : 512u;
+    const uint32_t warps = (uint32_t)(PPR_CTAS * PPR_WARPS) * (uint32_t)gg_sm_count();
+    uint32_t tile = g->ppr_tile;
+    if (!tile)
+    {
+        tile = g->E < 4u * 512u * warps ? 256u : 512u;
+        while (tile > 32u && (uint64_t)(tile / 2) * warps >= g->E) tile /= 2;
+    }
+    /* below 256 only while every warp has one tile at most */
+    if (tile < 256u && (uint64_t)tile * warps < g->E) tile = 256u;
+    return tile;
 }
 
 gg_status gg_ppr_round_prepare(gg_graph *g, uint32_t rs, int bf16, void **cb0, void **cb1, float **slots,
