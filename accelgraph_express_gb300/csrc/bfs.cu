@@ -50,6 +50,8 @@ struct Counters
     uint32_t nf;     /* bottom-up: vertices found */
     uint32_t nheavy; /* top-down: frontier vertices deferred to k_td_heavy */
     unsigned long long edges;
+    uint32_t nhuge; /* k_td: those of its second list */
+    uint32_t pad;
 };
 
 constexpr int BU_SERIAL = 4;  /* in-neighbours a lane checks before the warp helps */
@@ -236,8 +238,29 @@ __device__ __forceinline__ void td_enqueue_local(bool claimed, uint32_t u, uint3
 
 /* frontier vertices with more out-edges than `heavy_thr` (64 by default,
  * the tuned value per mapping otherwise) go to k_td_heavy, at most
- * TD_MAX_HEAVY of them per step (further ones stay with their warp) */
+ * TD_MAX_HEAVY of them per step (further ones stay with their warp).  k_td
+ * has a second list for the ones past that with more than TD_HUGE edges: a
+ * step of a frontier with 30K vertices of over 64 edges otherwise leaves a
+ * hub's 40K to one warp (push of R-MAT-20 1600 -> 675 us, slowest source 4500
+ * -> 740; R-MAT-22 4900 -> 2040, 11000 -> 2180) */
 #define TD_MAX_HEAVY 4096u
+#define TD_HUGE 512u
+#define TD_MAX_HUGE 65536u
+
+/* k_td's place in the two lists for a vertex of `degree` edges, past both when
+ * it stays with its warp.  A full list is not counted further (an addition to
+ * one address every 5 ns) */
+__device__ __forceinline__ uint32_t td_heavy_slot(uint32_t degree, Counters *c)
+{
+    if (*(volatile uint32_t *)&c->nheavy < TD_MAX_HEAVY)
+    {
+        const uint32_t slot = atomicAdd(&c->nheavy, 1u);
+        if (slot < TD_MAX_HEAVY) return slot;
+    }
+    if (degree <= TD_HUGE) return 0xffffffffu;
+    const uint32_t slot = atomicAdd(&c->nhuge, 1u);
+    return slot < TD_MAX_HUGE ? TD_MAX_HEAVY + slot : 0xffffffffu;
+}
 
 /* LOCAL: claims through the block's local queue.  Not inside the single-launch
  * search, where its registers made the bottom-up steps spill: a search of
@@ -267,9 +290,14 @@ __device__ __forceinline__ void td_body(const uint32_t *q, uint32_t qlen,
         if (e - s > heavy_thr)
         {
             uint32_t slot = 0;
-            if (lane == 0) slot = atomicAdd(&c->nheavy, 1u);
+            if constexpr (LOCAL)
+            {
+                if (lane == 0) slot = td_heavy_slot(e - s, c);
+            }
+            else if (lane == 0)
+                slot = atomicAdd(&c->nheavy, 1u);
             slot = __shfl_sync(0xffffffffu, slot, 0);
-            if (slot < TD_MAX_HEAVY)
+            if (slot < TD_MAX_HEAVY + (LOCAL ? TD_MAX_HUGE : 0u))
             {
                 if (lane == 0) heavy[slot] = make_uint4(v, s, e, 0u);
                 continue;
@@ -297,8 +325,10 @@ __device__ __forceinline__ void td_body(const uint32_t *q, uint32_t qlen,
 
 /* the deferred high-degree frontier vertices: their out-edges, concatenated,
  * are split evenly over the whole grid; every CTA scans the list's degrees
- * in shared memory and maps an edge index to its vertex by binary search */
-__device__ __forceinline__ void td_heavy_body(const uint4 *heavy, const uint32_t *__restrict__ adj,
+ * in shared memory and maps an edge index to its vertex by binary search.
+ * count, skip: the list's length, of which `skip` lie before `heavy` */
+__device__ __forceinline__ void td_heavy_body(const uint4 *heavy, const uint32_t *count, uint32_t skip,
+                                              const uint32_t *__restrict__ adj,
                                               int32_t *parents, uint32_t *dist, uint32_t newdist,
                                               uint32_t *visited, uint32_t *nq, uint32_t *nbm, Counters *c)
 {
@@ -308,7 +338,7 @@ __device__ __forceinline__ void td_heavy_body(const uint4 *heavy, const uint32_t
     __shared__ LocalQueue L;
     if (threadIdx.x == 0)
     {
-        s_nh = min(*(volatile uint32_t *)&c->nheavy, TD_MAX_HEAVY);
+        s_nh = min(*(volatile const uint32_t *)count - skip, TD_MAX_HEAVY);
         local_clear(L);
     }
     __syncthreads();
@@ -560,7 +590,14 @@ __global__ void __launch_bounds__(256) k_td_heavy(const uint4 *__restrict__ heav
                                                   int32_t *parents, uint32_t *dist, uint32_t newdist,
                                                   uint32_t *visited, uint32_t *nq, uint32_t *nbm, Counters *c)
 {
-    td_heavy_body(heavy, adj, parents, dist, newdist, visited, nq, nbm, c);
+    td_heavy_body(heavy, &c->nheavy, 0u, adj, parents, dist, newdist, visited, nq, nbm, c);
+    /* the second list lies behind the first */
+    const uint32_t more = min(*(volatile uint32_t *)&c->nhuge, TD_MAX_HUGE);
+    for (uint32_t at = 0; at < more; at += TD_MAX_HEAVY)
+    {
+        __syncthreads(); /* all have done with the block's queue */
+        td_heavy_body(heavy + TD_MAX_HEAVY + at, &c->nhuge, at, adj, parents, dist, newdist, visited, nq, nbm, c);
+    }
 }
 __global__ void __launch_bounds__(256) k_bu(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
                                             int32_t *parents, uint32_t *dist, int write_dist, uint32_t newdist,
@@ -589,12 +626,9 @@ __global__ void k_queue_to_bitmap(const uint32_t *__restrict__ q, uint32_t qlen,
  * last readers finished two barriers earlier. */
 
 /* control block of one search (work slot 7, CTL_BYTES, zeroed before the
- * launch): three counter slots at 0, the results at 256, the barrier's
- * root counter at 512, and per group of blocks an arrival counter at
- * 1024 + 128 g and a release word at 4096 + 128 g -- separate 128-byte
- * lines, so the spinning blocks of one group do not queue behind the
- * arrivals or the other groups at one L2 slice */
-constexpr size_t CTL_BYTES = 8192;
+ * launch): three counter slots at 0, the results at 512, the barrier's
+ * arrival counters behind (gg_device.cuh) */
+constexpr size_t CTL_BYTES = GG_BAR_BYTES;
 
 struct DoOut
 {
@@ -619,7 +653,7 @@ struct DoArgs
  * recorded in DoOut::err */
 __device__ __forceinline__ bool grid_barrier(char *ctl, unsigned long long limit_ns, unsigned int &gen)
 {
-    return gg::grid_barrier(ctl, &((DoOut *)(ctl + 256))->err, limit_ns, gen);
+    return gg::grid_barrier(ctl, &((DoOut *)(ctl + 512))->err, limit_ns, gen);
 }
 
 /* one read of a counter slot per block, shared with its threads */
@@ -716,7 +750,7 @@ __global__ void __launch_bounds__(256, 6) k_bfs_do(DoArgs a)
              * block reads the same final count, so all skip together) */
             if (read_counters_block(cs).nheavy)
             {
-                td_heavy_body(a.heavy, a.out_adj, a.parents, a.dist, level + 1, a.visited, a.q[qcur ^ 1], nullptr,
+                td_heavy_body(a.heavy, &cs->nheavy, 0u, a.out_adj, a.parents, a.dist, level + 1, a.visited, a.q[qcur ^ 1], nullptr,
                               cs);
                 if (!(ok = grid_barrier(a.ctl, a.bar_limit_ns, gen))) break;
             }
@@ -733,7 +767,7 @@ __global__ void __launch_bounds__(256, 6) k_bfs_do(DoArgs a)
     }
     if (blockIdx.x == 0 && threadIdx.x == 0)
     {
-        DoOut *out = (DoOut *)(a.ctl + 256);
+        DoOut *out = (DoOut *)(a.ctl + 512);
         out->processed = processed;
         out->levels = level;
         out->td = td;
@@ -857,9 +891,9 @@ gg_status bfs_setup(Bfs &B, gg_graph *g, void *stream, int profile)
     GG_CHECK(gg_work(g, 6, wb, &p)); B.visited = (uint32_t *)p;
     GG_CHECK(gg_work(g, 7, CTL_BYTES, &p)); B.c = (Counters *)p;
     GG_CHECK(gg_pinned(g, 256, &p)); B.h = (Counters *)p;
-    static_assert(3 * sizeof(Counters) <= 256 && sizeof(DoOut) <= 256 && GG_BAR_BYTES <= CTL_BYTES,
+    static_assert(3 * sizeof(Counters) <= 512 && sizeof(DoOut) <= 512 && GG_BAR_BYTES <= CTL_BYTES,
                   "control layout");
-    GG_CHECK(gg_work(g, 8, (size_t)TD_MAX_HEAVY * sizeof(uint4), &p)); B.heavy = (uint4 *)p;
+    GG_CHECK(gg_work(g, 8, (size_t)(TD_MAX_HEAVY + TD_MAX_HUGE) * sizeof(uint4), &p)); B.heavy = (uint4 *)p;
     return GG_OK;
 }
 
@@ -901,8 +935,8 @@ gg_status do_search(Bfs &B, const gg_bfs_params *p)
     void *args[] = {&a};
     GG_CUDA(cudaLaunchCooperativeKernel((const void *)k_bfs_do, dim3(gg_sm_count() * per_sm), dim3(256), args, 0, B.s));
     B.launches++;
-    DoOut *h = (DoOut *)((char *)B.h + 64);
-    GG_CUDA(cudaMemcpyAsync(h, ctl + 256, sizeof(DoOut), cudaMemcpyDeviceToHost, B.s));
+    DoOut *h = (DoOut *)((char *)B.h + 128);
+    GG_CUDA(cudaMemcpyAsync(h, ctl + 512, sizeof(DoOut), cudaMemcpyDeviceToHost, B.s));
     GG_CHECK(gg_wait(B.s));
     if (h->err) return gg_fail(GG_ERR_KERNEL, "BFS grid barrier timed out");
     B.res.processed_nodes = h->processed;

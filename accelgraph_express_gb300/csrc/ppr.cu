@@ -885,7 +885,9 @@ gg_status round_run(gg_graph *g, const gg_ppr_round_args &r, cudaStream_t s)
  * so a graph of few tiles per warp (3,040 resident) ends with the slowest:
  * 256 below four 512-edge tiles per warp (R-MAT-16, K = 64
  * BF16: 96 -> 78 us an iteration), 512 above (fewer rows
- * span tiles). */
+ * span tiles).  Down to 32 while every warp has one tile at most (K = 16 FP32, 20
+ * iterations: 32K R-MAT edges 351 us, 320K 962 -> 722): the gather asks for rows a
+ * few chunks ahead, past a next tile of so few only if there is none. */
 uint32_t gg_ppr_tile(const gg_graph *g)
 {
     const uint32_t warps = (uint32_t)(PPR_CTAS * PPR_WARPS) * (uint32_t)gg_sm_count();

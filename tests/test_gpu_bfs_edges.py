@@ -53,3 +53,23 @@ def test_two_levels_of_many_claims(gpu, mids, each):
         np.testing.assert_array_equal(dist, want)
         np.testing.assert_array_equal(parents, parent)
         assert res["processed_nodes"] == V
+
+
+@pytest.mark.parametrize("hubs,degree", [(4200, 65), (4096, 600), (4097, 513), (9000, 520)])
+def test_more_hubs_than_the_first_list(gpu, orc, hubs, degree):
+    """A frontier of `hubs` vertices with `degree` edges each, past the first
+    list's 4,096 and the second's chunks of as many."""
+    rng = np.random.default_rng(hubs)
+    V = 60000
+    a = np.concatenate([np.zeros(hubs, np.int64), np.repeat(np.arange(1, hubs + 1), degree)])
+    b = np.concatenate([np.arange(1, hubs + 1), rng.integers(hubs + 1, V, hubs * degree)])
+    g, o = pair(gpu, orc, gpu.Graph.from_edges(a.astype(np.uint32), b.astype(np.uint32), num_vertices=V))
+    dg = gpu.DeviceGraph(g, gpu.MAP_IN | gpu.MAP_OUT)
+    for mode, om in (("push", 1), ("push_bitmap", 3), ("do", 2)):
+        parents, dist, res = dg.bfs(0, mode)
+        _, rd, info = orc.bfs(o, om, 0)
+        np.testing.assert_array_equal(dist, rd)
+        assert res["processed_nodes"] == info["processed_nodes"]
+        reached = np.flatnonzero((parents >= 0) & (np.arange(V) != 0))
+        assert (dist[parents[reached]] + 1 == dist[reached]).all()
+    dg.free()
