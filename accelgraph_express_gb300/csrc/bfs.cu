@@ -239,7 +239,8 @@ __device__ __forceinline__ void td_enqueue_local(bool claimed, uint32_t u, uint3
 /* frontier vertices with more out-edges than `heavy_thr` (64 by default,
  * the tuned value per mapping otherwise) go to k_td_heavy, at most
  * TD_MAX_HEAVY of them per step (further ones stay with their warp).  k_td
- * has a second list for the ones past that with more than TD_HUGE edges: a
+ * has a second list, where the first may overflow, for the ones past that with
+ * more than TD_HUGE edges: a
  * step of a frontier with 30K vertices of over 64 edges otherwise leaves a
  * hub's 40K to one warp (push of R-MAT-20 1600 -> 675 us, slowest source 4500
  * -> 740; R-MAT-22 4900 -> 2040, 11000 -> 2180) */
@@ -248,24 +249,25 @@ __device__ __forceinline__ void td_enqueue_local(bool claimed, uint32_t u, uint3
 #define TD_MAX_HUGE 65536u
 
 /* k_td's place in the two lists for a vertex of `degree` edges, past both when
- * it stays with its warp.  A full list is not counted further (an addition to
- * one address every 5 ns) */
-__device__ __forceinline__ uint32_t td_heavy_slot(uint32_t degree, Counters *c)
+ * it stays with its warp.  A full list is not counted further by the block (an
+ * addition to one address every 5 ns) */
+__device__ __forceinline__ uint32_t td_heavy_slot(uint32_t degree, Counters *c, volatile bool *full)
 {
-    if (*(volatile uint32_t *)&c->nheavy < TD_MAX_HEAVY)
+    if (!*full)
     {
         const uint32_t slot = atomicAdd(&c->nheavy, 1u);
         if (slot < TD_MAX_HEAVY) return slot;
+        *full = true;
     }
     if (degree <= TD_HUGE) return 0xffffffffu;
     const uint32_t slot = atomicAdd(&c->nhuge, 1u);
     return slot < TD_MAX_HUGE ? TD_MAX_HEAVY + slot : 0xffffffffu;
 }
 
-/* LOCAL: claims through the block's local queue.  Not inside the single-launch
+/* HUGE: with the second list.  LOCAL: claims through the block's local queue.  Not inside the single-launch
  * search, where its registers made the bottom-up steps spill: a search of
  * R-MAT-22 lost 10 us while one of a graph without hubs won 55 */
-template <bool LOCAL>
+template <bool LOCAL, bool HUGE>
 __device__ __forceinline__ void td_body(const uint32_t *q, uint32_t qlen,
                                         const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
                                         int32_t *parents, uint32_t *dist, uint32_t newdist, uint32_t *visited,
@@ -277,9 +279,14 @@ __device__ __forceinline__ void td_body(const uint32_t *q, uint32_t qlen,
     uint32_t mf = 0;
     unsigned long long edges = 0;
     __shared__ LocalQueue L;
+    __shared__ bool s_full;
     if (LOCAL)
     {
-        if (threadIdx.x == 0) local_clear(L);
+        if (threadIdx.x == 0)
+        {
+            local_clear(L);
+            if (HUGE) s_full = false;
+        }
         __syncthreads();
     }
     for (uint32_t i = warp; i < qlen; i += nwarps)
@@ -290,14 +297,14 @@ __device__ __forceinline__ void td_body(const uint32_t *q, uint32_t qlen,
         if (e - s > heavy_thr)
         {
             uint32_t slot = 0;
-            if constexpr (LOCAL)
+            if constexpr (HUGE)
             {
-                if (lane == 0) slot = td_heavy_slot(e - s, c);
+                if (lane == 0) slot = td_heavy_slot(e - s, c, &s_full);
             }
             else if (lane == 0)
                 slot = atomicAdd(&c->nheavy, 1u);
             slot = __shfl_sync(0xffffffffu, slot, 0);
-            if (slot < TD_MAX_HEAVY + (LOCAL ? TD_MAX_HUGE : 0u))
+            if (slot < TD_MAX_HEAVY + (HUGE ? TD_MAX_HUGE : 0u))
             {
                 if (lane == 0) heavy[slot] = make_uint4(v, s, e, 0u);
                 continue;
@@ -578,25 +585,31 @@ __device__ __forceinline__ void q2bm_body(const uint32_t *q, uint32_t qlen, uint
     }
 }
 
+template <bool HUGE>
 __global__ void __launch_bounds__(256) k_td(const uint32_t *__restrict__ q, uint32_t qlen,
                                             const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
                                             int32_t *parents, uint32_t *dist, uint32_t newdist, uint32_t *visited,
                                             uint32_t *nq, uint32_t *nbm, Counters *c, uint4 *heavy,
                                             uint32_t heavy_thr)
 {
-    td_body<true>(q, qlen, off, adj, parents, dist, newdist, visited, nq, nbm, c, heavy, heavy_thr);
+    td_body<true, HUGE>(q, qlen, off, adj, parents, dist, newdist, visited, nq, nbm, c, heavy, heavy_thr);
 }
 __global__ void __launch_bounds__(256) k_td_heavy(const uint4 *__restrict__ heavy, const uint32_t *__restrict__ adj,
                                                   int32_t *parents, uint32_t *dist, uint32_t newdist,
                                                   uint32_t *visited, uint32_t *nq, uint32_t *nbm, Counters *c)
 {
     td_heavy_body(heavy, &c->nheavy, 0u, adj, parents, dist, newdist, visited, nq, nbm, c);
-    /* the second list lies behind the first */
+}
+/* k_td<true>'s second list, behind the first */
+__global__ void __launch_bounds__(256) k_td_huge(const uint4 *__restrict__ heavy, const uint32_t *__restrict__ adj,
+                                                 int32_t *parents, uint32_t *dist, uint32_t newdist,
+                                                 uint32_t *visited, uint32_t *nq, uint32_t *nbm, Counters *c)
+{
     const uint32_t more = min(*(volatile uint32_t *)&c->nhuge, TD_MAX_HUGE);
     for (uint32_t at = 0; at < more; at += TD_MAX_HEAVY)
     {
-        __syncthreads(); /* all have done with the block's queue */
         td_heavy_body(heavy + TD_MAX_HEAVY + at, &c->nhuge, at, adj, parents, dist, newdist, visited, nq, nbm, c);
+        __syncthreads(); /* all have done with the block's queue */
     }
 }
 __global__ void __launch_bounds__(256) k_bu(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
@@ -743,7 +756,7 @@ __global__ void __launch_bounds__(256, 6) k_bfs_do(DoArgs a)
             mu -= mf;
             Counters *cs = a.c + s % 3;
             clear_slot(a.c + (s + 1) % 3);
-            td_body<false>(a.q[qcur], qlen, a.out_off, a.out_adj, a.parents, a.dist, level + 1, a.visited, a.q[qcur ^ 1],
+            td_body<false, false>(a.q[qcur], qlen, a.out_off, a.out_adj, a.parents, a.dist, level + 1, a.visited, a.q[qcur ^ 1],
                     nullptr, cs, a.heavy, a.heavy_thr);
             if (!(ok = grid_barrier(a.ctl, a.bar_limit_ns, gen))) break;
             /* the deferred high-degree vertices, when there are any (every
@@ -826,11 +839,19 @@ gg_status td_step(Bfs &B, const uint32_t *q, uint32_t qlen, uint32_t *nq, uint32
     GG_CHECK(mark(B));
     if (qlen)
     {
-        k_td<<<cap_blocks((uint64_t)qlen * 32), 256, 0, B.s>>>(q, qlen, B.g->out_off, B.g->out_adj, B.parents, B.dist,
-                                                                newdist, B.visited, nq, nbm, B.c, B.heavy,
-                                                                B.g->bfs_heavy);
+        /* the second list only where the first may overflow: by the step's
+         * edges, the claims of the step before (the source has one vertex) */
+        const bool huge = qlen > TD_MAX_HEAVY && (uint64_t)B.h->mf > (uint64_t)TD_MAX_HEAVY * B.g->bfs_heavy;
+        (huge ? k_td<true> : k_td<false>)<<<cap_blocks((uint64_t)qlen * 32), 256, 0, B.s>>>(
+            q, qlen, B.g->out_off, B.g->out_adj, B.parents, B.dist, newdist, B.visited, nq, nbm, B.c, B.heavy, B.g->bfs_heavy);
         k_td_heavy<<<gg_sm_count() * 8, 256, 0, B.s>>>(B.heavy, B.g->out_adj, B.parents, B.dist, newdist, B.visited,
                                                        nq, nbm, B.c);
+        if (huge)
+        {
+            k_td_huge<<<gg_sm_count() * 8, 256, 0, B.s>>>(B.heavy, B.g->out_adj, B.parents, B.dist, newdist, B.visited,
+                                                          nq, nbm, B.c);
+            B.launches++;
+        }
         B.launches += 2;
     }
     GG_CHECK(mark(B));

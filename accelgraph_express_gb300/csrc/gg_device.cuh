@@ -711,7 +711,7 @@ __device__ __forceinline__ void push_scatter(const uint32_t *__restrict__ off, c
  * address takes an addition every 5 ns).  A block adds to its group's counter
  * and the lanes of its first warp each poll one group's: two memory round trips
  * (through a root counter and a release word per group it was five: a search of
- * 1,000 vertices 75 -> 69 us, of R-MAT-22 208 -> 199).  The counters only grow (barrier `gen` completes a group
+ * 1,000 vertices 71 -> 63 us, of R-MAT-22 207 -> 190).  The counters only grow (barrier `gen` completes a group
  * at (gen + 1) * group size arrivals), so no arrival waits for a counter to be
  * reset.  Ordering: the addition releases the block's writes, which the block
  * barrier before it has gathered; the polls acquire, and the block barrier
@@ -745,13 +745,17 @@ __device__ __forceinline__ bool grid_barrier(char *ctl, unsigned int *err, unsig
         const unsigned int want = lane < G ? (gen + 1) * ((gridDim.x - lane + G - 1) / G) : 0u;
         bool ok = true;
         const unsigned long long t0 = global_ns();
+        /* the polls of 900 blocks hold the arrivals up at the L2 (a search of 30K
+         * vertices: 77 us with 20 ns between polls, 69 with 150, 67 with 300 to
+         * 800), those of 300 do not (a batched PageRank: 618 against 635) */
+        const unsigned int pause = gridDim.x > 512u ? 400u : 20u;
         for (;;)
         {
             unsigned int v = want;
             if (lane < G) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(word) : "memory");
             /* a counter past `want` has arrivals at the next barrier already */
             if (__all_sync(0xffffffffu, (int)(v - want) >= 0)) break;
-            __nanosleep(20);
+            __nanosleep(pause);
             if (__shfl_sync(0xffffffffu, global_ns() - t0, 0) > limit_ns)
             {
                 if (lane == 0) atomicExch(err, 1u);
