@@ -39,11 +39,20 @@ struct SpmvGather
     __device__ __forceinline__ float value(const Raw &r) const { return __fmul_rn(to_f32(r.w), to_f32(r.x)); }
 };
 
+/* y of the next product: the gathers add the partials of rows that span tiles,
+ * so each clears the other one of two buffers, V floats (null: none follows) */
+__device__ __forceinline__ void clear_next(float *__restrict__ next, uint32_t V)
+{
+    if (!next) return;
+    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x) next[v] = 0.0f;
+}
+
 template <class T>
 __global__ void __launch_bounds__(GG_TILE_NT) k_spmv_pull(const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
                                                           const uint2 *__restrict__ coord, uint32_t ntiles, uint32_t V,
-                                                          float *y, SpmvGather<T> op)
+                                                          float *y, float *next, SpmvGather<T> op)
 {
+    clear_next(next, V);
     warp_pull_sums<GG_TILE_IPT, GG_TILE_WARPS>(off, adj, V, coord, ntiles, y, op);
 }
 
@@ -59,8 +68,9 @@ __global__ void k_spmv_hot_fill(const T *__restrict__ x, const uint32_t *__restr
 template <class T>
 __global__ void __launch_bounds__(GG_HOT_WARPS * 32, 1)
     k_spmv_pull_hot(HotArgs a, const T *__restrict__ x, const T *__restrict__ w, const T *__restrict__ table_src,
-                    float *y)
+                    float *y, float *next, uint32_t V)
 {
+    clear_next(next, V);
     extern __shared__ __align__(1024) unsigned char gg_dyn[];
     const uint32_t warps = blockDim.x >> 5, wid = threadIdx.x >> 5;
     const uint32_t ring = (uint32_t)__cvta_generic_to_shared(gg_dyn), table = ring + warps * HOT_RING;
@@ -235,9 +245,16 @@ gg_status spmv_fp(gg_graph *g, const gg_spmv_params *p, const float *x_dev, floa
         w = (const T *)w16;
         GG_CHECK(gg_work(g, 12, ((size_t)V + 16) * sizeof(T), &xs));
     }
-    k_spmv_x<T><<<grid_v(V), 256, 0, s>>>(g->out_deg, x_dev, xf, (T *)xs, nullptr, nullptr, y, V);
-    launches++;
     const T *xv = sizeof(T) == 4 ? (const T *)xf : (const T *)xs;
+    /* the products of a pull go to two buffers in turn, the last to y: a memset
+     * before each was a launch more (20 products: 128K edges 266 -> 180 us, 1M
+     * 397 -> 304, 3.2M 552 -> 493) */
+    void *other = nullptr;
+    if (pull && p->iterations > 1) GG_CHECK(gg_work(g, 14, ((size_t)V + 16) * 4, &other));
+    float *ys[2] = {y, (float *)other};
+    const uint32_t last = p->iterations ? p->iterations - 1 : 0;
+    k_spmv_x<T><<<grid_v(V), 256, 0, s>>>(g->out_deg, x_dev, xf, (T *)xs, nullptr, nullptr, pull ? ys[last & 1] : y, V);
+    launches++;
     /* the hot-vertex table, as for the PageRank pull */
     bool use_hot = false;
     void *hot_tab = nullptr;
@@ -264,16 +281,15 @@ gg_status spmv_fp(gg_graph *g, const gg_spmv_params *p, const float *x_dev, floa
         }
         if (pull)
         {
-            /* y is the row-sum array: zero, then the gather stores rows and
-             * adds the partials of rows spanning tiles */
-            GG_CUDA(cudaMemsetAsync(y, 0, (size_t)V * sizeof(float), s));
+            float *yi = ys[(last - it) & 1], *next = it < last ? ys[(last - it - 1) & 1] : nullptr;
             const int hg = use_hot ? spmv_hot_grid<T>(g->hot_ntiles, shape.hot_warps) : 0;
             if (hg)
                 k_spmv_pull_hot<T><<<hg, shape.hot_warps * 32, hot_smem_bytes<T>(shape.hot_warps), s>>>(
-                    HotArgs{g->hot_adj, g->rows_list, g->hot_seg0, g->E, g->hot_ntiles, g->hot_tile}, xv, w, (const T *)hot_tab, y);
+                    HotArgs{g->hot_adj, g->rows_list, g->hot_seg0, g->E, g->hot_ntiles, g->hot_tile}, xv, w, (const T *)hot_tab, yi,
+                    next, V);
             else
                 k_spmv_pull<T><<<gg_persistent_grid((const void *)k_spmv_pull<T>, t->ntiles, (int)shape.ctas),
-                                 GG_TILE_NT, 0, s>>>(g->in_off, g->in_adj, t->coord, t->ntiles, V, y, SpmvGather<T>{w, xv});
+                                 GG_TILE_NT, 0, s>>>(g->in_off, g->in_adj, t->coord, t->ntiles, V, yi, next, SpmvGather<T>{w, xv});
         }
         else
         {
@@ -510,7 +526,7 @@ extern "C" gg_status gg_spmv_pull_noalloc(uint32_t V, uint32_t E, const uint32_t
     GG_CHECK(gg_launch_tile_coords(in_off, V, E, ntiles, coord, s));
     GG_CUDA(cudaMemsetAsync(y, 0, (size_t)V * sizeof(float), s));
     k_spmv_pull<float><<<gg_persistent_grid((const void *)k_spmv_pull<float>, ntiles, GG_PULL_CTAS_PER_SM), GG_TILE_NT, 0, s>>>(
-        in_off, in_src, coord, ntiles, V, y, SpmvGather<float>{w, x});
+        in_off, in_src, coord, ntiles, V, y, nullptr, SpmvGather<float>{w, x});
     GG_CUDA(cudaGetLastError());
     return GG_OK;
 }
