@@ -950,17 +950,14 @@ def relabel_extras(gg, torch, peak, scale=24):
 
 
 def csr_radix_bytes(V, E):
-    """Bytes the device CSR + CSC build moves (unweighted): the CSR's keys
-    made (8E read, 8E written), per 8-bit pass a count read (8E) and a
-    scatter read + write (16E), ids and offsets split out (8E read, 4E + 4V
-    written); the CSC's fields swapped in place (16E), its passes over the
-    dst field only, and its split.  Returns (bytes, CSR passes)."""
+    """Bytes the device CSR + CSC build moves (unweighted): a field's sort is a
+    pass per 8 bits of the ids, each a count read (4E) and a scatter read +
+    write (16E); the CSR is two field sorts, the CSC a third; and each
+    direction's offsets from its sorted field (4E read, 4V written).  Returns
+    (bytes, CSR passes)."""
     b = max(1, (max(V, 2) - 1).bit_length())
-    passes = (2 * b + 7) // 8
-    csc_passes = (b + 7) // 8
-    csr = 16 * E + 24 * E * passes + 12 * E + 4 * V
-    csc = 16 * E + 24 * E * csc_passes + 12 * E + 4 * V
-    return csr + csc, passes
+    field = (b + 7) // 8
+    return 20 * E * 3 * field + 2 * (4 * E + 4 * V), 2 * field
 
 
 def csr_build_extras(gg, torch, peak, scale=24, edge_factor=16):
