@@ -240,10 +240,11 @@ __device__ __forceinline__ void td_enqueue_local(bool claimed, uint32_t u, uint3
  * the tuned value per mapping otherwise) go to k_td_heavy, at most
  * TD_MAX_HEAVY of them per step (further ones stay with their warp).  k_td
  * has a second list, where the first may overflow, for the ones past that with
- * more than TD_HUGE edges: a
- * step of a frontier with 30K vertices of over 64 edges otherwise leaves a
- * hub's 40K to one warp (push of R-MAT-20 1600 -> 675 us, slowest source 4500
- * -> 740; R-MAT-22 4900 -> 2040, 11000 -> 2180) */
+ * more than TD_HUGE edges: a step of a frontier with 30K vertices of over 64
+ * edges otherwise leaves a hub's 40K to one warp (push of R-MAT-20 1600 -> 574
+ * us, slowest of 24 sources 4500 -> 740; R-MAT-22 4900 -> 2040, 11000 -> 2180).
+ * Its edges are dealt by a launch of its own: in k_td_heavy its registers cost
+ * two of eight blocks per SM (30K vertices 187 -> 196 us) */
 #define TD_MAX_HEAVY 4096u
 #define TD_HUGE 512u
 #define TD_MAX_HUGE 65536u
@@ -264,9 +265,10 @@ __device__ __forceinline__ uint32_t td_heavy_slot(uint32_t degree, Counters *c, 
     return slot < TD_MAX_HUGE ? TD_MAX_HEAVY + slot : 0xffffffffu;
 }
 
-/* HUGE: with the second list.  LOCAL: claims through the block's local queue.  Not inside the single-launch
- * search, where its registers made the bottom-up steps spill: a search of
- * R-MAT-22 lost 10 us while one of a graph without hubs won 55 */
+/* HUGE: with the second list.  LOCAL: claims through the block's local queue;
+ * not inside the single-launch search, where its registers made the bottom-up
+ * steps spill: a search of R-MAT-22 lost 10 us while one of a graph without hubs
+ * won 55 */
 template <bool LOCAL, bool HUGE>
 __device__ __forceinline__ void td_body(const uint32_t *q, uint32_t qlen,
                                         const uint32_t *__restrict__ off, const uint32_t *__restrict__ adj,
@@ -763,8 +765,8 @@ __global__ void __launch_bounds__(256, 6) k_bfs_do(DoArgs a)
              * block reads the same final count, so all skip together) */
             if (read_counters_block(cs).nheavy)
             {
-                td_heavy_body(a.heavy, &cs->nheavy, 0u, a.out_adj, a.parents, a.dist, level + 1, a.visited, a.q[qcur ^ 1], nullptr,
-                              cs);
+                td_heavy_body(a.heavy, &cs->nheavy, 0u, a.out_adj, a.parents, a.dist, level + 1, a.visited,
+                              a.q[qcur ^ 1], nullptr, cs);
                 if (!(ok = grid_barrier(a.ctl, a.bar_limit_ns, gen))) break;
             }
             const Counters k = read_counters_block(cs);

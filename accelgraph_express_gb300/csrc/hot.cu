@@ -14,8 +14,9 @@
  * T and, up to H, vertices at T take slots by atomics (which of the ties win
  * does not matter: the table holds exact copies); one pass over the CSC
  * writes the encoded ids.  The gather (gg_hot.cuh) finds rows through the ids
- * themselves: passes over the row offsets list the rows that have edges, mark each one's last edge in the encoded ids, and note for every
- * tile of edges which row end comes first in it.
+ * themselves: passes over the row offsets list the rows that have edges, mark
+ * each one's last edge in the encoded ids, and note for every tile of edges which
+ * row end comes first in it.
  */
 #include <cuda_runtime.h>
 

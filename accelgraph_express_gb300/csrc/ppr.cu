@@ -740,6 +740,14 @@ gg_status ppr_tiles(gg_graph *g, cudaStream_t s, uint32_t *launches)
     return GG_OK;
 }
 
+/* tiles below 256 edges need a warp each (gg_ppr_tile) */
+gg_status ppr_tiles_fit(uint32_t tile, uint32_t ntiles, int grid)
+{
+    if (tile < 256u && (uint64_t)grid * PPR_WARPS < ntiles)
+        return gg_fail(GG_ERR_CUDA, "the batched gather has fewer resident warps than its tiles were made for");
+    return GG_OK;
+}
+
 /* one gather / fix-up as a launch of its own */
 template <int KP, int RS, class CT>
 gg_status launch_pull(const PprArgs<CT> &a, uint32_t *next, cudaStream_t s)
@@ -750,8 +758,9 @@ gg_status launch_pull(const PprArgs<CT> &a, uint32_t *next, cudaStream_t s)
     const void *fn = masked ? (const void *)k_ppr_pull<KP, RS, true, CT> : (const void *)k_ppr_pull<KP, RS, false, CT>;
     GG_CHECK(ppr_allow(fn, smem));
     void *args[] = {(void *)&a, &next};
-    GG_CUDA(cudaLaunchKernel(fn, dim3(occupancy_grid(fn, PPR_THREADS, smem, a.ntiles)), dim3(PPR_THREADS), args,
-                             smem, s));
+    const int grid = occupancy_grid(fn, PPR_THREADS, smem, a.ntiles);
+    GG_CHECK(ppr_tiles_fit(a.tile, a.ntiles, grid));
+    GG_CUDA(cudaLaunchKernel(fn, dim3(grid), dim3(PPR_THREADS), args, smem, s));
     return GG_OK;
 }
 template <int KP, int RS, class CT>
@@ -804,6 +813,7 @@ gg_status run_ppr(gg_graph *g, const gg_ppr_params *p, uint32_t nseedv, const ui
         if (per_sm < 1) return gg_fail(GG_ERR_CUDA, "k_ppr_persist cannot be resident");
         /* a warp per tile, or per 32 vertices (the rows without in-edges) */
         const int grid = occupancy_grid(fn, PPR_THREADS, smem, std::max<size_t>(ntiles, ((size_t)V + 31) / 32));
+        GG_CHECK(ppr_tiles_fit(a.tile, ntiles, grid));
         void *ctl;
         const size_t ctl_bytes = GG_BAR_BYTES + (size_t)p->iterations * 4;
         GG_CHECK(gg_work(g, 30, ctl_bytes, &ctl));

@@ -890,7 +890,7 @@ struct Run
     float eps_f = 0.0f, eps_fl = 0.0f;
     bool use_hot = false; /* pull gather through the hot-vertex table */
     const uint32_t *push_tags = nullptr; /* push scatter through the table of frequent destinations */
-    bool small = false;   /* every iteration in one cluster (small.cu) */
+    bool small = false;   /* every iteration in one launch (small.cu) */
     gg_pull_shape shape;  /* launch shape of the FP pull gather */
     uint32_t launches = 0;
     uint32_t gather_launches = 0;
@@ -1425,17 +1425,16 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
         GG_CHECK(gg_push_tags(g, iters, R.s, &R.push_tags));
 
     /* a graph of up to 2.5M edges and 262K vertices: every iteration in one
-     * launch, faster at every size it takes (small.cu); timed runs time each gather launch, and a table asked
-     * for is used */
+     * launch, faster at every size it takes (small.cu); timed runs time each
+     * gather launch, and a table asked for is used */
     R.small = p->mode == GG_PR_PULL && p->storage == GG_STORE_F32 && !ngraphs && !p->profile && !R.use_hot &&
               gg_small_fits(g);
 
-    /* with GG_PR_CUDA_GRAPH everything from here to the final normalisation
-     * is captured into one CUDA graph (over buffers reserved before) and
-     * instantiated; the
-     * instance stays with the mapping and is launched again by calls with
-     * the same parameters while no device memory of the mapping has been
-     * freed since (the buffers it writes are then the same) */
+    /* with GG_PR_CUDA_GRAPH everything from here to the final normalisation is
+     * captured into one CUDA graph (over buffers reserved before) and
+     * instantiated; the instance stays with the mapping and is launched again by
+     * calls with the same parameters while no device memory of the mapping has
+     * been freed since (the buffers it writes are then the same) */
     const bool as_graph = (p->flags & GG_PR_CUDA_GRAPH) != 0 && !R.small;
     gg_status st = GG_OK;
     if (as_graph)

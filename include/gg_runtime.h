@@ -72,7 +72,7 @@ const char *gg_last_error(void);
 void gg_set_wait_timeout_ms(uint32_t ms);
 /* Upper bound, in microseconds, of each device-side wait of the grid
  * barriers inside the single-launch kernels (direction-optimising BFS,
- * batched personalised PageRank); default 2,000,000 (2 s), 0 restores it.
+ * batched personalised PageRank, FP32 pull PageRank of up to 2.5M edges); default 2,000,000 (2 s), 0 restores it.
  * A wait that runs out ends the launch early and the call returns
  * GG_ERR_KERNEL with the context intact.  For diagnostics and tests of
  * that path: at a few microseconds the barriers give up before the other
@@ -190,9 +190,9 @@ typedef struct gg_pr_params
 /* The pull gather (every pull mode; SpMV pull in FP) serves the values of the
  * vertices with the most out-edges -- 40K FP32, 80K 16- or 8-bit, 20K 64-bit
  * ones -- from a shared-memory table (built once per mapping; an extra copy of
- * the CSC ids).  By default from 8M edges up, made once
- * the gathers done and asked for would repay it; HOT_OFF never, HOT_ON on any
- * graph with edges (below 2^30 vertices).  Results are the same. */
+ * the CSC ids).  By default from 8M edges up, made once the
+ * gathers done and asked for would repay it; HOT_OFF never, HOT_ON on any graph
+ * with edges (below 2^30 vertices).  Results are the same. */
 #define GG_PR_HOT_OFF 0x2u
 #define GG_PR_HOT_ON 0x4u
 /* gg_pagerank_batch: run the ordinary pull over the union of the graphs
