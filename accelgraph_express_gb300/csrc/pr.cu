@@ -1424,7 +1424,7 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
     if (p->mode == GG_PR_PUSH || p->mode == GG_PR_PUSH_FX64)
         GG_CHECK(gg_push_tags(g, iters, R.s, &R.push_tags));
 
-    /* a graph of up to 2.5M edges and 262K vertices: every iteration in one
+    /* a graph of up to 2.5M edges and 220K vertices: every iteration in one
      * launch, faster at every size it takes (small.cu); timed runs time each
      * gather launch, and a table asked for is used */
     R.small = p->mode == GG_PR_PULL && p->storage == GG_STORE_F32 && !ngraphs && !p->profile && !R.use_hot &&

@@ -649,9 +649,10 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_grid(GridArgs ga)
 
 /* Edges per thread (of 152 SMs: 2.5M edges) and vertices above which the
  * launches are faster: R-MAT with 2.4M edges 349 (launches) against 353 us, 2.9M
- * 403 against 440 -- the ids leave the L1 less room; 400K vertices with 5 edges
- * each 411 against 438, the update being half of it. */
-constexpr uint32_t GRID_RUN_MAX = 16, GRID_MAX_V = 1u << 18;
+ * 403 against 440 -- the ids leave the L1 less room; 250K vertices with 5 edges
+ * each 316 against 372, with 8 373 against 424, where 220K with 8 took 354
+ * against 341 -- the update and the contributions' lines take over. */
+constexpr uint32_t GRID_RUN_MAX = 16, GRID_MAX_V = 220000;
 constexpr size_t GRID_LIMIT = 220 * 1024;
 
 /* the shares of a graph of one CTA per SM, or false when it does not fit */

@@ -28,6 +28,10 @@ def edges(shape, E):
         V = 400000
         d = rng.integers(0, 40, E) * 10000 + rng.integers(0, 5000, E)
         return rng.integers(0, V, E), d, V
+    if shape == "gaps_in":  # the same within the vertices it takes: 3,000 empty rows between blocks, one of 60,000
+        V = 200000
+        d = rng.integers(0, 20, E) * 7000 + rng.integers(0, 4000, E)
+        return rng.integers(0, V, E), np.where(d < 70000, d, d + 57000), V
     V = max(3, E // 16) | 1
     return rng.integers(0, V, E), (rng.random(E) ** 3 * V).astype(np.int64), V
 
@@ -35,7 +39,9 @@ def edges(shape, E):
 S = 152 * 1024  # threads
 CASES = ([("skewed", E) for E in (163841, 4 * S, 4 * S + 1, 8 * S - 3, 8 * S + 1, 12 * S + 1, 16 * S, 20 * S + 1)] +
          [("one_row", E) for E in (200001, 8 * S + 5)] + [("degree_1", 200001), ("degree_1", 4 * S + 33)] +
-         [("sparse", E) for E in (170000, 300001)] + [("gaps", E) for E in (180000, 900000)])
+         [("sparse", E) for E in (170000, 300001)] + [("gaps", E) for E in (180000, 900000)] +
+         [("gaps_in", E) for E in (1000, 50000, 180000, 900000)] + [("sparse", E) for E in (40000, 109990)] +
+         [("sparse", 20), ("degree_1", 219999)])
 
 
 @pytest.mark.parametrize("shape,E", CASES)
