@@ -52,8 +52,10 @@ __global__ void __launch_bounds__(GG_TILE_NT) k_spmv_pull(const uint32_t *__rest
                                                           const uint2 *__restrict__ coord, uint32_t ntiles, uint32_t V,
                                                           float *y, float *next, SpmvGather<T> op)
 {
+    pdl_wait();
     clear_next(next, V);
     warp_pull_sums<GG_TILE_IPT, GG_TILE_WARPS>(off, adj, V, coord, ntiles, y, op);
+    pdl_trigger();
 }
 
 /* x of the hot vertices, contiguous (once per call: x does not change) */
@@ -70,6 +72,7 @@ __global__ void __launch_bounds__(GG_HOT_WARPS * 32, 1)
     k_spmv_pull_hot(HotArgs a, const T *__restrict__ x, const T *__restrict__ w, const T *__restrict__ table_src,
                     float *y, float *next, uint32_t V)
 {
+    pdl_wait();
     clear_next(next, V);
     extern __shared__ __align__(1024) unsigned char gg_dyn[];
     const uint32_t warps = blockDim.x >> 5, wid = threadIdx.x >> 5;
@@ -79,6 +82,7 @@ __global__ void __launch_bounds__(GG_HOT_WARPS * 32, 1)
                                hot_table_load(table, table_src, hot_table_bytes<T>());
                                return true;
                            });
+    pdl_trigger();
 }
 
 /* one CTA of `warps` warps per SM */
@@ -283,13 +287,28 @@ gg_status spmv_fp(gg_graph *g, const gg_spmv_params *p, const float *x_dev, floa
         {
             float *yi = ys[(last - it) & 1], *next = it < last ? ys[(last - it - 1) & 1] : nullptr;
             const int hg = use_hot ? spmv_hot_grid<T>(g->hot_ntiles, shape.hot_warps) : 0;
+            /* dependent launches, timed runs apart: 20 products of 16K edges
+             * 170 -> 120 us, of 1M 304 -> 249 */
             if (hg)
-                k_spmv_pull_hot<T><<<hg, shape.hot_warps * 32, hot_smem_bytes<T>(shape.hot_warps), s>>>(
-                    HotArgs{g->hot_adj, g->rows_list, g->hot_seg0, g->E, g->hot_ntiles, g->hot_tile}, xv, w, (const T *)hot_tab, yi,
-                    next, V);
+            {
+                const HotArgs ha{g->hot_adj, g->rows_list, g->hot_seg0, g->E, g->hot_ntiles, g->hot_tile};
+                const dim3 grid(hg), block(shape.hot_warps * 32);
+                const size_t smem = hot_smem_bytes<T>(shape.hot_warps);
+                if (p->profile)
+                    k_spmv_pull_hot<T><<<grid, block, smem, s>>>(ha, xv, w, (const T *)hot_tab, yi, next, V);
+                else
+                    GG_CUDA(gg_launch_pdl(k_spmv_pull_hot<T>, grid, block, smem, s, ha, xv, w, (const T *)hot_tab, yi, next, V));
+            }
             else
-                k_spmv_pull<T><<<gg_persistent_grid((const void *)k_spmv_pull<T>, t->ntiles, (int)shape.ctas),
-                                 GG_TILE_NT, 0, s>>>(g->in_off, g->in_adj, t->coord, t->ntiles, V, yi, next, SpmvGather<T>{w, xv});
+            {
+                const dim3 grid(gg_persistent_grid((const void *)k_spmv_pull<T>, t->ntiles, (int)shape.ctas)), block(GG_TILE_NT);
+                const SpmvGather<T> op{w, xv};
+                if (p->profile)
+                    k_spmv_pull<T><<<grid, block, 0, s>>>(g->in_off, g->in_adj, t->coord, t->ntiles, V, yi, next, op);
+                else
+                    GG_CUDA(gg_launch_pdl(k_spmv_pull<T>, grid, block, 0, s, g->in_off, g->in_adj, t->coord, t->ntiles, V, yi,
+                                          next, op));
+            }
         }
         else
         {
