@@ -343,26 +343,47 @@ gg_status gg_rows_tiles(gg_graph *g, cudaStream_t s, uint32_t tile, uint32_t **s
                         uint32_t *launches)
 {
     const uint32_t V = g->V, E = g->E;
-    const uint32_t nt = (uint32_t)(((uint64_t)E + tile - 1) / tile);
-    GG_CHECK(gg_dev_alloc(g, (void **)seg0, (size_t)nt * 4));
-    *ntiles = nt;
-    if (g->rows_list)
+    const uint32_t nt = (uint32_t)(((uint64_t)E + tile - 1) / tile), nb = (uint32_t)(((uint64_t)V + ROW_TILE - 1) / ROW_TILE);
+    /* all that is allocated here, before any of it is set on the mapping */
+    const bool list = !g->rows_list;
+    const size_t seg_bytes = (size_t)nt * 4;
+    void *counts = nullptr, *seg = nullptr, *rows = g->rows_list;
+    if (list) GG_CHECK(gg_work(g, 33, ((size_t)nb + 4) * 4, &counts));
+    GG_CHECK(gg_dev_alloc(g, &seg, seg_bytes));
+    if (list)
     {
-        k_rows_seg0<<<gg_sm_count() * 8, 256, 0, s>>>(g->in_off, V, g->rows_list, *seg0, tile);
-        GG_CUDA(cudaGetLastError());
-        *launches += 1;
-        return GG_OK;
+        const gg_status st = gg_dev_alloc(g, &rows, ((size_t)V + GG_ROW_PAD + 4) * 4);
+        if (st != GG_OK)
+        {
+            gg_dev_free(g, seg, seg_bytes);
+            return st;
+        }
     }
-    const uint32_t nb = (uint32_t)(((uint64_t)V + ROW_TILE - 1) / ROW_TILE);
-    void *counts;
-    GG_CHECK(gg_work(g, 33, ((size_t)nb + 4) * 4, &counts));
-    uint32_t *ticket = (uint32_t *)counts + nb;
-    GG_CUDA(cudaMemsetAsync(ticket, 0, 4, s));
-    GG_CHECK(gg_dev_alloc(g, (void **)&g->rows_list, ((size_t)V + GG_ROW_PAD + 4) * 4));
-    k_rows_count<<<nb, ROW_BLOCK, 0, s>>>(g->in_off, V, (uint32_t *)counts, ticket, g->rows_list + V + GG_ROW_PAD);
-    k_rows_write<<<nb, ROW_BLOCK, 0, s>>>(g->in_off, V, (const uint32_t *)counts, g->rows_list, *seg0, tile);
-    GG_CUDA(cudaGetLastError());
-    *launches += 2;
+    cudaError_t e = cudaSuccess;
+    uint32_t *r = (uint32_t *)rows;
+    if (list)
+    {
+        uint32_t *ticket = (uint32_t *)counts + nb;
+        e = cudaMemsetAsync(ticket, 0, 4, s);
+        if (e == cudaSuccess)
+        {
+            k_rows_count<<<nb, ROW_BLOCK, 0, s>>>(g->in_off, V, (uint32_t *)counts, ticket, r + V + GG_ROW_PAD);
+            k_rows_write<<<nb, ROW_BLOCK, 0, s>>>(g->in_off, V, (const uint32_t *)counts, r, (uint32_t *)seg, tile);
+        }
+    }
+    else
+        k_rows_seg0<<<gg_sm_count() * 8, 256, 0, s>>>(g->in_off, V, r, (uint32_t *)seg, tile);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess)
+    {
+        gg_dev_free(g, seg, seg_bytes);
+        if (list) gg_dev_free(g, rows, ((size_t)V + GG_ROW_PAD + 4) * 4);
+        return gg_cuda_fail(e, "rows and tiles");
+    }
+    g->rows_list = r;
+    *seg0 = (uint32_t *)seg;
+    *ntiles = nt;
+    *launches += list ? 2 : 1;
     return GG_OK;
 }
 
@@ -410,6 +431,7 @@ gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap)
     if (!g->hot_list) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_list, GG_HOT_LIST_BYTES));
     if (!g->hot_adj) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_adj, ((size_t)E + GG_EDGE_PAD) * 4));
     uint32_t *cnt = g->hot_list + GG_HOT_ENTRIES;
+    g->hot_cap = 0; /* until the list and the ids are written */
     GG_CUDA(cudaMemsetAsync(hist, 0, 65536 * 4, s));
     GG_CUDA(cudaMemsetAsync(cnt, 0, 16, s));
     const int grid = gg_sm_count() * 8;

@@ -735,6 +735,7 @@ gg_status ppr_tiles(gg_graph *g, cudaStream_t s, uint32_t *launches)
     if (g->ppr_seg0 && g->ppr_tiles_items == tile) return GG_OK;
     if (g->ppr_seg0) gg_dev_free(g, g->ppr_seg0, (size_t)g->ppr_ntiles * 4);
     g->ppr_seg0 = nullptr;
+    g->ppr_tiles_items = 0;
     GG_CHECK(gg_rows_tiles(g, s, tile, &g->ppr_seg0, &g->ppr_ntiles, launches));
     g->ppr_tiles_items = tile;
     return GG_OK;
