@@ -82,7 +82,7 @@ gg_status gg_push_tags(gg_graph *g, uint32_t iterations, cudaStream_t s, const u
         GG_CHECK(gg_dev_alloc(g, (void **)&g->push_tags, (PUSH_SLOTS + 4) * 4));
         GG_CUDA(cudaMemsetAsync(best, 0, (size_t)PUSH_SLOTS * 8, s));
         GG_CUDA(cudaMemsetAsync(counts, 0, (size_t)V * 4, s));
-        const uint32_t all = (E + 31) / 32, every = (all + SAMPLES / 32 - 1) / (SAMPLES / 32);
+        const uint32_t all = E / 32 + (E % 32 ? 1u : 0u), every = (all + SAMPLES / 32 - 1) / (SAMPLES / 32);
         const uint32_t groups = (all + every - 1) / every;
         const int grid = gg_sm_count() * 8;
         k_push_sample<<<grid, 256, 0, s>>>(g->out_adj, E, groups, every, counts);
