@@ -831,11 +831,15 @@ __global__ void k_perm_hits(const uint32_t *__restrict__ label, uint32_t V, uint
     }
 }
 
-/* out may be ids (in place: each slot is read, then written, by one thread) */
-__global__ void k_apply_labels(const uint32_t *ids, uint64_t n, const uint32_t *__restrict__ label, uint32_t *out)
+/* out may be ids (in place: each slot is read, then written, by one thread);
+ * an id >= V stays as it is, for the build to report */
+__global__ void k_apply_labels(const uint32_t *ids, uint64_t n, const uint32_t *__restrict__ label, uint32_t V, uint32_t *out)
 {
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x)
-        out[i] = label[ids[i]];
+    {
+        const uint32_t v = ids[i];
+        out[i] = v < V ? label[v] : v;
+    }
 }
 
 int bits_for64(uint64_t x)
@@ -939,9 +943,9 @@ gg_status gg_check_permutation(gg_graph *g, const uint32_t *label, uint32_t V, c
     return GG_OK;
 }
 
-gg_status gg_apply_labels(const uint32_t *ids, uint64_t n, const uint32_t *label, uint32_t *out, cudaStream_t s)
+gg_status gg_apply_labels(const uint32_t *ids, uint64_t n, const uint32_t *label, uint32_t V, uint32_t *out, cudaStream_t s)
 {
-    k_apply_labels<<<grid_for(n, 256), 256, 0, s>>>(ids, n, label, out);
+    k_apply_labels<<<grid_for(n, 256), 256, 0, s>>>(ids, n, label, V, out);
     GG_CUDA(cudaGetLastError());
     return GG_OK;
 }

@@ -213,7 +213,7 @@ gg_status gg_build_arrays(gg_graph *g, const uint32_t *src, const uint32_t *dst,
 gg_status gg_relabel_device(gg_graph *g, uint32_t V, uint64_t E, const uint32_t *src, const uint32_t *dst,
                             uint32_t mode, uint64_t seed, uint32_t *label, cudaStream_t s);
 gg_status gg_check_permutation(gg_graph *g, const uint32_t *label, uint32_t V, cudaStream_t s);
-gg_status gg_apply_labels(const uint32_t *ids, uint64_t n, const uint32_t *label, uint32_t *out, cudaStream_t s);
+gg_status gg_apply_labels(const uint32_t *ids, uint64_t n, const uint32_t *label, uint32_t V, uint32_t *out, cudaStream_t s);
 /* results of up to this many 4-byte values are read back through page-locked
  * scratch, one wait for all of a call's results */
 #define GG_STAGE_VALUES ((size_t)65536)

@@ -948,8 +948,8 @@ static gg_status build_common(uint32_t V, uint32_t E, const uint32_t *src, const
         /* relabel the uploaded ids in place: src' = label[src], dst' = label[dst] */
         st = upload(g, (void **)&dl, label_host, (size_t)V * 4, (size_t)V * 4 + 16, s);
         if (st == GG_OK) st = gg_check_permutation(g, dl, V, s);
-        if (st == GG_OK && E) st = gg_apply_labels(ds, E, dl, ds, s);
-        if (st == GG_OK && E) st = gg_apply_labels(dd, E, dl, dd, s);
+        if (st == GG_OK && E) st = gg_apply_labels(ds, E, dl, V, ds, s);
+        if (st == GG_OK && E) st = gg_apply_labels(dd, E, dl, V, dd, s);
     }
     if (st == GG_OK)
         st = gg_build_arrays(g, host ? ds : src, host ? dd : dst, want_w ? (host ? dw : w) : nullptr, what, s);

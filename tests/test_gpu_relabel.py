@@ -101,3 +101,16 @@ def test_relabel_from_file_labels_and_bad_permutation(gpu, orc):
         gpu.build_relabelled(s, d, bad, w, num_vertices=V)
     with pytest.raises(gpu.GgError):
         gpu.relabel_order(s, d, V, 12)
+
+
+@pytest.mark.parametrize("side", [0, 1])
+def test_labels_for_ids_out_of_range_are_refused(gpu, side):
+    """An edge list with an id >= num_vertices has no label: the build reports
+    it, without a read past the labels."""
+    V = 1000
+    e = [np.arange(V, dtype=np.uint32), np.arange(V, dtype=np.uint32)[::-1].copy()]
+    e[side][V // 2] = V
+    with pytest.raises(gpu.GgError, match="vertex id"):
+        gpu.build_relabelled(e[0], e[1], np.arange(V, dtype=np.uint32), num_vertices=V)
+    e[side][V // 2] = 0
+    gpu.build_relabelled(e[0], e[1], np.arange(V, dtype=np.uint32), num_vertices=V).free()
