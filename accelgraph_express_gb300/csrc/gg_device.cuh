@@ -97,55 +97,153 @@ template <class T> __device__ __forceinline__ T warp_sum(T v)
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
-/* A running sum of floats held as hi + lo (Knuth's two-sum: every rounding
- * error of hi is kept in lo), about 48 bits, in FP32 operations: the passes
- * that summed a residual per vertex in FP64 were bound by its issue rate
- * (k_pr_update of a 16.7M-vertex graph: 78 -> 60 us). */
-struct Sum2
+/* two FP32 additions or subtractions in one instruction, each rounded as FADD */
+__device__ __forceinline__ float2 add2(float2 a, float2 b)
 {
-    float hi, lo;
-    __device__ __forceinline__ Sum2() : hi(0.0f), lo(0.0f) {}
-    __device__ __forceinline__ void add(float x)
+    float2 r;
+    asm("{\n\t.reg .b64 ra, rb, rc;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+        "add.rn.f32x2 rc, ra, rb;\n\tmov.b64 {%0, %1}, rc;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+__device__ __forceinline__ float2 sub2(float2 a, float2 b)
+{
+    float2 r;
+    asm("{\n\t.reg .b64 ra, rb, rc;\n\tmov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
+        "sub.rn.f32x2 rc, ra, rb;\n\tmov.b64 {%0, %1}, rc;\n\t}"
+        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
+    return r;
+}
+
+/* A running sum of floats in three of them: hi takes the sum, mid the rounding
+ * errors of hi, lo those of mid (Knuth's two-sum), about 72 bits, in FP32
+ * operations: one FP64 addition per vertex bounds the passes that sum a residual
+ * (k_pr_update of a 16.7M-vertex graph: 78 us in FP64, 60 in FP32).  Where FP32
+ * ends -- sums past SUM_MAX, infinities, NaN -- the sum so far is added to the
+ * FP64 total `over` instead. */
+struct LongSum
+{
+    static constexpr float SUM_MAX = 8.507059173e37f; /* 2^126 */
+    float hi = 0.0f, mid = 0.0f, lo = 0.0f;
+    static __device__ __forceinline__ float two_sum(float &s, float x)
     {
-        const float t = __fadd_rn(hi, x), z = __fsub_rn(t, hi);
-        lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(t, z)), __fsub_rn(x, z)));
-        hi = t;
+        const float t = __fadd_rn(s, x), z = __fsub_rn(t, s);
+        const float e = __fadd_rn(__fsub_rn(s, __fsub_rn(t, z)), __fsub_rn(x, z));
+        s = t;
+        return e;
     }
-    /* an overflowed or NaN sum has no meaningful lo */
-    __device__ __forceinline__ double value() const
+    __device__ __forceinline__ void add(float x, double *over)
     {
-        return fabsf(hi) <= 3.402823466e38f ? (double)hi + (double)lo : (double)hi;
+        if (fabsf(__fadd_rn(hi, x)) <= SUM_MAX)
+            lo = __fadd_rn(lo, two_sum(mid, two_sum(hi, x)));
+        else
+        {
+            /* keeps the conversions to FP64 in this branch */
+            asm volatile("" : "+f"(hi), "+f"(mid), "+f"(lo), "+f"(x));
+            atomicAdd(over, value() + (double)x);
+            hi = mid = lo = 0.0f;
+        }
+    }
+    /* neither sum past SUM_MAX / 2 */
+    __device__ __forceinline__ void merge(float h, float m, float l)
+    {
+        const float e = two_sum(mid, two_sum(hi, h));
+        lo = __fadd_rn(__fadd_rn(lo, l), __fadd_rn(e, two_sum(mid, m)));
+    }
+    __device__ __forceinline__ double value() const { return (double)hi + ((double)mid + (double)lo); }
+};
+
+/* the same for the even and the odd vertex of a pair, by packed instructions */
+struct PairSum
+{
+    float2 hi = {0.0f, 0.0f}, mid = {0.0f, 0.0f}, lo = {0.0f, 0.0f};
+    static __device__ __forceinline__ float2 two_sum(float2 &s, float2 x, float2 t)
+    {
+        const float2 z = sub2(t, s), e = add2(sub2(s, sub2(t, z)), sub2(x, z));
+        s = t;
+        return e;
+    }
+    __device__ __forceinline__ void add(float x, float y, double *over)
+    {
+        float2 v = make_float2(x, y), t = add2(hi, v);
+        if (fabsf(t.x) <= LongSum::SUM_MAX && fabsf(t.y) <= LongSum::SUM_MAX)
+        {
+            const float2 e = two_sum(hi, v, t);
+            lo = add2(lo, two_sum(mid, e, add2(mid, e)));
+        }
+        else
+        {
+            asm volatile("" : "+f"(v.x), "+f"(v.y));
+            atomicAdd(over, part(0).value() + part(1).value() + (double)v.x + (double)v.y);
+            hi = mid = lo = make_float2(0.0f, 0.0f);
+        }
+    }
+    __device__ __forceinline__ LongSum part(int odd) const
+    {
+        LongSum s;
+        s.hi = odd ? hi.y : hi.x;
+        s.mid = odd ? mid.y : mid.x;
+        s.lo = odd ? lo.y : lo.x;
+        return s;
+    }
+    /* both together */
+    __device__ __forceinline__ LongSum total(double *over) const
+    {
+        LongSum s = part(0);
+        if (fabsf(hi.x) <= LongSum::SUM_MAX / 2 && fabsf(hi.y) <= LongSum::SUM_MAX / 2)
+            s.merge(hi.y, mid.y, lo.y);
+        else
+            atomicAdd(over, part(1).value());
+        return s;
     }
 };
 
-/* Block-wide sum of (Sum2, uint32) pairs in FP64; the result is valid in thread 0. */
-template <int NT>
-__device__ __forceinline__ void block_sum2(Sum2 s, uint32_t b, double &a, uint32_t &n)
+/* sum over the warp; the result is valid in lane 0 */
+__device__ __forceinline__ double warp_sum(LongSum s)
 {
-    __shared__ double sa[NT / 32];
-    __shared__ uint32_t sb[NT / 32];
-    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    /* within the warp in two-sum arithmetic, across warps in FP64 */
+    if (__any_sync(0xffffffffu, fabsf(s.hi) > LongSum::SUM_MAX / 64)) return warp_sum(s.value());
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
-    {
-        const float h = __shfl_down_sync(0xffffffffu, s.hi, o), e = __shfl_down_sync(0xffffffffu, s.lo, o);
-        s.add(h);
-        s.lo = __fadd_rn(s.lo, e);
-    }
-    b = warp_sum(b);
-    __syncthreads();
-    if (l == 0) { sa[w] = s.value(); sb[w] = b; }
+        s.merge(__shfl_down_sync(0xffffffffu, s.hi, o), __shfl_down_sync(0xffffffffu, s.mid, o),
+                __shfl_down_sync(0xffffffffu, s.lo, o));
+    return s.value();
+}
+
+/* Block-wide sum of (LongSum, uint32) pairs, once per kernel; the result is valid in thread 0.
+ * One warp joins the threads' sums: in every warp the merges took 1.5 us of a
+ * vertex pass. */
+template <int NT>
+__device__ __forceinline__ void block_sum2(const LongSum &s, uint32_t b, double &a, uint32_t &n)
+{
+    __shared__ float part[3][NT];
+    __shared__ uint32_t sb[NT / 32];
+    const uint32_t t = threadIdx.x, l = t & 31;
+    part[0][t] = s.hi;
+    part[1][t] = s.mid;
+    part[2][t] = s.lo;
+    b = __reduce_add_sync(0xffffffffu, b);
+    if (l == 0) sb[t >> 5] = b;
     __syncthreads();
     a = 0.0;
     n = 0u;
-    if (w == 0)
+    if (t >= 32) return;
+    LongSum all;
+    double wide = 0.0; /* of sums near the end of FP32 */
+#pragma unroll
+    for (uint32_t k = l; k < NT; k += 32)
     {
-        a = l < NT / 32 ? sa[l] : 0.0;
-        n = l < NT / 32 ? sb[l] : 0u;
-        a = warp_sum(a);
-        n = warp_sum(n);
+        const float h = part[0][k];
+        if (fabsf(h) <= LongSum::SUM_MAX / (2 * NT))
+            all.merge(h, part[1][k], part[2][k]);
+        else
+        {
+            asm volatile("" : "+d"(wide));
+            wide += (double)h + ((double)part[1][k] + (double)part[2][k]);
+        }
     }
+    a = warp_sum(all);
+    if (__any_sync(0xffffffffu, wide != 0.0)) a += warp_sum(wide);
+    n = __reduce_add_sync(0xffffffffu, l < NT / 32 ? sb[l] : 0u);
 }
 
 /* Asynchronous 4-byte global -> shared copy (cp.async, cached in L1): the

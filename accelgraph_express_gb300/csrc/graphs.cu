@@ -82,16 +82,18 @@ __device__ __forceinline__ uint32_t graph_iterations(const GraphsArgs &a, unsign
     typedef PullStage<IPT, float> S;
     __shared__ double s_err[32];
     __shared__ uint32_t s_act[32];
+    __shared__ double s_over;
     const uint32_t warps = blockDim.x >> 5, w = threadIdx.x >> 5;
     uint32_t it = 0, act = 0;
     double err = 0.0;
     for (; it < a.iterations; it++)
     {
+        if (threadIdx.x == 0) s_over = 0.0;
         warp_pull_sums_core<IPT>(reinterpret_cast<uint32_t *>(stage), reinterpret_cast<float *>(stage + S::OFF_BYTES),
                                  reinterpret_cast<float *>(stage + S::OFF_BYTES + S::VAL_BYTES), w, warps, a.off,
                                  a.adj, a.V, a.coord + cb, ntiles, sm - vb, GraphsGather{c - vb});
         __syncthreads();
-        Sum2 es;
+        LongSum es;
         uint32_t n_act = 0;
         constexpr uint32_t U = 2; /* measured: 4 was slower, and spills at IPT 9 */
         for (uint32_t v0 = threadIdx.x; v0 < Vg; v0 += U * blockDim.x)
@@ -119,27 +121,22 @@ __device__ __forceinline__ uint32_t graph_iterations(const GraphsArgs &a, unsign
                     const float nr = __fadd_rn(base, __fmul_rn(a.damp, sv[k]));
                     a.rank[vb + v] = nr;
                     const float e = fabsf(__fsub_rn(nr, pr[k]));
-                    es.add(e);
+                    es.add(e, &s_over);
                     n_act += e >= a.eps_f ? 1u : 0u;
                     c[v] = contrib_of_f(nr, dg[k]);
                 }
             }
         }
         /* CTA sums of the residual and the active count */
-        double e_sum = es.value();
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1)
-        {
-            e_sum += __shfl_down_sync(0xffffffffu, e_sum, o);
-            n_act += __shfl_down_sync(0xffffffffu, n_act, o);
-        }
+        const double e_sum = warp_sum(es);
+        n_act = warp_sum(n_act);
         if ((threadIdx.x & 31) == 0)
         {
             s_err[w] = e_sum;
             s_act[w] = n_act;
         }
         __syncthreads();
-        err = 0.0;
+        err = s_over;
         act = 0;
         for (uint32_t k = 0; k < warps; k++)
         {

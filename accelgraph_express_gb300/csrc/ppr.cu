@@ -72,12 +72,8 @@ struct F2
 };
 __device__ __forceinline__ F2 add2(F2 a, F2 b)
 {
-    F2 r;
-    asm("{\n\t.reg .b64 ra, rb, rc;\n\t"
-        "mov.b64 ra, {%2, %3};\n\tmov.b64 rb, {%4, %5};\n\t"
-        "add.rn.f32x2 rc, ra, rb;\n\tmov.b64 {%0, %1}, rc;\n\t}"
-        : "=f"(r.x), "=f"(r.y) : "f"(a.x), "f"(a.y), "f"(b.x), "f"(b.y));
-    return r;
+    const float2 r = gg::add2(make_float2(a.x, a.y), make_float2(b.x, b.y));
+    return F2{r.x, r.y};
 }
 
 /* One row of KP stored values, seen by a half warp: lane l of 16 reads the

@@ -370,7 +370,7 @@ __global__ void k_quantize(const float *__restrict__ cf, QT *__restrict__ q, uin
 __global__ void k_pr_finalize(float *__restrict__ rank, uint32_t V, int divide, double *sum)
 {
     pdl_wait();
-    Sum2 s;
+    PairSum s;
     const float fv = __uint2float_rn(V);
     const uint32_t P = V >> 1, stride = gridDim.x * blockDim.x, tid = blockIdx.x * blockDim.x + threadIdx.x;
     for (uint32_t p = tid; p < P; p += stride)
@@ -381,8 +381,7 @@ __global__ void k_pr_finalize(float *__restrict__ rank, uint32_t V, int divide, 
             r = make_float2(__fdiv_rn(r.x, fv), __fdiv_rn(r.y, fv));
             reinterpret_cast<float2 *>(rank)[p] = r;
         }
-        s.add(r.x);
-        s.add(r.y);
+        s.add(r.x, r.y, sum);
     }
     if ((V & 1u) && tid == 0)
     {
@@ -392,11 +391,11 @@ __global__ void k_pr_finalize(float *__restrict__ rank, uint32_t V, int divide, 
             r = __fdiv_rn(r, fv);
             rank[V - 1] = r;
         }
-        s.add(r);
+        s.add(r, 0.0f, sum);
     }
     double total;
     uint32_t none;
-    block_sum2<256>(s, 0u, total, none);
+    block_sum2<256>(s.total(sum), 0u, total, none);
     if (threadIdx.x == 0 && total != 0.0) atomicAdd(sum, total);
 }
 
@@ -405,7 +404,7 @@ __global__ void k_pr_finalize(float *__restrict__ rank, uint32_t V, int divide, 
 __global__ void k_pr_finalize_seg(float *__restrict__ rank, uint32_t V, const uint32_t *__restrict__ voff,
                                   uint32_t ngraphs, double *sum)
 {
-    Sum2 s;
+    LongSum s;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < V; v += gridDim.x * blockDim.x)
     {
         /* graph of v: the last g with voff[g] <= v */
@@ -420,7 +419,7 @@ __global__ void k_pr_finalize_seg(float *__restrict__ rank, uint32_t V, const ui
         }
         const float r = __fdiv_rn(rank[v], __uint2float_rn(voff[lo + 1] - voff[lo]));
         rank[v] = r;
-        s.add(r);
+        s.add(r, sum);
     }
     double total;
     uint32_t none;
@@ -486,21 +485,20 @@ struct UpdateStep
 {
     typedef typename Fmt<K>::Acc Acc;
     float base, damp, eps_f, qscale;
-    Sum2 err;
+    PairSum err;
     uint32_t act = 0, tmax = 0;
     /* pageRank.c:1057-1067: |rank' - rank| is a float difference; the sum of
      * the differences is divided by V once on the host (the reference
      * divides each term), and `error >= epsilon` is the same test as
      * e >= eps_f in FP32 */
-    __device__ __forceinline__ float rank(Acc s, float old)
+    __device__ __forceinline__ float rank(Acc s, float old, float &e)
     {
         float nr;
         if constexpr (K == K_Q8Z)
             nr = __fadd_rn(base, __fmul_rn(damp, (float)s));
         else
             nr = next_rank<K>(base, damp, s, qscale);
-        const float e = fabsf(__fsub_rn(nr, old));
-        err.add(e);
+        e = fabsf(__fsub_rn(nr, old));
         if (e >= eps_f) act++;
         return nr;
     }
@@ -535,20 +533,24 @@ __global__ void k_pr_update(PrCommon c, typename Fmt<K>::Acc *sums, typename Fmt
         const float2 pr = reinterpret_cast<const float2 *>(rank)[p];
         const uint2 d = reinterpret_cast<const uint2 *>(outdeg)[p];
         if (s.x != Acc(0) || s.y != Acc(0)) reinterpret_cast<Two<Acc> *>(sv)[p] = Two<Acc>{Acc(0), Acc(0)};
-        const float2 nr = make_float2(st.rank(s.x, pr.x), st.rank(s.y, pr.y));
+        float e0, e1;
+        const float2 nr = make_float2(st.rank(s.x, pr.x, e0), st.rank(s.y, pr.y, e1));
         reinterpret_cast<float2 *>(rank)[p] = nr;
         const float c0 = st.contribution(nr.x, d.x), c1 = st.contribution(nr.y, d.y);
         if constexpr (Fmt<K>::quant)
             reinterpret_cast<float2 *>(cf)[p] = make_float2(c0, c1);
         else
             reinterpret_cast<Two<CT> *>(cout)[p] = Two<CT>{encode<K>(c0, d.x), encode<K>(c1, d.y)};
+        st.err.add(e0, e1, &c.rec[c.it].err);
     }
     if ((c.V & 1u) && tid == 0)
     {
         const uint32_t v = c.V - 1, d = outdeg[v];
         const Acc s = sv[v];
         clear_after_read(&sv[v], s);
-        const float nr = st.rank(s, rank[v]);
+        float e;
+        const float nr = st.rank(s, rank[v], e);
+        st.err.add(e, 0.0f, &c.rec[c.it].err);
         rank[v] = nr;
         const float ctb = st.contribution(nr, d);
         if constexpr (Fmt<K>::quant)
@@ -559,7 +561,7 @@ __global__ void k_pr_update(PrCommon c, typename Fmt<K>::Acc *sums, typename Fmt
     if constexpr (Fmt<K>::quant) block_max_bits<256>(st.tmax, &c.rec[c.it + 1].maxbits);
     double err;
     uint32_t act;
-    block_sum2<256>(st.err, st.act, err, act);
+    block_sum2<256>(st.err.total(&c.rec[c.it].err), st.act, err, act);
     if (threadIdx.x == 0) c.reduce(err, act);
     pdl_trigger();
 }
@@ -640,9 +642,9 @@ struct DeltaStep
     float base, damp, init, in_inv, eps_f;
     int k;
     bool first;
-    Sum2 err;
+    PairSum err;
     uint32_t act = 0, tmax = 0;
-    __device__ __forceinline__ void operator()(float ds, float &s, float &ch, uint32_t deg, float &nr, CT &q)
+    __device__ __forceinline__ void operator()(float ds, float &s, float &ch, uint32_t deg, float &nr, CT &q, float &e)
     {
         const float s_old = s;
         s = __fadd_rn(s_old, __fmul_rn(ds, in_inv));
@@ -651,8 +653,7 @@ struct DeltaStep
          * sector whose read is still in flight stalls */
         const float pr = first ? init : __fadd_rn(base, __fmul_rn(damp, s_old));
         nr = __fadd_rn(base, __fmul_rn(damp, s));
-        const float e = fabsf(__fsub_rn(nr, pr));
-        err.add(e);
+        e = fabsf(__fsub_rn(nr, pr));
         if (e >= eps_f) act++;
         const float d = __fsub_rn(contrib_of(nr, deg), ch);
         ch = __fadd_rn(ch, store_delta<K>(d, k, &q));
@@ -705,20 +706,23 @@ __global__ void k_pr_update_delta(PrCommon c, float init, float *__restrict__ ds
         if (ds.x != 0.0f || ds.y != 0.0f) reinterpret_cast<float2 *>(dsum)[p] = make_float2(0.0f, 0.0f);
         float2 nr;
         CT q0, q1;
-        st(ds.x, s.x, ch.x, deg.x, nr.x, q0);
-        st(ds.y, s.y, ch.y, deg.y, nr.y, q1);
+        float e0, e1;
+        st(ds.x, s.x, ch.x, deg.x, nr.x, q0, e0);
+        st(ds.y, s.y, ch.y, deg.y, nr.y, q1, e1);
         reinterpret_cast<float2 *>(S)[p] = s;
         reinterpret_cast<float2 *>(rank)[p] = nr;
         reinterpret_cast<float2 *>(chat)[p] = ch;
         reinterpret_cast<typename Pair16<CT>::T *>(qout)[p] = Pair16<CT>::make(q0, q1);
+        st.err.add(e0, e1, &c.rec[c.it].err);
     }
     if ((c.V & 1u) && blockIdx.x == 0 && threadIdx.x == 0)
     {
         const uint32_t v = c.V - 1;
         const float ds = dsum[v];
         clear_after_read(&dsum[v], ds);
-        float s = S[v], ch = chat[v], nr;
-        st(ds, s, ch, outdeg[v], nr, qout[v]);
+        float s = S[v], ch = chat[v], nr, e;
+        st(ds, s, ch, outdeg[v], nr, qout[v], e);
+        st.err.add(e, 0.0f, &c.rec[c.it].err);
         S[v] = s;
         rank[v] = nr;
         chat[v] = ch;
@@ -727,7 +731,7 @@ __global__ void k_pr_update_delta(PrCommon c, float init, float *__restrict__ ds
     block_max_bits<256>(st.tmax, &c.rec[c.it + 1].maxbits);
     double err;
     uint32_t act;
-    block_sum2<256>(st.err, st.act, err, act);
+    block_sum2<256>(st.err.total(&c.rec[c.it].err), st.act, err, act);
     if (threadIdx.x == 0) c.reduce(err, act);
     pdl_trigger();
 }
@@ -767,7 +771,7 @@ __global__ void k_dd_update(PrCommon c, float *sums, const uint8_t *__restrict__
                             const uint32_t *__restrict__ out_off, const uint32_t *__restrict__ out_adj)
 {
     if (c.skip()) return;
-    Sum2 es;
+    LongSum es;
     uint32_t na = 0;
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < c.V; v += gridDim.x * blockDim.x)
     {
@@ -776,7 +780,7 @@ __global__ void k_dd_update(PrCommon c, float *sums, const uint8_t *__restrict__
         if (!wl_curr[v]) continue;
         float nr = __fadd_rn(c.base, __fmul_rn(c.damp, sum));
         float e = fabsf(__fsub_rn(nr, c.rank[v]));
-        es.add(e);
+        es.add(e, &c.rec[c.it].err);
         if (e >= c.eps_f)
         {
             c.rank[v] = nr;
@@ -823,7 +827,7 @@ __global__ void k_dd_push(PrCommon c, int pullpush, const uint32_t *__restrict__
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-    Sum2 es;
+    LongSum es;
     uint32_t na = 0;
     for (uint32_t v = warp; v < c.V; v += nwarps)
     {
@@ -855,7 +859,7 @@ __global__ void k_dd_push(PrCommon c, int pullpush, const uint32_t *__restrict__
         if (lane == 0)
         {
             float fv = __uint2float_rn(c.V);
-            es.add(fabsf(__fsub_rn(__fdiv_rn(new_pr, fv), __fdiv_rn(old_pr, fv))));
+            es.add(fabsf(__fsub_rn(__fdiv_rn(new_pr, fv), __fdiv_rn(old_pr, fv))), &c.rec[c.it].err);
             c.rank[v] = new_pr;
         }
         uint32_t deg = c.outdeg[v];

@@ -219,6 +219,38 @@ __device__ __forceinline__ void gather_run(const ID *run, uint32_t n, uint32_t s
     if (lane == 31) tail(ends != 0u, seg, sum);
 }
 
+/* the ranks of this CTA's vertices, their sum, and the residual of the last
+ * iteration run, for which every iteration leaves the ranks that it began with
+ * in a.rank: two FP64 sums of a few terms per thread, once */
+__device__ __forceinline__ void small_finish(const SmallArgs &a, const float *rank, uint32_t v0, uint32_t v1, uint32_t it)
+{
+    __shared__ double part[2][SM_WARPS];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
+    double err = 0.0, sum = 0.0;
+    for (uint32_t i = tid; i < v1 - v0; i += SM_THREADS)
+    {
+        float r = rank[i];
+        if (it > 0) err += (double)fabsf(__fsub_rn(r, a.rank[v0 + i]));
+        if (a.divide) r = __fdiv_rn(r, __uint2float_rn(a.V));
+        a.rank[v0 + i] = r;
+        sum += (double)r;
+    }
+    err = warp_sum(err);
+    sum = warp_sum(sum);
+    if (lane == 0)
+    {
+        part[0][w] = err;
+        part[1][w] = sum;
+    }
+    __syncthreads();
+    if (w < 2)
+    {
+        const double all = warp_sum(part[w][lane]);
+        double *to = w ? a.sum : &a.rec[it - 1].err;
+        if (lane == 0 && (w || it > 0)) atomicAdd(to, all);
+    }
+}
+
 struct SmallShape
 {
     size_t ids, rows, c, sums, rank, deg, total;
@@ -312,7 +344,6 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_small(SmallArgs a)
     }
     M::sync();
 
-    Sum2 err;
     uint32_t it = 0, total = 0;
     for (; it < a.iterations; it++)
     {
@@ -332,7 +363,6 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_small(SmallArgs a)
                     if (r < found && !(run[a.run - 1] & SM_END)) M::add(rows[r], v);
                 });
         M::sync();
-        err = Sum2();
         uint32_t act = 0;
         for (uint32_t i = tid; i < v1 - v0; i += SM_THREADS)
         {
@@ -340,8 +370,8 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_small(SmallArgs a)
             sums[i] = 0.0f;
             const float nr = __fadd_rn(a.base, __fmul_rn(a.damp, s));
             const float e = fabsf(__fsub_rn(nr, rank[i]));
+            a.rank[v0 + i] = rank[i];
             rank[i] = nr;
-            err.add(e);
             if (e >= a.eps_f) act++;
             const uint32_t d = deg[i];
             const float x = d ? __fdiv_rn(nr, __uint2float_rn(d)) : 0.0f;
@@ -362,22 +392,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_small(SmallArgs a)
             break;
         }
     }
-    /* the residual is only wanted of the last iteration run */
-    double e_sum;
-    uint32_t none;
-    block_sum2<SM_THREADS>(err, 0u, e_sum, none);
-    if (tid == 0 && it > 0) atomicAdd(&a.rec[it - 1].err, e_sum);
-    Sum2 rs;
-    for (uint32_t i = tid; i < v1 - v0; i += SM_THREADS)
-    {
-        float r = rank[i];
-        if (a.divide) r = __fdiv_rn(r, __uint2float_rn(a.V));
-        a.rank[v0 + i] = r;
-        rs.add(r);
-    }
-    double t_sum;
-    block_sum2<SM_THREADS>(rs, 0u, t_sum, none);
-    if (tid == 0 && t_sum != 0.0) atomicAdd(a.sum, t_sum);
+    small_finish(a, rank, v0, v1, it);
     M::sync(); /* no CTA leaves while another may still write its memory */
 }
 
@@ -557,7 +572,6 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_grid(GridArgs ga)
     uint32_t total;
     bool ok = counted_barrier(ga.words + a.iterations, 0u, ga.failed, ga.limit_ns, &total);
 
-    Sum2 err;
     uint32_t it = 0;
     for (; ok && it < a.iterations; it++)
     {
@@ -602,7 +616,6 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_grid(GridArgs ga)
         }
         if (tid == 0) s_total = 0u;
         if (!(ok = counted_barrier(ga.words + it, 0u, ga.failed, ga.limit_ns, &total))) break;
-        err = Sum2();
         uint32_t act = 0;
         for (uint32_t i = tid; i < v1 - v0; i += SM_THREADS)
         {
@@ -610,8 +623,8 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_grid(GridArgs ga)
             sums[v0 + i] = 0.0f;
             const float nr = __fadd_rn(a.base, __fmul_rn(a.damp, s));
             const float e = fabsf(__fsub_rn(nr, rank[i]));
+            a.rank[v0 + i] = rank[i];
             rank[i] = nr;
-            err.add(e);
             if (e >= a.eps_f) act++;
             const uint32_t d = deg[i];
             c[v0 + i] = d ? __fdiv_rn(nr, __uint2float_rn(d)) : 0.0f;
@@ -630,21 +643,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_grid(GridArgs ga)
         }
     }
     if (!ok) return; /* the host reports it */
-    double e_sum;
-    uint32_t none;
-    block_sum2<SM_THREADS>(err, 0u, e_sum, none);
-    if (tid == 0 && it > 0) atomicAdd(&a.rec[it - 1].err, e_sum);
-    Sum2 rs;
-    for (uint32_t i = tid; i < v1 - v0; i += SM_THREADS)
-    {
-        float r = rank[i];
-        if (a.divide) r = __fdiv_rn(r, __uint2float_rn(a.V));
-        a.rank[v0 + i] = r;
-        rs.add(r);
-    }
-    double t_sum;
-    block_sum2<SM_THREADS>(rs, 0u, t_sum, none);
-    if (tid == 0 && t_sum != 0.0) atomicAdd(a.sum, t_sum);
+    small_finish(a, rank, v0, v1, it);
 }
 
 /* Edges per thread (of 152 SMs: 2.5M edges) and vertices above which the
