@@ -360,10 +360,12 @@ void gg_tune_lookup(gg_graph *g, cudaStream_t s);
 
 /* FP32 pull PageRank of a small graph in one launch (small.cu): whether the
  * graph fits, and the run -- ranks (normalised), iteration records and the rank
- * sum as the launches of pr.cu write them (rec and sum zeroed before) */
+ * sum as the launches of pr.cu write them (rec and sum zeroed before), or
+ * *launched false where the device does not take the launch; rec[iterations +
+ * 1].pad is set when a grid barrier gave up */
 bool gg_small_fits(const gg_graph *g);
 gg_status gg_small_pagerank(gg_graph *g, const gg_pr_params *p, float *rank, void *rec, double *sum, float base,
-                            float init, float eps_f, cudaStream_t s);
+                            float init, float eps_f, cudaStream_t s, bool *launched);
 
 /* One iteration of the batched personalised PageRank on caller-held state
  * (ppr.cu; the server's continuous batch): the first kp (16/32/64) vectors

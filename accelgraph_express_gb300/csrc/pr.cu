@@ -1269,10 +1269,13 @@ gg_status pagerank_enqueue(Run &R, const gg_pr_params *p, IterRec *rec, float *r
 
     if (R.small)
     {
-        GG_CHECK(gg_small_pagerank(R.g, p, rank, rec, (double *)sum_v, base, init, R.eps_f, R.s));
-        R.launches++;
-        R.gather_launches += iters;
-        return GG_OK;
+        GG_CHECK(gg_small_pagerank(R.g, p, rank, rec, (double *)sum_v, base, init, R.eps_f, R.s, &R.small));
+        if (R.small)
+        {
+            R.launches++;
+            R.gather_launches += iters;
+            return GG_OK;
+        }
     }
     if (V > 0)
     {
@@ -1380,7 +1383,7 @@ gg_status graphs_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_re
  * graphs (vertex ranges h_voff[g] .. h_voff[g+1]) and the final
  * normalisation divides each vertex by its own graph's vertex count */
 gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_result *r, void *stream,
-                        uint32_t ngraphs, const uint32_t *h_voff)
+                        uint32_t ngraphs, const uint32_t *h_voff, bool one_launch = true)
 {
     GgRange range(ngraphs ? "gg_pagerank_batch" : "gg_pagerank");
     if (!g || !p) return gg_fail(GG_ERR_INVALID, "NULL argument");
@@ -1454,7 +1457,7 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
     /* a graph of up to 2.5M edges and 220K vertices: every iteration in one
      * launch, faster at every size it takes (small.cu); timed runs time each
      * gather launch, and a table asked for is used */
-    R.small = p->mode == GG_PR_PULL && p->storage == GG_STORE_F32 && !ngraphs && !p->profile && !R.use_hot &&
+    R.small = one_launch && p->mode == GG_PR_PULL && p->storage == GG_STORE_F32 && !ngraphs && !p->profile && !R.use_hot &&
               gg_small_fits(g);
 
     /* with GG_PR_CUDA_GRAPH everything from here to the final normalisation is
@@ -1543,6 +1546,9 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
         if (stage_rank) GG_CUDA(cudaMemcpyAsync(pin_rank, rank, (size_t)V * 4, cudaMemcpyDeviceToHost, R.s));
         GG_CHECK(gg_wait(R.s));
         h = (const IterRec *)pin;
+        /* a grid barrier of the one launch gave up: by launches, which wait for
+         * nothing on the device */
+        if (R.small && h[iters + 1].pad) return pagerank_impl(g, p, ranks, r, stream, ngraphs, h_voff, false);
         memcpy(&sum, (const char *)pin + rec_bytes, 8);
         if (stage_rank) memcpy(ranks, pin_rank, (size_t)V * 4);
     }
@@ -1554,11 +1560,11 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
         GG_CUDA(cudaMemcpyAsync(&sum, sum_v, sizeof(double), cudaMemcpyDeviceToHost, R.s));
         GG_CHECK(gg_wait(R.s));
         h = many.data();
+        if (R.small && h[iters + 1].pad) return pagerank_impl(g, p, ranks, r, stream, ngraphs, h_voff, false);
         if (stage_rank) GG_CHECK(gg_copy_d2h(ranks, rank, (size_t)V * 4, R.s));
     }
     if (ranks && V && !stage_rank) GG_CHECK(gg_copy_d2h(ranks, rank, (size_t)V * 4, R.s));
 
-    if (R.small && h[iters + 1].pad) return gg_fail(GG_ERR_KERNEL, "PageRank grid barrier timed out");
 
     /* reference loop convention: iterations = index of the breaking
      * iteration, or max when the loop ran out (pageRank.c:1021-1075) */

@@ -451,9 +451,9 @@ __device__ __forceinline__ uint32_t last_row(const uint32_t *__restrict__ off, u
 /* Grid barrier of k_pr_grid on a 64-bit word, zero at first: arrivals in the
  * high half, the sum of `add` in the low one, which is returned in *sum.  One
  * release add per CTA and acquire loads of the one word: two memory round
- * trips (the two-level barrier of gg_device.cuh, made for 900 blocks, takes
- * six).  False when the wait reached its limit, which sets *failed: the other
- * CTAs then leave at their next barrier. */
+ * trips, as the barrier of gg_device.cuh, which has sixteen words for 900 blocks
+ * and returns no sum.  False when the wait reached its limit, which sets
+ * *failed: the other CTAs then leave at their next barrier. */
 __device__ __forceinline__ bool counted_barrier(unsigned long long *word, uint32_t add, uint32_t *failed,
                                                 unsigned long long limit_ns, uint32_t *sum)
 {
@@ -712,8 +712,9 @@ bool gg_small_fits(const gg_graph *g)
 }
 
 gg_status gg_small_pagerank(gg_graph *g, const gg_pr_params *p, float *rank, void *rec, double *sum, float base,
-                            float init, float eps_f, cudaStream_t s)
+                            float init, float eps_f, cudaStream_t s, bool *launched)
 {
+    *launched = false;
     SmallArgs a{};
     uint32_t C;
     size_t smem;
@@ -738,7 +739,8 @@ gg_status gg_small_pagerank(gg_graph *g, const gg_pr_params *p, float *rank, voi
         ga.limit_ns = gg_barrier_limit_ns();
         GG_CUDA(cudaFuncSetAttribute((const void *)k_pr_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GRID_LIMIT));
         void *args[] = {&ga};
-        GG_CUDA(cudaLaunchCooperativeKernel((const void *)k_pr_grid, dim3(C), dim3(SM_THREADS), args, smem, s));
+        *launched = cudaLaunchCooperativeKernel((const void *)k_pr_grid, dim3(C), dim3(SM_THREADS), args, smem, s) == cudaSuccess;
+        if (!*launched) cudaGetLastError();
         return GG_OK;
     }
     void (*fn)(SmallArgs) = C > 1 ? k_pr_small<true> : k_pr_small<false>;
@@ -755,6 +757,7 @@ gg_status gg_small_pagerank(gg_graph *g, const gg_pr_params *p, float *rank, voi
     attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 1;
-    GG_CUDA(cudaLaunchKernelEx(&cfg, fn, a));
+    *launched = cudaLaunchKernelEx(&cfg, fn, a) == cudaSuccess;
+    if (!*launched) cudaGetLastError();
     return GG_OK;
 }

@@ -72,9 +72,10 @@ const char *gg_last_error(void);
 void gg_set_wait_timeout_ms(uint32_t ms);
 /* Upper bound, in microseconds, of each device-side wait of the grid
  * barriers inside the single-launch kernels (direction-optimising BFS,
- * batched personalised PageRank, FP32 pull PageRank of up to 2.5M edges); default 2,000,000 (2 s), 0 restores it.
- * A wait that runs out ends the launch early and the call returns
- * GG_ERR_KERNEL with the context intact.  For diagnostics and tests of
+ * batched personalised PageRank, FP32 pull PageRank of up to 2.5M edges);
+ * default 2,000,000 (2 s), 0 restores it.  A wait that runs out ends the launch
+ * early and the call returns GG_ERR_KERNEL with the context intact, or, for the
+ * pull PageRank, runs again as separate launches.  For diagnostics and tests of
  * that path: at a few microseconds the barriers give up before the other
  * blocks arrive. */
 void gg_set_barrier_limit_us(uint32_t us);
