@@ -463,15 +463,13 @@ __device__ __forceinline__ bool counted_barrier(unsigned long long *word, uint32
     {
         asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(word), "l"(((unsigned long long)1 << 32) | add)
                      : "memory");
-        unsigned long long v = 0, t0 = 0;
-        for (uint32_t n = 0;; n++)
+        const unsigned long long t0 = global_ns();
+        unsigned long long v = 0;
+        for (;;)
         {
             asm volatile("ld.acquire.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(word) : "memory");
             if ((uint32_t)(v >> 32) == gridDim.x) break;
-            if ((n & 63u) != 63u) continue;
-            const unsigned long long now = global_ns();
-            if (!t0) t0 = now;
-            if (now - t0 > limit_ns)
+            if (global_ns() - t0 > limit_ns)
             {
                 atomicExch(failed, 1u);
                 v = ~0ull;
