@@ -209,40 +209,48 @@ __device__ __forceinline__ double warp_sum(LongSum s)
     return s.value();
 }
 
-/* Block-wide sum of (LongSum, uint32) pairs, once per kernel; the result is valid in thread 0.
- * One warp joins the threads' sums: in every warp the merges took 1.5 us of a
- * vertex pass. */
+/* Block-wide sum of (LongSum, uint32) pairs, once per kernel; the result is valid in
+ * thread 0.  Groups of four lanes are joined in their warps, the rest by one
+ * warp: all of it in every warp took 1.5 us of a vertex pass, and a slot per
+ * thread (3 KB) kept the blocks off SMs whose shared memory the gather before
+ * them had sized for itself (a call on 7M edges 1.01 -> 1.10 ms). */
 template <int NT>
-__device__ __forceinline__ void block_sum2(const LongSum &s, uint32_t b, double &a, uint32_t &n)
+__device__ __forceinline__ void block_sum2(LongSum s, uint32_t b, double &a, uint32_t &n)
 {
-    __shared__ float part[3][NT];
+    constexpr uint32_t SLOTS = NT / 4;
+    __shared__ float part[3][SLOTS];
     __shared__ uint32_t sb[NT / 32];
+    __shared__ double s_wide; /* sums near the end of FP32 */
     const uint32_t t = threadIdx.x, l = t & 31;
-    part[0][t] = s.hi;
-    part[1][t] = s.mid;
-    part[2][t] = s.lo;
+    if (t == 0) s_wide = 0.0;
+    __syncthreads();
+    if (!(fabsf(s.hi) <= LongSum::SUM_MAX / (2 * NT)))
+    {
+        asm volatile("" : "+f"(s.hi), "+f"(s.mid), "+f"(s.lo));
+        atomicAdd(&s_wide, s.value());
+        s = LongSum();
+    }
+#pragma unroll
+    for (int o = 16; o >= 8; o >>= 1)
+        s.merge(__shfl_down_sync(0xffffffffu, s.hi, o), __shfl_down_sync(0xffffffffu, s.mid, o),
+                __shfl_down_sync(0xffffffffu, s.lo, o));
     b = __reduce_add_sync(0xffffffffu, b);
+    if (l < 8)
+    {
+        const uint32_t k = (t >> 5) * 8 + l;
+        part[0][k] = s.hi;
+        part[1][k] = s.mid;
+        part[2][k] = s.lo;
+    }
     if (l == 0) sb[t >> 5] = b;
     __syncthreads();
     a = 0.0;
     n = 0u;
     if (t >= 32) return;
     LongSum all;
-    double wide = 0.0; /* of sums near the end of FP32 */
 #pragma unroll
-    for (uint32_t k = l; k < NT; k += 32)
-    {
-        const float h = part[0][k];
-        if (fabsf(h) <= LongSum::SUM_MAX / (2 * NT))
-            all.merge(h, part[1][k], part[2][k]);
-        else
-        {
-            asm volatile("" : "+d"(wide));
-            wide += (double)h + ((double)part[1][k] + (double)part[2][k]);
-        }
-    }
-    a = warp_sum(all);
-    if (__any_sync(0xffffffffu, wide != 0.0)) a += warp_sum(wide);
+    for (uint32_t k = l; k < SLOTS; k += 32) all.merge(part[0][k], part[1][k], part[2][k]);
+    a = warp_sum(all) + s_wide;
     n = __reduce_add_sync(0xffffffffu, l < NT / 32 ? sb[l] : 0u);
 }
 
