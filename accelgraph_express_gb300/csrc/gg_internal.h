@@ -280,8 +280,12 @@ int gg_sm_count();
 /* persistent grid for a tile kernel: one CTA per resident slot, no more
  * CTAs than tiles need.  ctas_per_sm > 0 caps the resident CTAs per SM and
  * sets the kernel's shared-memory carve-out to just hold them, so the rest
- * of each SM's combined L1/shared array caches the gathered values. */
-int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm = 0);
+ * of each SM's combined L1/shared array caches the gathered values.  *pad:
+ * dynamic shared memory that keeps further CTAs off an SM, for dependent
+ * launches: they take the SMs in the order in which these become free, and one
+ * more per SM on the first of them left a sixth of the chip idle (PageRank,
+ * 4.2M vertices and 67M uniform random edges: 7.40 ms -> 6.67). */
+int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm = 0, size_t *pad = nullptr);
 /* Push scatters through a table of frequent destinations (push.cu,
  * gg_device.cuh) */
 #define PUSH_LOG 12

@@ -125,7 +125,27 @@ int gg_push_grid(const void *kernel, uint32_t ntiles, size_t smem)
     return need < (uint32_t)cap ? (int)need : cap;
 }
 
-int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm)
+/* The shared-memory share, in percent, of the smallest carve-out that holds
+ * `ctas` blocks of `block` bytes (the 1 KB that each reserves included), and the
+ * bytes that a block must take besides so that no further one fits.  The share is
+ * rounded down: a share above a carve-out selects the next one, which held a
+ * sixth block and left the L1 32 KB less (5 blocks of 20 KB are 43.9%). */
+static int carveout_for(size_t block, int ctas, size_t sm_bytes, size_t *pad)
+{
+    static const int kb[] = {8, 16, 32, 64, 100, 132, 164, 196, 228};
+    *pad = 0;
+    for (int k : kb)
+    {
+        const size_t bytes = (size_t)k * 1024;
+        if (bytes < block * (size_t)ctas || bytes > sm_bytes) continue;
+        if ((size_t)(ctas + 1) * block <= bytes) *pad = (bytes / (size_t)(ctas + 1) - block) / 128 * 128 + 128;
+        if ((block + *pad) * (size_t)ctas > bytes) *pad = 0;
+        return (int)(100 * bytes / sm_bytes);
+    }
+    return 100;
+}
+
+int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm, size_t *pad)
 {
     /* per (kernel, requested CTAs per SM): the resident CTAs per SM and the
      * carve-out that holds them; the carve-out is a kernel attribute, so it
@@ -135,6 +155,7 @@ int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm)
     {
         const void *kernel;
         int ctas, bps, pct;
+        size_t pad;
     };
     struct Applied
     {
@@ -146,6 +167,7 @@ int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm)
     static Applied applied[64];
     static int nshapes = 0, napplied = 0;
     int bps = 0, pct = 0;
+    size_t extra = 0;
     {
         std::lock_guard<std::mutex> lk(mu);
         int found = -1;
@@ -155,14 +177,13 @@ int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm)
         {
             bps = shapes[found].bps;
             pct = shapes[found].pct;
+            extra = shapes[found].pad;
         }
         else
         {
             cudaError_t e = cudaSuccess;
             if (ctas_per_sm > 0)
             {
-                /* carve-out: the smallest share of the SM's shared-memory
-                 * capacity that holds ctas_per_sm CTAs (1 KB reserved each) */
                 cudaFuncAttributes fa;
                 int dev = 0, smem_sm = 0;
                 e = cudaFuncGetAttributes(&fa, kernel);
@@ -170,9 +191,9 @@ int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm)
                 if (e == cudaSuccess) e = cudaDeviceGetAttribute(&smem_sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
                 if (e == cudaSuccess && smem_sm > 0)
                 {
-                    const double need = (double)ctas_per_sm * (double)(fa.sharedSizeBytes + 1024);
-                    pct = (int)ceil(100.0 * need / (double)smem_sm);
-                    pct = pct < 1 ? 1 : (pct > 100 ? 100 : pct);
+                    /* shared memory is given out in 128 bytes */
+                    pct = carveout_for((fa.sharedSizeBytes + 127) / 128 * 128 + 1024, ctas_per_sm, (size_t)smem_sm, &extra);
+                    if (fa.sharedSizeBytes + extra > 48 * 1024) extra = 0;
                     e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, pct);
                 }
             }
@@ -182,12 +203,13 @@ int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm)
                 cudaGetLastError();
                 bps = 1;
                 pct = 0;
+                extra = 0;
             }
             if (ctas_per_sm > 0 && bps > ctas_per_sm) bps = ctas_per_sm;
             if (getenv("GG_DEBUG"))
                 fprintf(stderr, "gg: kernel %p: %d CTAs of %d threads per SM (%s)\n", kernel, bps, GG_TILE_NT,
                         cudaGetErrorString(e));
-            if (nshapes < 128) shapes[nshapes++] = Shape{kernel, ctas_per_sm, bps, pct};
+            if (nshapes < 128) shapes[nshapes++] = Shape{kernel, ctas_per_sm, bps, pct, extra};
         }
         /* the carve-out applied to this kernel last */
         if (pct > 0)
@@ -209,6 +231,7 @@ int gg_persistent_grid(const void *kernel, uint32_t ntiles, int ctas_per_sm)
             }
         }
     }
+    if (pad) *pad = extra;
     const uint64_t need = ((uint64_t)ntiles + GG_TILE_WARPS - 1) / GG_TILE_WARPS;
     const uint64_t cap = (uint64_t)gg_sm_count() * (uint64_t)bps;
     const uint64_t g = need < cap ? need : cap;

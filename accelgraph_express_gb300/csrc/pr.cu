@@ -991,9 +991,10 @@ gg_status run_pull(Run &R, IterRec *rec, float *rank, uint32_t iters, float base
         }
         else
         {
-            const int pg = gg_persistent_grid((const void *)k_pr_pull<K>, t->ntiles, (int)R.shape.ctas);
+            size_t pad;
+            const int pg = gg_persistent_grid((const void *)k_pr_pull<K>, t->ntiles, (int)R.shape.ctas, &pad);
             if (pdl)
-                GG_CUDA(gg_launch_pdl(k_pr_pull<K>, dim3(pg), dim3(GG_TILE_NT), 0, R.s, g->in_off, g->in_adj, t->coord,
+                GG_CUDA(gg_launch_pdl(k_pr_pull<K>, dim3(pg), dim3(GG_TILE_NT), pad, R.s, g->in_off, g->in_adj, t->coord,
                                       t->ntiles, V, (Acc *)sums, PrGather<K>{cin}, (const IterRec *)rec, it));
             else
                 k_pr_pull<K><<<pg, GG_TILE_NT, 0, R.s>>>(g->in_off, g->in_adj, t->coord, t->ntiles, V, (Acc *)sums,

@@ -301,12 +301,13 @@ gg_status spmv_fp(gg_graph *g, const gg_spmv_params *p, const float *x_dev, floa
             }
             else
             {
-                const dim3 grid(gg_persistent_grid((const void *)k_spmv_pull<T>, t->ntiles, (int)shape.ctas)), block(GG_TILE_NT);
+                size_t pad;
+                const dim3 grid(gg_persistent_grid((const void *)k_spmv_pull<T>, t->ntiles, (int)shape.ctas, &pad)), block(GG_TILE_NT);
                 const SpmvGather<T> op{w, xv};
                 if (p->profile)
                     k_spmv_pull<T><<<grid, block, 0, s>>>(g->in_off, g->in_adj, t->coord, t->ntiles, V, yi, next, op);
                 else
-                    GG_CUDA(gg_launch_pdl(k_spmv_pull<T>, grid, block, 0, s, g->in_off, g->in_adj, t->coord, t->ntiles, V, yi,
+                    GG_CUDA(gg_launch_pdl(k_spmv_pull<T>, grid, block, pad, s, g->in_off, g->in_adj, t->coord, t->ntiles, V, yi,
                                           next, op));
             }
         }

@@ -28,16 +28,31 @@ API void fake_log_clear(void) { g_log_len = 0; g_log[0] = 0; }
 API const char *fake_log(void) { return g_log; }
 
 /* ---- kernels ---- */
-typedef struct { const void *fn; const char *name; } Kernel;
+typedef struct { const void *fn; const char *name; size_t smem; int carveout; } Kernel;
 static Kernel g_kernels[4096];
 static int g_nkernels;
 
-static cudaError_t launched(const void *fn)
+/* of the kernel whose name contains `name`: dynamic shared memory of its last
+ * launch, and its preferred carve-out in percent (0: never set) */
+static Kernel *by_name(const char *name)
+{
+    for (int i = 0; i < g_nkernels; i++)
+        if (strstr(g_kernels[i].name, name)) return &g_kernels[i];
+    abort();
+}
+API long fake_smem(const char *name) { return (long)by_name(name)->smem; }
+API int fake_carveout(const char *name) { return by_name(name)->carveout; }
+static size_t g_shared_size;
+/* static shared memory of every kernel */
+API void fake_shared_size(long n) { g_shared_size = (size_t)n; }
+
+static cudaError_t launched(const void *fn, size_t smem)
 {
     for (int i = 0; i < g_nkernels; i++)
         if (g_kernels[i].fn == fn)
         {
             const size_t n = strlen(g_kernels[i].name);
+            g_kernels[i].smem = smem;
             if (g_log_len + n + 2 > sizeof(g_log)) abort();
             memcpy(g_log + g_log_len, g_kernels[i].name, n);
             g_log_len += n;
@@ -79,33 +94,35 @@ API cudaError_t __cudaPopCallConfiguration(dim3 *g, dim3 *b, size_t *smem, void 
 API cudaError_t __cudaGetKernel(cudaKernel_t *k, const void *fn) { *k = (cudaKernel_t)fn; return cudaSuccess; }
 API cudaError_t __cudaLaunchKernel(cudaKernel_t k, dim3 g, dim3 b, void **a, size_t m, cudaStream_t s)
 {
-    (void)g; (void)b; (void)a; (void)m; (void)s;
-    return launched((const void *)k);
+    (void)g; (void)b; (void)a; (void)s;
+    return launched((const void *)k, m);
 }
 API cudaError_t cudaLaunchKernel(const void *f, dim3 g, dim3 b, void **a, size_t m, cudaStream_t s)
 {
-    (void)g; (void)b; (void)a; (void)m; (void)s;
-    return launched(f);
+    (void)g; (void)b; (void)a; (void)s;
+    return launched(f, m);
 }
 API cudaError_t cudaLaunchKernelExC(const cudaLaunchConfig_t *c, const void *f, void **a)
 {
-    (void)c; (void)a;
-    return launched(f);
+    (void)a;
+    return launched(f, c->dynamicSmemBytes);
 }
 API cudaError_t cudaLaunchCooperativeKernel(const void *f, dim3 g, dim3 b, void **a, size_t m, cudaStream_t s)
 {
-    (void)g; (void)b; (void)a; (void)m; (void)s;
-    return g_coop_error ? (cudaError_t)g_coop_error : launched(f);
+    (void)g; (void)b; (void)a; (void)s;
+    return g_coop_error ? (cudaError_t)g_coop_error : launched(f, m);
 }
 API cudaError_t cudaFuncSetAttribute(const void *f, enum cudaFuncAttribute a, int v)
 {
-    (void)f; (void)a; (void)v;
+    for (int i = 0; i < g_nkernels; i++)
+        if (g_kernels[i].fn == f && a == cudaFuncAttributePreferredSharedMemoryCarveout) g_kernels[i].carveout = v;
     return cudaSuccess;
 }
 API cudaError_t cudaFuncGetAttributes(struct cudaFuncAttributes *a, const void *f)
 {
     (void)f;
     memset(a, 0, sizeof(*a));
+    a->sharedSizeBytes = g_shared_size;
     return cudaSuccess;
 }
 API cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor(int *n, const void *f, int t, size_t m)

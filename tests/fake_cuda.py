@@ -23,6 +23,8 @@ F = gg.lib()
 F.fake_mallocs.restype = C.c_long
 F.fake_fail_mallocs_from.argtypes = [C.c_long]
 F.fake_log.restype = C.c_char_p
+F.fake_smem.restype = C.c_long
+F.fake_shared_size.argtypes = [C.c_long]
 
 def launches():
     return F.fake_log().decode().split()
