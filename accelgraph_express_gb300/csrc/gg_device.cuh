@@ -151,6 +151,20 @@ struct LongSum
         lo = __fadd_rn(__fadd_rn(lo, l), __fadd_rn(e, two_sum(mid, m)));
     }
     __device__ __forceinline__ double value() const { return (double)hi + ((double)mid + (double)lo); }
+    /* lane l: with lane l + o */
+    __device__ __forceinline__ void merge_down(int o)
+    {
+        merge(__shfl_down_sync(0xffffffffu, hi, o), __shfl_down_sync(0xffffffffu, mid, o),
+              __shfl_down_sync(0xffffffffu, lo, o));
+    }
+    /* to `over` if n sums of this size could leave FP32 */
+    __device__ __forceinline__ void spill(int n, double *over)
+    {
+        if (fabsf(hi) <= SUM_MAX / (2 * n)) return;
+        asm volatile("" : "+f"(hi), "+f"(mid), "+f"(lo));
+        atomicAdd(over, value());
+        hi = mid = lo = 0.0f;
+    }
 };
 
 /* the same for the even and the odd vertex of a pair, by packed instructions */
@@ -203,9 +217,7 @@ __device__ __forceinline__ double warp_sum(LongSum s)
 {
     if (__any_sync(0xffffffffu, fabsf(s.hi) > LongSum::SUM_MAX / 64)) return warp_sum(s.value());
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-        s.merge(__shfl_down_sync(0xffffffffu, s.hi, o), __shfl_down_sync(0xffffffffu, s.mid, o),
-                __shfl_down_sync(0xffffffffu, s.lo, o));
+    for (int o = 16; o > 0; o >>= 1) s.merge_down(o);
     return s.value();
 }
 
@@ -224,16 +236,9 @@ __device__ __forceinline__ void block_sum2(LongSum s, uint32_t b, double &a, uin
     const uint32_t t = threadIdx.x, l = t & 31;
     if (t == 0) s_wide = 0.0;
     __syncthreads();
-    if (!(fabsf(s.hi) <= LongSum::SUM_MAX / (2 * NT)))
-    {
-        asm volatile("" : "+f"(s.hi), "+f"(s.mid), "+f"(s.lo));
-        atomicAdd(&s_wide, s.value());
-        s = LongSum();
-    }
+    s.spill(NT, &s_wide);
 #pragma unroll
-    for (int o = 16; o >= 8; o >>= 1)
-        s.merge(__shfl_down_sync(0xffffffffu, s.hi, o), __shfl_down_sync(0xffffffffu, s.mid, o),
-                __shfl_down_sync(0xffffffffu, s.lo, o));
+    for (int o = 16; o >= 8; o >>= 1) s.merge_down(o);
     b = __reduce_add_sync(0xffffffffu, b);
     if (l < 8)
     {

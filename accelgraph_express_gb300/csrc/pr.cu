@@ -511,7 +511,7 @@ struct UpdateStep
 };
 
 template <int K>
-__global__ void k_pr_update(PrCommon c, typename Fmt<K>::Acc *sums, typename Fmt<K>::CT *cout, float *cf)
+__global__ void __launch_bounds__(256, 8) k_pr_update(PrCommon c, typename Fmt<K>::Acc *sums, typename Fmt<K>::CT *cout, float *cf)
 {
     typedef typename Fmt<K>::Acc Acc;
     typedef typename Fmt<K>::CT CT;
@@ -680,7 +680,7 @@ template <> struct Pair16<__half> { typedef __half2 T; static __device__ __force
  * flight to cover DRAM latency.  Every array is a whole allocation (8-byte
  * aligned); an odd last vertex is taken on its own. */
 template <int K>
-__global__ void k_pr_update_delta(PrCommon c, float init, float *__restrict__ dsum, float *__restrict__ S,
+__global__ void __launch_bounds__(256, 6) k_pr_update_delta(PrCommon c, float init, float *__restrict__ dsum, float *__restrict__ S,
                                   float *__restrict__ chat, typename Fmt<K>::CT *__restrict__ qout)
 {
     typedef typename Fmt<K>::CT CT;

@@ -36,7 +36,8 @@ using namespace gg;
 
 constexpr uint32_t SM_THREADS = 1024, SM_WARPS = SM_THREADS / 32;
 constexpr uint32_t SM_END = 0x8000u, SM_ID = 0x7fffu;
-constexpr size_t SM_LIMIT = 220 * 1024;
+constexpr size_t SM_LIMIT = 220 * 1024; /* graphs up to this are taken */
+constexpr size_t SM_MOST = 226 * 1024;  /* dynamic shared memory beside 1 KB of static */
 
 /* per-iteration record, as the launches of pr.cu write it */
 struct SmallRec
@@ -56,6 +57,7 @@ struct SmallArgs
     uint32_t V, E, iterations;
     uint32_t run, eq, vq; /* edges per thread, edges and vertices per CTA */
     uint32_t rows_cap;  /* entries of the row list */
+    uint32_t keep;      /* 1: the ranks an iteration began with stay in shared memory */
     float base, damp, init, eps_f;
     int divide;
 };
@@ -219,52 +221,77 @@ __device__ __forceinline__ void gather_run(const ID *run, uint32_t n, uint32_t s
     if (lane == 31) tail(ends != 0u, seg, sum);
 }
 
+/* shared memory in which small_finish joins the threads' sums */
+constexpr uint32_t SM_JOIN = 2 * 3 * (SM_THREADS / 4) * 4;
+
 /* the ranks of this CTA's vertices, their sum, and the residual of the last
- * iteration run, for which every iteration leaves the ranks that it began with
- * in a.rank: two FP64 sums of a few terms per thread, once */
-__device__ __forceinline__ void small_finish(const SmallArgs &a, const float *rank, uint32_t v0, uint32_t v1, uint32_t it)
+ * iteration run, which began with the ranks in `old`.  The sums stay in FP32 words
+ * (gg_device.cuh) up to one lane: a conversion to FP64 takes the SM about 64 clocks
+ * per warp (a call on 3,000 vertices lost 8 us to two per vertex).  join: SM_JOIN
+ * bytes, which nothing else uses any more */
+__device__ __forceinline__ void small_finish(const SmallArgs &a, const float *rank, const float *old, uint32_t v0,
+                                             uint32_t v1, uint32_t it, float *join)
 {
-    __shared__ double part[2][SM_WARPS];
+    constexpr uint32_t SLOTS = SM_THREADS / 4;
     const uint32_t tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-    double err = 0.0, sum = 0.0;
+    double *to[2] = {&a.rec[it ? it - 1 : 0].err, a.sum};
+    LongSum s[2];
     for (uint32_t i = tid; i < v1 - v0; i += SM_THREADS)
     {
         float r = rank[i];
-        if (it > 0) err += (double)fabsf(__fsub_rn(r, a.rank[v0 + i]));
+        if (it > 0) s[0].add(fabsf(__fsub_rn(r, old[i])), to[0]);
         if (a.divide) r = __fdiv_rn(r, __uint2float_rn(a.V));
         a.rank[v0 + i] = r;
-        sum += (double)r;
+        s[1].add(r, to[1]);
     }
-    err = warp_sum(err);
-    sum = warp_sum(sum);
-    if (lane == 0)
+    __syncthreads();
+#pragma unroll 1
+    for (int k = 0; k < 2; k++)
     {
-        part[0][w] = err;
-        part[1][w] = sum;
+        LongSum t = k ? s[1] : s[0];
+        t.spill(SM_THREADS, k ? to[1] : to[0]);
+#pragma unroll 1
+        for (int o = 16; o >= 8; o >>= 1) t.merge_down(o);
+        float *p = join + k * 3 * SLOTS + w * 8 + lane;
+        if (lane < 8)
+        {
+            p[0] = t.hi;
+            p[SLOTS] = t.mid;
+            p[2 * SLOTS] = t.lo;
+        }
     }
     __syncthreads();
     if (w < 2)
     {
-        const double all = warp_sum(part[w][lane]);
-        double *to = w ? a.sum : &a.rec[it - 1].err;
-        if (lane == 0 && (w || it > 0)) atomicAdd(to, all);
+        LongSum all;
+        const float *p = join + w * 3 * SLOTS + lane;
+#pragma unroll 1
+        for (uint32_t k = 0; k < SLOTS; k += 32) all.merge(p[k], p[SLOTS + k], p[2 * SLOTS + k]);
+#pragma unroll 1
+        for (int o = 16; o > 0; o >>= 1) all.merge_down(o);
+        if (lane == 0 && (w || it > 0)) atomicAdd(w ? to[1] : to[0], all.value());
     }
 }
 
 struct SmallShape
 {
-    size_t ids, rows, c, sums, rank, deg, total;
+    size_t ids, rows, c, sums, rank, deg, old, join, total;
 };
-__host__ __device__ inline SmallShape small_shape(uint32_t V, uint32_t eq, uint32_t vq, uint32_t rows_cap)
+/* keep: with the ranks that an iteration began with */
+__host__ __device__ inline SmallShape small_shape(uint32_t V, uint32_t eq, uint32_t vq, uint32_t rows_cap, uint32_t keep)
 {
     SmallShape s;
     s.c = 0;
     s.sums = s.c + ((size_t)V + 4) / 4 * 16;
     s.rank = s.sums + (size_t)vq * 4;
     s.deg = s.rank + (size_t)vq * 4;
-    s.ids = (s.deg + (size_t)vq * 4 + 15) / 16 * 16;
+    s.old = s.deg + (size_t)vq * 4;
+    s.ids = (s.old + (size_t)vq * 4 * keep + 15) / 16 * 16;
     s.rows = (s.ids + (size_t)eq * 2 + 15) / 16 * 16;
     s.total = (s.rows + (size_t)rows_cap * 4 + 15) / 16 * 16;
+    /* the sums are joined over the contributions, or behind everything */
+    s.join = ((size_t)V + 1) * 4 >= SM_JOIN ? s.c : s.total;
+    if (s.join) s.total += SM_JOIN;
     return s;
 }
 
@@ -276,7 +303,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_small(SmallArgs a)
     __shared__ uint32_t s_total;
     __shared__ uint32_t s_act[3]; /* active counts of the run, iteration mod 3 */
     __shared__ bool s_open;       /* this CTA's first edge continues a row of the CTA before */
-    const SmallShape sh = small_shape(a.V, a.eq, a.vq, a.rows_cap);
+    const SmallShape sh = small_shape(a.V, a.eq, a.vq, a.rows_cap, a.keep);
     float *c = reinterpret_cast<float *>(gg_dyn + sh.c);
     float *sums = reinterpret_cast<float *>(gg_dyn + sh.sums);
     float *rank = reinterpret_cast<float *>(gg_dyn + sh.rank);
@@ -287,6 +314,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_small(SmallArgs a)
     const uint32_t tid = threadIdx.x, lane = tid & 31;
     const uint32_t e0 = min(me * a.eq, a.E), e1 = min(e0 + a.eq, a.E), ne = e1 - e0;
     const uint32_t v0 = min(me * a.vq, a.V), v1 = min(v0 + a.vq, a.V);
+    float *old = a.keep ? reinterpret_cast<float *>(gg_dyn + sh.old) : a.rank + v0;
     /* the warps with edges; their threads' runs are padded with the id V,
      * whose contribution is 0 */
     const uint32_t wedges = 32 * a.run, nwork = (ne + wedges - 1) / wedges;
@@ -370,7 +398,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_small(SmallArgs a)
             sums[i] = 0.0f;
             const float nr = __fadd_rn(a.base, __fmul_rn(a.damp, s));
             const float e = fabsf(__fsub_rn(nr, rank[i]));
-            a.rank[v0 + i] = rank[i];
+            old[i] = rank[i];
             rank[i] = nr;
             if (e >= a.eps_f) act++;
             const uint32_t d = deg[i];
@@ -392,7 +420,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_small(SmallArgs a)
             break;
         }
     }
-    small_finish(a, rank, v0, v1, it);
+    small_finish(a, rank, old, v0, v1, it, reinterpret_cast<float *>(gg_dyn + sh.join));
     M::sync(); /* no CTA leaves while another may still write its memory */
 }
 
@@ -427,6 +455,7 @@ __host__ __device__ inline GridShape grid_shape(uint32_t eq, uint32_t vq, uint32
     GridShape s;
     s.rows = (size_t)eq * 4;
     s.rank = s.rows + (size_t)rows_cap * 4;
+    if (s.rank < SM_JOIN) s.rank = SM_JOIN; /* the sums are joined over the ids and rows */
     s.deg = s.rank + (size_t)vq * 4;
     s.total = (s.deg + (size_t)vq * 4 + 15) / 16 * 16;
     return s;
@@ -502,6 +531,9 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_grid(GridArgs ga)
     const uint32_t me = blockIdx.x, tid = threadIdx.x, lane = tid & 31;
     const uint32_t e0 = (uint32_t)min((uint64_t)me * a.eq, (uint64_t)a.E), e1 = min(e0 + a.eq, a.E), ne = e1 - e0;
     const uint32_t v0 = (uint32_t)min((uint64_t)me * a.vq, (uint64_t)a.V), v1 = min(v0 + a.vq, a.V);
+    /* the ranks that an iteration began with (in shared memory: 150K vertices, 750K
+     * edges 241 us a call against 226) */
+    float *old = a.rank + v0;
     const uint32_t wedges = 32 * a.run, nwork = (ne + wedges - 1) / wedges;
     const bool work = (tid >> 5) < nwork;
 
@@ -621,7 +653,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_grid(GridArgs ga)
             sums[v0 + i] = 0.0f;
             const float nr = __fadd_rn(a.base, __fmul_rn(a.damp, s));
             const float e = fabsf(__fsub_rn(nr, rank[i]));
-            a.rank[v0 + i] = rank[i];
+            old[i] = rank[i];
             rank[i] = nr;
             if (e >= a.eps_f) act++;
             const uint32_t d = deg[i];
@@ -641,7 +673,7 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_grid(GridArgs ga)
         }
     }
     if (!ok) return; /* the host reports it */
-    small_finish(a, rank, v0, v1, it);
+    small_finish(a, rank, old, v0, v1, it, reinterpret_cast<float *>(gg_dyn));
 }
 
 /* Edges per thread (of 152 SMs: 2.5M edges) and vertices above which the
@@ -695,8 +727,14 @@ bool small_plan(uint32_t V, uint32_t E, SmallArgs &a, uint32_t &C, size_t &smem)
     a.eq = ((E + C - 1) / C + wedges - 1) / wedges * wedges;
     a.vq = ((V + C - 1) / C + 3) / 4 * 4;
     a.rows_cap = std::min(V, a.eq) + 1;
-    smem = small_shape(V, a.eq, a.vq, a.rows_cap).total;
-    return smem <= SM_LIMIT;
+    smem = small_shape(V, a.eq, a.vq, a.rows_cap, 0).total;
+    if (smem > SM_LIMIT) return false;
+    /* without the room, the ranks that an iteration began with go to global memory
+     * (a call on 3,000 vertices with 15K edges: 101 us there, 92 in shared) */
+    const size_t with = small_shape(V, a.eq, a.vq, a.rows_cap, 1).total;
+    a.keep = with <= SM_MOST ? 1u : 0u;
+    if (a.keep) smem = with;
+    return true;
 }
 
 } // namespace
@@ -742,7 +780,7 @@ gg_status gg_small_pagerank(gg_graph *g, const gg_pr_params *p, float *rank, voi
         return GG_OK;
     }
     void (*fn)(SmallArgs) = C > 1 ? k_pr_small<true> : k_pr_small<false>;
-    GG_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_LIMIT));
+    GG_CUDA(cudaFuncSetAttribute((const void *)fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_MOST));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(C);
     cfg.blockDim = dim3(SM_THREADS);
