@@ -669,8 +669,8 @@ class DeviceGraph:
 
     def pagerank(self, mode="pull", storage="f32", iterations=20, epsilon=1e-4, init_one_over_n=False,
                  damp=0.85, profile=False, copy_out=True, stream=None, cuda_graph=False, hot=None):
-        """hot: None = the library's choice (hot-vertex table from 8M edges),
-        True / False = force it on / off (the pull modes)."""
+        """hot: None = the library's choice (hot-vertex table from 8M edges, by a
+        sample of the graph), True / False = force it on / off (the pull modes)."""
         p = PrParams(PR_MODES[mode] if isinstance(mode, str) else mode, STORE[storage], iterations,
                      int(init_one_over_n), epsilon, damp, int(profile), _pr_flags(cuda_graph, hot))
         r = PrResult()

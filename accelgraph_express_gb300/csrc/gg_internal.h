@@ -117,12 +117,14 @@ struct gg_graph
     uint32_t ppr_stride = 0;
     /* hot-vertex table: flag-encoded copy of in_adj and the slot -> vertex list */
     uint32_t *hot_adj = nullptr;
-    uint32_t *hot_list = nullptr;  /* GG_HOT_ENTRIES slots, then the counts (hot_taken) */
+    uint32_t *hot_list = nullptr;  /* GG_HOT_ENTRIES slots, then the counts (hot_taken) and the sample's */
     uint32_t hot_slots = 0;        /* slots there are: hot_cap, or V if that is less */
     uint32_t hot_cap = 0;          /* table capacity the encoding was made for */
     uint32_t *push_tags = nullptr; /* frequent destinations (gg_push_tags) */
     bool push_hubs = false;        /* they are frequent enough for the table */
     uint64_t push_edges = 0;       /* edges scattered without them */
+    uint32_t hot_threshold = 0;    /* table capacity that the threshold degree is of */
+    uint8_t hot_choice[2][6] = {}; /* by [weighted][log2 of the ids per 32-byte sector] */
     uint64_t plain_its = 0;        /* gathers done without the table since it was last made */
     uint32_t *hot_seg0 = nullptr;  /* per tile of hot_tile edges: its first row end (gg_hot.cuh) */
     uint32_t hot_ntiles = 0, hot_tile = 0; /* tiles and edges per tile */
@@ -219,14 +221,18 @@ gg_status gg_apply_labels(const uint32_t *ids, uint64_t n, const uint32_t *label
 #define GG_STAGE_VALUES ((size_t)65536)
 /* the mapping's page-locked host scratch, at least `bytes` long */
 gg_status gg_pinned(gg_graph *g, size_t bytes, void **out);
-/* build the hot-vertex table of the mapping for a table of `cap` entries
- * (<= GG_HOT_ENTRIES; rebuilt only when cap changes; needs GG_MAP_IN and
- * gg_hot_fits), and the rows and tiles of the hot kernels */
-gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap);
-/* whether a call of `iterations` gathers takes the table of `cap` entries:
- * asked for by the flags, chosen by the tuner (hot 0/1), or by the rule of
- * GG_HOT_MIN_E and GG_HOT_PAYS; the graph passes gg_hot_fits (hot.cu) */
-bool gg_hot_wanted(gg_graph *g, uint32_t flags, uint32_t hot, uint32_t cap, uint32_t iterations);
+/* whether a call of `iterations` gathers takes the hot-vertex table of `cap`
+ * entries (values of `bytes` bytes): asked for by the flags, chosen by the tuner
+ * (shape->hot 0/1), or by the rule of GG_HOT_MIN_E, GG_HOT_PAYS and a sample of the
+ * graph (hot.cu).  Then the table, rows and tiles are prepared (once per mapping and
+ * cap), and *use is set; where the sample says that the plain gather is the faster
+ * one, shape->ctas is set for it */
+struct gg_hot_ask
+{
+    uint32_t flags, cap, bytes, iterations;
+    bool weighted;
+};
+gg_status gg_hot_choose(gg_graph *g, cudaStream_t s, const gg_hot_ask &ask, gg_pull_shape *shape, bool *use);
 /* rows_list of the mapping, and for tiles of `tile` edges the first row end in
  * each (bit 31: that row began in an earlier tile) in a new allocation of
  * *ntiles words; adds its launches to *launches (hot.cu) */
@@ -234,6 +240,8 @@ bool gg_hot_wanted(gg_graph *g, uint32_t flags, uint32_t hot, uint32_t cap, uint
 gg_status gg_rows_tiles(gg_graph *g, cudaStream_t s, uint32_t tile, uint32_t **seg0, uint32_t *ntiles,
                         uint32_t *launches);
 cudaStream_t gg_stream(gg_graph *g, void *user_stream);
+/* host wait on a recorded event, bounded by the wait limit */
+gg_status gg_wait_event(cudaEvent_t ev);
 /* host wait on all work queued on `s`, bounded by the wait limit */
 gg_status gg_wait(cudaStream_t s);
 
@@ -309,6 +317,10 @@ int gg_occupancy(const void *kernel, int threads, size_t smem);
  * in-neighbours' values (skewed graphs concentrate most gathers on a few
  * thousand sectors); more hide more latency. */
 #define GG_PULL_CTAS_PER_SM 5
+/* ... and of graphs whose neighbours lie close together, which need less of the L1
+ * (20 iterations, 67M edges, neighbours within 1,000 ids 4.51 -> 4.27 ms, blocks of
+ * 4,096 4.80 -> 4.56; 904M edges of block-diagonal graphs 72.5 -> 70.8) */
+#define GG_PULL_CTAS_LOCAL 6
 
 /* control block bytes of gg::grid_barrier (gg_device.cuh) */
 #define GG_BAR_BYTES (1024 + 128 * 16)
@@ -346,7 +358,9 @@ unsigned long long gg_barrier_limit_ns();
 /* ids need two flag bits; edge numbers a tile round's headroom in 32 bits */
 #define GG_HOT_MAX_V 0x40000000u
 #define GG_HOT_MAX_E 0xfc000000u
-#define GG_HOT_LIST_BYTES (((size_t)GG_HOT_ENTRIES + 4) * 4)
+#define GG_HOT_LIST_BYTES (((size_t)GG_HOT_ENTRIES + 8) * 4)
+/* what the sample of a graph says (hot.cu) */
+enum { GG_HOT_UNKNOWN, GG_HOT_TABLE, GG_HOT_PLAIN };
 /* whether the hot-vertex gather can run on a graph of these sizes */
 inline bool gg_hot_fits(uint32_t V, uint32_t E) { return V > 0 && E > 0 && V < GG_HOT_MAX_V && E <= GG_HOT_MAX_E; }
 /* many-graphs PageRank (graphs.cu): tile coordinates and size order for the

@@ -514,7 +514,7 @@ cudaStream_t gg_stream(gg_graph *g, void *user_stream)
 }
 
 /* Bounded host wait on a recorded event. */
-static gg_status wait_event(cudaEvent_t ev)
+gg_status gg_wait_event(cudaEvent_t ev)
 {
     cudaError_t e;
     const auto t0 = std::chrono::steady_clock::now();
@@ -550,7 +550,7 @@ gg_status gg_wait(cudaStream_t s)
         cudaEvent_t ev;
         GG_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
         cudaError_t e = cudaEventRecord(ev, s);
-        const gg_status st = e == cudaSuccess ? wait_event(ev) : gg_cuda_fail(e, "cudaEventRecord");
+        const gg_status st = e == cudaSuccess ? gg_wait_event(ev) : gg_cuda_fail(e, "cudaEventRecord");
         cudaEventDestroy(ev);
         return st;
     }
@@ -565,7 +565,7 @@ gg_status gg_wait(cudaStream_t s)
         e = cudaEventRecord(ev, s);
         if (e != cudaSuccess) return gg_cuda_fail(e, "cudaEventRecord");
     }
-    return wait_event(ev);
+    return gg_wait_event(ev);
 }
 
 /* ---- copies between HBM and pageable host memory -------------------------
@@ -716,7 +716,7 @@ gg_status gg_copy_h2d(void *dst, const void *src, size_t bytes, cudaStream_t s)
     for (size_t off = 0, i = 0; off < bytes; off += STAGE_BYTES, i++)
     {
         const int b = (int)(i & 1);
-        if (used[b]) GG_CHECK(wait_event(g_stage_ev[b])); /* its last DMA has read the buffer */
+        if (used[b]) GG_CHECK(gg_wait_event(g_stage_ev[b])); /* its last DMA has read the buffer */
         const size_t n = bytes - off < STAGE_BYTES ? bytes - off : STAGE_BYTES;
         parallel_copy(g_stage[b], (const unsigned char *)src + off, n);
         GG_CUDA(cudaMemcpyAsync((unsigned char *)dst + off, g_stage[b], n, cudaMemcpyHostToDevice, s));
@@ -725,7 +725,7 @@ gg_status gg_copy_h2d(void *dst, const void *src, size_t bytes, cudaStream_t s)
     }
     /* the buffers go back to other callers only once their DMAs are done */
     for (int b = 0; b < 2; b++)
-        if (used[b]) GG_CHECK(wait_event(g_stage_ev[b]));
+        if (used[b]) GG_CHECK(gg_wait_event(g_stage_ev[b]));
     return GG_OK;
 }
 
@@ -790,7 +790,7 @@ gg_status gg_copy_d2h(void *dst, const void *src, size_t bytes, cudaStream_t s)
             const size_t k = i - 1;
             const int b = (int)(k & 1);
             const size_t off = k * STAGE_BYTES, n = bytes - off < STAGE_BYTES ? bytes - off : STAGE_BYTES;
-            GG_CHECK(wait_event(g_stage_ev[b]));
+            GG_CHECK(gg_wait_event(g_stage_ev[b]));
             parallel_copy((unsigned char *)dst + off, g_stage[b], n);
         }
     }

@@ -197,6 +197,51 @@ __global__ void __launch_bounds__(1024) k_hot_encode(const uint32_t *__restrict_
     if (blockIdx.x == 0 && threadIdx.x < GG_EDGE_PAD) out[n + threadIdx.x] = GG_HOT_FLAG | cap;
 }
 
+/* What the choice between the gathers turns on (gg_hot_choose): SAMPLE_WINDOWS
+ * windows of consecutive edges, evenly spaced.  out[0] += 32-byte sectors of the
+ * values in each window (L1 misses of a CTA of the plain gather, whose warps take
+ * about that many consecutive edges), out[1] += edges that the table would serve
+ * (threshold degree in cnt[2]). */
+constexpr uint32_t SAMPLE_WINDOWS = 304, SAMPLE_EDGES = GG_TILE_ITEMS * GG_TILE_WARPS, SAMPLE_SLOTS = 4096;
+constexpr uint32_t SAMPLE_PER = 3, SAMPLE_NT = SAMPLE_EDGES / SAMPLE_PER;
+static_assert(SAMPLE_NT * SAMPLE_PER == SAMPLE_EDGES && SAMPLE_NT % 32 == 0, "whole warps");
+
+/* E is at least GG_HOT_MIN_E: the windows do not overlap */
+__global__ void __launch_bounds__(SAMPLE_NT) k_hot_sample(const uint32_t *__restrict__ adj, uint32_t E,
+                                                    const uint32_t *__restrict__ outdeg,
+                                                    const uint32_t *__restrict__ cnt, uint32_t shift, uint32_t *out)
+{
+    __shared__ uint32_t seen[SAMPLE_SLOTS];
+    const uint32_t T = cnt[2], e0 = (uint32_t)((uint64_t)E * blockIdx.x / gridDim.x) + threadIdx.x;
+    uint32_t u[SAMPLE_PER], fresh = 0, served = 0;
+#pragma unroll
+    for (uint32_t k = 0; k < SAMPLE_PER; k++) u[k] = adj[e0 + k * SAMPLE_NT];
+    for (uint32_t i = threadIdx.x; i < SAMPLE_SLOTS; i += SAMPLE_NT) seen[i] = NO_SLOT; /* no sector: ids are below 2^30 */
+#pragma unroll
+    for (uint32_t k = 0; k < SAMPLE_PER; k++) served += min(outdeg[u[k]], 65535u) > T;
+    __syncthreads();
+#pragma unroll
+    for (uint32_t k = 0; k < SAMPLE_PER; k++)
+    {
+        const uint32_t sector = u[k] >> shift;
+        uint32_t at = (sector * 0x9E3779B1u) >> 20;
+        for (;;) /* at most SAMPLE_EDGES of SAMPLE_SLOTS are taken */
+        {
+            const uint32_t was = atomicCAS(&seen[at], NO_SLOT, sector);
+            fresh += was == NO_SLOT;
+            if (was == NO_SLOT || was == sector) break;
+            at = (at + 1u) & (SAMPLE_SLOTS - 1u);
+        }
+    }
+    fresh = __reduce_add_sync(0xffffffffu, fresh);
+    served = __reduce_add_sync(0xffffffffu, served);
+    if ((threadIdx.x & 31) == 0)
+    {
+        atomicAdd(out, fresh);
+        atomicAdd(out + 1, served);
+    }
+}
+
 /* ---- rows with edges ---- */
 
 constexpr uint32_t ROW_BLOCK = 256, ROW_PER = 8, ROW_TILE = ROW_BLOCK * ROW_PER;
@@ -398,45 +443,53 @@ static uint32_t hot_tile_for(uint32_t E)
     return tile;
 }
 
-bool gg_hot_wanted(gg_graph *g, uint32_t flags, uint32_t hot, uint32_t cap, uint32_t iterations)
+/* threshold degree of a table of `cap` entries, behind the hot list */
+static gg_status hot_threshold(gg_graph *g, cudaStream_t s, uint32_t cap)
 {
-    if (flags & GG_PR_HOT_OFF) return false;
-    if (flags & GG_PR_HOT_ON) return true;
-    if (hot != 2) return hot == 1;
-    if (g->E < GG_HOT_MIN_E) return false;
-    if (g->hot_adj && g->hot_cap == cap) return true;
-    const uint64_t its = g->plain_its + iterations;
-    if (its > 2 && (its - 2) * g->E >= GG_HOT_PAYS) return true;
-    g->plain_its = its;
-    return false;
+    if (g->hot_threshold == cap) return GG_OK;
+    const uint32_t V = g->V, H = V < cap ? V : cap;
+    void *hist;
+    GG_CHECK(gg_work(g, 25, 65536 * 4, &hist));
+    if (!g->hot_list) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_list, GG_HOT_LIST_BYTES));
+    g->hot_threshold = 0;
+    GG_CUDA(cudaMemsetAsync(hist, 0, 65536 * 4, s));
+    k_deg_hist<<<gg_sm_count() * 2, 256, 0, s>>>(g->out_deg, V, (uint32_t *)hist);
+    k_hot_threshold<<<1, 1024, 0, s>>>((const uint32_t *)hist, H, g->hot_list + GG_HOT_ENTRIES);
+    GG_CUDA(cudaGetLastError());
+    g->hot_threshold = cap;
+    return GG_OK;
 }
 
-gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap)
+/* the rows with edges and the first row end of every tile */
+static gg_status hot_rows(gg_graph *g, cudaStream_t s)
 {
-    if (!g->in_adj || !g->out_deg) return gg_fail(GG_ERR_INVALID, "the hot-vertex table needs GG_MAP_IN");
-    const uint32_t V = g->V, E = g->E;
-    if (!gg_hot_fits(V, E)) return gg_fail(GG_ERR_INVALID, "graph too large for flag-encoded ids");
-    if (cap < 1 || cap > GG_HOT_ENTRIES) return gg_fail(GG_ERR_INVALID, "hot table capacity out of range");
-    if (!g->hot_seg0)
-    {
-        uint32_t launches = 0;
-        g->hot_tile = hot_tile_for(E);
-        GG_CHECK(gg_rows_tiles(g, s, g->hot_tile, &g->hot_seg0, &g->hot_ntiles, &launches));
-    }
+    uint32_t launches = 0;
+    if (g->hot_seg0) return GG_OK;
+    g->hot_tile = hot_tile_for(g->E);
+    return gg_rows_tiles(g, s, g->hot_tile, &g->hot_seg0, &g->hot_ntiles, &launches);
+}
+
+/* the encoded ids' memory, and a slot per vertex */
+static gg_status hot_memory(gg_graph *g, void **slot_of)
+{
+    GG_CHECK(gg_work(g, 26, (size_t)g->V * 4, slot_of));
+    if (!g->hot_adj) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_adj, ((size_t)g->E + GG_EDGE_PAD) * 4));
+    return GG_OK;
+}
+
+/* the table's encoded ids and list, and the rows and tiles of its gathers */
+static gg_status hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap)
+{
+    const uint32_t V = g->V, E = g->E, H = V < cap ? V : cap;
+    GG_CHECK(hot_rows(g, s));
     if (g->hot_adj && g->hot_cap == cap) return GG_OK;
-    const uint32_t H = V < cap ? V : cap;
-    void *hist, *slot_of;
-    GG_CHECK(gg_work(g, 25, 65536 * 4, &hist));
-    GG_CHECK(gg_work(g, 26, (size_t)V * 4, &slot_of));
-    if (!g->hot_list) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_list, GG_HOT_LIST_BYTES));
-    if (!g->hot_adj) GG_CHECK(gg_dev_alloc(g, (void **)&g->hot_adj, ((size_t)E + GG_EDGE_PAD) * 4));
+    GG_CHECK(hot_threshold(g, s, cap));
+    void *slot_of;
+    GG_CHECK(hot_memory(g, &slot_of));
     uint32_t *cnt = g->hot_list + GG_HOT_ENTRIES;
     g->hot_cap = 0; /* until the list and the ids are written */
-    GG_CUDA(cudaMemsetAsync(hist, 0, 65536 * 4, s));
-    GG_CUDA(cudaMemsetAsync(cnt, 0, 16, s));
+    GG_CUDA(cudaMemsetAsync(cnt, 0, 8, s));
     const int grid = gg_sm_count() * 8;
-    k_deg_hist<<<gg_sm_count() * 2, 256, 0, s>>>(g->out_deg, V, (uint32_t *)hist);
-    k_hot_threshold<<<1, 1024, 0, s>>>((const uint32_t *)hist, H, cnt);
     k_hot_mark<<<grid, 256, 0, s>>>(g->out_deg, V, H, (uint32_t *)slot_of, g->hot_list, cnt);
     /* one CTA of 1024 threads per SM (60 registers a thread); adj and out are
      * whole allocations, 16-byte aligned for the vector loads */
@@ -448,5 +501,85 @@ gg_status gg_hot_prepare(gg_graph *g, cudaStream_t s, uint32_t cap)
     g->plain_its = 0;
     g->hot_slots = H;
     g->hot_cap = cap;
+    return GG_OK;
+}
+
+/* Whether the plain gather is the faster one on this graph.  It reads through L1,
+ * the table's does not (gg_hot.cuh), so it wins where most neighbours of nearby
+ * rows lie close together: meshes, orders with locality, unions of small graphs.
+ * With h the share of a window's edges that find their sector read already and s
+ * the share that the table serves, a gather takes, in ps per edge (PageRank /
+ * SpMV),
+ *     plain   2.55 / 2.9  +  4.0 / 4.5 V / E  +  1.8 / 2.3 (1 - h)^2
+ *     table   3.73 / 4.0 (1 - s)  +  0.52 / 0 h
+ * Measured us per gather of 67M edges between 4.2M vertices, plain : table.
+ * PageRank: neighbours within 1,000 ids (h 0.78) 191 : 271, 3,000 (0.49) 220 : 251,
+ * 10,000 (0.20) 265 : 250, uniform random (0) 295 : 252, R-MAT (0.14, s 0.48) 232 :
+ * 139, half R-MAT half within 1,000 (0.40, 0.25) 225 : 194.  SpMV: within 1,000 215 :
+ * 269, blocks of 4,096 (0.60) 226 : 266, within 10,000 312 : 266; a mesh of 16.7M
+ * vertices (0.90) 267 : 252. */
+static bool plain_is_faster(double V, double E, double h, double s, bool weighted)
+{
+    const double miss = (1.0 - h) * (1.0 - h);
+    return weighted ? 2.9 + 4.5 * V / E + 2.3 * miss < 4.0 * (1.0 - s)
+                    : 2.55 + 4.0 * V / E + 1.8 * miss < 3.73 * (1.0 - s) + 0.52 * h;
+}
+
+gg_status gg_hot_choose(gg_graph *g, cudaStream_t s, const gg_hot_ask &ask, gg_pull_shape *shape, bool *use)
+{
+    *use = false;
+    if ((ask.flags & GG_PR_HOT_OFF) || !gg_hot_fits(g->V, g->E)) return GG_OK;
+    if (!(ask.flags & GG_PR_HOT_ON) && shape->hot == 0) return GG_OK;
+    const bool by_rule = !(ask.flags & GG_PR_HOT_ON) && shape->hot == 2;
+    if (by_rule && g->E < GG_HOT_MIN_E) return GG_OK;
+    if (!g->in_adj || !g->out_deg) return gg_fail(GG_ERR_INVALID, "the hot-vertex table needs GG_MAP_IN");
+    if (by_rule)
+    {
+        uint32_t shift = 5; /* ids to sectors of 32 bytes */
+        while ((32u >> shift) < ask.bytes) shift--;
+        uint8_t &choice = g->hot_choice[ask.weighted ? 1 : 0][shift];
+        if (choice != GG_HOT_PLAIN && !(g->hot_adj && g->hot_cap == ask.cap))
+        {
+            const uint64_t its = g->plain_its + ask.iterations;
+            if (its <= 2 || (its - 2) * g->E < GG_HOT_PAYS)
+            {
+                g->plain_its = its;
+                return GG_OK;
+            }
+        }
+        if (choice == GG_HOT_UNKNOWN)
+        {
+            /* the host allocates, and waits for the sample, beside the passes over
+             * the degrees and rows */
+            void *pin, *slot_of;
+            const bool had = g->hot_adj != nullptr;
+            GG_CHECK(gg_pinned(g, 64, &pin));
+            GG_CHECK(hot_threshold(g, s, ask.cap));
+            uint32_t *cnt = g->hot_list + GG_HOT_ENTRIES, *out = cnt + 4;
+            GG_CUDA(cudaMemsetAsync(out, 0, 8, s));
+            k_hot_sample<<<SAMPLE_WINDOWS, SAMPLE_NT, 0, s>>>(g->in_adj, g->E, g->out_deg, cnt, shift, out);
+            GG_CUDA(cudaGetLastError());
+            GG_CUDA(cudaMemcpyAsync(pin, out, 8, cudaMemcpyDeviceToHost, s));
+            GG_CUDA(cudaEventRecord(g->ev_begin, s));
+            GG_CHECK(hot_rows(g, s));
+            GG_CHECK(hot_memory(g, &slot_of));
+            GG_CHECK(gg_wait_event(g->ev_begin));
+            const volatile uint32_t *got = (const volatile uint32_t *)pin;
+            const double n = (double)SAMPLE_WINDOWS * SAMPLE_EDGES;
+            choice = plain_is_faster(g->V, g->E, 1.0 - got[0] / n, got[1] / n, ask.weighted) ? GG_HOT_PLAIN : GG_HOT_TABLE;
+            if (choice == GG_HOT_PLAIN && !had)
+            {
+                gg_dev_free(g, g->hot_adj, ((size_t)g->E + GG_EDGE_PAD) * 4);
+                g->hot_adj = nullptr;
+            }
+        }
+        if (choice == GG_HOT_PLAIN)
+        {
+            shape->ctas = GG_PULL_CTAS_LOCAL;
+            return GG_OK;
+        }
+    }
+    GG_CHECK(hot_prepare(g, s, ask.cap));
+    *use = true;
     return GG_OK;
 }

@@ -1439,17 +1439,13 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
     gg_tune_lookup(g, R.s);
     R.shape = g->pr_shape;
     const uint32_t vb = value_bytes(p);
-    if (vb && gg_hot_fits(V, g->E))
+    if (vb)
     {
         const uint32_t cap = vb == 8   ? hot_cap<unsigned long long>()
                              : vb == 4 ? hot_cap<uint32_t>()
                              : vb == 2 ? hot_cap<uint16_t>()
                                        : hot_cap<uint8_t>();
-        if (gg_hot_wanted(g, p->flags, R.shape.hot, cap, p->max_iterations))
-        {
-            GG_CHECK(gg_hot_prepare(g, R.s, cap));
-            R.use_hot = true;
-        }
+        GG_CHECK(gg_hot_choose(g, R.s, gg_hot_ask{p->flags, cap, vb, iters, false}, &R.shape, &R.use_hot));
     }
 
     if (p->mode == GG_PR_PUSH || p->mode == GG_PR_PUSH_FX64)

@@ -266,14 +266,14 @@ gg_status spmv_fp(gg_graph *g, const gg_spmv_params *p, const float *x_dev, floa
     bool use_hot = false;
     void *hot_tab = nullptr;
     gg_tune_lookup(g, s);
-    const gg_pull_shape shape = g->spmv_shape;
-    if (pull && gg_hot_fits(V, g->E) && gg_hot_wanted(g, p->flags, shape.hot, hot_cap<T>(), p->iterations))
+    gg_pull_shape shape = g->spmv_shape;
+    if (pull)
+        GG_CHECK(gg_hot_choose(g, s, gg_hot_ask{p->flags, hot_cap<T>(), (uint32_t)sizeof(T), p->iterations, true}, &shape, &use_hot));
+    if (use_hot)
     {
-        GG_CHECK(gg_hot_prepare(g, s, hot_cap<T>()));
         GG_CHECK(gg_work(g, 32, GG_HOT_TABLE_BYTES + 16, &hot_tab));
         k_spmv_hot_fill<T><<<(hot_cap<T>() + 255) / 256, 256, 0, s>>>(xv, g->hot_list, g->hot_slots, hot_cap<T>(), (T *)hot_tab);
         launches++;
-        use_hot = true;
     }
     const uint32_t *tags = nullptr;
     if (!pull) GG_CHECK(gg_push_tags(g, p->iterations, s, &tags));

@@ -191,9 +191,10 @@ typedef struct gg_pr_params
 /* The pull gather (every pull mode; SpMV pull in FP) serves the values of the
  * vertices with the most out-edges -- 40K FP32, 80K 16- or 8-bit, 20K 64-bit
  * ones -- from a shared-memory table (built once per mapping; an extra copy of
- * the CSC ids).  By default from 8M edges up, made once the
- * gathers done and asked for would repay it; HOT_OFF never, HOT_ON on any graph
- * with edges (below 2^30 vertices).  Results are the same. */
+ * the CSC ids).  By default from 8M edges up, made once the gathers done and
+ * asked for would repay it, on graphs whose neighbours do not lie close together
+ * (a sample of the graph decides); HOT_OFF never, HOT_ON on any graph with edges
+ * (below 2^30 vertices).  Results are the same. */
 #define GG_PR_HOT_OFF 0x2u
 #define GG_PR_HOT_ON 0x4u
 /* gg_pagerank_batch: run the ordinary pull over the union of the graphs
