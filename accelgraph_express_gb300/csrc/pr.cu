@@ -1438,8 +1438,15 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
     /* the hot-vertex table of the pull modes (prepared before any capture) */
     gg_tune_lookup(g, R.s);
     R.shape = g->pr_shape;
+    /* a graph of up to 2.5M edges and 220K vertices: every iteration in one
+     * launch, faster at every size it takes (small.cu); timed runs time each
+     * gather launch, and a table asked for by the call is used (a tuned shape says
+     * which of the gather launches is fastest, and none of them is: 1M edges 249 us
+     * a call against 210) */
+    R.small = one_launch && p->mode == GG_PR_PULL && p->storage == GG_STORE_F32 && !ngraphs && !p->profile &&
+              !(p->flags & GG_PR_HOT_ON) && gg_small_fits(g);
     const uint32_t vb = value_bytes(p);
-    if (vb)
+    if (vb && !R.small)
     {
         const uint32_t cap = vb == 8   ? hot_cap<unsigned long long>()
                              : vb == 4 ? hot_cap<uint32_t>()
@@ -1450,12 +1457,6 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
 
     if (p->mode == GG_PR_PUSH || p->mode == GG_PR_PUSH_FX64)
         GG_CHECK(gg_push_tags(g, iters, R.s, &R.push_tags));
-
-    /* a graph of up to 2.5M edges and 220K vertices: every iteration in one
-     * launch, faster at every size it takes (small.cu); timed runs time each
-     * gather launch, and a table asked for is used */
-    R.small = one_launch && p->mode == GG_PR_PULL && p->storage == GG_STORE_F32 && !ngraphs && !p->profile && !R.use_hot &&
-              gg_small_fits(g);
 
     /* with GG_PR_CUDA_GRAPH everything from here to the final normalisation is
      * captured into one CUDA graph (over buffers reserved before) and

@@ -15,7 +15,8 @@
  *   PR, SPMV  the FP pull gather of PageRank / SpMV: the hot-vertex table off
  *             with 3, 4, 5, 6 or 8 resident CTAs per SM, or on with one CTA
  *             of 16, 24 or 32 warps per SM; measured: mean device time of a
- *             gather launch (profile events);
+ *             gather launch (profile events).  An FP32 PageRank of a graph that
+ *             one launch takes (small.cu) uses no gather launch, tuned or not;
  *   BFS       the top-down heavy-vertex threshold (32, 64, 128, 256, 1024
  *             out-edges) of the direction-optimising search; measured: device
  *             time of eight searches from fixed sources;
