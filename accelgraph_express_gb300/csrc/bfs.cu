@@ -833,17 +833,19 @@ gg_status read_counters(Bfs &B)
     return GG_OK;
 }
 
-/* top-down from queue `q` (qlen) into queue `nq` (and bitmap `nbm`) */
-gg_status td_step(Bfs &B, const uint32_t *q, uint32_t qlen, uint32_t *nq, uint32_t *nbm, uint32_t newdist)
+constexpr uint64_t EDGES_UNKNOWN = ~0ull;
+
+/* top-down from queue `q` (qlen vertices with `edges` out-edges) into queue `nq`
+ * (and bitmap `nbm`) */
+gg_status td_step(Bfs &B, const uint32_t *q, uint32_t qlen, uint64_t edges, uint32_t *nq, uint32_t *nbm, uint32_t newdist)
 {
     GG_CUDA(cudaMemsetAsync(B.c, 0, sizeof(Counters), B.s));
     if (nbm) GG_CUDA(cudaMemsetAsync(nbm, 0, (size_t)B.words * 4, B.s));
     GG_CHECK(mark(B));
     if (qlen)
     {
-        /* the second list only where the first may overflow: by the step's
-         * edges, the claims of the step before (the source has one vertex) */
-        const bool huge = qlen > TD_MAX_HEAVY && (uint64_t)B.h->mf > (uint64_t)TD_MAX_HEAVY * B.g->bfs_heavy;
+        /* the second list only where the first may overflow */
+        const bool huge = qlen > TD_MAX_HEAVY && edges > (uint64_t)TD_MAX_HEAVY * B.g->bfs_heavy;
         (huge ? k_td<true> : k_td<false>)<<<cap_blocks((uint64_t)qlen * 32), 256, 0, B.s>>>(
             q, qlen, B.g->out_off, B.g->out_adj, B.parents, B.dist, newdist, B.visited, nq, nbm, B.c, B.heavy, B.g->bfs_heavy);
         k_td_heavy<<<gg_sm_count() * 8, 256, 0, B.s>>>(B.heavy, B.g->out_adj, B.parents, B.dist, newdist, B.visited,
@@ -1043,9 +1045,11 @@ extern "C" gg_status gg_bfs(gg_graph *g, const gg_bfs_params *p, int32_t *parent
     case GG_BFS_PUSH_BITMAP:
     {
         /* BFS.c:424-523 (queue) and :841-930 (bitmap frontier) */
+        uint64_t edges = outdeg_src;
         while (qlen)
         {
-            GG_CHECK(td_step(B, q, qlen, nq, p->mode == GG_BFS_PUSH_BITMAP ? nbm : nullptr, level + 1));
+            GG_CHECK(td_step(B, q, qlen, edges, nq, p->mode == GG_BFS_PUSH_BITMAP ? nbm : nullptr, level + 1));
+            edges = B.h->mf; /* the out-edges of what the step claimed */
             qlen = B.h->qlen;
             std::swap(q, nq);
             std::swap(bm, nbm);
@@ -1065,6 +1069,7 @@ extern "C" gg_status gg_bfs(gg_graph *g, const gg_bfs_params *p, int32_t *parent
             break;
         }
         uint32_t mu = g->E, mf = outdeg_src, nf = 0, nf_prev = 0;
+        uint64_t edges = outdeg_src;
         const uint32_t n = V;
         while (qlen)
         {
@@ -1082,13 +1087,14 @@ extern "C" gg_status gg_bfs(gg_graph *g, const gg_bfs_params *p, int32_t *parent
                     level++;
                 } while ((nf > nf_prev) || (nf > (n / beta)));
                 GG_CHECK(compact(B, bm, q, &qlen));
-                mf = 1;
+                mf = 1; /* as the reference counts here */
+                edges = EDGES_UNKNOWN;
             }
             else
             {
                 mu -= mf;
-                GG_CHECK(td_step(B, q, qlen, nq, nullptr, level + 1));
-                mf = B.h->mf;
+                GG_CHECK(td_step(B, q, qlen, edges, nq, nullptr, level + 1));
+                edges = mf = B.h->mf;
                 qlen = B.h->qlen;
                 std::swap(q, nq);
                 processed += qlen;
@@ -1155,7 +1161,7 @@ extern "C" gg_status gg_bfs_step_host(gg_graph *g, int direction, const uint32_t
     if (direction == 0)
     {
         if (frontier_is_bitmap) GG_CHECK(compact(B, B.bma, B.qa, &qlen));
-        GG_CHECK(td_step(B, B.qa, qlen, B.qb, B.bmb, newdist));
+        GG_CHECK(td_step(B, B.qa, qlen, EDGES_UNKNOWN, B.qb, B.bmb, newdist));
         cnt = B.h->mf;
         nlen = B.h->qlen;
         if (next_queue && nlen) GG_CUDA(cudaMemcpyAsync(next_queue, B.qb, (size_t)nlen * 4, cudaMemcpyDeviceToHost, B.s));
