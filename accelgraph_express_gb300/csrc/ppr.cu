@@ -175,7 +175,8 @@ struct PprArgs
     const uint32_t *rows; /* the rows with edges, padded with V */
     const uint32_t *seg0; /* per tile: its first row end; bit 31: the row began earlier */
     uint32_t ntiles, V, E;
-    uint32_t tile; /* edges per tile, a power of two from 256 (512 by default, the tuned size otherwise) */
+    uint32_t tile; /* edges per tile (gg_ppr_tile): a power of two, at least a chunk's; below 256 every
+                    * tile needs a resident warp of its own (ppr_tiles_fit) */
     const CT *cin;
     CT *cout;
     float *rank;       /* [V][rs]: ranks of the vectors in rank_mask are written here */
@@ -899,7 +900,15 @@ uint32_t gg_ppr_tile(const gg_graph *g)
 {
     const uint32_t warps = (uint32_t)(PPR_CTAS * PPR_WARPS) * (uint32_t)gg_sm_count();
     uint32_t tile = g->ppr_tile;
-    if (!tile)
+    if (tile)
+    {
+        /* a size from a file may be any: the gather needs a power of two, no less
+         * than a chunk */
+        uint32_t pow2 = 32u;
+        while (pow2 <= tile / 2) pow2 *= 2;
+        tile = pow2;
+    }
+    else
     {
         tile = g->E < 4u * 512u * warps ? 256u : 512u;
         while (tile > 32u && (uint64_t)(tile / 2) * warps >= g->E) tile /= 2;
