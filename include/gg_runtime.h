@@ -186,7 +186,8 @@ typedef struct gg_pr_params
  * The instantiated graph stays with the mapping: a later call with the same
  * parameters relaunches it, unless device memory of the mapping has been
  * freed since (another algorithm regrowing a shared work buffer), in which
- * case it is captured again. */
+ * case it is captured again.  An FP32 pull of up to 2.5M edges and 220K vertices
+ * is one launch without it; the flag then changes nothing. */
 #define GG_PR_CUDA_GRAPH 0x1u
 /* The pull gather (every pull mode; SpMV pull in FP) serves the values of the
  * vertices with the most out-edges -- 40K FP32, 80K 16- or 8-bit, 20K 64-bit
@@ -210,7 +211,8 @@ typedef struct gg_pr_result
     double error_total;       /* last iteration's sum |delta| / V */
     double rank_sum;          /* sum of the returned ranks */
     float gather_ms;          /* profile: summed device time of the gather launches */
-    uint32_t gather_launches; /* gather launches timed */
+    uint32_t gather_launches; /* gathers queued: one per iteration, each timed with profile, also
+                               * where one launch runs all of them; 1 for the many-graphs kernel */
     uint32_t launches;        /* kernels launched by the call */
     uint32_t hot_table;       /* 1: the gather read the hot-vertex table (GG_PR_HOT_*) */
 } gg_pr_result;

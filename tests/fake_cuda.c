@@ -46,18 +46,23 @@ static size_t g_shared_size;
 /* static shared memory of every kernel */
 API void fake_shared_size(long n) { g_shared_size = (size_t)n; }
 
+static void log_line(const char *s)
+{
+    const size_t n = strlen(s);
+    if (g_log_len + n + 2 > sizeof(g_log)) abort();
+    memcpy(g_log + g_log_len, s, n);
+    g_log_len += n;
+    g_log[g_log_len++] = '\n';
+    g_log[g_log_len] = 0;
+}
+
 static cudaError_t launched(const void *fn, size_t smem)
 {
     for (int i = 0; i < g_nkernels; i++)
         if (g_kernels[i].fn == fn)
         {
-            const size_t n = strlen(g_kernels[i].name);
             g_kernels[i].smem = smem;
-            if (g_log_len + n + 2 > sizeof(g_log)) abort();
-            memcpy(g_log + g_log_len, g_kernels[i].name, n);
-            g_log_len += n;
-            g_log[g_log_len++] = '\n';
-            g_log[g_log_len] = 0;
+            log_line(g_kernels[i].name);
             return cudaSuccess;
         }
     return cudaErrorInvalidDeviceFunction;
@@ -208,7 +213,7 @@ API cudaError_t cudaEventDestroy(cudaEvent_t e) { free(e); return cudaSuccess; }
 API cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { (void)e; (void)s; return cudaSuccess; }
 API cudaError_t cudaEventQuery(cudaEvent_t e) { (void)e; return cudaSuccess; }
 API cudaError_t cudaEventElapsedTime(float *ms, cudaEvent_t a, cudaEvent_t b) { (void)a; (void)b; *ms = 0.1f; return cudaSuccess; }
-API cudaError_t cudaGraphInstantiate(cudaGraphExec_t *x, cudaGraph_t g, unsigned long long f) { (void)g; (void)f; *x = (cudaGraphExec_t)calloc(1, 8); return cudaSuccess; }
+API cudaError_t cudaGraphInstantiate(cudaGraphExec_t *x, cudaGraph_t g, unsigned long long f) { (void)g; (void)f; log_line("<instantiate>"); *x = (cudaGraphExec_t)calloc(1, 8); return cudaSuccess; }
 API cudaError_t cudaGraphDestroy(cudaGraph_t g) { free(g); return cudaSuccess; }
 API cudaError_t cudaGraphExecDestroy(cudaGraphExec_t x) { free(x); return cudaSuccess; }
-API cudaError_t cudaGraphLaunch(cudaGraphExec_t x, cudaStream_t s) { (void)x; (void)s; return cudaSuccess; }
+API cudaError_t cudaGraphLaunch(cudaGraphExec_t x, cudaStream_t s) { (void)x; (void)s; log_line("<graph>"); return cudaSuccess; }
