@@ -503,8 +503,7 @@ def c1_extras(gg, torch, scale=16, peak=6660.9):
     """The CPU-runnable configuration: PageRank pull on R-MAT-16 (65,536
     vertices, 1,048,576 edges), epsilon 1e-4, at most 20 iterations, in the
     reference's formulation (start 0.15, divide by V at the end) and with
-    1/N initialisation, in the gather shape the autotuner picks for the
-    graph; ranks against the FP64 oracle (L1, L-inf),
+    1/N initialisation (one launch each); ranks against the FP64 oracle (L1, L-inf),
     iterations against the reference's FP32 loop, GTEPS over the iterations
     run, the oracle's OpenMP loop timed beside it."""
     import numpy as np
@@ -515,26 +514,18 @@ def c1_extras(gg, torch, scale=16, peak=6660.9):
     a = g.arrays()
     o = O.Csr.from_arrays(V, E, a["out_off"], a["out_adj"], a["in_off"], a["in_adj"])
     dg = gg.DeviceGraph(g, gg.MAP_IN)
-    # the gather's launch shape picked by the autotuner for this graph class
-    # (setup; remembered for the class, so the drop-in calls below use it too)
-    tune = dg.autotune(gg.TUNE_PR, reps=3).get("pr")
-    out = {"graph": f"R-MAT-{scale}, V={V}, E={E}", "epsilon": 1e-4, "max_iterations": 20, "gather_shape": tune}
+    out = {"graph": f"R-MAT-{scale}, V={V}, E={E}", "epsilon": 1e-4, "max_iterations": 20}
     for name, one_over_n in (("reference_formulation", False), ("init_1_over_n", True)):
-        # per call (wall time, results left on the device): the call as one
-        # cached CUDA graph launch, and as stream launches
-        timed = {}
-        for as_graph in (True, False):
-            for _ in range(3):
-                dg.pagerank("pull", iterations=20, epsilon=1e-4, init_one_over_n=one_over_n, copy_out=False,
-                            cuda_graph=as_graph)
-            reps = 20
-            torch.cuda.synchronize()
-            t0 = time.perf_counter()
-            for _ in range(reps):
-                _, r = dg.pagerank("pull", iterations=20, epsilon=1e-4, init_one_over_n=one_over_n,
-                                   copy_out=False, cuda_graph=as_graph)
-            timed[as_graph] = (time.perf_counter() - t0) * 1e3 / reps
-        ms = timed[True]
+        # per call (wall time, results left on the device); every iteration is
+        # in one launch
+        for _ in range(3):
+            dg.pagerank("pull", iterations=20, epsilon=1e-4, init_one_over_n=one_over_n, copy_out=False)
+        reps = 20
+        torch.cuda.synchronize()
+        t0 = time.perf_counter()
+        for _ in range(reps):
+            dg.pagerank("pull", iterations=20, epsilon=1e-4, init_one_over_n=one_over_n, copy_out=False)
+        ms = (time.perf_counter() - t0) * 1e3 / reps
         ranks, r = dg.pagerank("pull", iterations=20, epsilon=1e-4, init_one_over_n=one_over_n)
         ref, info = O.pagerank(o, 0, 20, 1e-4, init_one_over_n=one_over_n)
         ex = O.pagerank_f64(o, info["executed"], init_one_over_n=one_over_n)
@@ -543,13 +534,11 @@ def c1_extras(gg, torch, scale=16, peak=6660.9):
         cpu_ms = (time.perf_counter() - t0) * 1e3
         alg = pr_bytes(V, E, 4) * info["executed"]
         out[name] = {"iterations": r["iterations"], "iterations_reference_loop": info["iterations"],
-                     "iterations_executed": info["executed"], "ms_per_call": ms,
+                     "iterations_executed": info["executed"], "ms_per_call": ms, "launches": r["launches"],
                      "gteps": E * (info["executed"]) / (ms / 1e3) / 1e9,
                      "roofline": {"alg_bytes_per_call": alg, "achieved_gbs": alg / (ms / 1e3) / 1e9,
                                   "frac": alg / (ms / 1e3) / 1e9 / peak,
-                                  "note": "R-MAT-16's 5.8 MB per iteration stays in L2; the call is launch-bound"},
-                     "ms_per_call_stream_launches": timed[False],
-                     "gteps_stream_launches": E * (info["executed"]) / (timed[False] / 1e3) / 1e9,
+                                  "note": "R-MAT-16's 5.8 MB per iteration stays in L2; one launch, bound by its grid barriers"},
                      "l1_vs_fp64": float(np.abs(ranks - ex).sum()), "linf_vs_fp64": float(np.abs(ranks - ex).max()),
                      "l1_reference_fp32_loop_vs_fp64": float(np.abs(ref - ex).sum()),
                      "cpu_gteps": E * info["executed"] / (cpu_ms / 1e3) / 1e9}
@@ -597,7 +586,7 @@ def batch_extras(gg, torch, peak, n=4096, iters=20):
     (one CTA per graph, largest first; graphs up to the bin threshold keep
     their contributions in shared memory), in the configuration the
     autotuner picks for this batch and in the default one; the union pull
-    (20 x 2 launches over the block-diagonal union, as one CUDA graph) is
+    (20 x 2 gathers and updates over the block-diagonal union, as one CUDA graph) is
     timed beside it.  Roofline: the algorithm's per-iteration bytes summed
     over the graphs.  Parity: the smallest, a middle and the largest graph
     against the FP64 oracle; CPU baseline: the oracle's OpenMP pull on 64
