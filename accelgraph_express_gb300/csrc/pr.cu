@@ -1438,11 +1438,11 @@ gg_status pagerank_impl(gg_graph *g, const gg_pr_params *p, float *ranks, gg_pr_
     /* the hot-vertex table of the pull modes (prepared before any capture) */
     gg_tune_lookup(g, R.s);
     R.shape = g->pr_shape;
-    /* a graph of up to 2.5M edges and 220K vertices: every iteration in one
-     * launch, faster at every size it takes (small.cu); timed runs time each
+    /* a graph of up to 2.5M edges and 200K vertices: every iteration in one
+     * launch, as fast or faster at the sizes it takes (small.cu); timed runs time each
      * gather launch, and a table asked for by the call is used (a tuned shape says
-     * which of the gather launches is fastest, and none of them is: 1M edges 249 us
-     * a call against 210) */
+     * which of the gather launches is fastest, and none of them is: 1M edges 212 us
+     * a call against 179) */
     R.small = one_launch && p->mode == GG_PR_PULL && p->storage == GG_STORE_F32 && !ngraphs && !p->profile &&
               !(p->flags & GG_PR_HOT_ON) && gg_small_fits(g);
     const uint32_t vb = value_bytes(p);

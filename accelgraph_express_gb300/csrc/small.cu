@@ -20,9 +20,9 @@
  * Bound by instruction issue (about ten instructions per edge and lane) and, in
  * a cluster, by its two barriers: one CTA up to SM_ONE edges, eight above.
  *
- * Measured per call of 20 iterations, R-MAT with 16 edges per vertex, against
- * the launches: 1.6K edges 144 -> 60 us, 16K 163 -> 96, 64K 169 -> 116 (some
- * 43 us of each are the call's host work).
+ * Measured per call of 20 iterations, R-MAT with 16 edges per vertex, ranks left on
+ * the device, against the launches: 1.6K edges 137 -> 43 us, 16K 140 -> 76, 32K 142 ->
+ * 101, 64K 144 -> 101, 96K 146 -> 126 (some 30 us of each are the call's host work).
  */
 #include <cuda_runtime.h>
 
@@ -434,9 +434,9 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_small(SmallArgs a)
  *
  * Bound by the two barriers (1.7 us each with the block's own) and, from 1M
  * edges, by the gather's L2 requests.  Measured per call of 20 iterations, R-MAT
- * with 16 edges per vertex, launches -> here: 128K edges 169 -> 151 us (the
- * cluster 163), 262K 191 -> 162, 1M 249 -> 210, 1.6M 283 -> 265; uniform random,
- * 1.9M 380 -> 327. */
+ * with 16 edges per vertex, launches -> here: 128K edges 151 -> 129 us (the
+ * cluster 140), 262K 156 -> 140, 524K 175 -> 151, 1M 212 -> 179, 1.6M 239 -> 215;
+ * uniform random, 1.9M 336 -> 286. */
 struct GridArgs
 {
     SmallArgs a;
@@ -677,11 +677,13 @@ __global__ void __launch_bounds__(SM_THREADS, 1) k_pr_grid(GridArgs ga)
 }
 
 /* Edges per thread (of 152 SMs: 2.5M edges) and vertices above which the
- * launches are faster: R-MAT with 2.4M edges 349 (launches) against 353 us, 2.9M
- * 403 against 440 -- the ids leave the L1 less room; 250K vertices with 5 edges
- * each 316 against 372, with 8 373 against 424, where 220K with 8 took 354
- * against 341 -- the update and the contributions' lines take over. */
-constexpr uint32_t GRID_RUN_MAX = 16, GRID_MAX_V = 220000;
+ * launches are faster.  One launch against launches, us per call of 20 iterations:
+ * R-MAT with 2.0M edges 253 : 273, 2.4M 301 : 310 -- the ids leave the L1 less room.
+ * By vertices (a thread has a second one from 156K), uniform random with 5 or 8
+ * edges each / R-MAT with 5 or 8: 150K 224 : 239, 249 : 278 / 225 : 215, 237 : 239;
+ * 200K 274 : 273, 312 : 333 / 254 : 249, 298 : 284; 219K 335 : 285, 360 : 346 / 323 :
+ * 255, 362 : 297. */
+constexpr uint32_t GRID_RUN_MAX = 16, GRID_MAX_V = 200000;
 constexpr size_t GRID_LIMIT = 220 * 1024;
 
 /* the shares of a graph of one CTA per SM, or false when it does not fit */

@@ -186,7 +186,7 @@ typedef struct gg_pr_params
  * The instantiated graph stays with the mapping: a later call with the same
  * parameters relaunches it, unless device memory of the mapping has been
  * freed since (another algorithm regrowing a shared work buffer), in which
- * case it is captured again.  An FP32 pull of up to 2.5M edges and 220K vertices
+ * case it is captured again.  An FP32 pull of up to 2.5M edges and 200K vertices
  * is one launch without it; the flag then changes nothing. */
 #define GG_PR_CUDA_GRAPH 0x1u
 /* The pull gather (every pull mode; SpMV pull in FP) serves the values of the
