@@ -313,8 +313,6 @@ __device__ __forceinline__ uint32_t stage_words(uint32_t *dst, const uint32_t *s
 
 __device__ __forceinline__ void atomic_add_acc(float *p, float v) { atomicAdd(p, v); }
 __device__ __forceinline__ void atomic_add_acc(unsigned long long *p, unsigned long long v) { atomicAdd(p, v); }
-__device__ __forceinline__ float atomic_take(float *p) { return atomicExch(p, 0.0f); }
-__device__ __forceinline__ unsigned long long atomic_take(unsigned long long *p) { return atomicExch(p, 0ull); }
 
 /* ---- merge-path tiles ------------------------------------------------------
  *

@@ -19,8 +19,8 @@
  * land in shared memory: a warp owns a tile of edges, asks for the rows of a
  * chunk of up to 32 edges with 16-byte asynchronous copies (cp.async.cg: L2
  * only, so rows rewritten inside the persistent launch are read fresh), and
- * sums a chunk while the next ones arrive; 8 KB of landing space per warp, 24
- * warps per SM.  The half warps take alternate edges, each lane KP / 16
+ * sums a chunk while the next ones arrive; up to 8 KB of landing space per warp
+ * (4 KB for 32-byte rows), 20 warps per SM.  The half warps take alternate edges, each lane KP / 16
  * columns, so one shared-memory read serves two edges and the additions are
  * packed (add.f32x2): issue slots are what is left to bound the loop.  The two
  * halves' sums are exchanged and added where the row ends, for every KP: the
