@@ -341,12 +341,13 @@ unsigned long long gg_barrier_limit_ns();
 #define GG_HOT_ENTRIES 81920u
 #define GG_HOT_WARPS 32
 #define GG_HOT_TILE_MAX 2048u
-/* From this many edges the pull gathers use the table by default.  Measured
- * per FP32 gather, table off -> on (its filling included): R-MAT with 4.2M
- * edges 20.5 -> 21.2 us, 11.2M 44.5 -> 35.0, 16.8M 63.5 -> 47.5, 67M 241 ->
- * 157, 268M 1,000 -> 662; uniform random graphs 28.7 -> 28.6, 61.5 -> 58.1,
- * 88 -> 78, 320 -> 268, 1,259 -> 1,043.  Below, the 25 MB of table that 152
- * SMs read per launch cost more than the requests they save. */
+/* From this many edges the pull gathers use the table by default (where a sample
+ * of the graph does not speak for the plain gather: hot.cu).  Measured per FP32
+ * iteration, update included, table off -> on: R-MAT with 4.2M edges 20.6 -> 18.9
+ * us, 11.2M 44.9 -> 33.1, 16.8M 64.1 -> 45.4, 67M 249 -> 158, 268M 1,051 -> 711;
+ * uniform random graphs 28.3 -> 27.5, 61.5 -> 55.7, 89 -> 75, 327 -> 269, 1,324 ->
+ * 1,093.  Below, what the 25 MB of table that 152 SMs read per launch cost is near
+ * what the requests they save are worth, and making the table is not repaid. */
 #define GG_HOT_MIN_E (1u << 23)
 /* ... and, while the table is not there, once the gathers done without it and
  * those of the call make (gathers - 2) * E reach this.  Making the table
